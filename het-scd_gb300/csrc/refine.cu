@@ -248,9 +248,35 @@ __global__ void k_pext_terms(uint32_t n, const uint32_t *__restrict__ indices, c
 // roundings + a block prefix sum give every in-binade partial sum exactly, and
 // only the first tie or binade crossing in a tile is done with a real DADD,
 // after which the tile restarts from the next term.
+//
+// Bound: one SM walks a graph's terms, so the rounding must not use the FP64
+// pipe (2 operations a clock and SM: scale, floor and subtract of 8192 terms
+// were 13 of the 25 us a tile took).  t/u is the term's 53-bit mantissa shifted
+// right by the exponent distance: the quotient, the remainder and the tie are
+// three 64-bit integer operations.  The first SEQ_HEAD terms, where s doubles
+// every few terms and each doubling would restart a tile, are added one by one.
 constexpr int SEQ_THREADS = 1024;
 constexpr int SEQ_ITEMS = 8;
 constexpr int SEQ_TILE = SEQ_THREADS * SEQ_ITEMS;
+constexpr uint32_t SEQ_HEAD = 32;
+
+// r = round-to-nearest of t / 2^(e-52) for 0 <= t < 2^(e+1); true: t needs a real
+// addition instead (negative or not finite, not below 2^(e+1), or halfway between
+// two multiples)
+__device__ __forceinline__ bool seq_round(double t, int e, long long *r) {
+    const unsigned long long b = (unsigned long long)__double_as_longlong(t);
+    *r = 0;
+    if ((b << 1) == 0) return false;   // +0 or -0
+    const int field = (int)(b >> 52) & 0x7ff;
+    if (b >> 63 || field == 0x7ff) return true;
+    const unsigned long long mant = (b & ((1ull << 52) - 1)) | (field ? 1ull << 52 : 0ull);
+    const int sh = e + 1023 - (field ? field : 1);   // t = mant * 2^(e - 52 - sh)
+    if (sh < 0) return true;
+    if (sh > 53) return false;         // t is below half a unit
+    const unsigned long long q = mant >> sh, twice = (mant - (q << sh)) << 1, unit = 1ull << sh;
+    *r = (long long)(q + (twice > unit));
+    return twice == unit;
+}
 
 __global__ void __launch_bounds__(SEQ_THREADS)
 k_sequential_sum_exact(const double *__restrict__ terms, const uint32_t *__restrict__ seg_off, double *out) {
@@ -263,20 +289,40 @@ k_sequential_sum_exact(const double *__restrict__ terms, const uint32_t *__restr
     __shared__ uint32_t s_pos, s_event;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const long long TWO53 = 1ll << 53;
+    __shared__ double head[SEQ_HEAD];
+    const uint32_t nhead = min(n, SEQ_HEAD);
+    if (threadIdx.x < nhead) head[threadIdx.x] = term[threadIdx.x];
+    __syncthreads();
     if (threadIdx.x == 0) {
         double s = 0.0;
-        uint32_t p = 0;
-        while (p < n && s == 0.0) s = dadd(s, term[p++]);   // leading zero terms
+        for (uint32_t p = 0; p < nhead; p++) s = dadd(s, head[p]);
         s_val = s;
-        s_pos = p;
+        s_pos = nhead;
     }
     __syncthreads();
     while (true) {
         const uint32_t pos = s_pos;
         if (pos >= n) break;
         const double s = s_val;
-        if (!(s >= 2.2250738585072014e-308) || s > 1e300) {
-            // not a positive normal number (e.g. after a negative term): one plain step
+        if (s == 0.0) {   // on to the first term that is not zero
+            __syncthreads();   // s_val and s_pos are read
+            if (threadIdx.x == 0) s_event = INVALID;
+            __syncthreads();
+            const uint32_t end = min(n, pos + (uint32_t)SEQ_TILE);
+            uint32_t at = INVALID;
+            for (uint32_t i = pos + threadIdx.x; i < end && at == INVALID; i += SEQ_THREADS)
+                if (term[i] != 0.0) at = i;
+            if (at != INVALID) atomicMin(&s_event, at);
+            __syncthreads();
+            if (threadIdx.x == 0) {
+                s_pos = s_event == INVALID ? end : s_event + 1;
+                if (s_event != INVALID) s_val = dadd(s, term[s_event]);
+            }
+            __syncthreads();
+            continue;
+        }
+        if (!(s >= 1e-290) || s > 1e300) {
+            // not a positive number well inside the normal range (e.g. after a negative term): one plain step
             __syncthreads();
             if (threadIdx.x == 0) {
                 s_val = dadd(s, term[pos]);
@@ -286,9 +332,8 @@ k_sequential_sum_exact(const double *__restrict__ terms, const uint32_t *__restr
             continue;
         }
         const int e = (int)((__double_as_longlong(s) >> 52) & 0x7ff) - 1023;   // s in [2^e, 2^(e+1))
-        const double scale = __longlong_as_double((long long)(1023 + 52 - e) << 52);   // 2^(52-e)
-        const double u = __longlong_as_double((long long)(1023 - 52 + e) << 52);       // 2^(e-52)
-        const long long S = __double2ll_rz(dmul(s, scale));
+        const double u = __longlong_as_double((long long)(1023 - 52 + e) << 52);   // 2^(e-52)
+        const long long S = (__double_as_longlong(s) & ((1ll << 52) - 1)) | (1ll << 52);   // s / u
         const uint32_t base = pos + threadIdx.x * SEQ_ITEMS;
         long long r[SEQ_ITEMS];
         bool ev[SEQ_ITEMS];
@@ -297,16 +342,7 @@ k_sequential_sum_exact(const double *__restrict__ terms, const uint32_t *__restr
         for (int i = 0; i < SEQ_ITEMS; i++) {
             r[i] = 0;
             ev[i] = false;
-            if (base + i < n) {
-                const double x = dmul(term[base + i], scale);   // exact: power-of-two scaling
-                if (!(x >= 0.0) || x >= 9007199254740992.0) {
-                    ev[i] = true;
-                } else {
-                    const double q = floor(x), f = dsub(x, q);
-                    ev[i] = f == 0.5;
-                    r[i] = (long long)q + (f > 0.5 ? 1 : 0);
-                }
-            }
+            if (base + i < n) ev[i] = seq_round(term[base + i], e, &r[i]);
             local += r[i];
         }
         // block exclusive scan of the per-thread totals
