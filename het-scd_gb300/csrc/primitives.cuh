@@ -46,73 +46,129 @@ struct DevBuf {
 
 // ---------------------------------------------------------------------------
 // exclusive scan: out[0..n] with out[n] = total (n+1 outputs)
+//
+// Most scans here are short (a run makes about a hundred, most of them over the
+// vertices or a list of them), so what bounds one is its launches, not its
+// bytes: up to SCAN_ONE outputs a single CTA does it in one launch; above, two
+// launches (every CTA's sum, then every CTA adds up the sums before its own and
+// scans its range), which also reads the input twice instead of writing the
+// output twice.
 
 constexpr int SCAN_THREADS = 256;
 constexpr int SCAN_ITEMS = 8;
 constexpr int SCAN_TILE = SCAN_THREADS * SCAN_ITEMS;
+constexpr int SCAN_ONE_THREADS = 1024;
+constexpr int SCAN_ONE_ITEMS = 16;
+constexpr size_t SCAN_ONE = (size_t)SCAN_ONE_THREADS * SCAN_ONE_ITEMS;
+constexpr size_t SCAN_MAX_CTAS = 152 * 8;   // each reads the sums of the ones before it
 
-template <typename T>
-__device__ __forceinline__ T block_exclusive_scan(T v, T *total, T *smem_warp /*[8]*/) {
+template <int THREADS, typename T>
+__device__ __forceinline__ T block_exclusive_scan(T v, T *total, T *smem_warp /*[THREADS / 32 + 1]*/) {
+    constexpr int WARPS = THREADS / 32;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     T inc = warp_inclusive_scan(v);
     if (lane == 31) smem_warp[warp] = inc;
     __syncthreads();
     if (warp == 0) {
-        T w = lane < (SCAN_THREADS / 32) ? smem_warp[lane] : T(0);
+        T w = lane < WARPS ? smem_warp[lane] : T(0);
         T wi = warp_inclusive_scan(w);
-        if (lane < (SCAN_THREADS / 32)) smem_warp[lane] = wi - w;
-        if (lane == (SCAN_THREADS / 32) - 1) smem_warp[SCAN_THREADS / 32] = wi;
+        if (lane < WARPS) smem_warp[lane] = wi - w;
+        if (lane == WARPS - 1) smem_warp[WARPS] = wi;
     }
     __syncthreads();
     T res = smem_warp[warp] + inc - v;
-    *total = smem_warp[SCAN_THREADS / 32];
+    *total = smem_warp[WARPS];
     __syncthreads();
     return res;
 }
 
-template <typename T, typename In>
-__global__ void __launch_bounds__(SCAN_THREADS) k_scan_tiles(In in, size_t n, T *out, T *tile_sums) {
-    __shared__ T sw[SCAN_THREADS / 32 + 1];
-    const size_t base = (size_t)blockIdx.x * SCAN_TILE + (size_t)threadIdx.x * SCAN_ITEMS;
-    T v[SCAN_ITEMS];
+// out[base .. base + THREADS * ITEMS) of the exclusive scan that starts at `run`; returns the tile's total
+template <int THREADS, int ITEMS, typename T, typename In>
+__device__ __forceinline__ T scan_tile(In in, size_t n, size_t base, T run, T *out, T *sw) {
+    const size_t first = base + (size_t)threadIdx.x * ITEMS;
+    T v[ITEMS];
     T sum = 0;
 #pragma unroll
-    for (int i = 0; i < SCAN_ITEMS; i++) {
-        size_t idx = base + i;
-        v[i] = idx < n ? T(in[idx]) : T(0);
+    for (int i = 0; i < ITEMS; i++) {
+        v[i] = first + i < n ? T(in[first + i]) : T(0);
         sum += v[i];
     }
     T total;
-    T run = block_exclusive_scan(sum, &total, sw);
+    run += block_exclusive_scan<THREADS>(sum, &total, sw);
 #pragma unroll
-    for (int i = 0; i < SCAN_ITEMS; i++) {
-        size_t idx = base + i;
-        if (idx <= n) out[idx] = run;
+    for (int i = 0; i < ITEMS; i++) {
+        if (first + i <= n) out[first + i] = run;
         run += v[i];
     }
-    if (threadIdx.x == 0) tile_sums[blockIdx.x] = total;
+    return total;
 }
 
-template <typename T>
-__global__ void k_scan_add(T *out, size_t n, const T *tile_offsets) {
-    size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    size_t stride = (size_t)gridDim.x * blockDim.x;
-    for (; i <= n; i += stride) out[i] += tile_offsets[i / SCAN_TILE];
+template <typename T, typename In>
+__global__ void __launch_bounds__(SCAN_THREADS) k_scan_tile(In in, size_t n, T *out) {
+    __shared__ T sw[SCAN_THREADS / 32 + 1];
+    scan_tile<SCAN_THREADS, SCAN_ITEMS>(in, n, 0, T(0), out, sw);
 }
 
-// in may be a pointer or any functor-like indexable; out must hold n+1 entries.
+template <typename T, typename In>
+__global__ void __launch_bounds__(SCAN_ONE_THREADS) k_scan_one(In in, size_t n, T *out) {
+    __shared__ T sw[SCAN_ONE_THREADS / 32 + 1];
+    scan_tile<SCAN_ONE_THREADS, SCAN_ONE_ITEMS>(in, n, 0, T(0), out, sw);
+}
+
+// sums[b] = sum of CTA b's range of per_cta tiles
+template <typename T, typename In>
+__global__ void __launch_bounds__(SCAN_THREADS) k_scan_sums(In in, size_t n, uint32_t per_cta, T *sums) {
+    __shared__ T sw[SCAN_THREADS / 32];
+    const size_t lo = (size_t)blockIdx.x * per_cta * SCAN_TILE;
+    const size_t hi = min(n, lo + (size_t)per_cta * SCAN_TILE);
+    T sum = 0;
+#pragma unroll 4
+    for (size_t i = lo + threadIdx.x; i < hi; i += SCAN_THREADS) sum += T(in[i]);
+    sum = warp_sum(sum);
+    if ((threadIdx.x & 31) == 0) sw[threadIdx.x >> 5] = sum;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        T t = 0;
+        for (int w = 0; w < SCAN_THREADS / 32; w++) t += sw[w];
+        sums[blockIdx.x] = t;
+    }
+}
+
+template <typename T, typename In>
+__global__ void __launch_bounds__(SCAN_THREADS) k_scan_out(In in, size_t n, uint32_t per_cta, const T *sums, T *out) {
+    __shared__ T sw[SCAN_THREADS / 32 + 1];
+    T before = 0, run;
+    for (uint32_t b = threadIdx.x; b < blockIdx.x; b += SCAN_THREADS) before += sums[b];
+    block_exclusive_scan<SCAN_THREADS>(before, &run, sw);   // run: the sums of all CTAs before this one
+    for (uint32_t k = 0; k < per_cta; k++) {
+        const size_t base = ((size_t)blockIdx.x * per_cta + k) * SCAN_TILE;
+        if (base > n) break;
+        run += scan_tile<SCAN_THREADS, SCAN_ITEMS>(in, n, base, run, out, sw);
+    }
+}
+
+// in may be a pointer or any functor-like indexable; out must hold n+1 entries
+// (out == in is allowed: every CTA reads its range before it writes it).
 template <typename T, typename In>
 void scan_exclusive(In in, T *out, size_t n, cudaStream_t s) {
-    size_t tiles = (n + 1 + SCAN_TILE - 1) / SCAN_TILE;
-    DevBuf<T> sums(tiles + 1, s);
-    k_scan_tiles<T, In><<<(unsigned)tiles, SCAN_THREADS, 0, s>>>(in, n, out, sums.get());
-    CK_LAUNCH("k_scan_tiles");
-    if (tiles > 1) {
-        DevBuf<T> offs(tiles + 1, s);
-        scan_exclusive<T, const T *>(sums.get(), offs.get(), tiles, s);
-        k_scan_add<T><<<grid_for(n + 1, 256), 256, 0, s>>>(out, n, offs.get());
-        CK_LAUNCH("k_scan_add");
+    if (n + 1 <= (size_t)SCAN_TILE) {
+        k_scan_tile<T, In><<<1, SCAN_THREADS, 0, s>>>(in, n, out);
+        CK_LAUNCH("k_scan_tile");
+        return;
     }
+    if (n + 1 <= SCAN_ONE) {
+        k_scan_one<T, In><<<1, SCAN_ONE_THREADS, 0, s>>>(in, n, out);
+        CK_LAUNCH("k_scan_one");
+        return;
+    }
+    const size_t tiles = (n + 1 + SCAN_TILE - 1) / SCAN_TILE;
+    const uint32_t per_cta = (uint32_t)((tiles + SCAN_MAX_CTAS - 1) / SCAN_MAX_CTAS);
+    const unsigned ctas = (unsigned)((tiles + per_cta - 1) / per_cta);
+    DevBuf<T> sums(ctas, s);
+    k_scan_sums<T, In><<<ctas, SCAN_THREADS, 0, s>>>(in, n, per_cta, sums.get());
+    CK_LAUNCH("k_scan_sums");
+    k_scan_out<T, In><<<ctas, SCAN_THREADS, 0, s>>>(in, n, per_cta, sums.get(), out);
+    CK_LAUNCH("k_scan_out");
 }
 
 // ---------------------------------------------------------------------------
