@@ -13,6 +13,7 @@
 // With de-duplication a repeated value of a row becomes INVALID and the number
 // of distinct values of the row is written out; the caller compacts.
 #include "engine.cuh"
+#include "lists.cuh"
 
 namespace scd {
 
@@ -210,19 +211,17 @@ k_sort_rows_cta(const uint32_t *__restrict__ list, uint32_t count, const uint32_
     }
 }
 
-struct RowLenIn {
+// the length classes of the longer rows: (32, 64], (64, 128], (128, 256], (256, 512],
+// (512, 4096], (4096, 16384] and above; shorter rows are in no class
+constexpr int ROW_CLASSES = 7;
+struct RowClassOf {
     const uint32_t *off;
-    uint32_t lo, hi;   // lo < len <= hi
     __device__ uint32_t operator[](size_t r) const {
         const uint32_t len = off[r + 1] - off[r];
-        return len > lo && len <= hi;
+        if (len <= WARP_ROW) return 0u;
+        return 1u << ((len > 64) + (len > 128) + (len > 256) + (len > MID_ROW) + (len > BIG_ROW) + (len > HUGE_ROW));
     }
 };
-
-__global__ void k_row_scatter(uint32_t nrows, RowLenIn f, const uint32_t *__restrict__ pos, uint32_t *list) {
-    for (uint32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < nrows; r += gridDim.x * blockDim.x)
-        if (f[r]) list[pos[r]] = r;
-}
 
 struct RowLenOf {
     const uint32_t *list, *off;
@@ -278,78 +277,71 @@ void sort_rows(Ctx &c, const uint32_t *off, uint32_t nrows, uint32_t *vals, bool
     CK_LAUNCH("k_sort_rows_warp");
     c.launches++;
     // the longer rows, listed by length class (one host read for all the counts)
-    constexpr int NC = 8;
-    const uint32_t bounds[NC + 1] = {WARP_ROW, 64, 128, 256, MID_ROW, BIG_ROW, HUGE_ROW, 0xffffffffu};
     prepare_sort_kernels();
-    DevBuf<uint32_t> pos[NC];
-    for (int k = 0; k < NC; k++) {
-        pos[k].alloc((size_t)nrows + 1, s);
-        scan_exclusive<uint32_t>(RowLenIn{off, bounds[k], bounds[k + 1]}, pos[k].get(), nrows, s);
-    }
-    uint32_t cnt[NC];
-    for (int k = 0; k < NC; k++) CK(cudaMemcpyAsync(cnt + k, pos[k].get() + nrows, 4, cudaMemcpyDeviceToHost, s));
+    DevBuf<uint32_t> lists(nrows, s), bounds(ROW_CLASSES + 1, s);
+    build_lists<ROW_CLASSES>(RowClassOf{off}, nrows, lists.get(), bounds.get(), s);
+    c.launches++;
+    uint32_t *hb = c.host_u32 + HOST_PLAN;
+    CK(cudaMemcpyAsync(hb, bounds.get(), 4 * (ROW_CLASSES + 1), cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
-    DevBuf<uint32_t> list[NC];
-    for (int k = 0; k < NC; k++) {
-        if (!cnt[k]) continue;
-        list[k].alloc(cnt[k], s);
-        k_row_scatter<<<grid_for(nrows, TPB), TPB, 0, s>>>(nrows, RowLenIn{off, bounds[k], bounds[k + 1]},
-                                                          pos[k].get(), list[k].get());
-        CK_LAUNCH("k_row_scatter");
-        c.launches++;
+    uint32_t cnt[ROW_CLASSES];
+    const uint32_t *list[ROW_CLASSES];
+    for (int k = 0; k < ROW_CLASSES; k++) {
+        cnt[k] = hb[k + 1] - hb[k];
+        list[k] = lists.get() + hb[k];
     }
     if (cnt[0]) {
-        k_sort_rows_warp_e<2><<<grid_for((uint64_t)cnt[0] * 32, TPB), TPB, 0, s>>>(list[0].get(), cnt[0], off, vals,
+        k_sort_rows_warp_e<2><<<grid_for((uint64_t)cnt[0] * 32, TPB), TPB, 0, s>>>(list[0], cnt[0], off, vals,
                                                                                 dedup, udeg);
         CK_LAUNCH("k_sort_rows_warp64");
         c.launches++;
     }
     if (cnt[1]) {
-        k_sort_rows_warp_e<4><<<grid_for((uint64_t)cnt[1] * 32, TPB), TPB, 0, s>>>(list[1].get(), cnt[1], off, vals,
+        k_sort_rows_warp_e<4><<<grid_for((uint64_t)cnt[1] * 32, TPB), TPB, 0, s>>>(list[1], cnt[1], off, vals,
                                                                                 dedup, udeg);
         CK_LAUNCH("k_sort_rows_warp128");
         c.launches++;
     }
     if (cnt[2]) {
-        k_sort_rows_warp_e<8><<<grid_for((uint64_t)cnt[2] * 32, TPB), TPB, 0, s>>>(list[2].get(), cnt[2], off, vals,
+        k_sort_rows_warp_e<8><<<grid_for((uint64_t)cnt[2] * 32, TPB), TPB, 0, s>>>(list[2], cnt[2], off, vals,
                                                                                 dedup, udeg);
         CK_LAUNCH("k_sort_rows_warp256");
         c.launches++;
     }
     if (cnt[3]) {
-        k_sort_rows_warp_e<16><<<grid_for((uint64_t)cnt[3] * 32, TPB), TPB, 0, s>>>(list[3].get(), cnt[3], off, vals,
+        k_sort_rows_warp_e<16><<<grid_for((uint64_t)cnt[3] * 32, TPB), TPB, 0, s>>>(list[3], cnt[3], off, vals,
                                                                                  dedup, udeg);
         CK_LAUNCH("k_sort_rows_warp512");
         c.launches++;
     }
     if (cnt[4]) {
-        k_sort_rows_cta<16, 8><<<grid_for(cnt[4], 1, 152 * 4), 512, BIG_ROW * 4, s>>>(list[4].get(), cnt[4], off, vals,
+        k_sort_rows_cta<16, 8><<<grid_for(cnt[4], 1, 152 * 4), 512, BIG_ROW * 4, s>>>(list[4], cnt[4], off, vals,
                                                                                     dedup, udeg);
         CK_LAUNCH("k_sort_rows_cta4096");
         c.launches++;
     }
     if (cnt[5]) {
-        k_sort_rows_cta<32, 16><<<grid_for(cnt[5], 1, 152 * 2), 1024, HUGE_ROW * 4, s>>>(list[5].get(), cnt[5], off,
+        k_sort_rows_cta<32, 16><<<grid_for(cnt[5], 1, 152 * 2), 1024, HUGE_ROW * 4, s>>>(list[5], cnt[5], off,
                                                                                       vals, dedup, udeg);
         CK_LAUNCH("k_sort_rows_cta16384");
         c.launches++;
     }
     if (cnt[6]) {
         DevBuf<uint32_t> koff((size_t)cnt[6] + 1, s);
-        scan_exclusive<uint32_t>(RowLenOf{list[6].get(), off}, koff.get(), cnt[6], s);
+        scan_exclusive<uint32_t>(RowLenOf{list[6], off}, koff.get(), cnt[6], s);
         uint32_t total = 0;
         CK(cudaMemcpyAsync(&total, koff.get() + cnt[6], 4, cudaMemcpyDeviceToHost, s));
         CK(cudaStreamSynchronize(s));
         DevBuf<uint64_t> keys(total, s);
-        k_big_keys<<<grid_for(cnt[6], 1, 152 * 8), TPB, 0, s>>>(list[6].get(), cnt[6], off, koff.get(), vals,
+        k_big_keys<<<grid_for(cnt[6], 1, 152 * 8), TPB, 0, s>>>(list[6], cnt[6], off, koff.get(), vals,
                                                                keys.get());
         CK_LAUNCH("k_big_keys");
         radix_sort<uint64_t>(keys.get(), nullptr, total, 0, 32 + ceil_log2(cnt[6] < 2 ? 2 : cnt[6]), s);
         if (udeg) {
-            k_zero_rows<<<grid_for(cnt[6], TPB), TPB, 0, s>>>(list[6].get(), cnt[6], udeg);
+            k_zero_rows<<<grid_for(cnt[6], TPB), TPB, 0, s>>>(list[6], cnt[6], udeg);
             CK_LAUNCH("k_zero_rows");
         }
-        k_big_back<<<grid_for(total, TPB), TPB, 0, s>>>(keys.get(), total, list[6].get(), off, koff.get(), vals,
+        k_big_back<<<grid_for(total, TPB), TPB, 0, s>>>(keys.get(), total, list[6], off, koff.get(), vals,
                                                         dedup, udeg);
         CK_LAUNCH("k_big_back");
         c.launches += 3;

@@ -7,6 +7,7 @@
 #include <new>
 
 #include "engine.cuh"
+#include "lists.cuh"
 
 namespace scd {
 
@@ -31,19 +32,21 @@ struct ChunksOf {   // RowWork chunks of a long row
     }
 };
 
-struct InClass {
+// the degree class of a vertex, and (bit K) whether its row is long (RowWork)
+struct DegreeMask {
     const uint32_t *indices;
-    uint32_t lo, hi;   // lo <= deg <= hi
+    uint32_t upper[DegreeClasses::K];
+    explicit DegreeMask(const uint32_t *ind) : indices(ind) {
+        for (int j = 0; j < DegreeClasses::K; j++) upper[j] = DegreeClasses::upper[j];
+    }
     __device__ uint32_t operator[](size_t v) const {
         const uint32_t d = indices[v + 1] - indices[v];
-        return d >= lo && d <= hi;
+        int k = 0;
+#pragma unroll
+        for (int j = 0; j < DegreeClasses::K - 1; j++) k += d > upper[j];
+        return (1u << k) | ((uint32_t)(d > RowWork::CHUNK) << DegreeClasses::K);
     }
 };
-
-__global__ void k_class_scatter(uint32_t n, InClass f, const uint32_t *__restrict__ pos, uint32_t *out) {
-    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x)
-        if (f[v]) out[pos[v]] = v;
-}
 
 struct TableWords {
     const uint32_t *verts, *indices;
@@ -147,29 +150,6 @@ __global__ void k_max_label(uint32_t n, const uint32_t *__restrict__ labels, uin
     }
     m = __reduce_max_sync(FULL, m);
     if ((threadIdx.x & 31) == 0) atomicMax(out, m);
-}
-
-// the vertex lists of K degree ranges (lo[k], hi[k]] with one host read for all counts
-void class_lists(Ctx &c, int K, const uint32_t *lo, const uint32_t *hi, uint32_t **out, uint32_t *cnt) {
-    const Graph &g = c.g;
-    cudaStream_t s = c.stream;
-    std::vector<DevBuf<uint32_t>> pos(K);
-    DevBuf<uint32_t> counts(K, s);
-    for (int k = 0; k < K; k++) {
-        pos[k].alloc((size_t)g.n + 1, s);
-        scan_exclusive<uint32_t>(InClass{g.indices, lo[k], hi[k]}, pos[k].get(), g.n, s);
-        CK(cudaMemcpyAsync(counts.get() + k, pos[k].get() + g.n, 4, cudaMemcpyDeviceToDevice, s));
-    }
-    CK(cudaMemcpyAsync(cnt, counts.get(), 4 * K, cudaMemcpyDeviceToHost, s));
-    CK(cudaStreamSynchronize(s));
-    for (int k = 0; k < K; k++) {
-        out[k] = c.alloc<uint32_t>(cnt[k]);
-        if (cnt[k]) {
-            k_class_scatter<<<grid_for(g.n, TPB), TPB, 0, s>>>(g.n, InClass{g.indices, lo[k], hi[k]}, pos[k].get(),
-                                                               out[k]);
-            CK_LAUNCH("k_class_scatter");
-        }
-    }
 }
 
 }  // namespace
@@ -305,43 +285,51 @@ void build_union_structure(Ctx &c, bool always_gid) {
         k_nlow<<<grid_for(n, TPB), TPB, 0, s>>>(n, g.indices, g.adj, g.nlow);
         CK_LAUNCH("k_nlow");
     }
-    {   // the degree classes and the long rows; class 0 includes degree 0 (possible in a
-        // transferred graph; convert never keeps one)
-        constexpr int K = DegreeClasses::K;
-        uint32_t lo[K + 1], hi[K + 1], cnt[K + 1];
-        uint32_t *lists[K + 1];
-        for (int k = 0; k < K; k++) {
-            lo[k] = k ? DegreeClasses::upper[k - 1] + 1 : 0u;
-            hi[k] = DegreeClasses::upper[k];
-        }
-        lo[K] = RowWork::CHUNK + 1;
-        hi[K] = 0xffffffffu;
-        class_lists(c, K + 1, lo, hi, lists, cnt);
-        for (int k = 0; k < K; k++) {
-            g.cls.list[k] = lists[k];
-            g.cls.count[k] = cnt[k];
-        }
-        g.rows.llong = lists[K];
-        g.rows.nlong = cnt[K];
-    }
+    // the degree classes (class 0 includes degree 0, possible in a transferred graph;
+    // convert never keeps one), the long rows and the WCC's triangle-counting buckets:
+    // every list is built before one host read of all their bounds
+    constexpr int K = DegreeClasses::K;
+    const Oriented o{g.indices, g.nlow, g.adj, n};
+    const uint64_t long_most = std::min<uint64_t>(n, 2 * (uint64_t)g.m / (RowWork::CHUNK + 1));
+    uint32_t *lists = c.alloc<uint32_t>(n + long_most), *tc_lists = c.alloc<uint32_t>(n);
+    uint32_t *hb = c.host_u32 + HOST_PLAN, *htc = hb + K + 2;
+    static_assert(HOST_PLAN + K + 2 + TC_LISTS + 1 <= HOST_WORDS, "planning words");
+    c.wplan = TcPlan();
     {
-        RowWork &rw = g.rows;
-        const uint32_t *llong = rw.llong;
-        uint32_t *coff = c.alloc<uint32_t>((size_t)rw.nlong + 1);
-        scan_exclusive<uint32_t>(ChunksOf{llong, g.indices}, coff, rw.nlong, s);
-        CK(cudaMemcpyAsync(&rw.nchunks, coff + rw.nlong, 4, cudaMemcpyDeviceToHost, s));
+        DevBuf<uint32_t> bounds(K + 2 + TC_LISTS + 1, s);
+        build_lists<K + 1>(DegreeMask{g.indices}, n, lists, bounds.get(), s);
+        tc_plan_lists(c, o, c.wplan, tc_lists, bounds.get() + K + 2, s, false, 0);
+        CK(cudaMemcpyAsync(hb, bounds.get(), 4 * (K + 2 + TC_LISTS + 1), cudaMemcpyDeviceToHost, s));
         CK(cudaStreamSynchronize(s));
-        rw.chunk_off = coff;
     }
-    const uint32_t n_big = g.cls.count[DegreeClasses::K - 1];
+    for (int k = 0; k < K; k++) {
+        g.cls.list[k] = lists + hb[k];
+        g.cls.count[k] = hb[k + 1] - hb[k];
+    }
+    g.rows.llong = lists + hb[K];
+    g.rows.nlong = hb[K + 1] - hb[K];
+    if (n) tc_plan_units(c, o, c.wplan, tc_lists, htc, s, true);
+    // the pieces of the long rows and the table words of the last class: one more read, if there are any
+    const uint32_t n_big = g.cls.count[K - 1];
+    uint32_t *coff = c.alloc<uint32_t>((size_t)g.rows.nlong + 1);
+    g.rows.chunk_off = coff;
+    g.rows.nchunks = 0;
     g.big_table_off = c.alloc<uint64_t>((size_t)n_big + 1);
     g.big_table_words = 0;
     c.big_tables = nullptr;
-    if (n_big) {
-        scan_exclusive<uint64_t>(TableWords{g.cls.list[DegreeClasses::K - 1], g.indices}, g.big_table_off, n_big, s);
-        CK(cudaMemcpyAsync(&g.big_table_words, g.big_table_off + n_big, 8, cudaMemcpyDeviceToHost, s));
+    scan_exclusive<uint32_t>(ChunksOf{g.rows.llong, g.indices}, coff, g.rows.nlong, s);
+    if (g.rows.nlong) {   // (a vertex of the last class has a long row)
+        CK(cudaMemcpyAsync(hb, coff + g.rows.nlong, 4, cudaMemcpyDeviceToHost, s));
+        if (n_big) {
+            scan_exclusive<uint64_t>(TableWords{g.cls.list[K - 1], g.indices}, g.big_table_off, n_big, s);
+            CK(cudaMemcpyAsync(hb + 2, g.big_table_off + n_big, 8, cudaMemcpyDeviceToHost, s));
+        }
         CK(cudaStreamSynchronize(s));
-        c.big_tables = c.alloc<uint32_t>(g.big_table_words);
+        g.rows.nchunks = hb[0];
+        if (n_big) {
+            memcpy(&g.big_table_words, hb + 2, 8);
+            c.big_tables = c.alloc<uint32_t>(g.big_table_words);
+        }
     }
     c.pin64 = c.alloc<double>(n);
     c.civ = c.alloc<int4>(n);
@@ -350,8 +338,6 @@ void build_union_structure(Ctx &c, bool always_gid) {
     c.itdeg = c.alloc<int32_t>(n);
     c.int_len = c.alloc<uint32_t>(n);
     c.int_adj = c.alloc<uint32_t>(2 * (size_t)g.m);
-    c.wplan = TcPlan();
-    if (n) tc_plan(c, Oriented{g.indices, g.nlow, g.adj, n}, c.wplan, s, true, false);
     c.wcc_part = c.alloc<double>(b.blocks + 1);
     c.launches += 3;
 }
@@ -645,7 +631,7 @@ int scd_create(scd_ctx **out, int device_id, int work_group_size, unsigned flags
         CK(cudaEventCreateWithFlags(&c.aux_join, cudaEventDisableTiming));
         CK(cudaMalloc((void **)&c.work_counter, 64));
         CK(cudaMallocHost((void **)&c.wcc_host, sizeof(double)));
-        CK(cudaMallocHost((void **)&c.host_u32, 32 * sizeof(uint32_t)));
+        CK(cudaMallocHost((void **)&c.host_u32, HOST_WORDS * sizeof(uint32_t)));
     } catch (const Error &e) {
         scd_destroy(ctx);
         return e.status;

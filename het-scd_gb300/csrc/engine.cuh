@@ -138,7 +138,9 @@ struct TcPlan {
     uint32_t nfwd[K] = {};
     uint32_t dir_lo = 0, dir_hi = 0, dir_amin = 0;   // b-centric iff d+(a) < d+(b),
                                                       // dir_lo < d+(b) <= dir_hi, d+(a) > dir_amin
-    DevBuf<uint32_t> tmp[2 * K];   // storage when the plan is temporary
+    DevBuf<uint32_t> tmp[4];   // storage when the plan is temporary: the lists, the unit offsets
+    // the buckets whose kernels take work units (unit_off is null for the others)
+    static constexpr bool has_units(int k) { return k >= 3 && k <= 5; }
     // Core map of the upper CTA bucket (tc_core_map): the vertices of degree >
     // cta_hi, numbered 0..core_n-1 in id order.  core_adj holds every out-list
     // in core numbers (core_n for a vertex outside the core), v's list at
@@ -163,6 +165,14 @@ void tc_plan(Ctx &c, const Oriented &o, TcPlan &plan, cudaStream_t s, bool owned
 // core's size, lcap: the bucket's longest out-list (both counted beforehand)
 void tc_core_map(Ctx &c, const Oriented &o, uint64_t slots, TcPlan &plan, uint32_t core_n, uint32_t lcap,
                  cudaStream_t s);
+// tc_plan in two parts around a host read the caller shares with other reads: the
+// bucket lists with their bounds (TC_LISTS + 1 device words), then, given the
+// bounds on the host, the plan's pointers and the work-unit offsets
+constexpr int TC_LISTS = TcPlan::K + 2;   // the two CTA buckets have an in-list part
+void tc_plan_lists(Ctx &c, const Oriented &o, TcPlan &plan, uint32_t *lists, uint32_t *bounds, cudaStream_t s,
+                   bool in_lists, uint32_t core_from);
+void tc_plan_units(Ctx &c, const Oriented &o, TcPlan &plan, uint32_t *lists, const uint32_t *host_bounds,
+                   cudaStream_t s, bool owned);
 // the plan of a full count (preprocessing) over out-lists o.adj[0..slots) with in-list
 // centres: the core split and its core map, or the hash kernels' split
 void tc_plan_counting(Ctx &c, const Oriented &o, uint64_t slots, TcPlan &plan, cudaStream_t s);
@@ -180,6 +190,8 @@ double autotune_tc(Ctx &c, std::vector<std::string> *report);
 // set kernel attributes (dynamic shared memory) once per device, outside any capture
 void prepare_tc_kernels();
 void prepare_improve_kernels();
+
+constexpr int HOST_PLAN = 2, HOST_WORDS = 64;   // pinned words of a context (Ctx::host_u32)
 
 struct Ctx;
 // records [start, end) of a phase on the context's stream when profiling
@@ -228,7 +240,7 @@ struct Ctx {
     uint32_t *int_adj = nullptr;      // and the internal out-lists at the CSR offsets (2m)
     TcPlan wplan;                     // triangle-counting plan of the resident graph
     double *wcc_part = nullptr, *wcc_host = nullptr;
-    uint32_t *host_u32 = nullptr;     // pinned: the active-graph count of an iteration [0, 2), planning words [2, 32)
+    uint32_t *host_u32 = nullptr;     // pinned words: the active-graph count of an iteration at 0, planning reads from HOST_PLAN on
     char *io_buf[2] = {};             // pinned pieces of a graph file on its way to the device
     cudaEvent_t io_done[2] = {};
     uint32_t *big_tables = nullptr;   // global hash tables of the last degree bucket

@@ -16,6 +16,7 @@
 //  5. the final symmetric CSR: rows of the kept edges in rank ids, placed by
 //     the known row lengths (tri_deg) and sorted row by row (src/convert.cpp:417-455).
 #include "engine.cuh"
+#include "lists.cuh"
 
 namespace scd {
 
@@ -96,12 +97,6 @@ struct LongRow {
     const uint32_t *off;
     __device__ uint32_t operator[](size_t u) const { return off[u + 1] - off[u] > LONG_ROW; }
 };
-
-__global__ void k_long_list(const uint32_t *__restrict__ off, uint32_t n, const uint32_t *__restrict__ lpos,
-                            uint32_t *longs) {
-    for (uint32_t u = blockIdx.x * blockDim.x + threadIdx.x; u < n; u += gridDim.x * blockDim.x)
-        if (off[u + 1] - off[u] > LONG_ROW) longs[lpos[u]] = u;
-}
 
 // out-slots of every short de-duplicated row (one warp per row; INVALID holes skipped)
 __global__ void k_row_out_count(const uint32_t *__restrict__ off, uint32_t n, const uint32_t *__restrict__ vals,
@@ -516,13 +511,11 @@ void convert_edges(Ctx &c, const uint32_t *pairs_in, uint64_t count, const std::
     //    ocol) and in-lists (icol) in row order; a warp per row, a CTA per row of
     //    more than LONG_ROW entries (a hub's row would be one warp's serial loop)
     DevBuf<uint32_t> olen(n1, s), obeg((size_t)n1 + 1, s), ibeg((size_t)n1 + 1, s);
-    DevBuf<uint32_t> lpos((size_t)n1 + 1, s), longs(n1, s);
-    scan_exclusive<uint32_t>(LongRow{off1.get()}, lpos.get(), n1, s);
-    k_long_list<<<grid_for(n1, TPB), TPB, 0, s>>>(off1.get(), n1, lpos.get(), longs.get());
-    CK_LAUNCH("k_long_list");
+    DevBuf<uint32_t> nlong(2, s), longs(n1, s);   // nlong[1]: long rows
+    build_lists<1>(LongRow{off1.get()}, n1, longs.get(), nlong.get(), s);
     k_row_out_count<<<grid_for((uint64_t)n1 * 32, TPB), TPB, 0, s>>>(off1.get(), n1, vals.get(), cnt.get(), olen.get());
     CK_LAUNCH("k_row_out_count");
-    k_long_out_count<<<152 * 2, LONG_THREADS, 0, s>>>(off1.get(), longs.get(), lpos.get() + n1, vals.get(), cnt.get(),
+    k_long_out_count<<<152 * 2, LONG_THREADS, 0, s>>>(off1.get(), longs.get(), nlong.get() + 1, vals.get(), cnt.get(),
                                                       olen.get());
     CK_LAUNCH("k_long_out_count");
     scan_exclusive<uint32_t>((const uint32_t *)olen.get(), obeg.get(), n1, s);
@@ -532,13 +525,13 @@ void convert_edges(Ctx &c, const uint32_t *pairs_in, uint64_t count, const std::
     k_row_orient<<<grid_for((uint64_t)n1 * 32, TPB), TPB, 0, s>>>(off1.get(), n1, vals.get(), cnt.get(), obeg.get(),
                                                                   ibeg.get(), orow.get(), ocol.get(), icol.get());
     CK_LAUNCH("k_row_orient");
-    k_long_orient<<<152 * 2, LONG_THREADS, 0, s>>>(off1.get(), longs.get(), lpos.get() + n1, vals.get(), cnt.get(),
+    k_long_orient<<<152 * 2, LONG_THREADS, 0, s>>>(off1.get(), longs.get(), nlong.get() + 1, vals.get(), cnt.get(),
                                                    obeg.get(), ibeg.get(), orow.get(), ocol.get(), icol.get());
     CK_LAUNCH("k_long_orient");
     c.launches += 8;
     vals.release();
     off1.release();
-    lpos.release();
+    nlong.release();
     longs.release();
     DevBuf<uint32_t> ilen(n1, s);
     k_in_len<<<grid_for(n1, TPB), TPB, 0, s>>>(cnt.get(), olen.get(), n1, ilen.get());
@@ -576,7 +569,7 @@ void convert_edges(Ctx &c, const uint32_t *pairs_in, uint64_t count, const std::
     CK(cudaMemsetAsync(dmax.get(), 0, 4, s));
     k_reduce_max<uint32_t><<<grid_for(n1, TPB, 152 * 8), TPB, 0, s>>>((const uint32_t *)tdeg1.get(), n1, dmax.get());
     CK_LAUNCH("k_reduce_max");
-    uint32_t *hk = c.host_u32 + 2;   // pinned words: kept vertices, largest tri_deg
+    uint32_t *hk = c.host_u32 + HOST_PLAN;   // kept vertices, largest tri_deg
     CK(cudaMemcpyAsync(hk, kscan.get() + n1, 4, cudaMemcpyDeviceToHost, s));
     CK(cudaMemcpyAsync(hk + 1, dmax.get(), 4, cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));

@@ -490,7 +490,8 @@ uint32_t rebuild(Ctx &c, ResidentSet &R, std::vector<ResidentSource *> &srcs) {
         for (int l = 0; l < NL; l++) list[l] = c.alloc<uint32_t>(lcnt[l]);
         off[NCLS - 1] = c.alloc<uint64_t>(lcnt[NCLS - 1] + 1);
         off[LONG] = c.alloc<uint32_t>(lcnt[LONG] + 1);
-        for (int k = 0; k < TcPlan::K; k++) off[BUCKET0 + k] = c.alloc<uint32_t>(lcnt[BUCKET0 + k] + 1);
+        for (int k = 0; k < TcPlan::K; k++)
+            if (TcPlan::has_units(k)) off[BUCKET0 + k] = c.alloc<uint32_t>(lcnt[BUCKET0 + k] + 1);
         for (int k = 0; k < NCLS; k++) {
             g.cls.list[k] = list[k];
             g.cls.count[k] = (uint32_t)lcnt[k];

@@ -44,6 +44,7 @@
 // T is the lowest of 64, 128, 256, 512, 1024 whose core has at most 128K
 // vertices (R-MAT scale 22: 128; Chung-Lu 8M: 256).
 #include "engine.cuh"
+#include "lists.cuh"
 
 namespace scd {
 
@@ -76,19 +77,25 @@ struct UnitsOf {
     }
 };
 
-struct InBucket {
+// the out-degree bucket of a vertex: bit k for bucket k < 4, bits 4 and 6 for the two CTA
+// buckets, 8 for the last; bit 5 or 7 (in-list centres) when a vertex of a CTA bucket also
+// has a non-empty in-list
+struct BucketMask {
     Oriented o;
-    uint32_t lo, hi;
-    bool in_list;   // in-list centres: also a non-empty in-list
+    uint32_t upper[TcPlan::K];   // ascending
+    bool in_lists;
     __device__ uint32_t operator[](size_t v) const {
-        return o.len[v] > lo && o.len[v] <= hi && (!in_list || o.in_len((uint32_t)v) > 0);
+        const uint32_t len = o.len[v];
+        if (len == 0) return 0u;
+        int k = 0;
+#pragma unroll
+        for (int j = 0; j < TcPlan::K - 1; j++) k += len > upper[j];
+        if (k < 4) return 1u << k;
+        if (k == 6) return 1u << 8;
+        const uint32_t both = in_lists && o.in_len((uint32_t)v) > 0;
+        return (1u | (both << 1)) << (k == 4 ? 4 : 6);
     }
 };
-
-__global__ void k_bucket_scatter(uint32_t n, InBucket f, const uint32_t *__restrict__ pos, uint32_t *out) {
-    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x)
-        if (f[v]) out[pos[v]] = v;
-}
 
 // Short out-lists (d+(a) <= G, G = 16 or 32): one group of G lanes per vertex
 // a, no table.  Lane i holds out(a)[i] in a register (out-lists are sorted
@@ -832,61 +839,59 @@ __global__ void k_core_pad(Oriented o, const uint32_t *__restrict__ cpos, uint32
 
 }  // namespace
 
-void tc_plan(Ctx &c, const Oriented &o, TcPlan &plan, cudaStream_t s, bool owned, bool in_lists, uint32_t core_from) {
+void tc_plan_lists(Ctx &c, const Oriented &o, TcPlan &plan, uint32_t *lists, uint32_t *bounds, cudaStream_t s,
+                   bool in_lists, uint32_t core_from) {
     const uint32_t sm = c.tc_small, s16 = sm < 16 ? sm : 16, s8 = sm < 8 ? sm : 8, b0 = c.tc_b0 > sm ? c.tc_b0 : sm;
     // the core-bitmap kernel takes the upper CTA bucket from core_from on; the hash
     // kernels' upper bucket (one CTA per SM, 16K-entry tables) from tc_b1 on
     const uint32_t b1 = core_from ? (core_from > b0 ? core_from : b0) : c.tc_b1;
-    const uint32_t bounds[TcPlan::K + 1] = {0, s8, s16, sm, b0, b1, B2, 0xffffffffu};
-    const uint32_t per_unit[TcPlan::K] = {1, 1, 1, 32, CTA1_THREADS * CTA1_ROUNDS, CTA2_THREADS * CTA2_ROUNDS, 1};
     const bool split = in_lists && !(c.flags & SCD_FLAG_TC_OUT_ONLY);
     plan.dir_lo = split ? b0 : 0;
     plan.dir_hi = split ? B2 : 0;
     plan.dir_amin = c.tc_amin < sm ? c.tc_amin : sm;
     plan.cta_lo = b0;
     plan.cta_hi = b1;
-    // every bucket's scans first, then one host read of all the counts
-    DevBuf<uint32_t> pos[TcPlan::K], ipos[TcPlan::K], counts(2 * TcPlan::K, s);
+    build_lists<TC_LISTS>(BucketMask{o, {s8, s16, sm, b0, b1, B2, 0xffffffffu}, split}, o.n, lists, bounds, s);
+}
+
+void tc_plan_units(Ctx &c, const Oriented &o, TcPlan &plan, uint32_t *lists, const uint32_t *hb, cudaStream_t s,
+                   bool owned) {
+    const uint32_t per_unit[TcPlan::K] = {1, 1, 1, 32, CTA1_THREADS * CTA1_ROUNDS, CTA2_THREADS * CTA2_ROUNDS, 1};
     for (int k = 0; k < TcPlan::K; k++) {
+        const int l = k < 5 ? k : k + (k == 5 ? 1 : 2);   // first list of bucket k
         const bool cta = k == 4 || k == 5;
-        pos[k].alloc((size_t)o.n + 1, s);
-        scan_exclusive<uint32_t>(InBucket{o, bounds[k], bounds[k + 1], false}, pos[k].get(), o.n, s);
-        CK(cudaMemcpyAsync(counts.get() + 2 * k, pos[k].get() + o.n, 4, cudaMemcpyDeviceToDevice, s));
-        if (split && cta) {
-            ipos[k].alloc((size_t)o.n + 1, s);
-            scan_exclusive<uint32_t>(InBucket{o, bounds[k], bounds[k + 1], true}, ipos[k].get(), o.n, s);
-            CK(cudaMemcpyAsync(counts.get() + 2 * k + 1, ipos[k].get() + o.n, 4, cudaMemcpyDeviceToDevice, s));
-        } else {
-            CK(cudaMemsetAsync(counts.get() + 2 * k + 1, 0, 4, s));
-        }
-    }
-    uint32_t cnts[2 * TcPlan::K];
-    CK(cudaMemcpyAsync(cnts, counts.get(), sizeof cnts, cudaMemcpyDeviceToHost, s));
-    CK(cudaStreamSynchronize(s));
-    for (int k = 0; k < TcPlan::K; k++) {
-        const InBucket fa{o, bounds[k], bounds[k + 1], false}, fb{o, bounds[k], bounds[k + 1], true};
-        const uint32_t na = cnts[2 * k], nb = cnts[2 * k + 1], cnt = na + nb;
-        plan.nverts[k] = cnt;
-        plan.nfwd[k] = na;
+        plan.verts[k] = lists + hb[l];
+        plan.nfwd[k] = hb[l + 1] - hb[l];
+        plan.nverts[k] = hb[l + 1 + cta] - hb[l];
+        plan.unit_off[k] = nullptr;
+        if (!TcPlan::has_units(k)) continue;
+        const uint32_t cnt = plan.nverts[k];
         if (owned) {
-            plan.verts[k] = c.alloc<uint32_t>(cnt);
             plan.unit_off[k] = c.alloc<uint32_t>((size_t)cnt + 1);
         } else {
-            plan.tmp[2 * k].alloc(cnt ? cnt : 1, s);
-            plan.tmp[2 * k + 1].alloc((size_t)cnt + 1, s);
-            plan.verts[k] = plan.tmp[2 * k].get();
-            plan.unit_off[k] = plan.tmp[2 * k + 1].get();
+            plan.tmp[k - 2].alloc((size_t)cnt + 1, s);
+            plan.unit_off[k] = plan.tmp[k - 2].get();
         }
-        if (na) {
-            k_bucket_scatter<<<grid_for(o.n, 256), 256, 0, s>>>(o.n, fa, pos[k].get(), plan.verts[k]);
-            CK_LAUNCH("k_bucket_scatter");
-        }
-        if (nb) {
-            k_bucket_scatter<<<grid_for(o.n, 256), 256, 0, s>>>(o.n, fb, ipos[k].get(), plan.verts[k] + na);
-            CK_LAUNCH("k_bucket_scatter");
-        }
-        scan_exclusive<uint32_t>(UnitsOf{o, plan.verts[k], per_unit[k], na}, plan.unit_off[k], cnt, s);
+        if (cnt || owned)
+            scan_exclusive<uint32_t>(UnitsOf{o, plan.verts[k], per_unit[k], plan.nfwd[k]}, plan.unit_off[k], cnt, s);
     }
+}
+
+void tc_plan(Ctx &c, const Oriented &o, TcPlan &plan, cudaStream_t s, bool owned, bool in_lists, uint32_t core_from) {
+    const size_t most = in_lists ? 2 * (size_t)o.n : o.n;   // an in-list centre is listed twice
+    uint32_t *lists;
+    if (owned) {
+        lists = c.alloc<uint32_t>(most);
+    } else {
+        plan.tmp[0].alloc(most ? most : 1, s);
+        lists = plan.tmp[0].get();
+    }
+    DevBuf<uint32_t> bounds(TC_LISTS + 1, s);
+    tc_plan_lists(c, o, plan, lists, bounds.get(), s, in_lists, core_from);
+    uint32_t *hb = c.host_u32 + HOST_PLAN;
+    CK(cudaMemcpyAsync(hb, bounds.get(), 4 * (TC_LISTS + 1), cudaMemcpyDeviceToHost, s));
+    CK(cudaStreamSynchronize(s));
+    tc_plan_units(c, o, plan, lists, hb, s, owned);
 }
 
 void tc_core_map(Ctx &c, const Oriented &o, uint64_t slots, TcPlan &plan, uint32_t core_n, uint32_t lcap,
@@ -936,7 +941,7 @@ void tc_plan_counting(Ctx &c, const Oriented &o, uint64_t slots, TcPlan &plan, c
     k_core_counts<<<grid_for(o.n, 256, 152 * 8), 256, 0, s>>>(o, cb, cnt.get());
     CK_LAUNCH("k_core_counts");
     c.launches++;
-    uint32_t *h = c.host_u32 + 2;   // pinned planning words
+    uint32_t *h = c.host_u32 + HOST_PLAN;
     CK(cudaMemcpyAsync(h, cnt.get(), 8 * K, cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
     int pick = -1;
