@@ -228,23 +228,25 @@ struct RowLenOf {
     __device__ uint32_t operator[](size_t i) const { return off[list[i] + 1] - off[list[i]]; }
 };
 
-// long rows: key = (rank of the row in the list) << 32 | value
+// long rows: key = (rank of the row in the list) << vbits | value (values are row numbers, < 2^vbits)
+template <typename K>
 __global__ void k_big_keys(const uint32_t *__restrict__ list, uint32_t count, const uint32_t *__restrict__ off,
-                           const uint32_t *__restrict__ koff, const uint32_t *__restrict__ vals, uint64_t *keys) {
+                           const uint32_t *__restrict__ koff, const uint32_t *__restrict__ vals, int vbits, K *keys) {
     for (uint32_t i = blockIdx.x; i < count; i += gridDim.x) {
         const uint32_t r = list[i], beg = off[r], len = off[r + 1] - beg, k0 = koff[i];
-        for (uint32_t t = threadIdx.x; t < len; t += blockDim.x) keys[k0 + t] = ((uint64_t)i << 32) | vals[beg + t];
+        for (uint32_t t = threadIdx.x; t < len; t += blockDim.x) keys[k0 + t] = ((K)i << vbits) | vals[beg + t];
     }
 }
 
-__global__ void k_big_back(const uint64_t *__restrict__ keys, uint32_t total, const uint32_t *__restrict__ list,
+template <typename K>
+__global__ void k_big_back(const K *__restrict__ keys, int vbits, uint32_t total, const uint32_t *__restrict__ list,
                            const uint32_t *__restrict__ off, const uint32_t *__restrict__ koff, uint32_t *vals,
                            bool dedup, uint32_t *udeg) {
     for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < total; p += gridDim.x * blockDim.x) {
-        const uint64_t key = keys[p];
-        const uint32_t i = (uint32_t)(key >> 32), v = (uint32_t)key;
+        const K key = keys[p];
+        const uint32_t i = (uint32_t)(key >> vbits), v = (uint32_t)(key & (((K)1 << vbits) - 1));
         const uint32_t t = p - koff[i], r = list[i];
-        const bool keep = !dedup || t == 0 || (uint32_t)keys[p - 1] != v;
+        const bool keep = !dedup || t == 0 || keys[p - 1] != key;
         vals[off[r] + t] = keep ? v : INVALID;
         if (udeg) {
             const unsigned peers = __match_any_sync(__activemask(), i);
@@ -256,6 +258,21 @@ __global__ void k_big_back(const uint64_t *__restrict__ keys, uint32_t total, co
 
 __global__ void k_zero_rows(const uint32_t *__restrict__ list, uint32_t count, uint32_t *udeg) {
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) udeg[list[i]] = 0;
+}
+
+template <typename K>
+void sort_big_rows(const uint32_t *list, uint32_t count, const uint32_t *off, const uint32_t *koff, uint32_t total,
+                   int vbits, int bits, uint32_t *vals, bool dedup, uint32_t *udeg, cudaStream_t s) {
+    DevBuf<K> keys(total, s);
+    k_big_keys<K><<<grid_for(count, 1, 152 * 8), TPB, 0, s>>>(list, count, off, koff, vals, vbits, keys.get());
+    CK_LAUNCH("k_big_keys");
+    radix_sort<K>(keys.get(), nullptr, total, 0, bits, s);
+    if (udeg) {
+        k_zero_rows<<<grid_for(count, TPB), TPB, 0, s>>>(list, count, udeg);
+        CK_LAUNCH("k_zero_rows");
+    }
+    k_big_back<K><<<grid_for(total, TPB), TPB, 0, s>>>(keys.get(), vbits, total, list, off, koff, vals, dedup, udeg);
+    CK_LAUNCH("k_big_back");
 }
 
 void prepare_sort_kernels() {
@@ -332,18 +349,10 @@ void sort_rows(Ctx &c, const uint32_t *off, uint32_t nrows, uint32_t *vals, bool
         uint32_t total = 0;
         CK(cudaMemcpyAsync(&total, koff.get() + cnt[6], 4, cudaMemcpyDeviceToHost, s));
         CK(cudaStreamSynchronize(s));
-        DevBuf<uint64_t> keys(total, s);
-        k_big_keys<<<grid_for(cnt[6], 1, 152 * 8), TPB, 0, s>>>(list[6], cnt[6], off, koff.get(), vals,
-                                                               keys.get());
-        CK_LAUNCH("k_big_keys");
-        radix_sort<uint64_t>(keys.get(), nullptr, total, 0, 32 + ceil_log2(cnt[6] < 2 ? 2 : cnt[6]), s);
-        if (udeg) {
-            k_zero_rows<<<grid_for(cnt[6], TPB), TPB, 0, s>>>(list[6], cnt[6], udeg);
-            CK_LAUNCH("k_zero_rows");
-        }
-        k_big_back<<<grid_for(total, TPB), TPB, 0, s>>>(keys.get(), total, list[6], off, koff.get(), vals,
-                                                        dedup, udeg);
-        CK_LAUNCH("k_big_back");
+        // the keys are as wide as the row ranks and the values need: in 32 bits a pass moves half the bytes
+        const int vbits = ceil_log2(nrows < 2 ? 2 : nrows), bits = vbits + ceil_log2(cnt[6] < 2 ? 2 : cnt[6]);
+        if (bits <= 32) sort_big_rows<uint32_t>(list[6], cnt[6], off, koff.get(), total, vbits, bits, vals, dedup, udeg, s);
+        else sort_big_rows<uint64_t>(list[6], cnt[6], off, koff.get(), total, vbits, bits, vals, dedup, udeg, s);
         c.launches += 3;
     }
 }

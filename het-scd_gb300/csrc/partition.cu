@@ -8,10 +8,12 @@
 // maximal independent set of that order); a seed's label is its rank among the
 // seeds; a non-seed takes the label of its earliest seed neighbour (that seed
 // reached it first).  The order comes from two stable LSD radix sorts:
-// (deg, id) then the cc bits (positive doubles order like their bit patterns).
+// the degree (from descending ids) then the cc bits (positive doubles order like their bit patterns).
 // The independent set is found in rounds: an undecided vertex becomes a
 // non-seed as soon as an earlier neighbour is a seed, and a seed once every
 // earlier neighbour is a decided non-seed.
+#include <algorithm>
+
 #include "engine.cuh"
 
 namespace scd {
@@ -21,11 +23,14 @@ namespace {
 constexpr unsigned TPB = 256;
 constexpr uint8_t UNDECIDED = 0, SEED = 1, NONSEED = 2;
 
-__global__ void k_order_keys(uint32_t n, const uint32_t *__restrict__ indices, uint64_t *keys, uint32_t *vals) {
-    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
-        const uint32_t d = indices[v + 1] - indices[v];
-        keys[v] = ((uint64_t)(0xffffffffu - d) << 32) | (0xffffffffu - v);
-        vals[v] = v;
+// the vertices in descending id order with the keys maxd - degree: a stable sort of
+// them gives (degree, id) descending
+__global__ void k_order_keys(uint32_t n, const uint32_t *__restrict__ indices, uint32_t maxd, uint32_t *keys,
+                             uint32_t *vals) {
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const uint32_t v = n - 1 - i;
+        keys[i] = maxd - (indices[v + 1] - indices[v]);
+        vals[i] = v;
     }
 }
 
@@ -207,9 +212,15 @@ void initial_partition(Ctx &c) {
     PhaseScope ph(c, "partition");
     DevBuf<uint64_t> keys(n, s);
     DevBuf<uint32_t> order(n, s), pos(n, s), undecided(1, s);
-    k_order_keys<<<grid_for(n, TPB), TPB, 0, s>>>(n, g.indices, keys.get(), order.get());
-    CK_LAUNCH("k_order_keys");
-    radix_sort<uint64_t>(keys.get(), order.get(), n, 0, 64, s);
+    {   // no degree is above the bound of the highest class that has a vertex, or 2m
+        uint32_t maxd = 2 * g.m;
+        for (int k = DegreeClasses::K - 1; k >= 0 && !g.cls.count[k]; k--)
+            if (k) maxd = std::min(maxd, DegreeClasses::upper[k - 1]);
+        DevBuf<uint32_t> dkeys(n, s);
+        k_order_keys<<<grid_for(n, TPB), TPB, 0, s>>>(n, g.indices, maxd, dkeys.get(), order.get());
+        CK_LAUNCH("k_order_keys");
+        radix_sort<uint32_t>(dkeys.get(), order.get(), n, 0, ceil_log2((uint64_t)maxd + 1), s);
+    }
     k_cc_keys<<<grid_for(n, TPB), TPB, 0, s>>>(n, order.get(), g.indices, g.tri, keys.get());
     CK_LAUNCH("k_cc_keys");
     radix_sort<uint64_t>(keys.get(), order.get(), n, 0, 64, s);

@@ -247,16 +247,16 @@ __global__ void k_tri_from_count(const uint32_t *__restrict__ tcount, uint32_t n
         tri[v] = (int32_t)(2u * tcount[v]);
 }
 
-// the kept vertices (tri_deg > 0) at their id-order positions kscan[v], with the
-// key ((maxd - tri_deg) << k) | (2^k-1 - v): ascending = (tri_deg, v) descending
+// the n2 kept vertices (tri_deg > 0) in descending id order (kscan: their positions in
+// ascending order) with the keys maxd - tri_deg: a stable sort of them gives
+// (tri_deg, v) descending
 __global__ void k_kept_keys(const int32_t *__restrict__ tri_deg, uint32_t n, const uint32_t *__restrict__ kscan,
-                            uint32_t maxd, int k, uint64_t *keys, uint32_t *vals) {
-    const uint64_t vmax = (1ull << k) - 1;
+                            uint32_t n2, uint32_t maxd, uint32_t *keys, uint32_t *vals) {
     for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
         const int32_t d = tri_deg[v];
         if (d > 0) {
-            const uint32_t i = kscan[v];
-            keys[i] = ((uint64_t)(maxd - (uint32_t)d) << k) | (vmax - v);
+            const uint32_t i = n2 - 1 - kscan[v];
+            keys[i] = maxd - (uint32_t)d;
             vals[i] = v;
         }
     }
@@ -384,7 +384,7 @@ __global__ void k_count_renamed(const uint32_t *__restrict__ rename, uint32_t n_
 }
 
 __global__ void k_graph_of_order(const uint32_t *__restrict__ order, uint32_t n, const uint32_t *__restrict__ ren_off,
-                                 uint32_t G, uint64_t *keys) {
+                                 uint32_t G, uint32_t *keys) {
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
         keys[i] = segment_of32(ren_off, G, order[i]);
 }
@@ -493,7 +493,6 @@ void convert_edges(Ctx &c, const uint32_t *pairs_in, uint64_t count, const std::
     }
 
     // 2. de-duplicated symmetric CSR over the renamed ids: rows by a counting sort, then sorted row by row
-    const int k1 = ceil_log2(n1 < 2 ? 2 : n1);
     DevBuf<uint32_t> cnt(n1, s), off1((size_t)n1 + 1, s);
     CK(cudaMemsetAsync(cnt.get(), 0, (size_t)n1 * 4, s));
     k_pair_degrees<<<G, TPB, 0, s>>>(pairs, count, rename.get(), cnt.get());
@@ -574,15 +573,14 @@ void convert_edges(Ctx &c, const uint32_t *pairs_in, uint64_t count, const std::
     CK(cudaMemcpyAsync(hk + 1, dmax.get(), 4, cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
     const uint32_t n2 = hk[0], maxd = hk[1];
-    DevBuf<uint64_t> dkeys(n2 ? n2 : 1, s);
-    DevBuf<uint32_t> order(n2 ? n2 : 1, s), rank(n1, s);
-    k_kept_keys<<<grid_for(n1, TPB), TPB, 0, s>>>(tdeg1.get(), n1, kscan.get(), maxd, k1, dkeys.get(), order.get());
+    DevBuf<uint32_t> dkeys(n2 ? n2 : 1, s), order(n2 ? n2 : 1, s), rank(n1, s);
+    k_kept_keys<<<grid_for(n1, TPB), TPB, 0, s>>>(tdeg1.get(), n1, kscan.get(), n2, maxd, dkeys.get(), order.get());
     CK_LAUNCH("k_kept_keys");
-    radix_sort<uint64_t>(dkeys.get(), order.get(), n2, 0, k1 + ceil_log2((uint64_t)maxd + 1), s);
+    radix_sort<uint32_t>(dkeys.get(), order.get(), n2, 0, ceil_log2((uint64_t)maxd + 1), s);
     if (NG > 1) {   // graph-major (stable): each graph's vertices stay contiguous
         k_graph_of_order<<<grid_for(n2 ? n2 : 1, TPB), TPB, 0, s>>>(order.get(), n2, ren_off.get(), NG, dkeys.get());
         CK_LAUNCH("k_graph_of_order");
-        radix_sort<uint64_t>(dkeys.get(), order.get(), n2, 0, ceil_log2(NG), s);
+        radix_sort<uint32_t>(dkeys.get(), order.get(), n2, 0, ceil_log2(NG), s);
     }
     dkeys.release();
 

@@ -188,22 +188,36 @@ __global__ void k_reduce_max(const T *in, size_t n, T *out) {
 }
 
 // ---------------------------------------------------------------------------
-// stable LSD radix sort, 8-bit digits, reduce-then-scan per pass.
+// stable LSD radix sort, 8-bit digits.
 //
 // A tile is RS_WARPS*32*RS_ITEMS keys; warp w of a tile owns the contiguous
 // run [w*32*RS_ITEMS, (w+1)*32*RS_ITEMS) and walks it 32 keys at a time, so
 // (step, lane) order equals input order and __match_any_sync ranking keeps the
 // sort stable.
+//
+// What bounds a sort is its launches for all but the largest graphs, so there are
+// three forms by size:
+//   one tile         one CTA makes every pass in shared memory, one launch;
+//   <= RS_FUSED      one launch a pass: every CTA adds up the digit counts of the
+//     tiles          tiles before its own (at most RS_FUSED reads a thread), and
+//                    counts the next pass's digits by output tile as it writes;
+//   more             per pass the tiles' digit counts, a scan of them, and the
+//                    move: the counts before a tile are too many to add up again
+//                    in every CTA.
 
 constexpr int RS_WARPS = 8;
 constexpr int RS_THREADS = RS_WARPS * 32;
 constexpr int RS_ITEMS = 8;
 constexpr int RS_TILE = RS_THREADS * RS_ITEMS;
+constexpr size_t RS_FUSED = 128;   // tiles
+static_assert(RS_THREADS == 256, "one thread per digit");
 
+// Digit counts of the tile at blockIdx.x: to hist[digit * tiles + tile] (for the scan)
+// or, tile_major, to hist[tile * 256 + digit].
 template <typename K>
 __global__ void __launch_bounds__(RS_THREADS) k_rs_upsweep(const K *keys, size_t n, int shift,
                                                            unsigned mask, uint32_t *hist,
-                                                           size_t tiles) {
+                                                           size_t tiles, bool tile_major) {
     __shared__ uint32_t cnt[RS_WARPS][256];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int i = threadIdx.x; i < RS_WARPS * 256; i += RS_THREADS) (&cnt[0][0])[i] = 0;
@@ -219,45 +233,29 @@ __global__ void __launch_bounds__(RS_THREADS) k_rs_upsweep(const K *keys, size_t
         __syncwarp();
     }
     __syncthreads();
-    for (int d = threadIdx.x; d < 256; d += RS_THREADS) {
-        uint32_t s = 0;
+    const int d = threadIdx.x;
+    uint32_t s = 0;
 #pragma unroll
-        for (int w = 0; w < RS_WARPS; w++) s += cnt[w][d];
-        hist[(size_t)d * tiles + blockIdx.x] = s;
-    }
+    for (int w = 0; w < RS_WARPS; w++) s += cnt[w][d];
+    hist[tile_major ? (size_t)blockIdx.x * 256 + d : (size_t)d * tiles + blockIdx.x] = s;
 }
 
-// Ranks every key of the tile stably by digit, reorders the tile in shared
-// memory, then writes it out in tile order so that keys of one digit leave as
-// one contiguous run (coalesced) at the digit's global offset.
-template <typename K, bool HAS_VALS>
-__global__ void __launch_bounds__(RS_THREADS, 4) k_rs_downsweep(const K *keys_in, const uint32_t *vals_in,
-                                                                K *keys_out, uint32_t *vals_out,
-                                                                size_t n, int shift, unsigned mask,
-                                                                const uint32_t *offsets, size_t tiles) {
-    __shared__ uint32_t cnt[RS_WARPS][256];
-    __shared__ uint32_t tile_start[256];   // first tile position of each digit
-    __shared__ uint32_t glob[256];         // global position of that first key
-    __shared__ K skeys[RS_TILE];
-    __shared__ uint32_t svals[HAS_VALS ? RS_TILE : 1];
+// Stable rank of every key of a tile within its digit and warp (rank[k]); cnt[w][d] becomes
+// the digit's keys in the warps before w, returns the tile's keys of digit threadIdx.x.
+// `count` keys of the tile are valid.  Starts and ends with a barrier's worth of order.
+template <typename K>
+__device__ __forceinline__ uint32_t rs_rank(const K (&key)[RS_ITEMS], uint32_t count, int shift, unsigned mask,
+                                            uint32_t (&cnt)[RS_WARPS][256], uint32_t (&rank)[RS_ITEMS]) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const unsigned lt = lanemask_lt();
     for (int i = threadIdx.x; i < RS_WARPS * 256; i += RS_THREADS) (&cnt[0][0])[i] = 0;
     __syncthreads();
-    const size_t tile_base = (size_t)blockIdx.x * RS_TILE;
-    const size_t base = tile_base + (size_t)warp * 32 * RS_ITEMS;
-    K key[RS_ITEMS];
-    uint32_t val[RS_ITEMS];
-    uint32_t rank[RS_ITEMS];
-    const unsigned lt = lanemask_lt();
 #pragma unroll
     for (int k = 0; k < RS_ITEMS; k++) {
-        size_t idx = base + (size_t)k * 32 + lane;
-        bool valid = idx < n;
-        key[k] = valid ? keys_in[idx] : K(0);
-        if (HAS_VALS) val[k] = valid ? vals_in[idx] : 0u;
-        unsigned d = valid ? (unsigned)(key[k] >> shift) & mask : 0xffffffffu;
-        unsigned peers = __match_any_sync(FULL, d);
-        int leader = __ffs(peers) - 1;
+        const bool valid = (uint32_t)(warp * 32 * RS_ITEMS + k * 32 + lane) < count;
+        const unsigned d = valid ? (unsigned)(key[k] >> shift) & mask : 0xffffffffu;
+        const unsigned peers = __match_any_sync(FULL, d);
+        const int leader = __ffs(peers) - 1;
         uint32_t before = 0;
         if (valid && lane == leader) {
             before = cnt[warp][d];
@@ -268,47 +266,191 @@ __global__ void __launch_bounds__(RS_THREADS, 4) k_rs_downsweep(const K *keys_in
         __syncwarp();
     }
     __syncthreads();
-    // per digit: exclusive prefix over warps (in place) and the digit's tile total
     uint32_t total = 0;
-    if (threadIdx.x < 256) {
-        const int d = threadIdx.x;
 #pragma unroll
-        for (int w = 0; w < RS_WARPS; w++) {
-            uint32_t c = cnt[w][d];
-            cnt[w][d] = total;
-            total += c;
+    for (int w = 0; w < RS_WARPS; w++) {
+        const uint32_t c = cnt[w][threadIdx.x];
+        cnt[w][threadIdx.x] = total;
+        total += c;
+    }
+    return total;
+}
+
+// exclusive sum over the 256 threads (sw: RS_WARPS words)
+__device__ __forceinline__ uint32_t rs_scan256(uint32_t v, uint32_t *sw) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t inc = warp_inclusive_scan(v);
+    if (lane == 31) sw[warp] = inc;
+    __syncthreads();
+    uint32_t off = 0;
+    for (int w = 0; w < warp; w++) off += sw[w];
+    __syncthreads();
+    return off + inc - v;
+}
+
+// Ranks every key of the tile stably by digit, reorders the tile in shared
+// memory, then writes it out in tile order so that keys of one digit leave as
+// one contiguous run (coalesced) at the digit's global offset.
+// FUSED: `hist` holds the tile-major digit counts of this pass (the offsets are
+// summed up here) and next_hist, if not null, receives those of the next pass;
+// else `hist` holds the scanned digit-major offsets.
+template <typename K, bool HAS_VALS, bool FUSED>
+__global__ void __launch_bounds__(RS_THREADS, 4) k_rs_downsweep(const K *keys_in, const uint32_t *vals_in,
+                                                                K *keys_out, uint32_t *vals_out,
+                                                                size_t n, int shift, unsigned mask,
+                                                                const uint32_t *hist, size_t tiles,
+                                                                uint32_t *next_hist, int next_shift,
+                                                                unsigned next_mask) {
+    __shared__ uint32_t cnt[RS_WARPS][256];
+    __shared__ uint32_t tile_start[256];   // first tile position of each digit
+    __shared__ uint32_t glob[256];         // global position of that first key
+    __shared__ uint32_t sw[RS_WARPS];
+    __shared__ K skeys[RS_TILE];
+    __shared__ uint32_t svals[HAS_VALS ? RS_TILE : 1];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const size_t tile_base = (size_t)blockIdx.x * RS_TILE;
+    const uint32_t count = (uint32_t)min((size_t)RS_TILE, n - tile_base);
+    const uint32_t first = warp * 32 * RS_ITEMS + lane;
+    K key[RS_ITEMS];
+    uint32_t val[RS_ITEMS], rank[RS_ITEMS];
+#pragma unroll
+    for (int k = 0; k < RS_ITEMS; k++) {
+        const bool valid = first + k * 32 < count;
+        key[k] = valid ? keys_in[tile_base + first + k * 32] : K(0);
+        if (HAS_VALS) val[k] = valid ? vals_in[tile_base + first + k * 32] : 0u;
+    }
+    if constexpr (FUSED) {
+        uint32_t before = 0, all = 0;
+#pragma unroll 8
+        for (uint32_t t = 0; t < (uint32_t)tiles; t++) {
+            const uint32_t h = hist[t * 256 + threadIdx.x];
+            if (t < blockIdx.x) before += h;
+            all += h;
         }
-        glob[d] = offsets[(size_t)d * tiles + blockIdx.x];
+        glob[threadIdx.x] = rs_scan256(all, sw) + before;
+    } else {
+        glob[threadIdx.x] = hist[(size_t)threadIdx.x * tiles + blockIdx.x];
     }
-    // exclusive scan of the 256 digit totals (RS_THREADS == 256: one per thread)
-    {
-        __shared__ uint32_t wsum[RS_WARPS];
-        uint32_t inc = warp_inclusive_scan(total);
-        if (lane == 31) wsum[warp] = inc;
-        __syncthreads();
-        uint32_t off = 0;
-        for (int w = 0; w < warp; w++) off += wsum[w];
-        tile_start[threadIdx.x] = off + inc - total;
-    }
+    const uint32_t total = rs_rank(key, count, shift, mask, cnt, rank);
+    tile_start[threadIdx.x] = rs_scan256(total, sw);
     __syncthreads();
 #pragma unroll
     for (int k = 0; k < RS_ITEMS; k++) {
-        size_t idx = base + (size_t)k * 32 + lane;
-        if (idx < n) {
-            unsigned d = (unsigned)(key[k] >> shift) & mask;
-            uint32_t p = tile_start[d] + cnt[warp][d] + rank[k];
+        if (first + k * 32 < count) {
+            const unsigned d = (unsigned)(key[k] >> shift) & mask;
+            const uint32_t p = tile_start[d] + cnt[warp][d] + rank[k];
             skeys[p] = key[k];
             if (HAS_VALS) svals[p] = val[k];
         }
     }
     __syncthreads();
-    const uint32_t count = (uint32_t)min((size_t)RS_TILE, n - tile_base);
-    for (uint32_t i = threadIdx.x; i < count; i += RS_THREADS) {
-        const K kk = skeys[i];
-        const unsigned d = (unsigned)(kk >> shift) & mask;
-        const uint32_t dst = glob[d] + (i - tile_start[d]);
-        keys_out[dst] = kk;
-        if (HAS_VALS) vals_out[dst] = svals[i];
+    for (uint32_t i0 = warp * 32; i0 < count; i0 += RS_THREADS) {
+        const uint32_t i = i0 + lane;
+        const bool valid = i < count;
+        const K kk = valid ? skeys[i] : K(0);
+        uint32_t dst = 0;
+        if (valid) {
+            const unsigned d = (unsigned)(kk >> shift) & mask;
+            dst = glob[d] + (i - tile_start[d]);
+            keys_out[dst] = kk;
+            if (HAS_VALS) vals_out[dst] = svals[i];
+        }
+        if (FUSED && next_hist) {   // equal keys leave together: one atomic per counter and warp
+            const uint32_t at = valid ? (dst / RS_TILE) * 256 + ((unsigned)(kk >> next_shift) & next_mask) : INVALID;
+            const unsigned peers = __match_any_sync(FULL, at);
+            if (valid && lane == __ffs(peers) - 1) atomicAdd(next_hist + at, (uint32_t)__popc(peers));
+        }
+    }
+}
+
+// up to one tile: every pass in one CTA
+template <typename K, bool HAS_VALS>
+__global__ void __launch_bounds__(RS_THREADS) k_rs_one(K *keys, uint32_t *vals, uint32_t n, int begin_bit, int end_bit) {
+    __shared__ uint32_t cnt[RS_WARPS][256];
+    __shared__ uint32_t tile_start[256], sw[RS_WARPS];
+    __shared__ K skeys[RS_TILE];
+    __shared__ uint32_t svals[HAS_VALS ? RS_TILE : 1];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t first = warp * 32 * RS_ITEMS + lane;
+    K key[RS_ITEMS];
+    uint32_t val[RS_ITEMS], rank[RS_ITEMS];
+#pragma unroll
+    for (int k = 0; k < RS_ITEMS; k++) {
+        const bool valid = first + k * 32 < n;
+        key[k] = valid ? keys[first + k * 32] : K(0);
+        val[k] = HAS_VALS && valid ? vals[first + k * 32] : 0u;
+    }
+    for (int b = begin_bit; b < end_bit; b += 8) {
+        const unsigned mask = (1u << (end_bit - b < 8 ? end_bit - b : 8)) - 1u;
+        const uint32_t total = rs_rank(key, n, b, mask, cnt, rank);
+        tile_start[threadIdx.x] = rs_scan256(total, sw);
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < RS_ITEMS; k++)
+            if (first + k * 32 < n) {
+                const unsigned d = (unsigned)(key[k] >> b) & mask;
+                const uint32_t p = tile_start[d] + cnt[warp][d] + rank[k];
+                skeys[p] = key[k];
+                if (HAS_VALS) svals[p] = val[k];
+            }
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < RS_ITEMS; k++)
+            if (first + k * 32 < n) {
+                key[k] = skeys[first + k * 32];
+                if (HAS_VALS) val[k] = svals[first + k * 32];
+            }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int k = 0; k < RS_ITEMS; k++)
+        if (first + k * 32 < n) {
+            keys[first + k * 32] = key[k];
+            if (HAS_VALS) vals[first + k * 32] = val[k];
+        }
+}
+
+template <typename K, bool HAS_VALS>
+void radix_sort_impl(K *keys, uint32_t *vals, size_t n, int begin_bit, int end_bit, cudaStream_t s) {
+    if (n <= (size_t)RS_TILE) {
+        k_rs_one<K, HAS_VALS><<<1, RS_THREADS, 0, s>>>(keys, vals, (uint32_t)n, begin_bit, end_bit);
+        CK_LAUNCH("k_rs_one");
+        return;
+    }
+    const size_t tiles = (n + RS_TILE - 1) / RS_TILE;
+    const int passes = (end_bit - begin_bit + 7) / 8;
+    const bool fused = tiles <= RS_FUSED;
+    DevBuf<K> kt(n, s);
+    DevBuf<uint32_t> vt(HAS_VALS ? n : 0, s);
+    DevBuf<uint32_t> hist(fused ? 256 * tiles * passes : 256 * tiles + 1, s);
+    K *kin = keys, *kout = kt.get();
+    uint32_t *vin = vals, *vout = vt.get(), *h = hist.get();
+    if (fused && passes > 1) CK(cudaMemsetAsync(h + 256 * tiles, 0, 4 * 256 * tiles * (passes - 1), s));
+    for (int p = 0; p < passes; p++) {
+        const int b = begin_bit + 8 * p, nb = b + 8;
+        const auto mask_at = [&](int bit) { return (1u << (end_bit - bit < 8 ? end_bit - bit : 8)) - 1u; };
+        if (!fused || p == 0) {
+            k_rs_upsweep<K><<<(unsigned)tiles, RS_THREADS, 0, s>>>(kin, n, b, mask_at(b), h, tiles, fused);
+            CK_LAUNCH("k_rs_upsweep");
+        }
+        if (fused) {
+            const bool more = p + 1 < passes;
+            k_rs_downsweep<K, HAS_VALS, true><<<(unsigned)tiles, RS_THREADS, 0, s>>>(
+                kin, vin, kout, vout, n, b, mask_at(b), h, tiles, more ? h + 256 * tiles : nullptr, more ? nb : 0,
+                more ? mask_at(nb) : 0u);
+            h += 256 * tiles;
+        } else {
+            scan_exclusive<uint32_t, const uint32_t *>(h, h, 256 * tiles, s);
+            k_rs_downsweep<K, HAS_VALS, false><<<(unsigned)tiles, RS_THREADS, 0, s>>>(kin, vin, kout, vout, n, b,
+                                                                                     mask_at(b), h, tiles, nullptr, 0, 0u);
+        }
+        CK_LAUNCH("k_rs_downsweep");
+        K *tk = kin; kin = kout; kout = tk;
+        uint32_t *tv = vin; vin = vout; vout = tv;
+    }
+    if (passes & 1) {
+        CK(cudaMemcpyAsync(keys, kin, n * sizeof(K), cudaMemcpyDeviceToDevice, s));
+        if (HAS_VALS) CK(cudaMemcpyAsync(vals, vin, n * sizeof(uint32_t), cudaMemcpyDeviceToDevice, s));
     }
 }
 
@@ -318,34 +460,8 @@ template <typename K>
 void radix_sort(K *keys, uint32_t *vals, size_t n, int begin_bit, int end_bit, cudaStream_t s) {
     if (n < 2 || end_bit <= begin_bit) return;
     if (n >= (size_t(1) << 32)) throw Error(SCD_ERR_LIMIT, "radix_sort: more than 2^32 keys");
-    const size_t tiles = (n + RS_TILE - 1) / RS_TILE;
-    DevBuf<K> kt(n, s);
-    DevBuf<uint32_t> vt(vals ? n : 0, s);
-    DevBuf<uint32_t> hist(256 * tiles + 1, s);
-    K *kin = keys, *kout = kt.get();
-    uint32_t *vin = vals, *vout = vt.get();
-    int passes = 0;
-    for (int b = begin_bit; b < end_bit; b += 8) {
-        int bits = end_bit - b < 8 ? end_bit - b : 8;
-        unsigned mask = (1u << bits) - 1u;
-        k_rs_upsweep<K><<<(unsigned)tiles, RS_THREADS, 0, s>>>(kin, n, b, mask, hist.get(), tiles);
-        CK_LAUNCH("k_rs_upsweep");
-        scan_exclusive<uint32_t, const uint32_t *>(hist.get(), hist.get(), 256 * tiles, s);
-        if (vals)
-            k_rs_downsweep<K, true><<<(unsigned)tiles, RS_THREADS, 0, s>>>(kin, vin, kout, vout, n, b, mask,
-                                                                           hist.get(), tiles);
-        else
-            k_rs_downsweep<K, false><<<(unsigned)tiles, RS_THREADS, 0, s>>>(kin, nullptr, kout, nullptr, n, b,
-                                                                            mask, hist.get(), tiles);
-        CK_LAUNCH("k_rs_downsweep");
-        K *tk = kin; kin = kout; kout = tk;
-        uint32_t *tv = vin; vin = vout; vout = tv;
-        passes++;
-    }
-    if (passes & 1) {
-        CK(cudaMemcpyAsync(keys, kin, n * sizeof(K), cudaMemcpyDeviceToDevice, s));
-        if (vals) CK(cudaMemcpyAsync(vals, vin, n * sizeof(uint32_t), cudaMemcpyDeviceToDevice, s));
-    }
+    if (vals) radix_sort_impl<K, true>(keys, vals, n, begin_bit, end_bit, s);
+    else radix_sort_impl<K, false>(keys, nullptr, n, begin_bit, end_bit, s);
 }
 
 }  // namespace scd
