@@ -16,7 +16,7 @@ ROOT = os.path.dirname(HERE)
 OUT = os.path.join(HERE, "_build")
 
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
-CU_SOURCES = ["engine.cu", "preprocess.cu", "csr.cu", "text.cu", "triangles.cu", "partition.cu", "refine.cu",
+CU_SOURCES = ["engine.cu", "preprocess.cu", "csr.cu", "text.cu", "triangles.cu", "tc_dense.cu", "partition.cu", "refine.cu",
               "improve.cu", "resident.cu", "wcc_static.cu"]
 
 

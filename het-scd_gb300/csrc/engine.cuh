@@ -126,6 +126,14 @@ struct LabelFilter {
     const uint8_t *active = nullptr;
     __device__ __forceinline__ bool frozen(uint32_t v) const { return active && !active[gid[v]]; }
 };
+// The dense core of a skewed graph (tc_dense.cu): the vertices of degree > bound.  The
+// triangles inside it, and those of two members and an outside vertex of a CTA bucket
+// below them, are counted by row bitmaps.
+struct DenseCore {
+    uint32_t n = 0, bound = 0;
+    DevBuf<uint32_t> verts, num;   // members ascending; number of each member (INVALID for the others)
+    DevBuf<uint32_t> walk;         // out-degree of every vertex, 0 for members
+};
 // out-degree buckets and their work-unit offsets (built once per oriented graph)
 // Bucket k lists its out-list centres first (nfwd[k] of them) and, for the CTA
 // buckets, then the in-list centres: a vertex b whose edges a -> b with
@@ -153,6 +161,8 @@ struct TcPlan {
     uint32_t core_n = 0, core_lcap = 0;
     uint32_t cta_lo = 0, cta_hi = 0;   // out-degree range (cta_lo, cta_hi] of the first CTA bucket
     DevBuf<uint32_t> core_buf, core_beg_buf;
+    DenseCore dense;   // counted by bitmaps instead of walks (n == 0: none)
+    const uint32_t *walk(const Oriented &o) const { return dense.n ? dense.walk.get() : o.len; }
 };
 struct Ctx;
 // in_lists: also in-list centres (b-centric edges) in the CTA buckets
@@ -173,6 +183,17 @@ void tc_plan_lists(Ctx &c, const Oriented &o, TcPlan &plan, uint32_t *lists, uin
                    bool in_lists, uint32_t core_from);
 void tc_plan_units(Ctx &c, const Oriented &o, TcPlan &plan, uint32_t *lists, const uint32_t *host_bounds,
                    cudaStream_t s, bool owned);
+// out-degree up to which the walks take a vertex by register groups or a warp
+uint32_t tc_short_lists(const Ctx &c);
+// tc_dense.cu.  pick (2 device words): members and degree bound of the dense core worth
+// having for the sorted symmetric rows off/vals (INVALID holes), out-degrees olen and
+// degrees deg; 0 members if none is
+void tc_dense_pick(Ctx &c, const uint32_t *off, const uint32_t *vals, uint64_t entries, const uint32_t *olen,
+                   const uint32_t *deg, uint32_t n, uint32_t *pick, cudaStream_t s);
+void tc_dense_setup(Ctx &c, const Oriented &o, const uint32_t *deg, uint32_t members, uint32_t bound, DenseCore &d,
+                    cudaStream_t s);
+void tc_dense_count(Ctx &c, const Oriented &o, const TcPlan &plan, uint32_t *tcount, uint8_t *flag, uint32_t *ctr,
+                    cudaStream_t s);
 // the plan of a full count (preprocessing) over out-lists o.adj[0..slots) with in-list
 // centres: the core split and its core map, or the hash kernels' split
 void tc_plan_counting(Ctx &c, const Oriented &o, uint64_t slots, TcPlan &plan, cudaStream_t s);

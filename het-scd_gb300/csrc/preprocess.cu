@@ -519,7 +519,17 @@ void convert_edges(Ctx &c, const uint32_t *pairs_in, uint64_t count, const std::
     CK_LAUNCH("k_long_out_count");
     scan_exclusive<uint32_t>((const uint32_t *)olen.get(), obeg.get(), n1, s);
     scan_exclusive<uint32_t>(InCount{cnt.get(), olen.get()}, ibeg.get(), n1, s);
-    const uint32_t m1 = read_scalar(obeg.get() + n1, s);
+    // the out-slots and, for the triangle count, the dense core worth having: one read
+    // (none under the flags that ask for the walks; smaller graphs have no use for one)
+    const bool dense = n1 >= 4096 && !(c.flags & (SCD_FLAG_TC_HASH | SCD_FLAG_TC_OUT_ONLY));
+    DevBuf<uint32_t> pick(2, s);
+    if (dense) tc_dense_pick(c, off1.get(), vals.get(), entries, olen.get(), cnt.get(), n1, pick.get(), s);
+    uint32_t *hm = c.host_u32 + HOST_PLAN;
+    hm[1] = hm[2] = 0;
+    CK(cudaMemcpyAsync(hm, obeg.get() + n1, 4, cudaMemcpyDeviceToHost, s));
+    if (dense) CK(cudaMemcpyAsync(hm + 1, pick.get(), 8, cudaMemcpyDeviceToHost, s));
+    CK(cudaStreamSynchronize(s));
+    const uint32_t m1 = hm[0], core_members = hm[1], core_bound = hm[2];
     DevBuf<uint32_t> orow(m1 ? m1 : 1, s), ocol(m1 ? m1 : 1, s), icol(m1 ? m1 : 1, s);
     k_row_orient<<<grid_for((uint64_t)n1 * 32, TPB), TPB, 0, s>>>(off1.get(), n1, vals.get(), cnt.get(), obeg.get(),
                                                                   ibeg.get(), orow.get(), ocol.get(), icol.get());
@@ -535,7 +545,6 @@ void convert_edges(Ctx &c, const uint32_t *pairs_in, uint64_t count, const std::
     DevBuf<uint32_t> ilen(n1, s);
     k_in_len<<<grid_for(n1, TPB), TPB, 0, s>>>(cnt.get(), olen.get(), n1, ilen.get());
     CK_LAUNCH("k_in_len");
-    cnt.release();
     DevBuf<uint32_t> tcount(n1, s);
     DevBuf<uint8_t> oflag(m1, s);
     CK(cudaMemsetAsync(tcount.get(), 0, (size_t)n1 * 4, s));
@@ -543,6 +552,8 @@ void convert_edges(Ctx &c, const uint32_t *pairs_in, uint64_t count, const std::
     Oriented o{obeg.get(), olen.get(), ocol.get(), n1, ibeg.get(), ilen.get(), icol.get()};
     {
         TcPlan plan;
+        tc_dense_setup(c, o, cnt.get(), core_members, core_bound, plan.dense, s);
+        cnt.release();
         tc_plan_counting(c, o, m1, plan, s);
         count_triangles(c, o, plan, LabelFilter{}, tcount.get(), oflag.get(), s);
     }

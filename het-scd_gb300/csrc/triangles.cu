@@ -84,16 +84,18 @@ struct BucketMask {
     Oriented o;
     uint32_t upper[TcPlan::K];   // ascending
     bool in_lists;
+    const uint32_t *walk;        // 0 for the members of the dense core, which are no out-list centres (nullptr: no core)
     __device__ uint32_t operator[](size_t v) const {
         const uint32_t len = o.len[v];
         if (len == 0) return 0u;
         int k = 0;
 #pragma unroll
         for (int j = 0; j < TcPlan::K - 1; j++) k += len > upper[j];
-        if (k < 4) return 1u << k;
-        if (k == 6) return 1u << 8;
-        const uint32_t both = in_lists && o.in_len((uint32_t)v) > 0;
-        return (1u | (both << 1)) << (k == 4 ? 4 : 6);
+        const uint32_t out = !walk || walk[v] > 0;
+        if (k < 4) return out << k;
+        if (k == 6) return out << 8;
+        const uint32_t in = in_lists && o.in_len((uint32_t)v) > 0;
+        return (out | (in << 1)) << (k == 4 ? 4 : 6);
     }
 };
 
@@ -350,13 +352,18 @@ k_tc_warp(Oriented o, const uint32_t *__restrict__ verts, const uint32_t *__rest
 // and flags are aggregated in shared memory.  The out-slot of a -> x (in-list
 // centre) is found by a binary search of x in out(a), for partners with hits.
 //
+// With a dense core (tc_dense.cu) the edges a -> b with b a member and d+(a) above
+// the warp kernel's are counted by bitmaps: a partner's walk length is walk[y], 0 for
+// members, and a member's in-list centre takes only the short out-lists.
+//
 // The table entries' hit counts are 16-bit halves of shared words (a count is at
 // most the unit's THREADS x ROUNDS partners), which with the register bound lets
 // MIN_CTAS CTAs share an SM.
 template <int THREADS, int ROUNDS, int TCAP, int LCAP, int FBITS, int MIN_CTAS>
 __global__ void __launch_bounds__(THREADS, MIN_CTAS)
 k_tc_cta(Oriented o, const uint32_t *__restrict__ verts, const uint32_t *__restrict__ unit_off, uint32_t nverts,
-         uint32_t nfwd, Dir dir, LabelFilter lf, uint32_t *tcount, uint8_t *flag, uint32_t *next_unit) {
+         uint32_t nfwd, const uint32_t *__restrict__ walk, Dir dir, LabelFilter lf, uint32_t *tcount, uint8_t *flag,
+         uint32_t *next_unit) {
     constexpr uint32_t PER_UNIT = (uint32_t)THREADS * ROUNDS;
     static_assert(PER_UNIT < 65536, "16-bit hit counts");
     const uint32_t *labels = lf.labels;
@@ -382,7 +389,7 @@ k_tc_cta(Oriented o, const uint32_t *__restrict__ verts, const uint32_t *__restr
         }
         const uint32_t vi = lo - 1;
         const uint32_t x = verts[vi], ch = unit - unit_off[vi];
-        const bool fwd = vi < nfwd;
+        const bool fwd = vi < nfwd, in_core = !fwd && walk[x] == 0;
         const uint32_t la = labels ? labels[x] : 0u;
         if (labels && (la == INVALID || lf.frozen(x))) {
             __syncthreads();
@@ -414,7 +421,8 @@ k_tc_cta(Oriented o, const uint32_t *__restrict__ verts, const uint32_t *__restr
             uint32_t wb = 0, bb = 0, y = 0;
             if (j < pend) {
                 y = padj[pbeg + j];
-                const uint32_t dy = o.len[y];
+                uint32_t dy = walk[y];
+                if (in_core && dy > dir.lo) dy = 0;
                 const bool here = fwd ? !dir.bcentric(xlen, dy) : dir.bcentric(dy, xlen);
                 if (here && (!labels || labels[y] == la)) {
                     wb = dy;
@@ -524,8 +532,8 @@ void launch_tc_cta(const Oriented &o, const TcPlan &plan, int k, LabelFilter lab
                    uint8_t *flag, uint32_t *ctr, unsigned grid, cudaStream_t s) {
     const size_t smem = tc_cta_smem<TCAP, LCAP, FBITS>();
     k_tc_cta<THREADS, ROUNDS, TCAP, LCAP, FBITS, MIN_CTAS><<<grid, THREADS, smem, s>>>(
-        o, plan.verts[k], plan.unit_off[k], plan.nverts[k], plan.nfwd[k], Dir{plan.dir_lo, plan.dir_hi, plan.dir_amin},
-        labels, tcount, flag, ctr);
+        o, plan.verts[k], plan.unit_off[k], plan.nverts[k], plan.nfwd[k], plan.walk(o),
+        Dir{plan.dir_lo, plan.dir_hi, plan.dir_amin}, labels, tcount, flag, ctr);
     CK_LAUNCH("k_tc_cta");
 }
 
@@ -554,8 +562,8 @@ template <int THREADS, int K>
 __global__ void __launch_bounds__(THREADS, 6)
 k_tc_core(Oriented o, const uint32_t *__restrict__ cpad, const uint32_t *__restrict__ cbeg, uint32_t core_n,
           uint32_t kwords, uint32_t lcap, const uint32_t *__restrict__ verts, const uint32_t *__restrict__ unit_off,
-          uint32_t nverts, uint32_t nfwd, uint32_t per_unit, Dir dir, uint32_t *tcount, uint8_t *flag,
-          uint32_t *next_unit) {
+          uint32_t nverts, uint32_t nfwd, const uint32_t *__restrict__ walk, uint32_t per_unit, Dir dir, uint32_t *tcount,
+          uint8_t *flag, uint32_t *next_unit) {
     extern __shared__ __align__(16) uint32_t sm[];
     uint32_t *bm = sm;                           // kwords
     uint32_t *cnt = bm + kwords;                 // lcap hit counts of the centre's members
@@ -582,7 +590,7 @@ k_tc_core(Oriented o, const uint32_t *__restrict__ cpad, const uint32_t *__restr
         }
         const uint32_t vi = lo - 1;
         const uint32_t x = verts[vi], ch = unit - unit_off[vi];
-        const bool fwd = vi < nfwd;
+        const bool fwd = vi < nfwd, in_core = !fwd && walk[x] == 0;
         const uint32_t xbeg = o.beg[x], xlen = o.len[x];
         const uint32_t *xc = cpad + cbeg[x];
         for (uint32_t i = threadIdx.x; i < xlen; i += THREADS) {
@@ -602,7 +610,8 @@ k_tc_core(Oriented o, const uint32_t *__restrict__ cpad, const uint32_t *__restr
             uint32_t y = 0, wb = 0, cb = 0, ob = 0;
             if (j < pend) {
                 y = padj[pbeg + j];
-                const uint32_t dy = o.len[y];
+                uint32_t dy = walk[y];
+                if (in_core && dy > dir.lo) dy = 0;
                 if (fwd ? !dir.bcentric(xlen, dy) : dir.bcentric(dy, xlen)) {
                     wb = dy;
                     cb = cbeg[y];
@@ -728,7 +737,8 @@ void launch_tc_core(const Oriented &o, const TcPlan &plan, int k, uint32_t lcap,
     CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     k_tc_core<CORE_THREADS, CORE_K><<<sms * per_sm, CORE_THREADS, smem, s>>>(
         o, plan.core_adj, plan.core_beg, plan.core_n, kwords, lcap, plan.verts[k], plan.unit_off[k], plan.nverts[k],
-        plan.nfwd[k], CTA2_THREADS * CTA2_ROUNDS, Dir{plan.dir_lo, plan.dir_hi, plan.dir_amin}, tcount, flag, ctr);
+        plan.nfwd[k], plan.walk(o), CTA2_THREADS * CTA2_ROUNDS, Dir{plan.dir_lo, plan.dir_hi, plan.dir_amin}, tcount,
+        flag, ctr);
     CK_LAUNCH("k_tc_core");
 }
 
@@ -839,9 +849,11 @@ __global__ void k_core_pad(Oriented o, const uint32_t *__restrict__ cpos, uint32
 
 }  // namespace
 
+uint32_t tc_short_lists(const Ctx &c) { return c.tc_b0 > c.tc_small ? c.tc_b0 : c.tc_small; }
+
 void tc_plan_lists(Ctx &c, const Oriented &o, TcPlan &plan, uint32_t *lists, uint32_t *bounds, cudaStream_t s,
                    bool in_lists, uint32_t core_from) {
-    const uint32_t sm = c.tc_small, s16 = sm < 16 ? sm : 16, s8 = sm < 8 ? sm : 8, b0 = c.tc_b0 > sm ? c.tc_b0 : sm;
+    const uint32_t sm = c.tc_small, s16 = sm < 16 ? sm : 16, s8 = sm < 8 ? sm : 8, b0 = tc_short_lists(c);
     // the core-bitmap kernel takes the upper CTA bucket from core_from on; the hash
     // kernels' upper bucket (one CTA per SM, 16K-entry tables) from tc_b1 on
     const uint32_t b1 = core_from ? (core_from > b0 ? core_from : b0) : c.tc_b1;
@@ -851,7 +863,9 @@ void tc_plan_lists(Ctx &c, const Oriented &o, TcPlan &plan, uint32_t *lists, uin
     plan.dir_amin = c.tc_amin < sm ? c.tc_amin : sm;
     plan.cta_lo = b0;
     plan.cta_hi = b1;
-    build_lists<TC_LISTS>(BucketMask{o, {s8, s16, sm, b0, b1, B2, 0xffffffffu}, split}, o.n, lists, bounds, s);
+    build_lists<TC_LISTS>(BucketMask{o, {s8, s16, sm, b0, b1, B2, 0xffffffffu}, split,
+                                     plan.dense.n ? plan.dense.walk.get() : nullptr},
+                          o.n, lists, bounds, s);
 }
 
 void tc_plan_units(Ctx &c, const Oriented &o, TcPlan &plan, uint32_t *lists, const uint32_t *hb, cudaStream_t s,
@@ -923,13 +937,12 @@ void tc_plan_counting(Ctx &c, const Oriented &o, uint64_t slots, TcPlan &plan, c
     }
     // the core kernel starts at the lowest candidate bound whose core fits the
     // bitmap budget (many CTAs per SM), else at the lowest one that fits at all
-    const uint32_t b0 = c.tc_b0 > c.tc_small ? c.tc_b0 : c.tc_small;
+    const uint32_t b0 = tc_short_lists(c);
     constexpr int K = CoreBounds::K;
     if (o.n <= CORE_BUDGET) {   // every core fits the budget: the lowest split, no host read
         tc_plan(c, o, plan, s, false, true, b0);
         tc_core_map(c, o, slots, plan, o.n, B2, s);   // core_n <= n; counts sized for the cap
         if (plan.core_n || !plan.nverts[5]) return;
-        plan = TcPlan();
         tc_plan(c, o, plan, s, false, true);
         return;
     }
@@ -954,7 +967,6 @@ void tc_plan_counting(Ctx &c, const Oriented &o, uint64_t slots, TcPlan &plan, c
         tc_plan(c, o, plan, s, false, true, cb.t[pick]);
         tc_core_map(c, o, slots, plan, core_n, lcap, s);
         if (plan.core_n || !plan.nverts[5]) return;
-        plan = TcPlan();
     }
     tc_plan(c, o, plan, s, false, true);   // no map: the hash kernels' split
 }
@@ -1050,7 +1062,7 @@ void count_triangles(Ctx &c, const Oriented &o, const TcPlan &plan, LabelFilter 
     PhaseScope ph(c, phase ? phase : labels.labels ? "wcc_tc" : "tc");
     prepare_tc_kernels();
     uint32_t *ctr = c.work_counter;
-    CK(cudaMemsetAsync(ctr, 0, 16, s));
+    CK(cudaMemsetAsync(ctr, 0, 24, s));
     const Dir dir{plan.dir_lo, plan.dir_hi, plan.dir_amin};
     const bool core = plan.nverts[5] && plan.core_n && !labels.labels;
     if (plan.nverts[0]) {
@@ -1089,6 +1101,7 @@ void count_triangles(Ctx &c, const Oriented &o, const TcPlan &plan, LabelFilter 
         launch_tc_cta<CTA2_THREADS, CTA2_ROUNDS, 16384, 8192, 17, 1>(o, plan, 5, labels, tcount, flag, ctr + 2, 152, s);
         c.launches++;
     }
+    if (plan.dense.n) tc_dense_count(c, o, plan, tcount, flag, ctr + 4, s);
     if (plan.nverts[6]) {
         k_tc_huge<<<152 * 4, 256, 0, s>>>(o, plan.verts[6], plan.nverts[6], labels, tcount, flag);
         CK_LAUNCH("k_tc_huge");
