@@ -24,6 +24,41 @@ __global__ void k_nlow(uint32_t n, const uint32_t *__restrict__ indices, const u
     }
 }
 
+// Is every entry (u, v) of the rows matched by its (v, u)?  Order-independent sums of two
+// 64-bit hashes of (smaller, larger) id, added from the smaller end's row and taken off from
+// the larger's: both are 0 for a symmetric graph, and for another only with the chance of
+// two hash sums meeting. sums[2] counts loops and descents of a row.
+__device__ __forceinline__ unsigned long long mix64(unsigned long long z) {   // splitmix64's finaliser
+    z = (z ^ (z >> 30)) * 0xbf58476d1ce4e5b9ull;
+    z = (z ^ (z >> 27)) * 0x94d049bb133111ebull;
+    return z ^ (z >> 31);
+}
+
+__global__ void k_symmetry(uint32_t n, const uint32_t *__restrict__ indices, const uint32_t *__restrict__ adj,
+                           unsigned long long *sums) {
+    const uint32_t lane = threadIdx.x & 31, warps = (gridDim.x * blockDim.x) >> 5;
+    unsigned long long a = 0, b = 0, bad = 0;
+    for (uint32_t v = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; v < n; v += warps) {
+        const uint32_t beg = indices[v], end = indices[v + 1];
+        for (uint32_t i = beg + lane; i < end; i += 32) {
+            const uint32_t w = adj[i];
+            bad += w == v || (i > beg && adj[i - 1] > w);
+            const unsigned long long key = v < w ? ((unsigned long long)v << 32) | w : ((unsigned long long)w << 32) | v;
+            const unsigned long long h = mix64(key + 0x9e3779b97f4a7c15ull), k = mix64(h ^ 0xd1b54a32d192ed03ull);
+            a += v < w ? h : 0ull - h;
+            b += v < w ? k : 0ull - k;
+        }
+    }
+    a = warp_sum(a);
+    b = warp_sum(b);
+    bad = warp_sum(bad);
+    if (lane == 0) {
+        if (a) atomicAdd(sums, a);
+        if (b) atomicAdd(sums + 1, b);
+        if (bad) atomicAdd(sums + 2, bad);
+    }
+}
+
 struct ChunksOf {   // RowWork chunks of a long row
     const uint32_t *verts, *indices;
     __device__ uint32_t operator[](size_t i) const {
@@ -251,7 +286,7 @@ void Ctx::free_all() {
 // the iteration's scratch arrays and the triangle-counting plan.  Needs
 // g.indices/adj, b.G, b.h_fin_off and b.fin_off; always_gid: a graph-id array even
 // for one graph (resident sets run every kernel in the skip-converged-graphs mode).
-void build_union_structure(Ctx &c, bool always_gid) {
+void build_union_structure(Ctx &c, bool always_gid, bool check_symmetry) {
     Graph &g = c.g;
     Batch &b = c.b;
     cudaStream_t s = c.stream;
@@ -293,14 +328,24 @@ void build_union_structure(Ctx &c, bool always_gid) {
     const uint64_t long_most = std::min<uint64_t>(n, 2 * (uint64_t)g.m / (RowWork::CHUNK + 1));
     uint32_t *lists = c.alloc<uint32_t>(n + long_most), *tc_lists = c.alloc<uint32_t>(n);
     uint32_t *hb = c.host_u32 + HOST_PLAN, *htc = hb + K + 2;
-    static_assert(HOST_PLAN + K + 2 + TC_LISTS + 1 <= HOST_WORDS, "planning words");
+    static_assert(HOST_PLAN + K + 2 + TC_LISTS + 1 <= HOST_SUMS, "planning words");
     c.wplan = TcPlan();
     {
         DevBuf<uint32_t> bounds(K + 2 + TC_LISTS + 1, s);
         build_lists<K + 1>(DegreeMask{g.indices}, n, lists, bounds.get(), s);
         tc_plan_lists(c, o, c.wplan, tc_lists, bounds.get() + K + 2, s, false, 0);
+        DevBuf<unsigned long long> sums(3, s);
+        unsigned long long *hs = (unsigned long long *)(c.host_u32 + HOST_SUMS);
+        hs[0] = hs[1] = hs[2] = 0;
+        if (check_symmetry && n) {
+            CK(cudaMemsetAsync(sums.get(), 0, 24, s));
+            k_symmetry<<<grid_for((uint64_t)n * 32, TPB, NUM_SMS_HINT * 16), TPB, 0, s>>>(n, g.indices, g.adj, sums.get());
+            CK_LAUNCH("k_symmetry");
+            CK(cudaMemcpyAsync(hs, sums.get(), 24, cudaMemcpyDeviceToHost, s));
+        }
         CK(cudaMemcpyAsync(hb, bounds.get(), 4 * (K + 2 + TC_LISTS + 1), cudaMemcpyDeviceToHost, s));
         CK(cudaStreamSynchronize(s));
+        g.symmetric = !(hs[0] | hs[1] | hs[2]);
     }
     for (int k = 0; k < K; k++) {
         g.cls.list[k] = lists + hb[k];
@@ -342,7 +387,7 @@ void build_union_structure(Ctx &c, bool always_gid) {
     c.launches += 3;
 }
 
-void finish_graph(Ctx &c) {
+void finish_graph(Ctx &c, bool transferred) {
     Graph &g = c.g;
     cudaStream_t s = c.stream;
     const uint32_t n = g.n;
@@ -380,7 +425,7 @@ void finish_graph(Ctx &c) {
         c.st[k].ext = c.alloc<int32_t>(n);
         c.st[k].intl = c.alloc<int32_t>(n);
     }
-    build_union_structure(c, false);
+    build_union_structure(c, false, transferred);
     compute_p_ext(c);
     c.launches++;
 }
@@ -392,13 +437,12 @@ void iterate_async(Ctx &c, double threshold, double *trace, int max_trace) {
     // converged graphs of a batch or a resident set keep their labels; their statistics
     // and WCC are not needed any more
     const bool frozen = c.b.G > 1 || c.resident;
-    improve(c, c.labels, c.st[c.cur], c.labels_next, frozen);
+    improve(c, c.labels, c.st[c.cur], c.labels_next, frozen, &c.st[c.cur ^ 1]);
     uint32_t *t = c.labels;
     c.labels = c.labels_next;
     c.labels_next = t;
     c.cur ^= 1;
-    collect_stats(c, c.labels, c.st[c.cur], frozen);
-    launch_wcc(c, c.labels, c.st[c.cur], frozen);
+    launch_stats_wcc(c, c.labels, c.st[c.cur], frozen);
     batch_step(c, threshold, trace, max_trace);
 }
 
@@ -478,13 +522,13 @@ void set_labels(Ctx &c, const uint32_t *host_labels) {
 double iterate(Ctx &c) {
     // improve (old labels -> labels_next), statistics and WCC of the new labels
     join_p_ext(c);
-    improve(c, c.labels, c.st[c.cur], c.labels_next);
+    improve(c, c.labels, c.st[c.cur], c.labels_next, false, &c.st[c.cur ^ 1]);
     uint32_t *t = c.labels;
     c.labels = c.labels_next;
     c.labels_next = t;
     c.cur ^= 1;
-    collect_stats(c, c.labels, c.st[c.cur]);
-    return compute_wcc(c, c.labels, c.st[c.cur]);
+    launch_stats_wcc(c, c.labels, c.st[c.cur], false);
+    return read_wcc(c);
 }
 
 double now_ms() {
@@ -728,7 +772,7 @@ void finish_loaded_graph(Ctx &c, double alpha) {
         throw Error(SCD_ERR_FORMAT, "indices do not match m");
     }
     c.alpha = alpha;
-    finish_graph(c);
+    finish_graph(c, true);
     c.has_graph = true;
     CK(cudaStreamSynchronize(c.stream));
 }

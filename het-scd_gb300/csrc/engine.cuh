@@ -44,7 +44,9 @@ struct Graph {
     uint32_t *indices = nullptr, *adj = nullptr, *nlow = nullptr;
     int32_t *tri = nullptr, *tri_deg = nullptr;
     double p_ext = 0.0;   // of graph 0 (the only graph of a plain context)
-    uint32_t max_deg = 0;
+    // every entry (u, v) has its (v, u), rows ascend, no loops: always so after convert, checked
+    // for a transferred graph
+    bool symmetric = true;
     // degree buckets of the improve kernels, built once per graph
     DegreeClasses cls;
     RowWork rows;
@@ -144,6 +146,7 @@ struct TcPlan {
     uint32_t *unit_off[K] = {};
     uint32_t nverts[K] = {};
     uint32_t nfwd[K] = {};
+    uint32_t small_max = 0;   // longest out-list of the register groups (buckets 0 to 2)
     uint32_t dir_lo = 0, dir_hi = 0, dir_amin = 0;   // b-centric iff d+(a) < d+(b),
                                                       // dir_lo < d+(b) <= dir_hi, d+(a) > dir_amin
     DevBuf<uint32_t> tmp[4];   // storage when the plan is temporary: the lists, the unit offsets
@@ -212,7 +215,7 @@ double autotune_tc(Ctx &c, std::vector<std::string> *report);
 void prepare_tc_kernels();
 void prepare_improve_kernels();
 
-constexpr int HOST_PLAN = 2, HOST_WORDS = 64;   // pinned words of a context (Ctx::host_u32)
+constexpr int HOST_PLAN = 2, HOST_SUMS = 56, HOST_WORDS = 64;   // pinned words of a context (Ctx::host_u32)
 
 struct Ctx;
 // records [start, end) of a phase on the context's stream when profiling
@@ -305,10 +308,11 @@ uint64_t parse_edge_text(Ctx &c, const char *text, uint64_t bytes, DevBuf<uint32
 void alloc_graph(Ctx &c, uint32_t n, uint32_t m);
 void upload_graph(Ctx &c, uint32_t n, uint32_t m, const uint32_t *indices, const uint32_t *adj,
                   const int32_t *tri, const int32_t *tri_deg);
-void finish_graph(Ctx &c);   // nlow, p_ext, degree classes, partition buffers
+// nlow, p_ext, degree classes, partition buffers; transferred: the rows are a caller's
+void finish_graph(Ctx &c, bool transferred);
 // the derived structure of the union graph (see engine.cu); always_gid: a graph-id
 // array even for one graph
-void build_union_structure(Ctx &c, bool always_gid);
+void build_union_structure(Ctx &c, bool always_gid, bool check_symmetry);
 // engine.cu: one refinement iteration of every running graph without host
 // synchronisation (capturable); kernel nodes of a captured CUDA graph
 void iterate_async(Ctx &c, double threshold, double *trace, int max_trace);
@@ -324,9 +328,14 @@ void initial_partition(Ctx &c);
 void collect_stats(Ctx &c, const uint32_t *labels, Stats &st, bool frozen_graphs = false);
 double compute_wcc(Ctx &c, const uint32_t *labels, const Stats &st);
 // frozen_graphs: vertices of graphs whose loop has ended keep their labels
-void improve(Ctx &c, const uint32_t *labels, const Stats &st, uint32_t *next, bool frozen_graphs = false);
+// clear (nullable): statistics to clear for the labels this call makes
+void improve(Ctx &c, const uint32_t *labels, const Stats &st, uint32_t *next, bool frozen_graphs, Stats *clear);
+// statistics (st cleared by improve) and WCC of an iteration's labels
+void launch_stats_wcc(Ctx &c, const uint32_t *labels, Stats &st, bool frozen_graphs);
+double read_wcc(Ctx &c);   // waits for the WCC of graph 0
 // per-graph WCC in c.b.wcc (device); frozen_graphs: skip the graphs of a batch that stopped iterating
-void launch_wcc(Ctx &c, const uint32_t *labels, const Stats &st, bool frozen_graphs = false);
+// with_stats: also adds the labels' statistics to st
+void launch_wcc(Ctx &c, const uint32_t *labels, const Stats &st, bool frozen_graphs = false, bool with_stats = false);
 void compute_p_ext(Ctx &c);   // launches on the side stream
 void join_p_ext(Ctx &c);      // main stream waits for p_ext (outside captures)
 void host_p_ext(Ctx &c);      // host copies of p_ext (b.h_p_ext, g.p_ext)

@@ -125,12 +125,14 @@ __device__ __forceinline__ uint32_t decide(double best_gain, uint32_t best_label
     return mine;
 }
 
-__global__ void k_comm_prep(uint32_t nc, Stats st, double *pin64, int4 *civ) {
+// clear: the statistics of the labels this iteration makes start from 0 (nullptrs: none)
+__global__ void k_comm_prep(uint32_t nc, Stats st, double *pin64, int4 *civ, Stats clear) {
     for (uint32_t l = blockIdx.x * blockDim.x + threadIdx.x; l < nc; l += gridDim.x * blockDim.x) {
         const double p = community_p_in(st.sizes[l], st.intl[l] / 2);
         pin64[l] = p;
         civ[l] = make_int4(st.sizes[l], st.ext[l], __float_as_int(__double2float_rd(p)),
                            __float_as_int(__double2float_ru(p)));
+        if (clear.sizes) clear.sizes[l] = clear.ext[l] = clear.intl[l] = 0;
     }
 }
 
@@ -800,14 +802,14 @@ void launch_cta(const uint32_t *verts, uint32_t count, const ImproveArgs &a, cud
 
 }  // namespace
 
-void improve(Ctx &c, const uint32_t *labels, const Stats &st, uint32_t *next, bool frozen_graphs) {
+void improve(Ctx &c, const uint32_t *labels, const Stats &st, uint32_t *next, bool frozen_graphs, Stats *clear) {
     const Graph &g = c.g;
     cudaStream_t s = c.stream;
     if (g.n == 0) return;
     PhaseScope ph(c, "improve");
     prepare_improve_kernels();
     if (c.num_comms) {
-        k_comm_prep<<<grid_for(c.num_comms, TPB), TPB, 0, s>>>(c.num_comms, st, c.pin64, c.civ);
+        k_comm_prep<<<grid_for(c.num_comms, TPB), TPB, 0, s>>>(c.num_comms, st, c.pin64, c.civ, clear ? *clear : Stats());
         CK_LAUNCH("k_comm_prep");
         c.launches++;
     }

@@ -15,6 +15,7 @@
 #include <algorithm>
 
 #include "engine.cuh"
+#include "rows.cuh"
 
 namespace scd {
 
@@ -68,28 +69,13 @@ constexpr uint32_t HUB_DEG = 4096, HUB_TPB = 1024;
 
 // The vertices of degree 33 .. HUB_DEG (four degree classes, the longest rows first) have a
 // warp each; several of their rows in one warp, consecutive in id order, would be a long
-// serial tail.
-struct WarpRows {
-    static constexpr int K = 4;
-    const uint32_t *list[K];
-    uint32_t count[K], total;
-    __device__ uint32_t operator[](uint32_t i) const {
-#pragma unroll
-        for (int k = 0; k < K - 1; k++) {
-            if (i < count[k]) return list[k][i];
-            i -= count[k];
-        }
-        return list[K - 1][i];
-    }
-};
-
-// Rows of up to 32 neighbours are taken `rows` at a time by a warp (k_mis_round,
-// k_claim_labels): its lanes read the state, position and bounds of consecutive vertices in
-// one coalesced step, and the next row's neighbours are fetched while a row is looked at,
-// so a row costs two dependent gathers instead of five loads in a chain (these kernels are
-// bound by that latency, not by their bytes: the first round of 96 planted graphs, 2.6 M
-// vertices, took 1.58 ms with a warp and the whole chain per row, 0.67 ms so). Few rows for
-// small graphs, so that every SM has warps.
+// serial tail. Rows of up to 32 neighbours are taken `rows` at a time by a warp
+// (k_mis_round, k_claim_labels): its lanes read the state, position and bounds of
+// consecutive vertices in one coalesced step, and the next row's neighbours are fetched
+// while a row is looked at, so a row costs two dependent gathers instead of five loads in a
+// chain (these kernels are bound by that latency, not by their bytes: the first round of 96
+// planted graphs, 2.6 M vertices, took 1.58 ms with a warp and the whole chain per row, 0.67
+// ms so). Few rows for small graphs, so that every SM has warps.
 inline uint32_t rows_per_warp(uint32_t n) {
     uint32_t r = 1;
     while (r < 32 && (uint64_t)r * 2 * NUM_SMS_HINT * 32 <= n) r <<= 1;
@@ -364,11 +350,8 @@ void initial_partition(Ctx &c) {
     const uint32_t nhubs = g.cls.count[DegreeClasses::K - 1];
     const uint32_t rows = rows_per_warp(n);
     WarpRows wr{};
-    for (int k = 0; k < WarpRows::K; k++) {
-        wr.list[k] = g.cls.list[DegreeClasses::K - 2 - k];
-        wr.count[k] = g.cls.count[DegreeClasses::K - 2 - k];
-        wr.total += wr.count[k];
-    }
+    for (int k = 0; k < WarpRows::K; k++)
+        wr.set(k, g.cls.list[DegreeClasses::K - 2 - k], g.cls.count[DegreeClasses::K - 2 - k]);
     static_assert(DegreeClasses::upper[DegreeClasses::K - 2 - WarpRows::K] == 32, "rows of more than 32");
     const unsigned G = grid_for((((uint64_t)n + rows - 1) / rows + wr.total) * 32, TPB, 152 * 16);
     static_assert(DegreeClasses::upper[DegreeClasses::K - 2] == HUB_DEG, "hub class");

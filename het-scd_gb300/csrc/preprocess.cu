@@ -623,7 +623,7 @@ void convert_edges(Ctx &c, const uint32_t *pairs_in, uint64_t count, const std::
         sort_rows(c, g.indices, n2, g.adj, false, nullptr, s);
         c.launches++;
     }
-    finish_graph(c);
+    finish_graph(c, false);
     c.has_graph = true;   // only once every array exists: a failure above leaves no graph
 }
 
@@ -657,7 +657,7 @@ void upload_graph(Ctx &c, uint32_t n, uint32_t m, const uint32_t *indices, const
     } else {
         CK(cudaMemsetAsync(g.indices, 0, ((size_t)n + 1) * 4, s));
     }
-    finish_graph(c);
+    finish_graph(c, true);
     c.has_graph = true;
 }
 

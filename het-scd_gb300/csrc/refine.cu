@@ -174,7 +174,11 @@ __device__ __forceinline__ double wcc_term(uint32_t p, const uint32_t *labels, c
     if (size <= 2 || td == 0) return 0.0;
     const int it = (int)(2u * itcount[p]), itd = itdeg[p];   // int_tri = 2 x internal triangles
     const double nom = (double)imul_wrap(it, td);
-    const double den = dmul((double)tri[p], dadd((double)td, dmul(alpha, (double)(size - 1 - itd))));
+    // (the FP64 pipe bounds this kernel on large graphs: with alpha 1, the default, the sum of
+    // two integers below 2^31 is made in integers, where it is the same exact value)
+    const int out = size - 1 - itd;
+    const double sum = alpha == 1.0 ? (double)((long long)td + out) : dadd((double)td, dmul(alpha, (double)out));
+    const double den = dmul((double)tri[p], sum);
     return den != 0.0 ? ddiv(nom, den) : 0.0;
 }
 
@@ -473,6 +477,140 @@ void batch_reset(Ctx &c) {
     c.launches++;
 }
 
+namespace {
+
+// One pass over the out-lists of a labelling, for the label-mode triangle count and for
+// the community statistics.
+//
+// LISTS: the internal out-lists, i.e. the out-neighbours of v that carry v's (valid)
+// label, in order, at v's CSR offset (length 0 for unlabelled vertices and those of
+// converged graphs). The internal triangles of compute_wcc (src/wcc.cpp:84-127) are
+// exactly the triangles of that subgraph, so the count walks internal lists only instead
+// of filtering whole out-lists. The counters and flags the count starts from are cleared
+// on the way.
+// STATS: collect_stats (src/scd.cpp:57-111) of a symmetric graph without loops. An
+// internal edge is an out-edge of one of its two ends and internal for both, so with c
+// internal out-edges at v the row's share of the sums is +1 vertex, +2c internal and
+// +deg - 2c external entries: half the neighbours are looked at, and in one iteration
+// the same look gives the lists.
+//
+// Out-lists above the register groups' (the vertices of `longer`) have a warp each. Of the
+// others a warp takes `rows` vertices: its lanes read their labels and bounds in one
+// coalesced step; then a group of 8 lanes walks one out-list (most are short, and ids being
+// degree ranks, the vertices of a warp have lists of similar length), the next four lists'
+// neighbours on their way meanwhile. Bound by the latency of the dependent loads (label,
+// bounds, neighbour, its label), which one vertex per group at a time paid in full.
+// Measured (statistics + lists of a step): 96 planted graphs, 2.6 M vertices, 130 + 227 ->
+// 195 us; Chung-Lu 500k, statistics alone 123 -> 30 us; R-MAT scale 20 89 + 40 -> 80 us.
+// a vertex of label l and degree deg with c internal out-edges
+__device__ __forceinline__ void add_stats(const Stats &st, uint32_t l, uint32_t deg, uint32_t c) {
+    atomicAdd(st.sizes + l, 1);
+    if (deg - 2 * c) atomicAdd(st.ext + l, (int)(deg - 2 * c));
+    if (c) atomicAdd(st.intl + l, (int)(2 * c));
+}
+
+template <bool LISTS, bool STATS>
+__global__ void __launch_bounds__(TPB)
+k_internal_lists(uint32_t n, uint32_t rows, WarpRows longer, uint32_t most_short,
+                 const uint32_t *__restrict__ indices, const uint32_t *__restrict__ nlow, const uint32_t *__restrict__ adj, LabelFilter lf, uint32_t *ilen, uint32_t *iadj, uint8_t *flag,
+                 uint32_t *itcount, int32_t *itdeg, Stats st) {
+    const uint32_t lane = threadIdx.x & 31, gl = lane & 7, grp = lane >> 3;
+    const uint32_t warps = (gridDim.x * blockDim.x) >> 5, units = (n + rows - 1) / rows;
+    const unsigned gmask = 0xffu << (grp * 8), lt = (1u << lane) - 1u;
+    for (uint32_t unit = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; unit < longer.total + units; unit += warps) {
+        if (unit < longer.total) {
+            const uint32_t v = longer[unit], l = lf.labels[v], beg = indices[v], len = nlow[v];
+            const bool on = l != INVALID && !lf.frozen(v);
+            uint32_t c = 0;
+            if (on) {
+                uint32_t w = lane < len ? adj[beg + lane] : INVALID;
+                for (uint32_t i = lane; i - lane < len; i += 32) {
+                    const uint32_t cw = w;
+                    w = i + 32 < len ? adj[beg + i + 32] : INVALID;
+                    const bool keep = cw != INVALID && lf.labels[cw] == l;
+                    const unsigned kb = __ballot_sync(FULL, keep);
+                    if (LISTS && keep) {
+                        const uint32_t p = beg + c + __popc(kb & lt);
+                        iadj[p] = cw;
+                        flag[p] = 0;
+                    }
+                    c += __popc(kb);
+                }
+            }
+            if (LISTS && lane == 0) ilen[v] = c;
+            if (STATS && on && lane == 0) add_stats(st, l, indices[v + 1] - beg, c);
+            continue;
+        }
+        const uint32_t u = unit - longer.total, v = u * rows + lane, nrows = min(rows, n - u * rows);
+        const bool in = lane < nrows;
+        const uint32_t l = in ? lf.labels[v] : INVALID;
+        bool on = l != INVALID && !lf.frozen(v);
+        uint32_t beg = 0, len = in ? nlow[v] : 0u, deg = 0, cnt = 0;
+        const bool shorter = len <= most_short;   // (the others have a warp)
+        on = on && shorter;
+        if (!on) len = 0;
+        if (on) {
+            beg = indices[v];
+            if (STATS) deg = indices[v + 1] - beg;
+        }
+        uint32_t b = __shfl_sync(FULL, beg, grp), ln = __shfl_sync(FULL, len, grp);
+        uint32_t w = gl < ln ? adj[b + gl] : INVALID;   // rows beyond nrows have length 0
+        for (uint32_t s0 = 0; s0 < nrows; s0 += 4) {
+            const uint32_t lr = __shfl_sync(FULL, l, s0 + grp), cb = b, cln = ln;
+            uint32_t cw = w;
+            if (s0 + 4 < nrows) {
+                b = __shfl_sync(FULL, beg, s0 + 4 + grp);
+                ln = __shfl_sync(FULL, len, s0 + 4 + grp);
+                w = gl < ln ? adj[b + gl] : INVALID;
+            }
+            const uint32_t most = __reduce_max_sync(FULL, cln);
+            uint32_t c = 0;
+            for (uint32_t i = 0; i < most; i += 8) {
+                const bool keep = cw != INVALID && lf.labels[cw] == lr;
+                const unsigned kb = __ballot_sync(FULL, keep) & gmask;
+                if (LISTS && keep) {
+                    const uint32_t p = cb + c + __popc(kb & lt);
+                    iadj[p] = cw;
+                    flag[p] = 0;
+                }
+                c += __popc(kb);
+                cw = i + 8 + gl < cln ? adj[cb + i + 8 + gl] : INVALID;
+            }
+            const uint32_t mine = __shfl_sync(FULL, c, ((lane - s0) & 3) * 8);
+            if (lane >= s0 && lane < s0 + 4) cnt = mine;
+        }
+        if (LISTS && in) {
+            if (shorter) ilen[v] = cnt;
+            itcount[v] = 0;
+            itdeg[v] = 0;
+        }
+        if (STATS && on) add_stats(st, l, deg, cnt);
+    }
+}
+
+template <bool LISTS, bool STATS>
+void launch_internal_lists(Ctx &c, LabelFilter lf, const Stats &st) {
+    const Graph &g = c.g;
+    uint32_t rows = 4;   // as many as leave every SM its 32 warps
+    while (rows < 32 && (uint64_t)rows * 2 * NUM_SMS_HINT * 32 <= g.n) rows <<= 1;
+    WarpRows longer{};
+    for (int k = 0; k < WarpRows::K; k++)   // the longest first
+        longer.set(k, c.wplan.verts[TcPlan::K - 1 - k], c.wplan.nverts[TcPlan::K - 1 - k]);
+    static_assert(TcPlan::K - WarpRows::K == 3, "the buckets above the register groups");
+    k_internal_lists<LISTS, STATS><<<grid_for((((uint64_t)g.n + rows - 1) / rows + longer.total) * 32, TPB,
+                                              NUM_SMS_HINT * 16), TPB, 0, c.stream>>>(
+        g.n, rows, longer, c.wplan.small_max, g.indices, g.nlow, g.adj, lf, c.int_len, c.int_adj, c.slot_flag, c.itcount,
+        c.itdeg, st);
+    CK_LAUNCH("k_internal_lists");
+}
+
+// statistics from the out-lists alone: a symmetric graph (Graph::symmetric) whose longest
+// out-list is no hub's whole row (a graph whose ids are not degree ranks may have such ones,
+// and k_stats spreads them over warps)
+bool stats_from_out_lists(const Ctx &c) { return c.g.symmetric && c.wplan.nverts[TcPlan::K - 1] == 0; }
+
+}  // namespace
+
 void collect_stats(Ctx &c, const uint32_t *labels, Stats &st, bool frozen_graphs) {
     const Graph &g = c.g;
     cudaStream_t s = c.stream;
@@ -483,51 +621,17 @@ void collect_stats(Ctx &c, const uint32_t *labels, Stats &st, bool frozen_graphs
     if (g.n == 0) return;
     PhaseScope ph(c, "stats");
     const LabelFilter skip{nullptr, c.b.gid, frozen_graphs ? c.b.active : nullptr};
-    k_stats<<<grid_for(((uint64_t)(g.n + 31) / 32 + g.rows.nchunks) * 32, TPB), TPB, 0, s>>>(
-        g.n, g.rows, g.indices, g.adj, labels, st, skip);
-    CK_LAUNCH("k_stats");
+    if (stats_from_out_lists(c)) {
+        launch_internal_lists<false, true>(c, LabelFilter{labels, skip.gid, skip.active}, st);
+    } else {
+        k_stats<<<grid_for(((uint64_t)(g.n + 31) / 32 + g.rows.nchunks) * 32, TPB), TPB, 0, s>>>(
+            g.n, g.rows, g.indices, g.adj, labels, st, skip);
+        CK_LAUNCH("k_stats");
+    }
     c.launches++;
 }
 
-// Internal out-lists for the label-mode triangle count: the out-neighbours of v
-// that carry v's (valid) label, in order, at v's CSR offset; length 0 for
-// unlabelled vertices and those of converged graphs.  The internal triangles of
-// compute_wcc (src/wcc.cpp:84-127) are exactly the triangles of this subgraph, so
-// the count walks internal lists only instead of filtering whole out-lists.
-template <int G>
-__global__ void __launch_bounds__(TPB)
-k_internal_outlists(uint32_t n, const uint32_t *__restrict__ indices, const uint32_t *__restrict__ nlow,
-                    const uint32_t *__restrict__ adj, LabelFilter lf, uint32_t *ilen, uint32_t *iadj) {
-    // a group of G lanes per vertex (out-lists of most vertices are short; ids are
-    // degree ranks, so the vertices of a warp have out-lists of similar length)
-    const int lane = threadIdx.x & 31, gl = lane % G, g0 = lane - gl;
-    const unsigned gmask = (G == 32) ? FULL : (((1u << G) - 1u) << g0);
-    const unsigned lt = (1u << lane) - 1u;
-    const uint32_t groups = (gridDim.x * blockDim.x) / G;
-    for (uint32_t base = (blockIdx.x * blockDim.x + threadIdx.x) / G - (lane / G); base < n;
-         base += groups) {
-        const uint32_t v = base + lane / G;   // (base: the warp's first vertex)
-        const bool live = v < n;
-        const uint32_t l = live ? lf.labels[v] : INVALID;
-        const bool on = live && l != INVALID && !lf.frozen(v);
-        const uint32_t beg = on ? indices[v] : 0u, len = on ? nlow[v] : 0u;
-        uint32_t steps = (len + G - 1) / G;
-#pragma unroll
-        for (int d = G; d < 32; d <<= 1) steps = max(steps, __shfl_xor_sync(FULL, steps, d));
-        uint32_t cnt = 0;
-        for (uint32_t s = 0; s < steps; s++) {
-            const uint32_t i = s * G + gl;
-            const uint32_t w = i < len ? adj[beg + i] : 0u;
-            const bool keep = i < len && lf.labels[w] == l;
-            const unsigned kb = __ballot_sync(FULL, keep) & gmask;
-            if (keep) iadj[beg + cnt + __popc(kb & lt)] = w;
-            cnt += __popc(kb);
-        }
-        if (live && gl == 0) ilen[v] = cnt;
-    }
-}
-
-void launch_wcc(Ctx &c, const uint32_t *labels, const Stats &st, bool frozen_graphs) {
+void launch_wcc(Ctx &c, const uint32_t *labels, const Stats &st, bool frozen_graphs, bool with_stats) {
     const Graph &g = c.g;
     cudaStream_t s = c.stream;
     if (g.n == 0) {
@@ -535,15 +639,11 @@ void launch_wcc(Ctx &c, const uint32_t *labels, const Stats &st, bool frozen_gra
         return;
     }
     PhaseScope ph(c, "wcc");
-    CK(cudaMemsetAsync(c.slot_flag, 0, 2 * (size_t)g.m, s));
-    CK(cudaMemsetAsync(c.itcount, 0, (size_t)g.n * 4, s));
-    CK(cudaMemsetAsync(c.itdeg, 0, (size_t)g.n * 4, s));
     const Batch &b = c.b;
     const uint8_t *active = frozen_graphs ? b.active : nullptr;
     const LabelFilter lf{labels, b.gid, active};
-    k_internal_outlists<8><<<grid_for((uint64_t)g.n * 8, TPB), TPB, 0, s>>>(g.n, g.indices, g.nlow, g.adj, lf, c.int_len,
-                                                                        c.int_adj);
-    CK_LAUNCH("k_internal_outlists");
+    if (with_stats) launch_internal_lists<true, true>(c, lf, st);
+    else launch_internal_lists<true, false>(c, lf, st);
     // the plan's buckets (by full out-degree) stay valid: internal lists are never longer
     const Oriented o{g.indices, c.int_len, c.int_adj, g.n};
     count_triangles(c, o, c.wplan, LabelFilter{}, c.itcount, c.slot_flag, s, "wcc_tc");
@@ -561,11 +661,22 @@ void launch_wcc(Ctx &c, const uint32_t *labels, const Stats &st, bool frozen_gra
     c.launches += 3;
 }
 
-double compute_wcc(Ctx &c, const uint32_t *labels, const Stats &st) {
-    launch_wcc(c, labels, st);
+// statistics (st cleared by improve) and WCC of the labels of an iteration
+void launch_stats_wcc(Ctx &c, const uint32_t *labels, Stats &st, bool frozen_graphs) {
+    const bool fused = stats_from_out_lists(c);
+    if (!fused) collect_stats(c, labels, st, frozen_graphs);
+    launch_wcc(c, labels, st, frozen_graphs, fused);
+}
+
+double read_wcc(Ctx &c) {
     CK(cudaMemcpyAsync(c.wcc_host, c.b.wcc, sizeof(double), cudaMemcpyDeviceToHost, c.stream));
     CK(cudaStreamSynchronize(c.stream));
     return *c.wcc_host;
+}
+
+double compute_wcc(Ctx &c, const uint32_t *labels, const Stats &st) {
+    launch_wcc(c, labels, st);
+    return read_wcc(c);
 }
 
 // FP32 enclosure of every p_ext (directed conversions), for the interval gains

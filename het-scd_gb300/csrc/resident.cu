@@ -197,6 +197,7 @@ struct ResidentSource {
     std::vector<uint32_t> fin_off, comm_off, m;   // per graph of the source union
     UnionLists lists{};
     const uint32_t *nlow = nullptr;
+    bool symmetric = true;
     std::vector<GraphLists> gl;                  // per graph of the source union
     std::vector<uint64_t> ids;
     std::vector<double> wcc0;
@@ -435,7 +436,11 @@ uint32_t rebuild(Ctx &c, ResidentSet &R, std::vector<ResidentSource *> &srcs) {
     c.owned.clear();
     c.bytes = 0;
     R.drop_exec();
+    bool symmetric = true;   // statistics from out-lists: only if every graph's rows allow it
+    for (const ResidentGraph &x : R.graphs) symmetric = symmetric && (x.taken || c.g.symmetric);
+    for (const ResidentSource *ps : srcs) symmetric = symmetric && ps->symmetric;
     c.g = Graph();
+    c.g.symmetric = symmetric;
     c.b = Batch();
     c.wplan = TcPlan();
     c.has_graph = c.has_labels = false;
@@ -509,6 +514,7 @@ uint32_t rebuild(Ctx &c, ResidentSet &R, std::vector<ResidentSource *> &srcs) {
             pl.unit_off[k] = (uint32_t *)off[BUCKET0 + k];
             pl.nverts[k] = pl.nfwd[k] = (uint32_t)lcnt[BUCKET0 + k];
         }
+        pl.small_max = R.split[0];
         pl.dir_lo = pl.dir_hi = 0;   // out-list centres only, as tc_plan builds the WCC plan
         pl.dir_amin = c.tc_amin < c.tc_small ? c.tc_amin : c.tc_small;
         // scratch of the iteration
@@ -753,6 +759,7 @@ int scd_resident_add(scd_ctx *set, scd_ctx *src, uint64_t *ids) {
         }
         ps->lists = lists_of(s);
         ps->nlow = s.g.nlow;
+        ps->symmetric = s.g.symmetric;
         ps->gl = graph_lists(s);
         ps->a = arrays_of(s);
         ps->fin_off = s.b.h_fin_off;

@@ -1,10 +1,30 @@
-// Row streams: a warp walks the entries of 32 consecutive CSR rows as one
+// Work shapes over CSR rows: lists of rows that have a warp each, and row streams: a warp walks the entries of 32 consecutive CSR rows as one
 // stream (see RowStream).
 #pragma once
 
 #include "common.cuh"
 
 namespace scd {
+
+// Four vertex lists one after the other: the rows of a kernel that have a warp each
+struct WarpRows {
+    static constexpr int K = 4;
+    const uint32_t *list[K];
+    uint32_t count[K], total;
+    void set(int k, const uint32_t *l, uint32_t c) {   // (total starts at 0)
+        list[k] = l;
+        count[k] = c;
+        total += c;
+    }
+    __device__ uint32_t operator[](uint32_t i) const {
+#pragma unroll
+        for (int k = 0; k < K - 1; k++) {
+            if (i < count[k]) return list[k][i];
+            i -= count[k];
+        }
+        return list[K - 1][i];
+    }
+};
 
 // A warp takes 32 consecutive rows (lane k: row r0 + k, its entries [b_k, b_k + len_k))
 // and walks their concatenated entries 32 at a time: coalesced loads and many

@@ -858,6 +858,7 @@ void tc_plan_lists(Ctx &c, const Oriented &o, TcPlan &plan, uint32_t *lists, uin
     // kernels' upper bucket (one CTA per SM, 16K-entry tables) from tc_b1 on
     const uint32_t b1 = core_from ? (core_from > b0 ? core_from : b0) : c.tc_b1;
     const bool split = in_lists && !(c.flags & SCD_FLAG_TC_OUT_ONLY);
+    plan.small_max = sm;
     plan.dir_lo = split ? b0 : 0;
     plan.dir_hi = split ? B2 : 0;
     plan.dir_amin = c.tc_amin < sm ? c.tc_amin : sm;
