@@ -147,9 +147,10 @@ constexpr unsigned GROUP_GRID = 152 * 4;   // resident CTAs (64 registers x 256 
 // of the pending vertices.  The interval of every candidate is evaluated 32 at
 // a time with all lanes busy (a vertex of degree <= 32 has only a few distinct
 // labels, so evaluating them where they arise would leave most lanes idle);
-// then one lane per vertex decides from the intervals, and the rare vertices
-// that need exact gains are evaluated one at a time, lane-parallel over their
-// candidates.
+// then one lane per vertex decides from the intervals. The candidates whose exact
+// gain is needed are gathered over all vertices of the queue and evaluated 32 at a
+// time too: an FP64 instruction holds its pipe as long for one lane as for 32, so the
+// gains' cost is the number of passes through the model, not the number of gains.
 constexpr int CQ = 64;
 
 struct CandQueue {
@@ -157,8 +158,13 @@ struct CandQueue {
     float lo[CQ], hi[CQ];
     uint8_t vert[CQ], need[CQ];
     uint32_t p[CQ], deg[CQ], mine[CQ], gp[CQ];   // pending vertices (each has >= 1 candidate)
-    uint8_t first[CQ], cnt[CQ], exact[CQ];
+    uint8_t first[CQ], cnt[CQ], exact[CQ];   // exact: 0 decided, 1 exact gains of the foreign survivors, 2 the own one too
+    float m[CQ];                             // best lower bound among the vertex's foreign labels
+    uint8_t items[CQ];                       // candidates whose exact gain is needed
+    double gain[CQ];
 };
+
+__device__ __forceinline__ bool survives(float hi, float m) { return hi > 0.f && hi >= m; }
 
 __device__ __forceinline__ void process_candidates(const ImproveArgs &a, CandQueue &q, uint32_t cn, uint32_t vn,
                                                 int lane, Iv al) {
@@ -193,67 +199,68 @@ __device__ __forceinline__ void process_candidates(const ImproveArgs &a, CandQue
             }
         }
         uint32_t survivors = 0;
-        for (uint32_t k = f; k < e; k++)
-            survivors += q.label[k] != mine && (q.need[k] || (q.hi[k] > 0.f && q.hi[k] >= m));
+        for (uint32_t k = f; k < e; k++) survivors += q.label[k] != mine && (q.need[k] || survives(q.hi[k], m));
         uint32_t dec = UNDECIDED;
         if (survivors == 1 && !need_any && m > 0.f && !(has_own && own_need))
             dec = decide_iv(Iv{m, m_hi}, m_label, has_own, own, mine);
         else if (survivors == 0 && !(has_own && !own_sign_known(own, own_need)))
             dec = (has_own && own.hi < 0.f) ? INVALID : mine;   // no foreign label can have a positive gain
-        q.exact[v] = dec == UNDECIDED;
+        // (undecided with no survivor: the own label's sign is not known)
+        q.exact[v] = dec != UNDECIDED ? 0 : has_own ? 2 : 1;
+        q.m[v] = m;
         if (dec != UNDECIDED) a.next[q.p[v]] = dec;
     }
     __syncwarp();
-    // exact gains: one vertex at a time, a lane per candidate (<= 32 of them)
-    for (uint32_t v0 = 0; v0 < vn; v0 += 32) {
-        unsigned xb = __ballot_sync(FULL, v0 + lane < vn && q.exact[v0 + lane]);
-        while (xb) {
-            const uint32_t v = v0 + __ffs(xb) - 1;
-            xb &= xb - 1;
-            const uint32_t mine = q.mine[v], c = q.cnt[v], k = q.first[v] + lane;
-            const bool in = (uint32_t)lane < c;
-            const uint32_t l = in ? q.label[k] : INVALID;
-            const bool is_own = in && l == mine, need = in && q.need[k];
-            const float lo = in ? q.lo[k] : -INFINITY, hi = in ? q.hi[k] : -INFINITY;
-            float m = (in && !is_own && !need) ? lo : -INFINITY;
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(FULL, m, o));
-            const bool survive = in && !is_own && (need || (hi > 0.f && hi >= m));
-            const bool any_survivor = __any_sync(FULL, survive);
-            const bool own_item = is_own && (any_survivor || !own_sign_known(Iv{lo, hi}, need));
-            const double p_ext = a.p_ext[q.gp[v]];
-            double g = 0.0;
-            if (survive || own_item) g = exact_gain(a, l, q.freq[k], q.deg[v], mine, p_ext);
-            const unsigned own_lanes = __ballot_sync(FULL, is_own);
-            const double own_g = __shfl_sync(FULL, g, own_lanes ? __ffs(own_lanes) - 1 : 0);
-            // remove gain: exact if evaluated; else only its sign matters (nothing survives)
-            const bool own_eval = __shfl_sync(FULL, own_item, own_lanes ? __ffs(own_lanes) - 1 : 0);
-            const float own_hi = __shfl_sync(FULL, hi, own_lanes ? __ffs(own_lanes) - 1 : 0);
-            const double rg = !own_lanes ? 0.0 : own_eval ? -own_g : (own_hi < 0.f ? 1.0 : 0.0);
-            double bg = 0.0;
-            uint32_t bl = INVALID;
-            if (survive && g > 0.0) {
+    // the candidates whose exact gain is needed
+    uint32_t items = 0;
+    for (uint32_t i0 = 0; i0 < cn; i0 += 32) {
+        const uint32_t i = i0 + lane;
+        bool need = false;
+        if (i < cn) {
+            const uint32_t v = q.vert[i], x = q.exact[v];
+            if (x) need = q.label[i] == q.mine[v] ? x == 2 : (q.need[i] || survives(q.hi[i], q.m[v]));
+            if (x && !need) q.gain[i] = 0.0;
+        }
+        const unsigned b = __ballot_sync(FULL, need);
+        if (need) q.items[items + __popc(b & ((1u << lane) - 1u))] = (uint8_t)i;
+        items += __popc(b);
+    }
+    __syncwarp();
+    if (items == 0) return;
+    for (uint32_t t = lane; t < items; t += 32) {
+        const uint32_t i = q.items[t], v = q.vert[i];
+        q.gain[i] = exact_gain(a, q.label[i], q.freq[i], q.deg[v], q.mine[v], a.p_ext[q.gp[v]]);
+    }
+    __syncwarp();
+    for (uint32_t v = lane; v < vn; v += 32) {
+        if (!q.exact[v]) continue;
+        const uint32_t mine = q.mine[v], f = q.first[v], e = f + q.cnt[v];
+        double bg = 0.0, rg = 0.0;
+        uint32_t bl = INVALID;
+        for (uint32_t k = f; k < e; k++) {
+            const uint32_t l = q.label[k];
+            const double g = q.gain[k];   // 0: not a survivor
+            if (l == mine) {
+                rg = -g;
+            } else if (g > 0.0 && (bl == INVALID || better(g, l, bg, bl))) {
                 bg = g;
                 bl = l;
             }
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                const double og = __shfl_xor_sync(FULL, bg, o);
-                const uint32_t olb = __shfl_xor_sync(FULL, bl, o);
-                if (olb != INVALID && (bl == INVALID || better(og, olb, bg, bl))) {
-                    bg = og;
-                    bl = olb;
-                }
-            }
-            if (lane == 0) a.next[q.p[v]] = decide(bl == INVALID ? 0.0 : bg, bl == INVALID ? 0u : bl, rg, mine);
         }
+        a.next[q.p[v]] = decide(bl == INVALID ? 0.0 : bg, bl == INVALID ? 0u : bl, rg, mine);
     }
     __syncwarp();
 }
 
+// A warp takes `take` (a multiple of its groups) vertices of the list at a time: its lanes
+// read their bounds, labels and graphs in one coalesced step, vertices of converged graphs
+// are done with there, and then each group's next neighbours and their labels are on
+// their way while a round of groups is looked at. (One vertex per group at a time paid the
+// whole chain list -> bounds, label, graph -> active -> neighbour -> its label: with one
+// resident round of warps it, and not the gains, set the time.)
 template <int G>
-__global__ void __launch_bounds__(TPB)
-k_improve_group(const uint32_t *__restrict__ verts, uint32_t count, ImproveArgs a) {
+__global__ void __launch_bounds__(TPB, 4)
+k_improve_group(const uint32_t *__restrict__ verts, uint32_t count, uint32_t take, ImproveArgs a) {
     constexpr int PER_WARP = 32 / G;
     __shared__ CandQueue queues[TPB / 32];
     const int lane = threadIdx.x & 31, gl = lane % G, g0 = lane - gl;
@@ -263,40 +270,66 @@ k_improve_group(const uint32_t *__restrict__ verts, uint32_t count, ImproveArgs 
     const Iv al = iv_of(a.alpha);
     const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
     uint32_t cn = 0, vn = 0;   // warp-uniform
-    for (uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;; w += warps) {
-        const bool done = w * PER_WARP >= count;
+    uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, here = 0, r0 = 0;
+    uint32_t p = 0, mine = INVALID, gp = 0, beg = 0, deg = 0, x = INVALID, l_next = INVALID;
+    bool live = false;
+    const auto neighbour = [&](uint32_t row0) {   // of the group's vertex in the round from row0 on
+        const uint32_t r = row0 + lane / G, b = __shfl_sync(FULL, beg, r & 31), d = __shfl_sync(FULL, deg, r & 31);
+        return r < here && (uint32_t)gl < d ? a.adj[b + gl] : INVALID;
+    };
+    while (true) {
+        while (r0 >= here && w * (uint64_t)take < count) {   // the next vertices, until some are live
+            const uint32_t slot = w * take + lane;
+            here = min(take, count - w * take);
+            w += warps;
+            const bool in = (uint32_t)lane < here;
+            p = in ? verts[slot] : 0u;
+            mine = in ? a.labels[p] : INVALID;
+            gp = in ? graph_of(a, p) : 0u;
+            live = in && !(a.active && !a.active[gp]);   // its graph has not converged
+            beg = deg = 0;
+            if (live) {
+                beg = a.indices[p];
+                deg = a.indices[p + 1] - beg;
+            } else if (in) {
+                a.next[p] = mine;
+            }
+            r0 = __any_sync(FULL, live) ? 0u : here;
+            if (r0 == 0) {   // neighbours of round 0 with their labels, neighbours of round 1
+                x = neighbour(0);
+                l_next = x != INVALID ? a.labels[x] : INVALID;
+                x = neighbour(PER_WARP);
+            }
+        }
+        const bool done = r0 >= here;
         if (cn > CQ - 32 || (done && cn)) {   // one call site: the evaluation is inlined once
             process_candidates(a, q, cn, vn, lane, al);
             cn = vn = 0;
         }
         if (done) break;
-        const uint32_t slot = w * PER_WARP + lane / G;
-        const bool active = slot < count;
-        const uint32_t p = active ? verts[slot] : 0;
-        const uint32_t beg = active ? a.indices[p] : 0;
-        const uint32_t deg = active ? a.indices[p + 1] - beg : 0;
-        const uint32_t mine = active ? a.labels[p] : INVALID;
-        const uint32_t gp = active ? graph_of(a, p) : 0u;
-        const bool frozen = active && a.active && !a.active[gp];   // graph already converged
-        const uint32_t l = (uint32_t)gl < deg && !frozen ? a.labels[a.adj[beg + gl]] : INVALID;
+        const uint32_t l = l_next;
+        l_next = x != INVALID ? a.labels[x] : INVALID;
+        x = neighbour(r0 + 2 * PER_WARP);
         const unsigned peers = __match_any_sync(FULL, l) & gmask;
         const bool owner = l != INVALID && lane == __ffs(peers) - 1;
         const uint32_t freq = __popc(peers);
         const unsigned ob = __ballot_sync(FULL, owner);
         const uint32_t gcnt = __popc(ob & gmask);
-        // no labelled neighbour (or the graph converged): the label stays
-        if (active && gl == 0 && gcnt == 0) a.next[p] = mine;
-        const unsigned vb = __ballot_sync(FULL, active && gl == 0 && gcnt != 0);
-        const uint32_t vidx = vn + __popc(vb & below);
-        if (active && gl == 0 && gcnt != 0) {
-            q.p[vidx] = p;
-            q.deg[vidx] = deg;
-            q.mine[vidx] = mine;
-            q.gp[vidx] = gp;
-            q.first[vidx] = (uint8_t)(cn + __popc(ob & ((1u << g0) - 1u)));
-            q.cnt[vidx] = (uint8_t)gcnt;
+        // the lane that read the vertex of row r0 + g enters it: its group's labels and where they start
+        const uint32_t got = __shfl_sync(FULL, (gcnt << 8) | (cn + __popc(ob & ((1u << g0) - 1u))), (lane - r0) * G);
+        const bool row = (uint32_t)lane - r0 < PER_WARP && live;
+        if (row && got < 256) a.next[p] = mine;   // no labelled neighbour: the label stays
+        const unsigned vb = __ballot_sync(FULL, row && got >= 256);
+        if (row && got >= 256) {
+            const uint32_t v = vn + __popc(vb & below);
+            q.p[v] = p;
+            q.deg[v] = deg;
+            q.mine[v] = mine;
+            q.gp[v] = gp;
+            q.first[v] = (uint8_t)got;
+            q.cnt[v] = (uint8_t)(got >> 8);
         }
-        const uint32_t my_v = __shfl_sync(FULL, vidx, g0);
+        const uint32_t my_v = vn + __popc(vb & ((1u << ((r0 + lane / G) & 31)) - 1u));
         if (owner) {
             const uint32_t pos = cn + __popc(ob & below);
             q.label[pos] = l;
@@ -305,6 +338,7 @@ k_improve_group(const uint32_t *__restrict__ verts, uint32_t count, ImproveArgs 
         }
         cn += __popc(ob);
         vn += __popc(vb);
+        r0 += PER_WARP;
     }
 }
 
@@ -334,16 +368,15 @@ struct WarpTable {
     uint32_t n;
 };
 
-__device__ __forceinline__ bool survives(float hi, float m) { return hi > 0.f && hi >= m; }
-
 // a vertex with more than 32 distinct labels, on its own
 __device__ __forceinline__ void improve_many_labels(const ImproveArgs &a, WarpTable &T, uint32_t nl, uint32_t p,
                                                     uint32_t gp, uint32_t mine, uint32_t deg, Iv al, int lane) {
     const double p_ext = a.p_ext[gp];
     const Iv pe = pe_of(a, gp);
-    float m = -INFINITY, mh = -INFINITY, m_hi = -INFINITY;   // m_hi: upper bound of the label holding m
+    float m = -INFINITY, m_hi = -INFINITY;   // m_hi: upper bound of the label holding m
     uint32_t m_label = INVALID;
     bool need_any = false, has_own = false, own_need = false;
+    uint32_t own_k = 0;
     Iv own_iv = {0.f, 0.f};
     for (uint32_t k = lane; k < nl; k += 32) {
         const uint32_t h = T.list[k], l = T.keys[h], f = T.vals[h];
@@ -353,6 +386,7 @@ __device__ __forceinline__ void improve_many_labels(const ImproveArgs &a, WarpTa
             has_own = true;
             own_need = need;
             own_iv = iv;
+            own_k = k;
             T.hi[k] = -INFINITY;
         } else if (need) {
             need_any = true;
@@ -363,7 +397,6 @@ __device__ __forceinline__ void improve_many_labels(const ImproveArgs &a, WarpTa
                 m_hi = iv.hi;
                 m_label = l;
             }
-            mh = fmaxf(mh, iv.hi);
             T.hi[k] = iv.hi;
         }
     }
@@ -376,7 +409,6 @@ __device__ __forceinline__ void improve_many_labels(const ImproveArgs &a, WarpTa
             m_hi = omh;
             m_label = oml;
         }
-        mh = fmaxf(mh, __shfl_xor_sync(FULL, mh, o));
     }
     need_any = __any_sync(FULL, need_any);
     const unsigned own_lanes = __ballot_sync(FULL, has_own);
@@ -384,12 +416,19 @@ __device__ __forceinline__ void improve_many_labels(const ImproveArgs &a, WarpTa
     own_need = __shfl_sync(FULL, own_need, ol);
     own_iv.lo = __shfl_sync(FULL, own_iv.lo, ol);
     own_iv.hi = __shfl_sync(FULL, own_iv.hi, ol);
+    own_k = __shfl_sync(FULL, own_k, ol);
     __syncwarp();
-    const bool any_survivor = need_any || (mh > 0.f && mh >= m);
+    // the survivors' places in the list, one after the other, in the memory of the bounds
+    // (a survivor's place is never after its own bound, and a chunk's bounds are read first)
+    uint32_t *items = reinterpret_cast<uint32_t *>(T.hi);
     uint32_t survivors = 0;
     for (uint32_t kb = 0; kb < nl; kb += 32) {
         const uint32_t k = kb + lane;
-        survivors += __popc(__ballot_sync(FULL, k < nl && survives(T.hi[k], m)));
+        const bool s = k < nl && survives(T.hi[k], m);
+        const unsigned b = __ballot_sync(FULL, s);
+        if (s) items[survivors + __popc(b & ((1u << lane) - 1u))] = k;
+        survivors += __popc(b);
+        __syncwarp();
     }
     uint32_t dec = UNDECIDED;
     if (survivors == 1 && !need_any && m > 0.f && !(own_lanes && own_need))
@@ -400,24 +439,22 @@ __device__ __forceinline__ void improve_many_labels(const ImproveArgs &a, WarpTa
         if (lane == 0) a.next[p] = dec;
         return;
     }
-    // exact gains of the survivors and of the own label, lane-parallel over the list
-    const bool own_item = own_lanes && (own_need || !own_sign_known(own_iv, own_need) || any_survivor);
+    // exact gains of the survivors and of the own label (the last item, if it is among the
+    // neighbours), 32 at a time: as few passes through the FP64 model as there can be
     double bg = 0.0, rg = 0.0;
     uint32_t bl = INVALID;
-    for (uint32_t k = lane; k < nl; k += 32) {
-        const uint32_t h = T.list[k], l = T.keys[h];
+    const uint32_t total = survivors + (own_lanes != 0);
+    for (uint32_t t = lane; t < total; t += 32) {
+        const uint32_t h = T.list[t < survivors ? items[t] : own_k], l = T.keys[h];
+        const double g = exact_gain(a, l, T.vals[h], deg, mine, p_ext);
         if (l == mine) {
-            if (own_item) rg = -exact_gain(a, l, T.vals[h], deg, mine, p_ext);
-        } else if (survives(T.hi[k], m)) {
-            const double g = exact_gain(a, l, T.vals[h], deg, mine, p_ext);
-            if (g > 0.0 && (bl == INVALID || better(g, l, bg, bl))) {
-                bg = g;
-                bl = l;
-            }
+            rg = -g;
+        } else if (g > 0.0 && (bl == INVALID || better(g, l, bg, bl))) {
+            bg = g;
+            bl = l;
         }
     }
-    rg = __shfl_sync(FULL, rg, ol);
-    if (own_lanes && !own_item) rg = own_iv.hi < 0.f ? 1.0 : 0.0;   // only its sign matters then
+    rg = __shfl_sync(FULL, rg, survivors & 31);   // the own label's lane (0 if there is none)
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         const double og = __shfl_xor_sync(FULL, bg, o);
@@ -431,7 +468,7 @@ __device__ __forceinline__ void improve_many_labels(const ImproveArgs &a, WarpTa
 }
 
 __global__ void __launch_bounds__(WWARPS * 32)
-k_improve_warp(const uint32_t *__restrict__ verts, uint32_t count, ImproveArgs a) {
+k_improve_warp(const uint32_t *__restrict__ verts, uint32_t count, uint32_t take, ImproveArgs a) {
     __shared__ WarpTable tabs[WWARPS];
     __shared__ CandQueue queues[WWARPS];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -446,53 +483,95 @@ k_improve_warp(const uint32_t *__restrict__ verts, uint32_t count, ImproveArgs a
     __syncwarp();
     uint32_t cn = 0, vn = 0;   // warp-uniform
     const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
-    for (uint32_t vi = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;; vi += warps) {
-        const bool done = vi >= count;
+    // as in k_improve_group, `take` vertices' bounds, labels and graphs are read in one step,
+    // and the first neighbours of the next vertex are on their way while one is looked at
+    uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    uint32_t my_p = 0, my_mine = INVALID, my_gp = 0, my_beg = 0, my_deg = 0;
+    unsigned todo = 0;
+    constexpr int LB = 4;   // neighbours of a lane whose labels are gathered together
+    uint32_t x[LB];
+    while (true) {
+        while (!todo && w * (uint64_t)take < count) {
+            const uint32_t slot = w * take + lane, here = min(take, count - w * take);
+            w += warps;
+            const bool in = (uint32_t)lane < here;
+            my_p = in ? verts[slot] : 0u;
+            my_mine = in ? a.labels[my_p] : INVALID;
+            my_gp = in ? graph_of(a, my_p) : 0u;
+            const bool live = in && !(a.active && !a.active[my_gp]);
+            if (live) {
+                my_beg = a.indices[my_p];
+                my_deg = a.indices[my_p + 1] - my_beg;
+            } else if (in) {   // converged graph: the label stays
+                a.next[my_p] = my_mine;
+            }
+            todo = __ballot_sync(FULL, live);
+            if (todo) {
+                const int j = __ffs(todo) - 1;
+                const uint32_t beg = __shfl_sync(FULL, my_beg, j), deg = __shfl_sync(FULL, my_deg, j);
+#pragma unroll
+                for (int k = 0; k < LB; k++) x[k] = lane + 32 * k < deg ? a.adj[beg + lane + 32 * k] : INVALID;
+            }
+        }
+        const bool done = !todo;
         // the label table of this vertex, before a flush needs the queue
         uint32_t p = 0, gp = 0, mine = INVALID, deg = 0, nl = 0;
-        bool frozen = false;
         if (!done) {
-            p = verts[vi];
-            gp = graph_of(a, p);
-            mine = a.labels[p];
-            frozen = a.active && !a.active[gp];
-        }
-        if (!done && !frozen) {
-            const uint32_t beg = a.indices[p];
-            deg = a.indices[p + 1] - beg;
+            const int j = __ffs(todo) - 1;
+            todo &= todo - 1;
+            p = __shfl_sync(FULL, my_p, j);
+            gp = __shfl_sync(FULL, my_gp, j);
+            mine = __shfl_sync(FULL, my_mine, j);
+            deg = __shfl_sync(FULL, my_deg, j);
+            const uint32_t beg = __shfl_sync(FULL, my_beg, j);
             uint32_t cap = 64;
             while (cap < 2 * deg) cap <<= 1;
             const uint32_t mask = cap - 1;
-            for (uint32_t k = lane; k < deg; k += 32) {
-                const uint32_t l = a.labels[a.adj[beg + k]];
-                if (l == INVALID) continue;
-                uint32_t h = hash32(l) & mask;
-                while (true) {
-                    uint32_t key = T.keys[h];
-                    if (key == INVALID) {
-                        key = atomicCAS(T.keys + h, INVALID, l);
+            for (uint32_t i0 = 0; i0 < deg; i0 += 32 * LB) {
+                uint32_t lb[LB];
+#pragma unroll
+                for (int k = 0; k < LB; k++) lb[k] = x[k] != INVALID ? a.labels[x[k]] : INVALID;
+                // the next neighbours: of this vertex, or the first ones of the next
+                uint32_t nb = beg + i0 + 32 * LB, nd = deg - min(deg, i0 + 32 * LB);
+                if (nd == 0 && todo) {
+                    const int n = __ffs(todo) - 1;
+                    nb = __shfl_sync(FULL, my_beg, n);
+                    nd = __shfl_sync(FULL, my_deg, n);
+                }
+#pragma unroll
+                for (int k = 0; k < LB; k++) x[k] = lane + 32 * k < nd ? a.adj[nb + lane + 32 * k] : INVALID;
+#pragma unroll
+                for (int k = 0; k < LB; k++) {
+                    const uint32_t l = lb[k];
+                    if (l == INVALID) continue;
+                    uint32_t h = hash32(l) & mask;
+                    while (true) {
+                        uint32_t key = T.keys[h];
                         if (key == INVALID) {
-                            T.list[atomicAdd(&T.n, 1u)] = (uint16_t)h;
-                            key = l;
+                            key = atomicCAS(T.keys + h, INVALID, l);
+                            if (key == INVALID) {
+                                T.list[atomicAdd(&T.n, 1u)] = (uint16_t)h;
+                                key = l;
+                            }
                         }
+                        if (key == l) {
+                            atomicAdd(T.vals + h, 1u);
+                            break;
+                        }
+                        h = (h + 1) & mask;
                     }
-                    if (key == l) {
-                        atomicAdd(T.vals + h, 1u);
-                        break;
-                    }
-                    h = (h + 1) & mask;
                 }
             }
             __syncwarp();
             nl = T.n;
         }
-        const bool queued = !done && !frozen && nl > 0 && nl <= 32;
+        const bool queued = !done && nl > 0 && nl <= 32;
         if ((queued && cn + nl > (uint32_t)CQ) || (done && cn)) {   // one call site
             process_candidates(a, q, cn, vn, lane, al);
             cn = vn = 0;
         }
         if (done) break;
-        if (frozen || nl == 0) {   // converged graph, or no labelled neighbour: the label stays
+        if (nl == 0) {   // no labelled neighbour: the label stays
             if (lane == 0) a.next[p] = mine;
         } else if (queued) {
             if ((uint32_t)lane < nl) {
@@ -543,7 +622,9 @@ __device__ void improve_cta(const ImproveArgs &a, uint32_t p, uint32_t *keys, ui
     __shared__ float s_own_lo, s_own_hi;
     __shared__ uint32_t s_own_i;  // the own label's position in the entry list
     __shared__ float s_mhi[THREADS / 32];
-    __shared__ uint32_t s_mlab[THREADS / 32], s_surv[THREADS / 32];
+    __shared__ uint32_t s_mlab[THREADS / 32];
+    constexpr uint32_t ITEMS = 256;
+    __shared__ uint32_t s_surv, s_items[ITEMS];   // foreign labels that can hold the maximum, their places in the list
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t beg = a.indices[p], deg = a.indices[p + 1] - beg, mine = a.labels[p];
     const uint32_t mask = cap - 1;
@@ -556,6 +637,7 @@ __device__ void improve_cta(const ImproveArgs &a, uint32_t p, uint32_t *keys, ui
         s_n = 0;
         s_need = 0;
         s_own = 0;
+        s_surv = 0;
     }
     __syncthreads();
     // LB neighbour labels per thread are gathered before any is inserted, so their
@@ -657,46 +739,49 @@ __device__ void improve_cta(const ImproveArgs &a, uint32_t p, uint32_t *keys, ui
     // a foreign label survives iff its interval is unusable or hi > 0 and hi >= m;
     // the one with the largest hi decides whether any does
     const bool any_survivor = s_need || (mh > 0.f && mh >= m);
-    // the intervals alone decide when the label holding m > 0 is the only survivor
-    // and the own label's interval is usable (decide_iv); no exact gain is then needed
-    if (!s_need && m > 0.f && s_own != 2) {
-        uint32_t surv = 0;
+    if (any_survivor) {
         for (uint32_t i0 = 0; i0 < nl; i0 += THREADS) {
             const uint32_t i = i0 + threadIdx.x;
-            const float hi = i < nl ? hi_of[i] : -INFINITY;
-            surv += __popc(__ballot_sync(FULL, hi > 0.f && hi >= m));
-        }
-        if (lane == 0) s_surv[warp] = surv;
-        __syncthreads();
-        surv = 0;
-#pragma unroll
-        for (int w = 0; w < THREADS / 32; w++) surv += s_surv[w];
-        if (surv == 1) {
-            const uint32_t dec = decide_iv(Iv{m, m_hi}, m_label, s_own != 0, Iv{s_own_lo, s_own_hi}, mine);
-            if (dec != UNDECIDED) {
-                if (threadIdx.x == 0) a.next[p] = dec;
-                __syncthreads();
-                return;
-            }
+            const bool sv = i < nl && survives(hi_of[i], m);   // (hi_of: -inf for the own label)
+            const unsigned b = __ballot_sync(FULL, sv);
+            uint32_t at = 0;
+            if (lane == 0 && b) at = atomicAdd(&s_surv, (uint32_t)__popc(b));
+            at = __shfl_sync(FULL, at, 0) + __popc(b & ((1u << lane) - 1u));
+            if (sv && at < ITEMS) s_items[at] = i;
         }
     }
-    // pass 2: exact gains of the survivors and, if needed, of the own label (remove gain)
+    __syncthreads();
+    const uint32_t survivors = s_surv;
+    // the intervals alone decide when the label holding m > 0 is the only survivor and the
+    // own label's interval is usable (decide_iv), or when nothing survives and the own
+    // label's sign is known; no exact gain is then needed
+    uint32_t dec = UNDECIDED;
+    if (survivors == 1 && !s_need && m > 0.f && s_own != 2)
+        dec = decide_iv(Iv{m, m_hi}, m_label, s_own != 0, Iv{s_own_lo, s_own_hi}, mine);
+    else if (survivors == 0 && s_own != 2)
+        dec = (s_own && s_own_hi < 0.f) ? INVALID : mine;
+    if (dec != UNDECIDED) {
+        if (threadIdx.x == 0) a.next[p] = dec;
+        __syncthreads();
+        return;
+    }
+    // pass 2: exact gains of the survivors and of the own label (remove gain), packed into as
+    // few warps as hold them: an FP64 instruction holds its pipe as long for one lane as for 32,
+    // and most vertices that come here have a handful of survivors
     double bg = 0.0;
     uint32_t bl = INVALID;
-    if (s_own && threadIdx.x == (s_own_i & (THREADS - 1))) {   // the own label (remove gain)
-        const uint32_t h = list[s_own_i];
-        if (any_survivor || s_own == 2) s_remove = -exact_gain(a, mine, vals[h], deg, mine, p_ext);
-        else if (s_own_hi < 0.f) s_remove = 1.0;   // only its sign matters when nothing survives
-    }
-    for (uint32_t i = threadIdx.x; i < nl; i += THREADS) {
-        const float hi = hi_of[i];   // -inf for the own label
-        if (hi > 0.f && hi >= m) {
-            const uint32_t h = list[i], l = keys[h];
-            const double g = exact_gain(a, l, vals[h], deg, mine, p_ext);
-            if (g > 0.0 && (bl == INVALID || better(g, l, bg, bl))) {
-                bg = g;
-                bl = l;
-            }
+    const bool packed = survivors <= ITEMS;
+    const uint32_t total = (packed ? survivors : nl) + (packed && s_own);   // unpacked: every place of the list
+    for (uint32_t t = threadIdx.x; t < total; t += THREADS) {
+        const uint32_t i = !packed ? t : t < survivors ? s_items[t] : s_own_i;
+        if (!packed && !survives(hi_of[i], m) && !(s_own && i == s_own_i)) continue;
+        const uint32_t h = list[i], l = keys[h];
+        const double g = exact_gain(a, l, vals[h], deg, mine, p_ext);
+        if (l == mine) {
+            s_remove = -g;
+        } else if (g > 0.0 && (bl == INVALID || better(g, l, bg, bl))) {
+            bg = g;
+            bl = l;
         }
     }
 #pragma unroll
@@ -794,6 +879,23 @@ void prepare_improve_kernels() {
 
 namespace {
 
+// vertices a warp takes at a time: at least `least`, and as many as leave every one of `warps`
+// eight turns (with two, R-MAT's uneven gains left a third of the warps idle at the end)
+uint32_t take_of(uint32_t count, uint32_t least, uint64_t warps) {
+    uint32_t take = least;
+    while (take < 32 && count >= 16ull * take * warps) take <<= 1;
+    return take;
+}
+
+template <int G>
+void launch_group(Ctx &c, const uint32_t *verts, uint32_t count, const ImproveArgs &a, cudaStream_t s) {
+    const uint32_t take = take_of(count, 32 / G, GROUP_GRID * (TPB / 32));
+    k_improve_group<G><<<grid_for(((uint64_t)count + take - 1) / take * 32, TPB, GROUP_GRID), TPB, 0, s>>>(verts, count,
+                                                                                                        take, a);
+    CK_LAUNCH("k_improve_group");
+    c.launches++;
+}
+
 template <int THREADS, uint32_t CAP>
 void launch_cta(const uint32_t *verts, uint32_t count, const ImproveArgs &a, cudaStream_t s, unsigned max_grid) {
     k_improve_cta<THREADS, CAP><<<grid_for(count, 1, max_grid), THREADS, cta_smem<THREADS, CAP>(), s>>>(verts, count, a);
@@ -829,24 +931,13 @@ void improve(Ctx &c, const uint32_t *labels, const Stats &st, uint32_t *next, bo
         CK(cudaEventRecord(c.aux_join, c.aux));
         c.launches++;
     }
-    if (k.count[0]) {
-        k_improve_group<8><<<grid_for((uint64_t)k.count[0] * 8, TPB, GROUP_GRID), TPB, 0, s>>>(k.list[0], k.count[0], a);
-        CK_LAUNCH("k_improve_group8");
-        c.launches++;
-    }
-    if (k.count[1]) {
-        k_improve_group<16><<<grid_for((uint64_t)k.count[1] * 16, TPB, GROUP_GRID), TPB, 0, s>>>(k.list[1], k.count[1], a);
-        CK_LAUNCH("k_improve_group16");
-        c.launches++;
-    }
-    if (k.count[2]) {
-        k_improve_group<32><<<grid_for((uint64_t)k.count[2] * 32, TPB, GROUP_GRID), TPB, 0, s>>>(k.list[2], k.count[2], a);
-        CK_LAUNCH("k_improve_group32");
-        c.launches++;
-    }
+    if (k.count[0]) launch_group<8>(c, k.list[0], k.count[0], a, s);
+    if (k.count[1]) launch_group<16>(c, k.list[1], k.count[1], a, s);
+    if (k.count[2]) launch_group<32>(c, k.list[2], k.count[2], a, s);
     if (k.count[3]) {
-        k_improve_warp<<<grid_for((uint64_t)k.count[3] * 32, WWARPS * 32, 152 * 7), WWARPS * 32, 0, s>>>(
-            k.list[3], k.count[3], a);
+        const uint32_t take = take_of(k.count[3], 1, 152 * 7 * WWARPS);
+        k_improve_warp<<<grid_for(((uint64_t)k.count[3] + take - 1) / take * 32, WWARPS * 32, 152 * 7), WWARPS * 32, 0, s>>>(
+            k.list[3], k.count[3], take, a);
         CK_LAUNCH("k_improve_warp");
         c.launches++;
     }
