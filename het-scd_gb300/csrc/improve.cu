@@ -95,6 +95,23 @@ __device__ __forceinline__ Iv interval_any_gain(const ImproveArgs &a, uint32_t l
     return g;
 }
 
+// Can a foreign label seen once never have a positive gain?  With d_in = 1 the terms A and B
+// of the model are 0 (their numerators hold d_in - 1), and the gain is (r - 1) C with
+//   C = -(r-1)(r-2) p_in^3 (q + t) alpha / den
+// for q = (r-1) p_in, t = (ext - 1) / r. Every factor of den is >= 0 if t is 0 or at least 1
+// (p_in <= 1 makes r - q - 1 >= 0; t (t - 1) is the one term that could be negative), and
+// (r-1)(r-2) does not wrap up to r = 46340; for r <= 2 the numerator is 0. Rounding to
+// nearest keeps all these signs, so the FP64 gain is <= 0 and the label is never chosen.
+// `signs`: alpha >= 0 and p_ext >= 0. Most labels of a skewed graph's long rows are seen once
+// (R-MAT scale 21, degree 257..1024: 460 labels a vertex, nearly one per neighbour), and this
+// costs a tenth of an interval.
+__device__ __forceinline__ bool never_gains(const ImproveArgs &a, uint32_t l, uint32_t freq, uint32_t mine, bool signs) {
+    if (freq != 1 || l == mine || !signs) return false;
+    const int4 cv = a.civ[l];
+    const int r = cv.x, ext = cv.y;
+    return r >= 1 && r <= 46340 && ext >= 1 && __int_as_float(cv.z) >= 0.f && (r <= 2 || ext == 1 || ext - 1 >= r);
+}
+
 // The own label's exact gain is needed unless no foreign label survives the
 // interval test and the interval alone fixes the sign of the remove gain
 // (remove gain > 0 exactly when the own gain is < 0).
@@ -160,7 +177,7 @@ struct CandQueue {
     uint32_t p[CQ], deg[CQ], mine[CQ], gp[CQ];   // pending vertices (each has >= 1 candidate)
     uint8_t first[CQ], cnt[CQ], exact[CQ];   // exact: 0 decided, 1 exact gains of the foreign survivors, 2 the own one too
     float m[CQ];                             // best lower bound among the vertex's foreign labels
-    uint8_t items[CQ];                       // candidates whose exact gain is needed
+    uint8_t items[CQ];                       // candidates whose interval, then whose exact gain is needed
     double gain[CQ];
 };
 
@@ -169,8 +186,25 @@ __device__ __forceinline__ bool survives(float hi, float m) { return hi > 0.f &&
 __device__ __forceinline__ void process_candidates(const ImproveArgs &a, CandQueue &q, uint32_t cn, uint32_t vn,
                                                 int lane, Iv al) {
     __syncwarp();
-    for (uint32_t i = lane; i < cn; i += 32) {
-        const uint32_t v = q.vert[i], l = q.label[i];
+    uint32_t wide = 0;   // candidates that need an interval, packed
+    for (uint32_t i0 = 0; i0 < cn; i0 += 32) {
+        const uint32_t i = i0 + lane;
+        bool keep = false;
+        if (i < cn) {
+            const uint32_t v = q.vert[i];
+            keep = !never_gains(a, q.label[i], q.freq[i], q.mine[v], al.lo >= 0.f && pe_of(a, q.gp[v]).lo >= 0.f);
+            if (!keep) {
+                q.lo[i] = q.hi[i] = -INFINITY;
+                q.need[i] = 0;
+            }
+        }
+        const unsigned b = __ballot_sync(FULL, keep);
+        if (keep) q.items[wide + __popc(b & ((1u << lane) - 1u))] = (uint8_t)i;
+        wide += __popc(b);
+    }
+    __syncwarp();
+    for (uint32_t t = lane; t < wide; t += 32) {
+        const uint32_t i = q.items[t], v = q.vert[i], l = q.label[i];
         bool need = false;
         const Iv iv = interval_any_gain(a, l, l == q.mine[v], q.freq[i], q.deg[v], pe_of(a, q.gp[v]), al, &need);
         q.lo[i] = iv.lo;
@@ -361,8 +395,37 @@ __device__ __forceinline__ uint32_t hash32(uint32_t x) {
 // list and, where they do not settle it, its exact gains too.
 constexpr int WCAP = 512, WLIST = 256, WWARPS = 4;
 
+// For every k < nl of this warp's (first, first + stride, ... in steps of 32 lanes): test(k) says
+// whether its interval is needed, eval(k) evaluates it; the ones that need it are packed so
+// that a warp evaluates 32 at a time (queue: 64 words of shared memory of this warp).
+template <typename Test, typename Eval>
+__device__ __forceinline__ void for_wide(uint32_t nl, int lane, uint32_t first, uint32_t stride, uint32_t *queue, Test test,
+                                         Eval eval) {
+    uint32_t n = 0;
+    for (uint32_t k0 = first;; k0 += stride) {
+        const bool more = k0 < nl;
+        if (more) {
+            const uint32_t k = k0 + lane;
+            const bool keep = k < nl && test(k);
+            const unsigned b = __ballot_sync(FULL, keep);
+            if (keep) queue[n + __popc(b & ((1u << lane) - 1u))] = k;
+            n += __popc(b);
+        }
+        if (n < 32 && more) continue;
+        __syncwarp();
+        const uint32_t k = (uint32_t)lane < n ? queue[lane] : INVALID;
+        const uint32_t rest = 32 + (uint32_t)lane < n ? queue[32 + lane] : INVALID;
+        __syncwarp();
+        if (rest != INVALID) queue[lane] = rest;
+        n -= min(n, 32u);
+        if (k != INVALID) eval(k);
+        __syncwarp();
+        if (!more && n == 0) break;
+    }
+}
+
 struct WarpTable {
-    uint32_t keys[WCAP], vals[WCAP];
+    uint32_t keys[WCAP], vals[WCAP], wide[64];
     float hi[WLIST];   // upper bound of each listed foreign label (+inf: interval unusable)
     uint16_t list[WLIST];
     uint32_t n;
@@ -378,28 +441,36 @@ __device__ __forceinline__ void improve_many_labels(const ImproveArgs &a, WarpTa
     bool need_any = false, has_own = false, own_need = false;
     uint32_t own_k = 0;
     Iv own_iv = {0.f, 0.f};
-    for (uint32_t k = lane; k < nl; k += 32) {
-        const uint32_t h = T.list[k], l = T.keys[h], f = T.vals[h];
-        bool need = false;
-        const Iv iv = interval_any_gain(a, l, l == mine, f, deg, pe, al, &need);
-        if (l == mine) {
-            has_own = true;
-            own_need = need;
-            own_iv = iv;
-            own_k = k;
-            T.hi[k] = -INFINITY;
-        } else if (need) {
-            need_any = true;
-            T.hi[k] = INFINITY;
-        } else {
-            if (iv.lo > m) {
-                m = iv.lo;
-                m_hi = iv.hi;
-                m_label = l;
-            }
-            T.hi[k] = iv.hi;
-        }
-    }
+    const bool signs = al.lo >= 0.f && pe.lo >= 0.f;
+    for_wide(nl, lane, 0, 32, T.wide,
+             [&](uint32_t k) {
+                 const uint32_t h = T.list[k];
+                 const bool no = never_gains(a, T.keys[h], T.vals[h], mine, signs);
+                 if (no) T.hi[k] = -INFINITY;
+                 return !no;
+             },
+             [&](uint32_t k) {
+                 const uint32_t h = T.list[k], l = T.keys[h], f = T.vals[h];
+                 bool need = false;
+                 const Iv iv = interval_any_gain(a, l, l == mine, f, deg, pe, al, &need);
+                 if (l == mine) {
+                     has_own = true;
+                     own_need = need;
+                     own_iv = iv;
+                     own_k = k;
+                     T.hi[k] = -INFINITY;
+                 } else if (need) {
+                     need_any = true;
+                     T.hi[k] = INFINITY;
+                 } else {
+                     if (iv.lo > m) {
+                         m = iv.lo;
+                         m_hi = iv.hi;
+                         m_label = l;
+                     }
+                     T.hi[k] = iv.hi;
+                 }
+             });
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         const float om = __shfl_xor_sync(FULL, m, o), omh = __shfl_xor_sync(FULL, m_hi, o);
@@ -624,6 +695,7 @@ __device__ void improve_cta(const ImproveArgs &a, uint32_t p, uint32_t *keys, ui
     __shared__ float s_mhi[THREADS / 32];
     __shared__ uint32_t s_mlab[THREADS / 32];
     constexpr uint32_t ITEMS = 256;
+    __shared__ uint32_t s_wide[THREADS / 32][64];
     __shared__ uint32_t s_surv, s_items[ITEMS];   // foreign labels that can hold the maximum, their places in the list
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t beg = a.indices[p], deg = a.indices[p + 1] - beg, mine = a.labels[p];
@@ -680,31 +752,37 @@ __device__ void improve_cta(const ImproveArgs &a, uint32_t p, uint32_t *keys, ui
     // interval; hi_of[i] keeps label i's upper bound for pass 2 (+inf: unusable)
     float m = -INFINITY, mh = -INFINITY, m_hi = -INFINITY;   // m_hi: upper bound of the label holding m
     uint32_t m_label = INVALID;
-    for (uint32_t i = threadIdx.x; i < nl; i += THREADS) {
-        const uint32_t h = list[i], l = keys[h];
-        bool need = false;
-        const Iv iv = interval_any_gain(a, l, l == mine, vals[h], deg, pe, al, &need);
-        if (l == mine) {
-            s_own = own_sign_known(iv, need) ? 1 : 2;
-            s_own_lo = iv.lo;
-            s_own_hi = iv.hi;
-            s_own_i = i;
-            hi_of[i] = -INFINITY;
-            continue;
-        }
-        if (need) {
-            s_need = 1;
-            hi_of[i] = INFINITY;
-        } else {
-            if (iv.lo > m || (iv.lo == m && l < m_label)) {
-                m = iv.lo;
-                m_hi = iv.hi;
-                m_label = l;
-            }
-            mh = fmaxf(mh, iv.hi);
-            hi_of[i] = iv.hi;
-        }
-    }
+    const bool signs = al.lo >= 0.f && pe.lo >= 0.f;
+    for_wide(nl, lane, warp * 32, THREADS, s_wide[warp],
+             [&](uint32_t i) {
+                 const uint32_t h = list[i];
+                 const bool no = never_gains(a, keys[h], vals[h], mine, signs);
+                 if (no) hi_of[i] = -INFINITY;
+                 return !no;
+             },
+             [&](uint32_t i) {
+                 const uint32_t h = list[i], l = keys[h];
+                 bool need = false;
+                 const Iv iv = interval_any_gain(a, l, l == mine, vals[h], deg, pe, al, &need);
+                 if (l == mine) {
+                     s_own = own_sign_known(iv, need) ? 1 : 2;
+                     s_own_lo = iv.lo;
+                     s_own_hi = iv.hi;
+                     s_own_i = i;
+                     hi_of[i] = -INFINITY;
+                 } else if (need) {
+                     s_need = 1;
+                     hi_of[i] = INFINITY;
+                 } else {
+                     if (iv.lo > m || (iv.lo == m && l < m_label)) {
+                         m = iv.lo;
+                         m_hi = iv.hi;
+                         m_label = l;
+                     }
+                     mh = fmaxf(mh, iv.hi);
+                     hi_of[i] = iv.hi;
+                 }
+             });
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         const float om = __shfl_xor_sync(FULL, m, o), omh = __shfl_xor_sync(FULL, m_hi, o);
