@@ -6,12 +6,13 @@
 // (row lengths, offsets, one scatter) and then every row is sorted on its own:
 //   rows of length <= 512     a warp, bitonic network in registers and
 //                             shuffles (1, 2, 4, 8 or 16 values per lane);
-//   513 .. 4096, .. 16384     a CTA, 8 or 16 values per thread: the stages
-//                             whose partner is in the same warp in registers
-//                             and shuffles, the cross-warp ones in shared memory;
-//   longer rows               one radix sort of (row rank, value) keys.
-// With de-duplication a repeated value of a row becomes INVALID and the number
-// of distinct values of the row is written out; the caller compacts.
+//   513 .. 4096               a CTA, radix sort in shared memory (as many
+//                             8-bit passes as the row numbers have bytes);
+//   longer rows               a CTA sets a bit per value in a shared bitmap of
+//                             the row numbers and reads it back in order.
+// With de-duplication a repeated value of a row becomes INVALID (anywhere in the
+// row) and the number of distinct values of the row is written out; the callers
+// skip the holes.
 #include "engine.cuh"
 #include "lists.cuh"
 
@@ -20,7 +21,7 @@ namespace scd {
 namespace {
 
 constexpr unsigned TPB = 256;
-constexpr uint32_t WARP_ROW = 32, MID_ROW = 512, BIG_ROW = 4096, HUGE_ROW = 16384;
+constexpr uint32_t WARP_ROW = 32, MID_ROW = 512, HALF_ROW = 2048, BIG_ROW = 4096;
 
 __device__ __forceinline__ uint32_t bitonic32(uint32_t v, int lane) {
 #pragma unroll
@@ -113,113 +114,160 @@ k_sort_rows_warp_e(const uint32_t *__restrict__ list, uint32_t count, const uint
     }
 }
 
-// rows of one list, one CTA of W warps per row, E values per thread in index
-// order (value index = threadIdx.x * E + i); bitonic network over the next power
-// of two P >= len: stages with partner distance j < E in registers, E <= j < 32E
-// by shuffles, j >= 32E through shared memory (pairs enumerated directly)
-template <int W, int E>
-__global__ void __launch_bounds__(W * 32)
-k_sort_rows_cta(const uint32_t *__restrict__ list, uint32_t count, const uint32_t *__restrict__ off, uint32_t *vals,
-                bool dedup, uint32_t *udeg) {
-    constexpr int THREADS = W * 32;
-    constexpr uint32_t WSPAN = 32u * E;
-    extern __shared__ uint32_t sh[];   // THREADS * E values
-    __shared__ uint32_t wsum[W];
-    const uint32_t base = threadIdx.x * E;
+// rows of one list with len <= 256 * W: one CTA of W warps per row, LSD radix sort of the row
+// numbers (`bits` of them) in shared memory. (A bitonic network over 4096 values is 78
+// exchange stages, three radix passes are a third of its instructions; the counters of a
+// pass are W x 256 whatever the row's length, hence the two sizes. R-MAT scale 22, both
+// sorts, rows of 513 to 4096: 2.5 ms by the network, 2.2 with one size of 16 warps and ranks
+// by __match_any_sync, 1.66 ms so.)
+template <int W>
+__global__ void __launch_bounds__(W * 32, 64 / W)
+k_sort_rows_radix(const uint32_t *__restrict__ list, uint32_t count, const uint32_t *__restrict__ off, int bits,
+                  uint32_t *vals, bool dedup, uint32_t *udeg) {
+    __shared__ uint32_t cnt[W][256];
+    __shared__ uint32_t start[256], sw[RS_WARPS], sh[W * 32 * RS_ITEMS], kept_at[W];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int width = (bits + (bits + 7) / 8 - 1) / ((bits + 7) / 8);   // even digits
     for (uint32_t i = blockIdx.x; i < count; i += gridDim.x) {
         const uint32_t r = list[i], beg = off[r], len = off[r + 1] - beg;
-        uint32_t P = WSPAN;
-        while (P < len) P <<= 1;
-        for (uint32_t t = threadIdx.x; t < P; t += THREADS) sh[t] = t < len ? vals[beg + t] : INVALID;
-        __syncthreads();
-        uint32_t v[E];
+        const uint32_t items = (len + (W * 32) - 1) / (W * 32), first = warp * 32 * items + lane;
+        uint32_t key[RS_ITEMS], rank[RS_ITEMS];
 #pragma unroll
-        for (int e = 0; e < E; e++) v[e] = base + e < P ? sh[base + e] : INVALID;
-        const bool live = base < P;   // warp-uniform: P is a multiple of the warp span
-        for (uint32_t k = 2; k <= P; k <<= 1) {
-            if (k > WSPAN) {   // distances j >= 32E: shared memory
+        for (int k = 0; k < RS_ITEMS; k++)
+            key[k] = (uint32_t)k < items && first + k * 32 < len ? vals[beg + first + k * 32] : 0u;
+        for (int b = 0; b < bits; b += width) {
+            const unsigned mask = (1u << min(width, bits - b)) - 1u;
+            const uint32_t total = rs_rank<W>(key, len, items, b, mask, cnt, rank);
+            const uint32_t at = rs_scan256(total, sw);
+            if (threadIdx.x < 256) start[threadIdx.x] = at;
+            __syncthreads();
+#pragma unroll
+            for (int k = 0; k < RS_ITEMS; k++)
+                if ((uint32_t)k < items && first + k * 32 < len) {
+                    const unsigned d = (key[k] >> b) & mask;
+                    sh[start[d] + cnt[warp][d] + rank[k]] = key[k];
+                }
+            __syncthreads();
+            if (b + width < bits) {
+#pragma unroll
+                for (int k = 0; k < RS_ITEMS; k++)
+                    if ((uint32_t)k < items && first + k * 32 < len) key[k] = sh[first + k * 32];
                 __syncthreads();
-#pragma unroll
-                for (int e = 0; e < E; e++)
-                    if (live) sh[base + e] = v[e];
-                __syncthreads();
-                for (uint32_t j = k >> 1; j >= WSPAN; j >>= 1) {
-                    for (uint32_t q = threadIdx.x; q < P / 2; q += THREADS) {
-                        const uint32_t t = ((q & ~(j - 1)) << 1) | (q & (j - 1)), x = t | j;
-                        const uint32_t a = sh[t], b = sh[x];
-                        if ((a > b) == ((t & k) == 0)) {
-                            sh[t] = b;
-                            sh[x] = a;
-                        }
-                    }
-                    __syncthreads();
-                }
-#pragma unroll
-                for (int e = 0; e < E; e++)
-                    if (live) v[e] = sh[base + e];
-            }
-            if (!live) continue;
-#pragma unroll
-            for (int j = 16 * E; j >= E; j >>= 1) {   // partner in lane ^ (j / E)
-                if ((uint32_t)j >= k) continue;
-#pragma unroll
-                for (int e = 0; e < E; e++) {
-                    const uint32_t idx = base + e;
-                    const uint32_t o = __shfl_xor_sync(FULL, v[e], j / E);
-                    const bool asc = (idx & k) == 0, low = (idx & j) == 0;
-                    v[e] = (low == asc) ? min(v[e], o) : max(v[e], o);
-                }
-            }
-#pragma unroll
-            for (int j = E / 2; j > 0; j >>= 1) {    // partner in this thread: e ^ j
-                if ((uint32_t)j >= k) continue;
-#pragma unroll
-                for (int e = 0; e < E; e++) {
-                    const int q = e ^ j;
-                    if (q > e) {
-                        const bool asc = ((base + e) & k) == 0;
-                        const uint32_t x = v[e], y = v[q];
-                        if ((x > y) == asc) {
-                            v[e] = y;
-                            v[q] = x;
-                        }
-                    }
-                }
             }
         }
-        __syncthreads();
-#pragma unroll
-        for (int e = 0; e < E; e++)
-            if (live) sh[base + e] = v[e];
-        __syncthreads();
         uint32_t kept = 0;
-        for (uint32_t t = threadIdx.x; t < len; t += THREADS) {
+        for (uint32_t t = threadIdx.x; t < len; t += W * 32) {
             const uint32_t v = sh[t];
             const bool keep = !dedup || t == 0 || v != sh[t - 1];
             vals[beg + t] = keep ? v : INVALID;
             kept += keep;
         }
         kept = warp_sum(kept);
-        if ((threadIdx.x & 31) == 0) wsum[threadIdx.x >> 5] = kept;
+        if (lane == 0) kept_at[warp] = kept;
         __syncthreads();
         if (threadIdx.x == 0 && udeg) {
-            uint32_t tot = 0;
-            for (int w = 0; w < THREADS / 32; w++) tot += wsum[w];
-            udeg[r] = tot;
+            uint32_t t = 0;
+            for (int w = 0; w < W; w++) t += kept_at[w];
+            udeg[r] = t;
         }
         __syncthreads();
     }
 }
 
+// Rows of one list with len > 4096, all of distinct values or to be de-duplicated: one CTA per
+// row. A row's values, row numbers below nrows, set bits in a shared bitmap; the warps count
+// and then list its blocks of 32 words in turn, a word a lane (in turn, because the ids of
+// the densest part of a skewed graph are close together). The distinct values come first in
+// the row, INVALID after them. Bound by shared memory: a row costs len bit sets and twice
+// nrows/32 word reads, whatever its order; the network and radix passes it replaces cost
+// log^2 or five rounds of len (R-MAT scale 22, both sorts, rows above 4096: 3.3 -> 0.93 ms).
+// Row numbers beyond the bitmap are taken in ranges, each of which reads the row again
+// from its copy in `src` (src_off: the rows' places in it; nullptr: one range, from vals).
+constexpr int BITMAP_THREADS = 1024;
+constexpr uint32_t BITMAP_WORDS = 54 * 1024;   // 216 KB (at most two blocks of 32 a thread)
+constexpr uint32_t BITMAP_RANGES = 16;         // beyond: radix sort (every range walks the bitmap once more)
+static_assert(BITMAP_WORDS / 32 <= 2 * BITMAP_THREADS, "a scan of two counts a thread");
+constexpr size_t bitmap_bytes(uint64_t words) { return (words + words / 32) * 4; }
+
+__global__ void __launch_bounds__(BITMAP_THREADS)
+k_sort_rows_bitmap(const uint32_t *__restrict__ list, uint32_t count, const uint32_t *__restrict__ off, uint32_t nrows,
+                   uint32_t words, const uint32_t *__restrict__ src, const uint32_t *__restrict__ src_off,
+                   uint32_t *vals, uint32_t *udeg) {
+    extern __shared__ uint32_t bits[];   // words (a multiple of 32), then a count per block of 32 words
+    __shared__ uint32_t sw[BITMAP_THREADS / 32 + 1];
+    uint32_t *blk = bits + words;
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, blocks = words / 32;
+    for (uint32_t w = threadIdx.x; w < words; w += BITMAP_THREADS) bits[w] = 0;
+    __syncthreads();
+    for (uint32_t i = blockIdx.x; i < count; i += gridDim.x) {
+        const uint32_t r = list[i], beg = off[r], len = off[r + 1] - beg;
+        const uint32_t *row = src ? src + src_off[i] : vals + beg;
+        uint32_t done = 0;
+        for (uint64_t lo = 0; lo < nrows; lo += (uint64_t)words * 32) {
+#pragma unroll 4
+            for (uint32_t t = threadIdx.x; t < len; t += BITMAP_THREADS) {
+                const uint32_t v = row[t] - (uint32_t)lo;   // (below the range: wraps to above it)
+                if (v >> 5 < words) atomicOr(bits + (v >> 5), 1u << (v & 31));
+            }
+            __syncthreads();
+#pragma unroll 4
+            for (uint32_t b = warp; b < blocks; b += BITMAP_THREADS / 32) {
+                const uint32_t c = __reduce_add_sync(FULL, (uint32_t)__popc(bits[b * 32 + lane]));
+                if (lane == 0) blk[b] = c;
+            }
+            __syncthreads();
+            const uint32_t b0 = 2 * threadIdx.x, c0 = b0 < blocks ? blk[b0] : 0u, c1 = b0 + 1 < blocks ? blk[b0 + 1] : 0u;
+            uint32_t total;
+            const uint32_t at0 = block_exclusive_scan<BITMAP_THREADS>(c0 + c1, &total, sw);
+            if (b0 < blocks) blk[b0] = at0;
+            if (b0 + 1 < blocks) blk[b0 + 1] = at0 + c0;
+            __syncthreads();
+            for (uint32_t b = warp; b < blocks; b += BITMAP_THREADS / 32) {
+                uint32_t w = bits[b * 32 + lane];
+                if (!__any_sync(FULL, w != 0)) continue;
+                const uint32_t c = __popc(w);
+                uint32_t at = beg + done + blk[b] + warp_inclusive_scan(c) - c;
+                if (w) bits[b * 32 + lane] = 0;
+                for (; w; w &= w - 1) vals[at++] = (uint32_t)lo + (b * 32 + lane) * 32 + __ffs(w) - 1;
+            }
+            done += total;
+            __syncthreads();
+        }
+        for (uint32_t t = done + threadIdx.x; t < len; t += BITMAP_THREADS) vals[beg + t] = INVALID;
+        if (threadIdx.x == 0 && udeg) udeg[r] = done;
+    }
+}
+
+// the listed rows one after the other (koff: their places), in pieces of 4096 entries
+__global__ void k_copy_rows(const uint32_t *__restrict__ list, uint32_t count, const uint32_t *__restrict__ off,
+                            const uint32_t *__restrict__ koff, uint32_t total, const uint32_t *__restrict__ vals,
+                            uint32_t *out) {
+    constexpr uint32_t PIECE = 4096;
+    for (uint64_t p0 = (uint64_t)blockIdx.x * PIECE; p0 < total; p0 += (uint64_t)gridDim.x * PIECE) {
+        const uint32_t p1 = (uint32_t)min((uint64_t)total, p0 + PIECE);
+        uint32_t lo = 0, hi = count;   // last row that starts at or before p0
+        while (hi - lo > 1) {
+            const uint32_t mid = (lo + hi) >> 1;
+            if (koff[mid] <= p0) lo = mid;
+            else hi = mid;
+        }
+        for (uint32_t i = lo; i < count && koff[i] < p1; i++) {
+            const uint32_t beg = off[list[i]], k0 = koff[i], a = max((uint32_t)p0, k0), e = min(p1, koff[i + 1]);
+            for (uint32_t p = a + threadIdx.x; p < e; p += blockDim.x) out[p] = vals[beg + (p - k0)];
+        }
+    }
+}
+
 // the length classes of the longer rows: (32, 64], (64, 128], (128, 256], (256, 512],
-// (512, 4096], (4096, 16384] and above; shorter rows are in no class
+// (512, 2048], (2048, 4096] and above; shorter rows are in no class
 constexpr int ROW_CLASSES = 7;
 struct RowClassOf {
     const uint32_t *off;
     __device__ uint32_t operator[](size_t r) const {
         const uint32_t len = off[r + 1] - off[r];
         if (len <= WARP_ROW) return 0u;
-        return 1u << ((len > 64) + (len > 128) + (len > 256) + (len > MID_ROW) + (len > BIG_ROW) + (len > HUGE_ROW));
+        return 1u << ((len > 64) + (len > 128) + (len > 256) + (len > MID_ROW) + (len > HALF_ROW) +
+                     (len > BIG_ROW));
     }
 };
 
@@ -228,7 +276,8 @@ struct RowLenOf {
     __device__ uint32_t operator[](size_t i) const { return off[list[i] + 1] - off[list[i]]; }
 };
 
-// long rows: key = (rank of the row in the list) << vbits | value (values are row numbers, < 2^vbits)
+// long rows of a graph of very many rows: key = (rank of the row in the list) << vbits | value
+// (values are row numbers, < 2^vbits)
 template <typename K>
 __global__ void k_big_keys(const uint32_t *__restrict__ list, uint32_t count, const uint32_t *__restrict__ off,
                            const uint32_t *__restrict__ koff, const uint32_t *__restrict__ vals, int vbits, K *keys) {
@@ -280,8 +329,8 @@ void prepare_sort_kernels() {
     int dev = 0;
     CK(cudaGetDevice(&dev));
     if (done_device == dev) return;
-    CK(cudaFuncSetAttribute((const void *)k_sort_rows_cta<32, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                            (int)(HUGE_ROW * 4)));
+    CK(cudaFuncSetAttribute((const void *)k_sort_rows_bitmap, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                            (int)bitmap_bytes(BITMAP_WORDS)));
     done_device = dev;
 }
 
@@ -331,30 +380,52 @@ void sort_rows(Ctx &c, const uint32_t *off, uint32_t nrows, uint32_t *vals, bool
         CK_LAUNCH("k_sort_rows_warp512");
         c.launches++;
     }
+    const int vbits = ceil_log2(nrows < 2 ? 2 : nrows);   // values are row numbers
     if (cnt[4]) {
-        k_sort_rows_cta<16, 8><<<grid_for(cnt[4], 1, 152 * 4), 512, BIG_ROW * 4, s>>>(list[4], cnt[4], off, vals,
-                                                                                    dedup, udeg);
-        CK_LAUNCH("k_sort_rows_cta4096");
+        k_sort_rows_radix<8><<<grid_for(cnt[4], 1, 152 * 8), 256, 0, s>>>(list[4], cnt[4], off, vbits, vals, dedup, udeg);
+        CK_LAUNCH("k_sort_rows_radix2048");
         c.launches++;
     }
     if (cnt[5]) {
-        k_sort_rows_cta<32, 16><<<grid_for(cnt[5], 1, 152 * 2), 1024, HUGE_ROW * 4, s>>>(list[5], cnt[5], off,
-                                                                                      vals, dedup, udeg);
-        CK_LAUNCH("k_sort_rows_cta16384");
+        k_sort_rows_radix<16><<<grid_for(cnt[5], 1, 152 * 4), 512, 0, s>>>(list[5], cnt[5], off, vbits, vals, dedup, udeg);
+        CK_LAUNCH("k_sort_rows_radix4096");
         c.launches++;
     }
-    if (cnt[6]) {
-        DevBuf<uint32_t> koff((size_t)cnt[6] + 1, s);
-        scan_exclusive<uint32_t>(RowLenOf{list[6], off}, koff.get(), cnt[6], s);
-        uint32_t total = 0;
-        CK(cudaMemcpyAsync(&total, koff.get() + cnt[6], 4, cudaMemcpyDeviceToHost, s));
-        CK(cudaStreamSynchronize(s));
-        // the keys are as wide as the row ranks and the values need: in 32 bits a pass moves half the bytes
-        const int vbits = ceil_log2(nrows < 2 ? 2 : nrows), bits = vbits + ceil_log2(cnt[6] < 2 ? 2 : cnt[6]);
-        if (bits <= 32) sort_big_rows<uint32_t>(list[6], cnt[6], off, koff.get(), total, vbits, bits, vals, dedup, udeg, s);
-        else sort_big_rows<uint64_t>(list[6], cnt[6], off, koff.get(), total, vbits, bits, vals, dedup, udeg, s);
-        c.launches += 3;
+    if (!cnt[6]) return;
+    const uint64_t words = ((uint64_t)nrows + 1023) / 1024 * 32, ranges = (words + BITMAP_WORDS - 1) / BITMAP_WORDS;
+    if (ranges == 1) {
+        int per_sm = 0;
+        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void *)k_sort_rows_bitmap, BITMAP_THREADS,
+                                                         bitmap_bytes(words)));
+        k_sort_rows_bitmap<<<grid_for(cnt[6], 1, 152 * (per_sm > 0 ? per_sm : 1)), BITMAP_THREADS, bitmap_bytes(words), s>>>(
+            list[6], cnt[6], off, nrows, (uint32_t)words, nullptr, nullptr, vals, udeg);
+        CK_LAUNCH("k_sort_rows_bitmap");
+        c.launches++;
+        return;
     }
+    DevBuf<uint32_t> koff((size_t)cnt[6] + 1, s);
+    scan_exclusive<uint32_t>(RowLenOf{list[6], off}, koff.get(), cnt[6], s);
+    uint32_t *htotal = c.host_u32 + HOST_PLAN;
+    CK(cudaMemcpyAsync(htotal, koff.get() + cnt[6], 4, cudaMemcpyDeviceToHost, s));
+    CK(cudaStreamSynchronize(s));
+    const uint32_t total = *htotal;
+    if (ranges <= BITMAP_RANGES) {
+        const uint32_t per_range = (uint32_t)((words / 32 + ranges - 1) / ranges * 32);   // even ranges
+        DevBuf<uint32_t> copy(total, s);
+        k_copy_rows<<<grid_for(total, 4096, 152 * 8), TPB, 0, s>>>(list[6], cnt[6], off, koff.get(), total, vals,
+                                                                copy.get());
+        CK_LAUNCH("k_copy_rows");
+        k_sort_rows_bitmap<<<grid_for(cnt[6], 1, 152), BITMAP_THREADS, bitmap_bytes(per_range), s>>>(
+            list[6], cnt[6], off, nrows, per_range, copy.get(), koff.get(), vals, udeg);
+        CK_LAUNCH("k_sort_rows_bitmap");
+        c.launches += 2;
+        return;
+    }
+    // the keys are as wide as the row ranks and the values need: in 32 bits a pass moves half the bytes
+    const int bits = vbits + ceil_log2(cnt[6] < 2 ? 2 : cnt[6]);
+    if (bits <= 32) sort_big_rows<uint32_t>(list[6], cnt[6], off, koff.get(), total, vbits, bits, vals, dedup, udeg, s);
+    else sort_big_rows<uint64_t>(list[6], cnt[6], off, koff.get(), total, vbits, bits, vals, dedup, udeg, s);
+    c.launches += 3;
 }
 
 }  // namespace scd

@@ -227,10 +227,8 @@ __global__ void __launch_bounds__(RS_THREADS) k_rs_upsweep(const K *keys, size_t
     for (int k = 0; k < RS_ITEMS; k++) {
         size_t idx = base + (size_t)k * 32 + lane;
         bool valid = idx < n;
-        unsigned d = valid ? (unsigned)(keys[idx] >> shift) & mask : 0xffffffffu;
-        unsigned peers = __match_any_sync(FULL, d);
-        if (valid && lane == __ffs(peers) - 1) cnt[warp][d] += __popc(peers);
-        __syncwarp();
+        unsigned d = valid ? (unsigned)(keys[idx] >> shift) & mask : 0u;
+        if (valid) atomicAdd(&cnt[warp][d], 1u);
     }
     __syncthreads();
     const int d = threadIdx.x;
@@ -240,22 +238,38 @@ __global__ void __launch_bounds__(RS_THREADS) k_rs_upsweep(const K *keys, size_t
     hist[tile_major ? (size_t)blockIdx.x * 256 + d : (size_t)d * tiles + blockIdx.x] = s;
 }
 
+// The lanes that hold the same digit (below mask + 1, a power of two) as this one, among the
+// lanes of `valid`: a vote per bit. (__match_any_sync goes once round per distinct value, and
+// the digits of a warp's 32 keys are nearly all distinct.)
+__device__ __forceinline__ unsigned same_digit(unsigned d, unsigned mask, unsigned valid) {
+    unsigned peers = valid;
+#pragma unroll
+    for (int b = 0; b < 8; b++) {
+        if (!((mask >> b) & 1u)) break;
+        const unsigned vote = __ballot_sync(FULL, (d >> b) & 1u);
+        peers &= (d >> b) & 1u ? vote : ~vote;
+    }
+    return peers;
+}
+
 // Stable rank of every key of a tile within its digit and warp (rank[k]); cnt[w][d] becomes
 // the digit's keys in the warps before w, returns the tile's keys of digit threadIdx.x.
 // `count` keys of the tile are valid.  Starts and ends with a barrier's worth of order.
-template <typename K>
-__device__ __forceinline__ uint32_t rs_rank(const K (&key)[RS_ITEMS], uint32_t count, int shift, unsigned mask,
-                                            uint32_t (&cnt)[RS_WARPS][256], uint32_t (&rank)[RS_ITEMS]) {
+// A warp's keys are `items` (<= RS_ITEMS) rounds of 32 consecutive ones from warp * 32 * items on.
+template <int WARPS, typename K>
+__device__ __forceinline__ uint32_t rs_rank(const K (&key)[RS_ITEMS], uint32_t count, uint32_t items, int shift,
+                                            unsigned mask, uint32_t (&cnt)[WARPS][256], uint32_t (&rank)[RS_ITEMS]) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const unsigned lt = lanemask_lt();
-    for (int i = threadIdx.x; i < RS_WARPS * 256; i += RS_THREADS) (&cnt[0][0])[i] = 0;
+    for (int i = threadIdx.x; i < WARPS * 256; i += WARPS * 32) (&cnt[0][0])[i] = 0;
     __syncthreads();
 #pragma unroll
     for (int k = 0; k < RS_ITEMS; k++) {
-        const bool valid = (uint32_t)(warp * 32 * RS_ITEMS + k * 32 + lane) < count;
-        const unsigned d = valid ? (unsigned)(key[k] >> shift) & mask : 0xffffffffu;
-        const unsigned peers = __match_any_sync(FULL, d);
-        const int leader = __ffs(peers) - 1;
+        if ((uint32_t)k >= items) break;
+        const bool valid = (uint32_t)(warp * 32 * items + k * 32 + lane) < count;
+        const unsigned d = valid ? (unsigned)(key[k] >> shift) & mask : 0u;
+        const unsigned peers = same_digit(d, mask, __ballot_sync(FULL, valid));   // (of an invalid lane: unused)
+        const int leader = (__ffs(peers) - 1) & 31;
         uint32_t before = 0;
         if (valid && lane == leader) {
             before = cnt[warp][d];
@@ -267,23 +281,25 @@ __device__ __forceinline__ uint32_t rs_rank(const K (&key)[RS_ITEMS], uint32_t c
     }
     __syncthreads();
     uint32_t total = 0;
+    if (WARPS == 8 || threadIdx.x < 256) {
 #pragma unroll
-    for (int w = 0; w < RS_WARPS; w++) {
-        const uint32_t c = cnt[w][threadIdx.x];
-        cnt[w][threadIdx.x] = total;
-        total += c;
+        for (int w = 0; w < WARPS; w++) {
+            const uint32_t c = cnt[w][threadIdx.x];
+            cnt[w][threadIdx.x] = total;
+            total += c;
+        }
     }
     return total;
 }
 
-// exclusive sum over the 256 threads (sw: RS_WARPS words)
+// exclusive sum over the first 256 threads (sw: RS_WARPS words; v is 0 in any others)
 __device__ __forceinline__ uint32_t rs_scan256(uint32_t v, uint32_t *sw) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t inc = warp_inclusive_scan(v);
-    if (lane == 31) sw[warp] = inc;
+    if (lane == 31 && warp < RS_WARPS) sw[warp] = inc;
     __syncthreads();
     uint32_t off = 0;
-    for (int w = 0; w < warp; w++) off += sw[w];
+    for (int w = 0; w < RS_WARPS && w < warp; w++) off += sw[w];
     __syncthreads();
     return off + inc - v;
 }
@@ -331,7 +347,7 @@ __global__ void __launch_bounds__(RS_THREADS, 4) k_rs_downsweep(const K *keys_in
     } else {
         glob[threadIdx.x] = hist[(size_t)threadIdx.x * tiles + blockIdx.x];
     }
-    const uint32_t total = rs_rank(key, count, shift, mask, cnt, rank);
+    const uint32_t total = rs_rank<RS_WARPS>(key, count, RS_ITEMS, shift, mask, cnt, rank);
     tile_start[threadIdx.x] = rs_scan256(total, sw);
     __syncthreads();
 #pragma unroll
@@ -382,7 +398,7 @@ __global__ void __launch_bounds__(RS_THREADS) k_rs_one(K *keys, uint32_t *vals, 
     }
     for (int b = begin_bit; b < end_bit; b += 8) {
         const unsigned mask = (1u << (end_bit - b < 8 ? end_bit - b : 8)) - 1u;
-        const uint32_t total = rs_rank(key, n, b, mask, cnt, rank);
+        const uint32_t total = rs_rank<RS_WARPS>(key, n, RS_ITEMS, b, mask, cnt, rank);
         tile_start[threadIdx.x] = rs_scan256(total, sw);
         __syncthreads();
 #pragma unroll
