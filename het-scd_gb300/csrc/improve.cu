@@ -293,18 +293,16 @@ __device__ __forceinline__ void process_candidates(const ImproveArgs &a, CandQue
 // whole chain list -> bounds, label, graph -> active -> neighbour -> its label: with one
 // resident round of warps it, and not the gains, set the time.)
 template <int G>
-__global__ void __launch_bounds__(TPB, 4)
-k_improve_group(const uint32_t *__restrict__ verts, uint32_t count, uint32_t take, ImproveArgs a) {
+__device__ __forceinline__ void improve_group(const uint32_t *__restrict__ verts, uint32_t count, uint32_t take,
+                                              uint32_t block, uint32_t blocks, CandQueue &q, const ImproveArgs &a) {
     constexpr int PER_WARP = 32 / G;
-    __shared__ CandQueue queues[TPB / 32];
     const int lane = threadIdx.x & 31, gl = lane % G, g0 = lane - gl;
     const unsigned gmask = (G == 32) ? FULL : (((1u << G) - 1u) << g0);
     const unsigned below = (1u << lane) - 1u;
-    CandQueue &q = queues[threadIdx.x >> 5];
     const Iv al = iv_of(a.alpha);
-    const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
+    const uint32_t warps = blocks * (TPB / 32);
     uint32_t cn = 0, vn = 0;   // warp-uniform
-    uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, here = 0, r0 = 0;
+    uint32_t w = (block * TPB + threadIdx.x) >> 5, here = 0, r0 = 0;
     uint32_t p = 0, mine = INVALID, gp = 0, beg = 0, deg = 0, x = INVALID, l_next = INVALID;
     bool live = false;
     const auto neighbour = [&](uint32_t row0) {   // of the group's vertex in the round from row0 on
@@ -374,6 +372,24 @@ k_improve_group(const uint32_t *__restrict__ verts, uint32_t count, uint32_t tak
         vn += __popc(vb);
         r0 += PER_WARP;
     }
+}
+
+// The three group classes in one launch, the longest rows' blocks first: a small graph's step
+// is a chain of launches, and a large one's classes fill each other's tails.
+struct GroupWork {
+    const uint32_t *verts[3];   // degree 17..32, 9..16, up to 8
+    uint32_t count[3], take[3], blocks[3];
+};
+
+__global__ void __launch_bounds__(TPB, 4) k_improve_groups(GroupWork w, ImproveArgs a) {
+    __shared__ CandQueue queues[TPB / 32];
+    CandQueue &q = queues[threadIdx.x >> 5];
+    uint32_t b = blockIdx.x;
+    if (b < w.blocks[0]) return improve_group<32>(w.verts[0], w.count[0], w.take[0], b, w.blocks[0], q, a);
+    b -= w.blocks[0];
+    if (b < w.blocks[1]) return improve_group<16>(w.verts[1], w.count[1], w.take[1], b, w.blocks[1], q, a);
+    b -= w.blocks[1];
+    improve_group<8>(w.verts[2], w.count[2], w.take[2], b, w.blocks[2], q, a);
 }
 
 // ---- degree 33 .. 256: one warp per vertex, (label, count) hash table -------
@@ -554,7 +570,7 @@ k_improve_warp(const uint32_t *__restrict__ verts, uint32_t count, uint32_t take
     __syncwarp();
     uint32_t cn = 0, vn = 0;   // warp-uniform
     const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
-    // as in k_improve_group, `take` vertices' bounds, labels and graphs are read in one step,
+    // as in improve_group, `take` vertices' bounds, labels and graphs are read in one step,
     // and the first neighbours of the next vertex are on their way while one is looked at
     uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     uint32_t my_p = 0, my_mine = INVALID, my_gp = 0, my_beg = 0, my_deg = 0;
@@ -965,15 +981,6 @@ uint32_t take_of(uint32_t count, uint32_t least, uint64_t warps) {
     return take;
 }
 
-template <int G>
-void launch_group(Ctx &c, const uint32_t *verts, uint32_t count, const ImproveArgs &a, cudaStream_t s) {
-    const uint32_t take = take_of(count, 32 / G, GROUP_GRID * (TPB / 32));
-    k_improve_group<G><<<grid_for(((uint64_t)count + take - 1) / take * 32, TPB, GROUP_GRID), TPB, 0, s>>>(verts, count,
-                                                                                                        take, a);
-    CK_LAUNCH("k_improve_group");
-    c.launches++;
-}
-
 template <int THREADS, uint32_t CAP>
 void launch_cta(const uint32_t *verts, uint32_t count, const ImproveArgs &a, cudaStream_t s, unsigned max_grid) {
     k_improve_cta<THREADS, CAP><<<grid_for(count, 1, max_grid), THREADS, cta_smem<THREADS, CAP>(), s>>>(verts, count, a);
@@ -1009,9 +1016,19 @@ void improve(Ctx &c, const uint32_t *labels, const Stats &st, uint32_t *next, bo
         CK(cudaEventRecord(c.aux_join, c.aux));
         c.launches++;
     }
-    if (k.count[0]) launch_group<8>(c, k.list[0], k.count[0], a, s);
-    if (k.count[1]) launch_group<16>(c, k.list[1], k.count[1], a, s);
-    if (k.count[2]) launch_group<32>(c, k.list[2], k.count[2], a, s);
+    GroupWork gw{};
+    for (int j = 0; j < 3; j++) {   // classes 2, 1, 0: groups of 32, 16 and 8 lanes
+        const uint32_t n = k.count[2 - j];
+        gw.verts[j] = k.list[2 - j];
+        gw.count[j] = n;
+        gw.take[j] = take_of(n, 1u << j, GROUP_GRID * (TPB / 32));
+        gw.blocks[j] = n ? grid_for(((uint64_t)n + gw.take[j] - 1) / gw.take[j] * 32, TPB, GROUP_GRID) : 0u;
+    }
+    if (const unsigned blocks = gw.blocks[0] + gw.blocks[1] + gw.blocks[2]) {
+        k_improve_groups<<<blocks, TPB, 0, s>>>(gw, a);
+        CK_LAUNCH("k_improve_groups");
+        c.launches++;
+    }
     if (k.count[3]) {
         const uint32_t take = take_of(k.count[3], 1, 152 * 7 * WWARPS);
         k_improve_warp<<<grid_for(((uint64_t)k.count[3] + take - 1) / take * 32, WWARPS * 32, 152 * 7), WWARPS * 32, 0, s>>>(

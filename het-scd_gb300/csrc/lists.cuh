@@ -20,35 +20,41 @@ constexpr uint32_t LISTS_TILE = LISTS_WARPS * 32 * LISTS_STEPS;
 constexpr int LISTS_ONE_WARPS = 32, LISTS_ONE_STEPS = 16;
 constexpr uint32_t LISTS_ONE = LISTS_ONE_WARPS * 32 * LISTS_ONE_STEPS;
 
-// The class masks of a warp's STEPS x 32 consecutive ids from `first` on (bit k: the
-// id is in class k), and in lane k < K the number of the warp's ids in class k.
+// The class masks of a warp's steps x 32 (steps <= STEPS) consecutive ids from `first` on (bit
+// k: the id is in class k), and in lane k < K the number of the warp's ids in class k. (A
+// vote for every class: a loop over only the classes that some lane has, its bound from a
+// warp reduction, lost list entries.)
 template <int K, int STEPS, typename F>
-__device__ __forceinline__ uint32_t warp_masks(F f, uint32_t n, uint32_t first, uint32_t (&m)[STEPS]) {
+__device__ __forceinline__ uint32_t warp_masks(F f, uint32_t n, uint32_t first, uint32_t steps, uint32_t (&m)[STEPS]) {
     static_assert(K <= 32, "a lane per class");
     const uint32_t lane = threadIdx.x & 31;
     uint32_t cnt = 0;
 #pragma unroll
     for (int i = 0; i < STEPS; i++) {
         const uint32_t id = first + i * 32 + lane;
-        m[i] = id < n ? f[id] : 0u;
+        m[i] = (uint32_t)i < steps && id < n ? f[id] : 0u;
     }
 #pragma unroll
-    for (int i = 0; i < STEPS; i++)
+    for (int i = 0; i < STEPS; i++) {
+        if ((uint32_t)i >= steps) break;
 #pragma unroll
         for (int k = 0; k < K; k++) {
             const uint32_t c = __popc(__ballot_sync(FULL, (m[i] >> k) & 1u));
             if (lane == (uint32_t)k) cnt += c;
         }
+    }
     return cnt;
 }
 
 // writes the warp's ids; lane k holds the list position of the warp's first id of class k
 template <int K, int STEPS>
-__device__ __forceinline__ void warp_scatter(uint32_t first, const uint32_t (&m)[STEPS], uint32_t pos, uint32_t *lists) {
+__device__ __forceinline__ void warp_scatter(uint32_t first, uint32_t steps, const uint32_t (&m)[STEPS], uint32_t pos,
+                                             uint32_t *lists) {
     const uint32_t lane = threadIdx.x & 31;
     const unsigned lt = lanemask_lt();
 #pragma unroll
-    for (int i = 0; i < STEPS; i++)
+    for (int i = 0; i < STEPS; i++) {
+        if ((uint32_t)i >= steps) break;
 #pragma unroll
         for (int k = 0; k < K; k++) {
             const unsigned b = __ballot_sync(FULL, (m[i] >> k) & 1u);
@@ -56,6 +62,7 @@ __device__ __forceinline__ void warp_scatter(uint32_t first, const uint32_t (&m)
             if ((m[i] >> k) & 1u) lists[p + __popc(b & lt)] = first + i * 32 + lane;
             if (lane == (uint32_t)k) pos += __popc(b);
         }
+    }
 }
 
 template <int K, typename F>
@@ -64,7 +71,7 @@ k_lists_count(F f, uint32_t n, uint32_t tiles, uint32_t *hist) {
     __shared__ uint32_t sm[LISTS_WARPS][K];
     const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     uint32_t m[LISTS_STEPS];
-    const uint32_t cnt = warp_masks<K>(f, n, blockIdx.x * LISTS_TILE + w * 32 * LISTS_STEPS, m);
+    const uint32_t cnt = warp_masks<K>(f, n, blockIdx.x * LISTS_TILE + w * 32 * LISTS_STEPS, LISTS_STEPS, m);
     if (lane < K) sm[w][lane] = cnt;
     __syncthreads();
     if (threadIdx.x < K) {
@@ -81,7 +88,7 @@ k_lists_scatter(F f, uint32_t n, uint32_t tiles, const uint32_t *__restrict__ at
     const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const uint32_t first = blockIdx.x * LISTS_TILE + w * 32 * LISTS_STEPS;
     uint32_t m[LISTS_STEPS];
-    const uint32_t cnt = warp_masks<K>(f, n, first, m);
+    const uint32_t cnt = warp_masks<K>(f, n, first, LISTS_STEPS, m);
     if (lane < K) sm[w][lane] = cnt;
     __syncthreads();
     if (threadIdx.x < K) {
@@ -94,7 +101,7 @@ k_lists_scatter(F f, uint32_t n, uint32_t tiles, const uint32_t *__restrict__ at
     }
     if (blockIdx.x == 0 && threadIdx.x <= K) bounds[threadIdx.x] = at[(size_t)threadIdx.x * tiles];
     __syncthreads();
-    warp_scatter<K>(first, m, lane < K ? sm[w][lane] : 0u, lists);
+    warp_scatter<K>(first, LISTS_STEPS, m, lane < K ? sm[w][lane] : 0u, lists);
 }
 
 // up to LISTS_ONE ids: counts and lists in one CTA
@@ -102,9 +109,10 @@ template <int K, typename F>
 __global__ void __launch_bounds__(LISTS_ONE_WARPS * 32)
 k_lists_one(F f, uint32_t n, uint32_t *lists, uint32_t *bounds) {
     __shared__ uint32_t sm[LISTS_ONE_WARPS][K], base[K + 1];
-    const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5, first = w * 32 * LISTS_ONE_STEPS;
+    const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const uint32_t steps = (n + LISTS_ONE_WARPS * 32 - 1) / (LISTS_ONE_WARPS * 32), first = w * 32 * steps;
     uint32_t m[LISTS_ONE_STEPS];
-    const uint32_t cnt = warp_masks<K>(f, n, first, m);
+    const uint32_t cnt = warp_masks<K>(f, n, first, steps, m);
     if (lane < K) sm[w][lane] = cnt;
     __syncthreads();
     if (threadIdx.x < K) {
@@ -127,7 +135,7 @@ k_lists_one(F f, uint32_t n, uint32_t *lists, uint32_t *bounds) {
         }
     }
     __syncthreads();
-    warp_scatter<K>(first, m, lane < K ? sm[w][lane] + base[lane] : 0u, lists);
+    warp_scatter<K>(first, steps, m, lane < K ? sm[w][lane] + base[lane] : 0u, lists);
 }
 
 // The K lists into `lists` (room for every membership), list k at

@@ -196,24 +196,40 @@ __device__ __forceinline__ double block_sum_fixed(double v, double *sh) {
 
 // Graph-aligned blocks: block b sums WCC_CHUNK consecutive vertices of graph
 // blk_gid[b], counted from that graph's first vertex, so every graph's sum has
-// the same shape as when the graph is processed alone.
-__global__ void __launch_bounds__(TPB)
+// the same shape as when the graph is processed alone: eight consecutive terms by one
+// thread, 32 threads by shuffles, eight warps in order. The terms themselves (a chain of
+// FP64 operations that ends in a division) are made two by a thread, not eight: a small graph
+// has few blocks, and the chains were its time (1000 vertices, one block: 15 -> 8 us).
+constexpr int WCC_TERM_THREADS = 1024;
+
+__global__ void __launch_bounds__(WCC_TERM_THREADS)
 k_wcc_partial(const uint32_t *__restrict__ fin_off, const uint32_t *__restrict__ blk_off,
               const uint32_t *__restrict__ blk_gid, const uint32_t *__restrict__ labels, Stats st,
               const int32_t *__restrict__ tri, const int32_t *__restrict__ tri_deg,
               const uint32_t *__restrict__ itcount, const int32_t *__restrict__ itdeg, double alpha,
               double *partial, const uint8_t *__restrict__ active) {
     __shared__ double sh[TPB / 32];
+    __shared__ double terms[WCC_CHUNK + WCC_CHUNK / WCC_ITEMS];   // a gap after every thread's eight: no bank conflicts
     const uint32_t g = blk_gid[blockIdx.x];
     if (active && !active[g]) return;   // a graph of the batch that stopped iterating
-    const uint32_t end = fin_off[g + 1];
-    const uint32_t base = fin_off[g] + (blockIdx.x - blk_off[g]) * WCC_CHUNK + threadIdx.x * WCC_ITEMS;
+    const uint32_t end = fin_off[g + 1], base = fin_off[g] + (blockIdx.x - blk_off[g]) * WCC_CHUNK;
+    for (uint32_t i = threadIdx.x; i < WCC_CHUNK; i += WCC_TERM_THREADS)
+        terms[i + i / WCC_ITEMS] =
+            base + i < end ? wcc_term(base + i, labels, st, tri, tri_deg, itcount, itdeg, alpha) : 0.0;
+    __syncthreads();
+    if (threadIdx.x >= TPB) return;
     double s = 0.0;
 #pragma unroll
-    for (int i = 0; i < WCC_ITEMS; i++)
-        if (base + i < end) s = dadd(s, wcc_term(base + i, labels, st, tri, tri_deg, itcount, itdeg, alpha));
-    double r = block_sum_fixed(s, sh);
-    if (threadIdx.x == 0) partial[blockIdx.x] = r;
+    for (int i = 0; i < WCC_ITEMS; i++) s = dadd(s, terms[threadIdx.x * (WCC_ITEMS + 1) + i]);   // (+ 0.0 past the end)
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s = dadd(s, __shfl_xor_sync(FULL, s, o));
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = s;
+    asm volatile("bar.sync 1, %0;" ::"n"(TPB) : "memory");   // the first TPB threads only
+    if (threadIdx.x == 0) {
+        double r = 0.0;
+        for (int w = 0; w < TPB / 32; w++) r = dadd(r, sh[w]);
+        partial[blockIdx.x] = r;
+    }
 }
 
 // one block per graph: fixed-order sum of the graph's partials, divided by its n
@@ -652,7 +668,7 @@ void launch_wcc(Ctx &c, const uint32_t *labels, const Stats &st, bool frozen_gra
     CK_LAUNCH("k_internal_degrees");
     c.launches++;
     if (b.blocks) {
-        k_wcc_partial<<<b.blocks, TPB, 0, s>>>(b.fin_off, b.blk_off, b.blk_gid, labels, st, g.tri, g.tri_deg,
+        k_wcc_partial<<<b.blocks, WCC_TERM_THREADS, 0, s>>>(b.fin_off, b.blk_off, b.blk_gid, labels, st, g.tri, g.tri_deg,
                                                c.itcount, c.itdeg, c.alpha, c.wcc_part, active);
         CK_LAUNCH("k_wcc_partial");
     }

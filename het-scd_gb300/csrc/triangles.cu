@@ -109,17 +109,15 @@ struct BucketMask {
 // least 4x longer than out(a) (a hub's) is not walked: every lane searches its
 // out(a) entry in out(b) instead (alen searches of log2 d+(b) steps).
 template <int G>
-__global__ void __launch_bounds__(256)
-k_tc_small(Oriented o, const uint32_t *__restrict__ verts, uint32_t nverts, Dir dir, LabelFilter lf,
-           uint32_t *tcount, uint8_t *flag) {
+__device__ __forceinline__ void tc_small(Oriented o, const uint32_t *__restrict__ verts, uint32_t nverts, Dir dir,
+                                         LabelFilter lf, uint32_t *tcount, uint8_t *flag, uint32_t block,
+                                         uint32_t blocks, uint32_t (&acc)[8][32]) {
     constexpr int PER_WARP = 32 / G;
-    __shared__ uint32_t acc[8][32];
     const uint32_t *labels = lf.labels;
     const int lane = threadIdx.x & 31, gl = lane % G, g0 = lane - gl, w = threadIdx.x >> 5;
     const unsigned gmask = (G == 32) ? FULL : (((1u << G) - 1u) << g0);
-    const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
-    for (uint32_t base = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * PER_WARP; base < nverts;
-         base += warps * PER_WARP) {
+    const uint32_t warps = blocks * 8;
+    for (uint32_t base = ((block * 256 + threadIdx.x) >> 5) * PER_WARP; base < nverts; base += warps * PER_WARP) {
         const uint32_t vi = base + lane / G;
         bool live = vi < nverts;
         const uint32_t a = live ? verts[vi] : 0u;
@@ -217,6 +215,23 @@ k_tc_small(Oriented o, const uint32_t *__restrict__ verts, uint32_t nverts, Dir 
         if (gl == 0 && hits) atomicAdd(tcount + a, hits);
         __syncwarp();
     }
+}
+
+// The three register-group buckets in one launch, the longest out-lists' blocks first
+struct SmallWork {
+    const uint32_t *verts[3];   // buckets 2, 1, 0: groups of 32, 16 and 8 lanes
+    uint32_t nverts[3], blocks[3];
+};
+
+__global__ void __launch_bounds__(256)
+k_tc_small(Oriented o, SmallWork w, Dir dir, LabelFilter lf, uint32_t *tcount, uint8_t *flag) {
+    __shared__ uint32_t acc[8][32];
+    uint32_t b = blockIdx.x;
+    if (b < w.blocks[0]) return tc_small<32>(o, w.verts[0], w.nverts[0], dir, lf, tcount, flag, b, w.blocks[0], acc);
+    b -= w.blocks[0];
+    if (b < w.blocks[1]) return tc_small<16>(o, w.verts[1], w.nverts[1], dir, lf, tcount, flag, b, w.blocks[1], acc);
+    b -= w.blocks[1];
+    tc_small<8>(o, w.verts[2], w.nverts[2], dir, lf, tcount, flag, b, w.blocks[2], acc);
 }
 
 // Warp units.  Per warp: table of TCAP (key, index) entries, LCAP counters.
@@ -1066,22 +1081,15 @@ void count_triangles(Ctx &c, const Oriented &o, const TcPlan &plan, LabelFilter 
     CK(cudaMemsetAsync(ctr, 0, 24, s));
     const Dir dir{plan.dir_lo, plan.dir_hi, plan.dir_amin};
     const bool core = plan.nverts[5] && plan.core_n && !labels.labels;
-    if (plan.nverts[0]) {
-        k_tc_small<8><<<grid_for((uint64_t)plan.nverts[0] * 8, 256, 152 * 8), 256, 0, s>>>(
-            o, plan.verts[0], plan.nverts[0], dir, labels, tcount, flag);
-        CK_LAUNCH("k_tc_small8");
-        c.launches++;
+    SmallWork sw{};
+    for (int j = 0; j < 3; j++) {
+        sw.verts[j] = plan.verts[2 - j];
+        sw.nverts[j] = plan.nverts[2 - j];
+        sw.blocks[j] = sw.nverts[j] ? grid_for((uint64_t)sw.nverts[j] * (32 >> j), 256, 152 * 8) : 0u;
     }
-    if (plan.nverts[1]) {
-        k_tc_small<16><<<grid_for((uint64_t)plan.nverts[1] * 16, 256, 152 * 8), 256, 0, s>>>(
-            o, plan.verts[1], plan.nverts[1], dir, labels, tcount, flag);
-        CK_LAUNCH("k_tc_small16");
-        c.launches++;
-    }
-    if (plan.nverts[2]) {
-        k_tc_small<32><<<grid_for((uint64_t)plan.nverts[2] * 32, 256, 152 * 8), 256, 0, s>>>(
-            o, plan.verts[2], plan.nverts[2], dir, labels, tcount, flag);
-        CK_LAUNCH("k_tc_small32");
+    if (const unsigned blocks = sw.blocks[0] + sw.blocks[1] + sw.blocks[2]) {
+        k_tc_small<<<blocks, 256, 0, s>>>(o, sw, dir, labels, tcount, flag);
+        CK_LAUNCH("k_tc_small");
         c.launches++;
     }
     if (plan.nverts[3]) {
