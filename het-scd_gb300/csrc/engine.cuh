@@ -113,6 +113,7 @@ struct Oriented {
     // ibeg, beg is the offset array of a symmetric CSR whose rows hold the
     // out-list first and the in-list after it
     const uint32_t *ibeg = nullptr, *ilen = nullptr, *iadj = nullptr;
+    Spread at;   // where a vertex's triangle count lies in tcount
     __device__ __forceinline__ uint32_t in_beg(uint32_t u) const { return ibeg ? ibeg[u] : beg[u] + len[u]; }
     __device__ __forceinline__ uint32_t in_len(uint32_t u) const {
         return ibeg ? ilen[u] : beg[u + 1] - beg[u] - len[u];
@@ -200,7 +201,7 @@ void tc_dense_count(Ctx &c, const Oriented &o, const TcPlan &plan, uint32_t *tco
 // the plan of a full count (preprocessing) over out-lists o.adj[0..slots) with in-list
 // centres: the core split and its core map, or the hash kernels' split
 void tc_plan_counting(Ctx &c, const Oriented &o, uint64_t slots, TcPlan &plan, cudaStream_t s);
-// tcount[v] += triangles at v; flag[slot] = 1 for out-slots on a triangle.
+// tcount[o.at(v)] += triangles at v; flag[slot] = 1 for out-slots on a triangle.
 // With labels: internal triangles only.  tcount and flag must be zeroed.
 // Sorts every row of a CSR (offsets off[nrows+1], values vals) ascending in place;
 // with dedup, repeated values of a row become INVALID and udeg[r] receives the

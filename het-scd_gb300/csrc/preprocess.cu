@@ -60,26 +60,26 @@ __global__ void k_rename(uint32_t *first, uint32_t n_raw, const uint32_t *__rest
 
 // row lengths of the renamed, loop-free pairs in both directions
 __global__ void k_pair_degrees(const uint32_t *__restrict__ pairs, uint64_t count, const uint32_t *__restrict__ rename,
-                               uint32_t *cnt) {
+                               Spread at, uint32_t *cnt) {
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < count;
          i += (uint64_t)gridDim.x * blockDim.x) {
         const uint32_t a = rename[pairs[2 * i]], b = rename[pairs[2 * i + 1]];
         if (a != b) {   // (input lists are often sorted by the first id: aggregate its increments)
-            warp_atomic_inc(cnt + a, __activemask());
-            atomicAdd(cnt + b, 1u);
+            warp_atomic_inc(cnt + at(a), __activemask());
+            atomicAdd(cnt + at(b), 1u);
         }
     }
 }
 
 // both directions of every pair into their rows (order inside a row is fixed by the row sort)
 __global__ void k_pair_fill(const uint32_t *__restrict__ pairs, uint64_t count, const uint32_t *__restrict__ rename,
-                            const uint32_t *__restrict__ off, uint32_t *fill, uint32_t *vals) {
+                            const uint32_t *__restrict__ off, Spread at, uint32_t *fill, uint32_t *vals) {
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < count;
          i += (uint64_t)gridDim.x * blockDim.x) {
         const uint32_t a = rename[pairs[2 * i]], b = rename[pairs[2 * i + 1]];
         if (a != b) {
-            vals[off[a] + warp_atomic_inc(fill + a, __activemask())] = b;
-            vals[off[b] + atomicAdd(fill + b, 1u)] = a;
+            vals[off[a] + warp_atomic_inc(fill + at(a), __activemask())] = b;
+            vals[off[b] + atomicAdd(fill + at(b), 1u)] = a;
         }
     }
 }
@@ -231,20 +231,23 @@ __global__ void k_in_len(const uint32_t *__restrict__ deg, const uint32_t *__res
 
 // tri_deg[v] = number of v's edges that lie on a triangle (src/convert.cpp:327-340)
 __global__ void k_flag_degrees(const uint32_t *__restrict__ orow, const uint32_t *__restrict__ ocol,
-                               const uint8_t *__restrict__ flag, uint32_t count, int32_t *tri_deg) {
+                               const uint8_t *__restrict__ flag, uint32_t count, Spread at, uint32_t *tri_deg) {
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
         if (flag[i]) {   // out-slots are grouped by row: one atomic per row and warp for that side
-            warp_atomic_inc((uint32_t *)(tri_deg + orow[i]), __activemask());
-            atomicAdd(tri_deg + ocol[i], 1);
+            warp_atomic_inc(tri_deg + at(orow[i]), __activemask());
+            atomicAdd(tri_deg + at(ocol[i]), 1u);
         }
     }
 }
 
 // tri[v] = sum of the per-edge counts at v = 2 x triangles at v, in int32
-// two's-complement arithmetic like the reference's int accumulator
-__global__ void k_tri_from_count(const uint32_t *__restrict__ tcount, uint32_t n, int32_t *tri) {
-    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x)
+// two's-complement arithmetic like the reference's int accumulator; tri_deg in id order
+__global__ void k_tri_from_count(SpreadCounters tcount, SpreadCounters deg, uint32_t n, int32_t *tri,
+                                 int32_t *tri_deg) {
+    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
         tri[v] = (int32_t)(2u * tcount[v]);
+        tri_deg[v] = (int32_t)deg[v];
+    }
 }
 
 // the n2 kept vertices (tri_deg > 0) in descending id order (kscan: their positions in
@@ -277,12 +280,12 @@ __global__ void k_rank_of(const uint32_t *__restrict__ order, uint32_t n2, const
 // the kept (flagged) edges in rank ids into the rows of the final CSR, both directions
 __global__ void k_final_fill(const uint32_t *__restrict__ orow, const uint32_t *__restrict__ ocol,
                              const uint8_t *__restrict__ flag, uint32_t count, const uint32_t *__restrict__ rank,
-                             const uint32_t *__restrict__ ind, uint32_t *fill, uint32_t *adj) {
+                             const uint32_t *__restrict__ ind, Spread at, uint32_t *fill, uint32_t *adj) {
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
         if (flag[i]) {
             const uint32_t a = rank[orow[i]], b = rank[ocol[i]];
-            adj[ind[a] + warp_atomic_inc(fill + a, __activemask())] = b;
-            adj[ind[b] + atomicAdd(fill + b, 1u)] = a;
+            adj[ind[a] + warp_atomic_inc(fill + at(a), __activemask())] = b;
+            adj[ind[b] + atomicAdd(fill + at(b), 1u)] = a;
         }
     }
 }
@@ -493,15 +496,16 @@ void convert_edges(Ctx &c, const uint32_t *pairs_in, uint64_t count, const std::
     }
 
     // 2. de-duplicated symmetric CSR over the renamed ids: rows by a counting sort, then sorted row by row
-    DevBuf<uint32_t> cnt(n1, s), off1((size_t)n1 + 1, s);
-    CK(cudaMemsetAsync(cnt.get(), 0, (size_t)n1 * 4, s));
-    k_pair_degrees<<<G, TPB, 0, s>>>(pairs, count, rename.get(), cnt.get());
+    const Spread at1(n1, NG == 1);
+    DevBuf<uint32_t> cnt(at1.size(), s), off1((size_t)n1 + 1, s);
+    CK(cudaMemsetAsync(cnt.get(), 0, at1.size() * 4, s));
+    k_pair_degrees<<<G, TPB, 0, s>>>(pairs, count, rename.get(), at1, cnt.get());
     CK_LAUNCH("k_pair_degrees");
-    scan_exclusive<uint32_t>((const uint32_t *)cnt.get(), off1.get(), n1, s);
+    scan_exclusive<uint32_t>(SpreadCounters{cnt.get(), at1}, off1.get(), n1, s);
     const uint32_t entries = read_scalar(off1.get() + n1, s);
     DevBuf<uint32_t> vals(entries ? entries : 1, s);
-    CK(cudaMemsetAsync(cnt.get(), 0, (size_t)n1 * 4, s));
-    k_pair_fill<<<G, TPB, 0, s>>>(pairs, count, rename.get(), off1.get(), cnt.get(), vals.get());
+    CK(cudaMemsetAsync(cnt.get(), 0, at1.size() * 4, s));
+    k_pair_fill<<<G, TPB, 0, s>>>(pairs, count, rename.get(), off1.get(), at1, cnt.get(), vals.get());
     CK_LAUNCH("k_pair_fill");
     rename.release();
     sort_rows(c, off1.get(), n1, vals.get(), true, cnt.get(), s);   // cnt := distinct values of each row
@@ -545,11 +549,11 @@ void convert_edges(Ctx &c, const uint32_t *pairs_in, uint64_t count, const std::
     DevBuf<uint32_t> ilen(n1, s);
     k_in_len<<<grid_for(n1, TPB), TPB, 0, s>>>(cnt.get(), olen.get(), n1, ilen.get());
     CK_LAUNCH("k_in_len");
-    DevBuf<uint32_t> tcount(n1, s);
+    DevBuf<uint32_t> tcount(at1.size(), s);
     DevBuf<uint8_t> oflag(m1, s);
-    CK(cudaMemsetAsync(tcount.get(), 0, (size_t)n1 * 4, s));
+    CK(cudaMemsetAsync(tcount.get(), 0, at1.size() * 4, s));
     CK(cudaMemsetAsync(oflag.get(), 0, m1, s));
-    Oriented o{obeg.get(), olen.get(), ocol.get(), n1, ibeg.get(), ilen.get(), icol.get()};
+    Oriented o{obeg.get(), olen.get(), ocol.get(), n1, ibeg.get(), ilen.get(), icol.get(), at1};
     {
         TcPlan plan;
         tc_dense_setup(c, o, cnt.get(), core_members, core_bound, plan.dense, s);
@@ -561,11 +565,14 @@ void convert_edges(Ctx &c, const uint32_t *pairs_in, uint64_t count, const std::
     ibeg.release();
     ilen.release();
     DevBuf<int32_t> tri1(n1, s), tdeg1(n1, s);
-    CK(cudaMemsetAsync(tdeg1.get(), 0, (size_t)n1 * 4, s));
-    k_tri_from_count<<<grid_for(n1, TPB), TPB, 0, s>>>(tcount.get(), n1, tri1.get());
-    CK_LAUNCH("k_tri_from_count");
-    k_flag_degrees<<<grid_for(m1, TPB), TPB, 0, s>>>(orow.get(), ocol.get(), oflag.get(), m1, tdeg1.get());
+    DevBuf<uint32_t> sdeg(at1.size(), s);
+    CK(cudaMemsetAsync(sdeg.get(), 0, at1.size() * 4, s));
+    k_flag_degrees<<<grid_for(m1, TPB), TPB, 0, s>>>(orow.get(), ocol.get(), oflag.get(), m1, at1, sdeg.get());
     CK_LAUNCH("k_flag_degrees");
+    k_tri_from_count<<<grid_for(n1, TPB), TPB, 0, s>>>(SpreadCounters{tcount.get(), at1}, SpreadCounters{sdeg.get(), at1}, n1,
+                                                       tri1.get(), tdeg1.get());
+    CK_LAUNCH("k_tri_from_count");
+    sdeg.release();
     tcount.release();
     obeg.release();
     olen.release();
@@ -615,10 +622,11 @@ void convert_edges(Ctx &c, const uint32_t *pairs_in, uint64_t count, const std::
     c.b.h_fin_off.resize(NG + 1);
     CK(cudaMemcpyAsync(c.b.h_fin_off.data(), c.b.fin_off, 4 * (NG + 1), cudaMemcpyDeviceToHost, s));
     if (m2 > 0) {
-        DevBuf<uint32_t> fill(n2, s);
-        CK(cudaMemsetAsync(fill.get(), 0, (size_t)n2 * 4, s));
+        const Spread at2(n2, NG == 1);
+        DevBuf<uint32_t> fill(at2.size(), s);
+        CK(cudaMemsetAsync(fill.get(), 0, at2.size() * 4, s));
         k_final_fill<<<grid_for(m1, TPB), TPB, 0, s>>>(orow.get(), ocol.get(), oflag.get(), m1, rank.get(), g.indices,
-                                                      fill.get(), g.adj);
+                                                      at2, fill.get(), g.adj);
         CK_LAUNCH("k_final_fill");
         sort_rows(c, g.indices, n2, g.adj, false, nullptr, s);
         c.launches++;

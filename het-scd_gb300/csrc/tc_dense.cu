@@ -395,7 +395,7 @@ k_tc_fringe(Oriented o, const uint32_t *__restrict__ va, uint32_t na, const uint
             const uint32_t t = row_counts<Q>(ra, bits, c, who);
             if (c != INVALID && t) {
                 flag[beg + j] = 1;
-                atomicAdd(tcount + b, t);
+                atomicAdd(tcount + o.at(b), t);
                 total += t;
             }
             // open edges of b that end at another of a's members lie on a triangle with a
@@ -409,15 +409,15 @@ k_tc_fringe(Oriented o, const uint32_t *__restrict__ va, uint32_t na, const uint
             }
         }
         total = warp_sum(total);   // every triangle at a is counted at both of its edges there
-        if (lane == 0 && total) atomicAdd(tcount + a, total / 2);
+        if (lane == 0 && total) atomicAdd(tcount + o.at(a), total / 2);
     }
 }
 
 // the triangles at a member: half the counts of its edges
 __global__ void k_dense_counts(const uint32_t *__restrict__ verts, uint32_t k, const uint32_t *__restrict__ sums,
-                               uint32_t *tcount) {
+                               Spread at, uint32_t *tcount) {
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < k; i += gridDim.x * blockDim.x)
-        if (sums[i]) atomicAdd(tcount + verts[i], sums[i] / 2);
+        if (sums[i]) atomicAdd(tcount + at(verts[i]), sums[i] / 2);
 }
 
 template <typename F>
@@ -512,7 +512,7 @@ void tc_dense_count(Ctx &c, const Oriented &o, const TcPlan &plan, uint32_t *tco
     case 7: launch_dense<7>(o, d, plan, m, tcount, flag, ctr, s); break;
     default: launch_dense<8>(o, d, plan, m, tcount, flag, ctr, s); break;
     }
-    k_dense_counts<<<grid_for(d.n, 256), 256, 0, s>>>(d.verts.get(), d.n, sums.get(), tcount);
+    k_dense_counts<<<grid_for(d.n, 256), 256, 0, s>>>(d.verts.get(), d.n, sums.get(), o.at, tcount);
     CK_LAUNCH("k_dense_counts");
     c.launches += 6;
 }

@@ -7,7 +7,7 @@
 // (src/convert.cpp:290-340): tri[v] = sum of the per-edge counts at v =
 // 2 x (triangles at v), and tri_deg[v] and the filter need only whether an
 // edge's count is > 0.  So the kernels produce
-//   tcount[v]  triangles at v (tri = 2 tcount),
+//   tcount[o.at(v)]  triangles at v (tri = 2 tcount),
 //   flag[slot] 1 if the edge of that out-slot lies on a triangle,
 // and never a per-edge counter: the centre's, the partners' and the table
 // entries' counts and flags are aggregated in shared memory per work unit; the
@@ -207,12 +207,12 @@ __device__ __forceinline__ void tc_small(Oriented o, const uint32_t *__restrict_
         __syncwarp();
         const uint32_t hc = acc[w][lane] + selfc;
         if (hc && in_a) {
-            atomicAdd(tcount + x, hc);
+            atomicAdd(tcount + o.at(x), hc);
             flag[abeg + gl] = 1;
         }
 #pragma unroll
         for (int d = G / 2; d > 0; d >>= 1) hits += __shfl_xor_sync(FULL, hits, d);
-        if (gl == 0 && hits) atomicAdd(tcount + a, hits);
+        if (gl == 0 && hits) atomicAdd(tcount + o.at(a), hits);
         __syncwarp();
     }
 }
@@ -342,15 +342,15 @@ k_tc_warp(Oriented o, const uint32_t *__restrict__ verts, const uint32_t *__rest
         __syncwarp();
         const uint32_t hb = j < alen ? bhits[w][lane] : 0;
         if (hb) {
-            atomicAdd(tcount + b, hb);
+            atomicAdd(tcount + o.at(b), hb);
             flag[abeg + j] = 1;
         }
         const uint32_t sa = warp_sum(hb);
-        if (lane == 0 && sa) atomicAdd(tcount + a, sa);
+        if (lane == 0 && sa) atomicAdd(tcount + o.at(a), sa);
         for (uint32_t i = lane; i < alen; i += 32) {
             const uint32_t cc = cnt[w][i];
             if (cc) {
-                atomicAdd(tcount + o.adj[abeg + i], cc);
+                atomicAdd(tcount + o.at(o.adj[abeg + i]), cc);
                 flag[abeg + i] = 1;
             }
         }
@@ -511,18 +511,18 @@ k_tc_cta(Oriented o, const uint32_t *__restrict__ verts, const uint32_t *__restr
             __syncthreads();
             const uint32_t hb = j < pend ? bhits[threadIdx.x] : 0;
             if (hb) {
-                atomicAdd(tcount + y, hb);
+                atomicAdd(tcount + o.at(y), hb);
                 const uint32_t yb = o.beg[y];
                 flag[fwd ? xbeg + j : yb + lower_bound(o.adj + yb, o.len[y], x)] = 1;
             }
             xhits += hb;
         }
         const uint32_t sa = warp_sum(xhits);
-        if (lane == 0 && sa) atomicAdd(tcount + x, sa);
+        if (lane == 0 && sa) atomicAdd(tcount + o.at(x), sa);
         for (uint32_t i = threadIdx.x; i < xlen; i += THREADS) {
             const uint32_t cc = (cnt[i >> 1] >> ((i & 1) << 4)) & 0xffffu;
             if (cc) {
-                atomicAdd(tcount + o.adj[xbeg + i], cc);
+                atomicAdd(tcount + o.at(o.adj[xbeg + i]), cc);
                 flag[xbeg + i] = 1;
             }
         }
@@ -708,7 +708,7 @@ k_tc_core(Oriented o, const uint32_t *__restrict__ cpad, const uint32_t *__restr
             __syncthreads();
             const uint32_t hb = j < pend ? sh[threadIdx.x] : 0u;
             if (hb) {
-                atomicAdd(tcount + y, hb);
+                atomicAdd(tcount + o.at(y), hb);
                 flag[fwd ? xbeg + j : ob + lower_bound(o.adj + ob, wb, x)] = 1;
                 xh += hb;
             }
@@ -716,12 +716,12 @@ k_tc_core(Oriented o, const uint32_t *__restrict__ cpad, const uint32_t *__restr
         xh = warp_sum(xh);
         if (lane == 0 && xh) atomicAdd(&s_xhits, xh);
         __syncthreads();
-        if (threadIdx.x == 0 && s_xhits) atomicAdd(tcount + x, s_xhits);
+        if (threadIdx.x == 0 && s_xhits) atomicAdd(tcount + o.at(x), s_xhits);
         const uint32_t *xa = o.adj + xbeg;
         for (uint32_t i = threadIdx.x; i < xlen; i += THREADS) {
             const uint32_t cc = cnt[i];
             if (cc) {
-                atomicAdd(tcount + xa[i], cc);
+                atomicAdd(tcount + o.at(xa[i]), cc);
                 flag[xbeg + i] = 1;
             }
             const uint32_t c = xc[i];
@@ -782,15 +782,15 @@ k_tc_huge(Oriented o, const uint32_t *__restrict__ verts, uint32_t nverts, Label
                 const uint32_t ic = lower_bound(A, alen, c);
                 if (ic < alen && A[ic] == c && (!labels || labels[c] == la)) {
                     hits++;
-                    atomicAdd(tcount + c, 1u);
+                    atomicAdd(tcount + o.at(c), 1u);
                     flag[abeg + ic] = 1;
                     flag[bbeg + i] = 1;
                 }
             }
             hits = warp_sum(hits);
             if (lane == 0 && hits) {
-                atomicAdd(tcount + a, hits);
-                atomicAdd(tcount + b, hits);
+                atomicAdd(tcount + o.at(a), hits);
+                atomicAdd(tcount + o.at(b), hits);
                 flag[abeg + j] = 1;
             }
         }
