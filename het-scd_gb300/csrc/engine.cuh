@@ -137,6 +137,19 @@ struct DenseCore {
     DevBuf<uint32_t> verts, num;   // members ascending; number of each member (INVALID for the others)
     DevBuf<uint32_t> walk;         // out-degree of every vertex, 0 for members
 };
+// The vertices above the register groups' buckets by the length of their internal out-list,
+// listed anew for every labelling by the pass that makes the internal lists: a community
+// holds a few dozen of a hub's neighbours, so nearly all of them belong to a cheaper kernel
+// than their whole out-list's, or to none (fewer than two internal out-neighbours).
+// Measured, the CTA kernels of a step by whole out-lists -> by this list: R-MAT scale 22
+// 650 -> 4-21 us, scale 20 210 -> 5 us; 96 planted graphs (register groups only) unchanged.
+struct InternalWork {
+    static constexpr int K = 4;   // register groups, warp units, 128-thread CTA units, 256-thread CTA units
+    static constexpr uint32_t SMALL = 32, MID = 64, CTA = 1024, LONGEST = 8192, CHUNK = 512;
+    uint32_t *verts[K] = {}, *chunk[K] = {};   // chunk (CTA units only): 512 partners each
+    uint32_t *count = nullptr;                 // K words
+    // (out-lists above LONGEST keep k_tc_huge)
+};
 // out-degree buckets and their work-unit offsets (built once per oriented graph)
 // Bucket k lists its out-list centres first (nfwd[k] of them) and, for the CTA
 // buckets, then the in-list centres: a vertex b whose edges a -> b with
@@ -151,8 +164,6 @@ struct TcPlan {
     uint32_t dir_lo = 0, dir_hi = 0, dir_amin = 0;   // b-centric iff d+(a) < d+(b),
                                                       // dir_lo < d+(b) <= dir_hi, d+(a) > dir_amin
     DevBuf<uint32_t> tmp[4];   // storage when the plan is temporary: the lists, the unit offsets
-    // the buckets whose kernels take work units (unit_off is null for the others)
-    static constexpr bool has_units(int k) { return k >= 3 && k <= 5; }
     // Core map of the upper CTA bucket (tc_core_map): the vertices of degree >
     // cta_hi, numbered 0..core_n-1 in id order.  core_adj holds every out-list
     // in core numbers (core_n for a vertex outside the core), v's list at
@@ -181,12 +192,13 @@ void tc_core_map(Ctx &c, const Oriented &o, uint64_t slots, TcPlan &plan, uint32
                  cudaStream_t s);
 // tc_plan in two parts around a host read the caller shares with other reads: the
 // bucket lists with their bounds (TC_LISTS + 1 device words), then, given the
-// bounds on the host, the plan's pointers and the work-unit offsets
+// bounds on the host, the plan's pointers and (not owned: the WCC lists its units itself,
+// InternalWork) the work-unit offsets
 constexpr int TC_LISTS = TcPlan::K + 2;   // the two CTA buckets have an in-list part
 void tc_plan_lists(Ctx &c, const Oriented &o, TcPlan &plan, uint32_t *lists, uint32_t *bounds, cudaStream_t s,
                    bool in_lists, uint32_t core_from);
-void tc_plan_units(Ctx &c, const Oriented &o, TcPlan &plan, uint32_t *lists, const uint32_t *host_bounds,
-                   cudaStream_t s, bool owned);
+void tc_plan_units(const Oriented &o, TcPlan &plan, uint32_t *lists, const uint32_t *host_bounds, cudaStream_t s,
+                   bool owned);
 // out-degree up to which the walks take a vertex by register groups or a warp
 uint32_t tc_short_lists(const Ctx &c);
 // tc_dense.cu.  pick (2 device words): members and degree bound of the dense core worth
@@ -209,7 +221,11 @@ void tc_plan_counting(Ctx &c, const Oriented &o, uint64_t slots, TcPlan &plan, c
 void sort_rows(Ctx &c, const uint32_t *off, uint32_t nrows, uint32_t *vals, bool dedup, uint32_t *udeg,
                cudaStream_t s);
 void count_triangles(Ctx &c, const Oriented &o, const TcPlan &plan, LabelFilter labels, uint32_t *tcount,
-                     uint8_t *flag, cudaStream_t s, const char *phase = nullptr);
+                     uint8_t *flag, cudaStream_t s);
+// lists for the resident graph's WCC plan (InternalWork), and the count of the internal
+// out-lists o by that plan and those lists
+void alloc_internal_work(Ctx &c);
+void count_internal_triangles(Ctx &c, const Oriented &o, uint32_t *tcount, uint8_t *flag);
 // times the triangle-counting bucket splits on the resident graph, keeps the fastest
 double autotune_tc(Ctx &c, std::vector<std::string> *report);
 // set kernel attributes (dynamic shared memory) once per device, outside any capture
@@ -264,6 +280,7 @@ struct Ctx {
     uint32_t *int_len = nullptr;      // label-mode count: internal out-list lengths (n)
     uint32_t *int_adj = nullptr;      // and the internal out-lists at the CSR offsets (2m)
     TcPlan wplan;                     // triangle-counting plan of the resident graph
+    InternalWork iwork;
     double *wcc_part = nullptr, *wcc_host = nullptr;
     uint32_t *host_u32 = nullptr;     // pinned words: the active-graph count of an iteration at 0, planning reads from HOST_PLAN on
     char *io_buf[2] = {};             // pinned pieces of a graph file on its way to the device

@@ -529,10 +529,23 @@ template <bool LISTS, bool STATS>
 __global__ void __launch_bounds__(TPB)
 k_internal_lists(uint32_t n, uint32_t rows, WarpRows longer, uint32_t most_short,
                  const uint32_t *__restrict__ indices, const uint32_t *__restrict__ nlow, const uint32_t *__restrict__ adj, LabelFilter lf, uint32_t *ilen, uint32_t *iadj, uint8_t *flag,
-                 uint32_t *itcount, int32_t *itdeg, Stats st) {
+                 uint32_t *itcount, int32_t *itdeg, Stats st, InternalWork work) {
     const uint32_t lane = threadIdx.x & 31, gl = lane & 7, grp = lane >> 3;
     const uint32_t warps = (gridDim.x * blockDim.x) >> 5, units = (n + rows - 1) / rows;
     const unsigned gmask = 0xffu << (grp * 8), lt = (1u << lane) - 1u;
+    // entries of the work lists, a warp's 32 at a time (one atomic a vertex on one address would
+    // be the kernel's time): lane i of the pending ones holds entry i
+    uint32_t pend_v[InternalWork::K] = {}, pend_c[InternalWork::K] = {}, pend[InternalWork::K] = {};
+    const auto flush = [&](int k) {
+        uint32_t at = 0;
+        if (lane == 0) at = atomicAdd(work.count + k, pend[k]);
+        at = __shfl_sync(FULL, at, 0) + lane;
+        if (lane < pend[k]) {
+            work.verts[k][at] = pend_v[k];
+            if (k >= 2) work.chunk[k][at] = pend_c[k];
+        }
+        pend[k] = 0;
+    };
     for (uint32_t unit = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; unit < longer.total + units; unit += warps) {
         if (unit < longer.total) {
             const uint32_t v = longer[unit], l = lf.labels[v], beg = indices[v], len = nlow[v];
@@ -554,6 +567,21 @@ k_internal_lists(uint32_t n, uint32_t rows, WarpRows longer, uint32_t most_short
                 }
             }
             if (LISTS && lane == 0) ilen[v] = c;
+            if (LISTS && c >= 2 && len <= InternalWork::LONGEST) {
+                const uint32_t chunks = c <= InternalWork::MID ? 1u : (c + InternalWork::CHUNK - 1) / InternalWork::CHUNK;
+                for (uint32_t ch = 0; ch < chunks; ch++) {
+#pragma unroll
+                    for (int k = 0; k < InternalWork::K; k++) {
+                        const uint32_t kk = (c > InternalWork::SMALL) + (c > InternalWork::MID) + (c > InternalWork::CTA);
+                        if (kk != (uint32_t)k) continue;
+                        if (lane == pend[k]) {
+                            pend_v[k] = v;
+                            pend_c[k] = ch;
+                        }
+                        if (++pend[k] == 32) flush(k);
+                    }
+                }
+            }
             if (STATS && on && lane == 0) add_stats(st, l, indices[v + 1] - beg, c);
             continue;
         }
@@ -602,6 +630,11 @@ k_internal_lists(uint32_t n, uint32_t rows, WarpRows longer, uint32_t most_short
         }
         if (STATS && on) add_stats(st, l, deg, cnt);
     }
+    if (LISTS) {
+#pragma unroll
+        for (int k = 0; k < InternalWork::K; k++)
+            if (pend[k]) flush(k);
+    }
 }
 
 template <bool LISTS, bool STATS>
@@ -616,7 +649,7 @@ void launch_internal_lists(Ctx &c, LabelFilter lf, const Stats &st) {
     k_internal_lists<LISTS, STATS><<<grid_for((((uint64_t)g.n + rows - 1) / rows + longer.total) * 32, TPB,
                                               NUM_SMS_HINT * 16), TPB, 0, c.stream>>>(
         g.n, rows, longer, c.wplan.small_max, g.indices, g.nlow, g.adj, lf, c.int_len, c.int_adj, c.slot_flag, c.itcount,
-        c.itdeg, st);
+        c.itdeg, st, c.iwork);
     CK_LAUNCH("k_internal_lists");
 }
 
@@ -658,11 +691,12 @@ void launch_wcc(Ctx &c, const uint32_t *labels, const Stats &st, bool frozen_gra
     const Batch &b = c.b;
     const uint8_t *active = frozen_graphs ? b.active : nullptr;
     const LabelFilter lf{labels, b.gid, active};
+    CK(cudaMemsetAsync(c.work_counter, 0, 64, s));   // the lists' counts and the kernels' unit counters
     if (with_stats) launch_internal_lists<true, true>(c, lf, st);
     else launch_internal_lists<true, false>(c, lf, st);
     // the plan's buckets (by full out-degree) stay valid: internal lists are never longer
     const Oriented o{g.indices, c.int_len, c.int_adj, g.n};
-    count_triangles(c, o, c.wplan, LabelFilter{}, c.itcount, c.slot_flag, s, "wcc_tc");
+    count_internal_triangles(c, o, c.itcount, c.slot_flag);
     k_internal_degrees<<<grid_for(((uint64_t)(g.n + 31) / 32 + g.rows.nchunks) * 32, TPB), TPB, 0, s>>>(
         g.n, g.rows, g.indices, c.int_len, c.int_adj, c.slot_flag, c.itdeg, lf);
     CK_LAUNCH("k_internal_degrees");

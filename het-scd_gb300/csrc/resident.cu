@@ -104,8 +104,7 @@ UnionArrays arrays_of(const Ctx &c) {
 // The vertex lists of a union's structure, each sorted by vertex id (so each
 // graph's entries are one contiguous piece): the degree classes, the long rows,
 // the WCC triangle-counting buckets; with the offset array that goes with some
-// of them (table words of the last class, pieces of the long rows, work units of
-// the buckets).
+// of them (table words of the last class, pieces of the long rows).
 constexpr int NCLS = DegreeClasses::K, LONG = NCLS, BUCKET0 = NCLS + 1, NL = NCLS + 1 + TcPlan::K;
 struct UnionLists {
     const uint32_t *list[NL];
@@ -128,13 +127,12 @@ UnionLists lists_of(const Ctx &c) {
     for (int k = 0; k < TcPlan::K; k++) {
         L.list[BUCKET0 + k] = c.wplan.verts[k];
         L.count[BUCKET0 + k] = c.wplan.nverts[k];
-        L.off[BUCKET0 + k] = c.wplan.unit_off[k];
     }
     return L;
 }
 
 // A graph's share of each list: entries, and the span of the offsets (table
-// words, long-row pieces, work units) they cover.
+// words, long-row pieces) they cover.
 struct GraphLists {
     uint32_t cnt[NL] = {};
     uint64_t span[NL] = {};
@@ -495,8 +493,6 @@ uint32_t rebuild(Ctx &c, ResidentSet &R, std::vector<ResidentSource *> &srcs) {
         for (int l = 0; l < NL; l++) list[l] = c.alloc<uint32_t>(lcnt[l]);
         off[NCLS - 1] = c.alloc<uint64_t>(lcnt[NCLS - 1] + 1);
         off[LONG] = c.alloc<uint32_t>(lcnt[LONG] + 1);
-        for (int k = 0; k < TcPlan::K; k++)
-            if (TcPlan::has_units(k)) off[BUCKET0 + k] = c.alloc<uint32_t>(lcnt[BUCKET0 + k] + 1);
         for (int k = 0; k < NCLS; k++) {
             g.cls.list[k] = list[k];
             g.cls.count[k] = (uint32_t)lcnt[k];
@@ -511,10 +507,10 @@ uint32_t rebuild(Ctx &c, ResidentSet &R, std::vector<ResidentSource *> &srcs) {
         TcPlan &pl = c.wplan;
         for (int k = 0; k < TcPlan::K; k++) {
             pl.verts[k] = list[BUCKET0 + k];
-            pl.unit_off[k] = (uint32_t *)off[BUCKET0 + k];
             pl.nverts[k] = pl.nfwd[k] = (uint32_t)lcnt[BUCKET0 + k];
         }
         pl.small_max = R.split[0];
+        alloc_internal_work(c);
         pl.dir_lo = pl.dir_hi = 0;   // out-list centres only, as tc_plan builds the WCC plan
         pl.dir_amin = c.tc_amin < c.tc_small ? c.tc_amin : c.tc_small;
         // scratch of the iteration

@@ -99,6 +99,34 @@ struct BucketMask {
     }
 };
 
+// The work units of a kernel: those of a plan's bucket (unit_off), or a list made on the device
+// (count set): with `chunk` a (vertex, chunk) per entry, else `per` chunks of every vertex.
+struct UnitList {
+    const uint32_t *verts, *unit_off;
+    uint32_t nverts;
+    const uint32_t *count, *chunk;
+    uint32_t per;
+    __device__ __forceinline__ uint32_t total() const { return count ? *count * per : unit_off[nverts]; }
+    // vertex v, chunk ch and place vi in the list of a unit
+    __device__ __forceinline__ void find(uint32_t unit, uint32_t &vi, uint32_t &v, uint32_t &ch) const {
+        if (count) {
+            vi = unit / per;
+            v = verts[vi];
+            ch = chunk ? chunk[vi] : unit % per;
+            return;
+        }
+        uint32_t lo = 0, hi = nverts + 1;   // unit_off[vi] <= unit < unit_off[vi + 1]
+        while (lo < hi) {
+            const uint32_t mid = (lo + hi) >> 1;
+            if (unit_off[mid] <= unit) lo = mid + 1;
+            else hi = mid;
+        }
+        vi = lo - 1;
+        v = verts[vi];
+        ch = unit - unit_off[vi];
+    }
+};
+
 // Short out-lists (d+(a) <= G, G = 16 or 32): one group of G lanes per vertex
 // a, no table.  Lane i holds out(a)[i] in a register (out-lists are sorted
 // ascending); the (b, c in out(b)) items of a are flattened by a group scan
@@ -221,12 +249,16 @@ __device__ __forceinline__ void tc_small(Oriented o, const uint32_t *__restrict_
 struct SmallWork {
     const uint32_t *verts[3];   // buckets 2, 1, 0: groups of 32, 16 and 8 lanes
     uint32_t nverts[3], blocks[3];
+    const uint32_t *list, *count;   // and a list made on the device, groups of 32
+    uint32_t list_blocks;
 };
 
 __global__ void __launch_bounds__(256)
 k_tc_small(Oriented o, SmallWork w, Dir dir, LabelFilter lf, uint32_t *tcount, uint8_t *flag) {
     __shared__ uint32_t acc[8][32];
     uint32_t b = blockIdx.x;
+    if (b < w.list_blocks) return tc_small<32>(o, w.list, *w.count, dir, lf, tcount, flag, b, w.list_blocks, acc);
+    b -= w.list_blocks;
     if (b < w.blocks[0]) return tc_small<32>(o, w.verts[0], w.nverts[0], dir, lf, tcount, flag, b, w.blocks[0], acc);
     b -= w.blocks[0];
     if (b < w.blocks[1]) return tc_small<16>(o, w.verts[1], w.nverts[1], dir, lf, tcount, flag, b, w.blocks[1], acc);
@@ -237,8 +269,7 @@ k_tc_small(Oriented o, SmallWork w, Dir dir, LabelFilter lf, uint32_t *tcount, u
 // Warp units.  Per warp: table of TCAP (key, index) entries, LCAP counters.
 template <int WARPS, int TCAP, int LCAP, int FBITS>
 __global__ void __launch_bounds__(WARPS * 32)
-k_tc_warp(Oriented o, const uint32_t *__restrict__ verts, const uint32_t *__restrict__ unit_off, uint32_t nverts,
-          Dir dir, LabelFilter lf, uint32_t *tcount, uint8_t *flag, uint32_t *next_unit) {
+k_tc_warp(Oriented o, UnitList units, Dir dir, LabelFilter lf, uint32_t *tcount, uint8_t *flag, uint32_t *next_unit) {
     const uint32_t *labels = lf.labels;
     __shared__ uint32_t filt[WARPS][(1 << FBITS) / 32];
     __shared__ uint32_t keys[WARPS][TCAP];
@@ -246,20 +277,14 @@ k_tc_warp(Oriented o, const uint32_t *__restrict__ verts, const uint32_t *__rest
     __shared__ uint32_t cnt[WARPS][LCAP];
     __shared__ uint32_t pre[WARPS][32], bbase[WARPS][32], bhits[WARPS][32];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const uint32_t n_units = unit_off[nverts];
+    const uint32_t n_units = units.total();
     while (true) {
         uint32_t unit = 0;
         if (lane == 0) unit = atomicAdd(next_unit, 1u);
         unit = __shfl_sync(FULL, unit, 0);
         if (unit >= n_units) break;
-        uint32_t lo = 0, hi = nverts + 1;   // vertex index: unit_off[i] <= unit < unit_off[i+1]
-        while (lo < hi) {
-            const uint32_t mid = (lo + hi) >> 1;
-            if (unit_off[mid] <= unit) lo = mid + 1;
-            else hi = mid;
-        }
-        const uint32_t vi = lo - 1;
-        const uint32_t a = verts[vi], ch = unit - unit_off[vi];
+        uint32_t vi, a, ch;
+        units.find(unit, vi, a, ch);
         const uint32_t la = labels ? labels[a] : 0u;
         if (labels && (la == INVALID || lf.frozen(a))) continue;
         const uint32_t abeg = o.beg[a], alen = o.len[a];
@@ -376,8 +401,7 @@ k_tc_warp(Oriented o, const uint32_t *__restrict__ verts, const uint32_t *__rest
 // MIN_CTAS CTAs share an SM.
 template <int THREADS, int ROUNDS, int TCAP, int LCAP, int FBITS, int MIN_CTAS>
 __global__ void __launch_bounds__(THREADS, MIN_CTAS)
-k_tc_cta(Oriented o, const uint32_t *__restrict__ verts, const uint32_t *__restrict__ unit_off, uint32_t nverts,
-         uint32_t nfwd, const uint32_t *__restrict__ walk, Dir dir, LabelFilter lf, uint32_t *tcount, uint8_t *flag,
+k_tc_cta(Oriented o, UnitList units, uint32_t nfwd, const uint32_t *__restrict__ walk, Dir dir, LabelFilter lf, uint32_t *tcount, uint8_t *flag,
          uint32_t *next_unit) {
     constexpr uint32_t PER_UNIT = (uint32_t)THREADS * ROUNDS;
     static_assert(PER_UNIT < 65536, "16-bit hit counts");
@@ -390,20 +414,14 @@ k_tc_cta(Oriented o, const uint32_t *__restrict__ verts, const uint32_t *__restr
     __shared__ uint32_t pre[THREADS], bbase[THREADS], bhits[THREADS], wsum[THREADS / 32];
     __shared__ uint32_t s_unit, s_total;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const uint32_t n_units = unit_off[nverts];
+    const uint32_t n_units = units.total();
     while (true) {
         if (threadIdx.x == 0) s_unit = atomicAdd(next_unit, 1u);
         __syncthreads();
         const uint32_t unit = s_unit;
         if (unit >= n_units) break;
-        uint32_t lo = 0, hi = nverts + 1;
-        while (lo < hi) {
-            const uint32_t mid = (lo + hi) >> 1;
-            if (unit_off[mid] <= unit) lo = mid + 1;
-            else hi = mid;
-        }
-        const uint32_t vi = lo - 1;
-        const uint32_t x = verts[vi], ch = unit - unit_off[vi];
+        uint32_t vi, x, ch;
+        units.find(unit, vi, x, ch);
         const bool fwd = vi < nfwd, in_core = !fwd && walk[x] == 0;
         const uint32_t la = labels ? labels[x] : 0u;
         if (labels && (la == INVALID || lf.frozen(x))) {
@@ -543,12 +561,11 @@ void set_tc_attr() {
 }
 
 template <int THREADS, int ROUNDS, int TCAP, int LCAP, int FBITS, int MIN_CTAS>
-void launch_tc_cta(const Oriented &o, const TcPlan &plan, int k, LabelFilter labels, uint32_t *tcount,
-                   uint8_t *flag, uint32_t *ctr, unsigned grid, cudaStream_t s) {
+void launch_tc_cta(const Oriented &o, const UnitList &units, uint32_t nfwd, const TcPlan &plan, LabelFilter labels,
+                   uint32_t *tcount, uint8_t *flag, uint32_t *ctr, unsigned grid, cudaStream_t s) {
     const size_t smem = tc_cta_smem<TCAP, LCAP, FBITS>();
     k_tc_cta<THREADS, ROUNDS, TCAP, LCAP, FBITS, MIN_CTAS><<<grid, THREADS, smem, s>>>(
-        o, plan.verts[k], plan.unit_off[k], plan.nverts[k], plan.nfwd[k], plan.walk(o),
-        Dir{plan.dir_lo, plan.dir_hi, plan.dir_amin}, labels, tcount, flag, ctr);
+        o, units, nfwd, plan.walk(o), Dir{plan.dir_lo, plan.dir_hi, plan.dir_amin}, labels, tcount, flag, ctr);
     CK_LAUNCH("k_tc_cta");
 }
 
@@ -884,8 +901,7 @@ void tc_plan_lists(Ctx &c, const Oriented &o, TcPlan &plan, uint32_t *lists, uin
                           o.n, lists, bounds, s);
 }
 
-void tc_plan_units(Ctx &c, const Oriented &o, TcPlan &plan, uint32_t *lists, const uint32_t *hb, cudaStream_t s,
-                   bool owned) {
+void tc_plan_units(const Oriented &o, TcPlan &plan, uint32_t *lists, const uint32_t *hb, cudaStream_t s, bool owned) {
     const uint32_t per_unit[TcPlan::K] = {1, 1, 1, 32, CTA1_THREADS * CTA1_ROUNDS, CTA2_THREADS * CTA2_ROUNDS, 1};
     for (int k = 0; k < TcPlan::K; k++) {
         const int l = k < 5 ? k : k + (k == 5 ? 1 : 2);   // first list of bucket k
@@ -894,16 +910,11 @@ void tc_plan_units(Ctx &c, const Oriented &o, TcPlan &plan, uint32_t *lists, con
         plan.nfwd[k] = hb[l + 1] - hb[l];
         plan.nverts[k] = hb[l + 1 + cta] - hb[l];
         plan.unit_off[k] = nullptr;
-        if (!TcPlan::has_units(k)) continue;
         const uint32_t cnt = plan.nverts[k];
-        if (owned) {
-            plan.unit_off[k] = c.alloc<uint32_t>((size_t)cnt + 1);
-        } else {
-            plan.tmp[k - 2].alloc((size_t)cnt + 1, s);
-            plan.unit_off[k] = plan.tmp[k - 2].get();
-        }
-        if (cnt || owned)
-            scan_exclusive<uint32_t>(UnitsOf{o, plan.verts[k], per_unit[k], plan.nfwd[k]}, plan.unit_off[k], cnt, s);
+        if (k < 3 || k > 5 || !cnt || owned) continue;
+        plan.tmp[k - 2].alloc((size_t)cnt + 1, s);
+        plan.unit_off[k] = plan.tmp[k - 2].get();
+        scan_exclusive<uint32_t>(UnitsOf{o, plan.verts[k], per_unit[k], plan.nfwd[k]}, plan.unit_off[k], cnt, s);
     }
 }
 
@@ -921,7 +932,7 @@ void tc_plan(Ctx &c, const Oriented &o, TcPlan &plan, cudaStream_t s, bool owned
     uint32_t *hb = c.host_u32 + HOST_PLAN;
     CK(cudaMemcpyAsync(hb, bounds.get(), 4 * (TC_LISTS + 1), cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
-    tc_plan_units(c, o, plan, lists, hb, s, owned);
+    tc_plan_units(o, plan, lists, hb, s, owned);
 }
 
 void tc_core_map(Ctx &c, const Oriented &o, uint64_t slots, TcPlan &plan, uint32_t core_n, uint32_t lcap,
@@ -1072,50 +1083,120 @@ double autotune_tc(Ctx &c, std::vector<std::string> *report) {
     return best;
 }
 
-void count_triangles(Ctx &c, const Oriented &o, const TcPlan &plan, LabelFilter labels, uint32_t *tcount,
-                     uint8_t *flag, cudaStream_t s, const char *phase) {
-    if (o.n == 0) return;
-    PhaseScope ph(c, phase ? phase : labels.labels ? "wcc_tc" : "tc");
-    prepare_tc_kernels();
-    uint32_t *ctr = c.work_counter;
-    CK(cudaMemsetAsync(ctr, 0, 24, s));
-    const Dir dir{plan.dir_lo, plan.dir_hi, plan.dir_amin};
-    const bool core = plan.nverts[5] && plan.core_n && !labels.labels;
-    SmallWork sw{};
+namespace {
+
+UnitList bucket_units(const TcPlan &plan, int k) {
+    return UnitList{plan.verts[k], plan.unit_off[k], plan.nverts[k], nullptr, nullptr, 1};
+}
+
+void launch_small(Ctx &c, const Oriented &o, const TcPlan &plan, SmallWork sw, LabelFilter labels, uint32_t *tcount,
+                  uint8_t *flag, cudaStream_t s) {
     for (int j = 0; j < 3; j++) {
         sw.verts[j] = plan.verts[2 - j];
         sw.nverts[j] = plan.nverts[2 - j];
         sw.blocks[j] = sw.nverts[j] ? grid_for((uint64_t)sw.nverts[j] * (32 >> j), 256, 152 * 8) : 0u;
     }
-    if (const unsigned blocks = sw.blocks[0] + sw.blocks[1] + sw.blocks[2]) {
-        k_tc_small<<<blocks, 256, 0, s>>>(o, sw, dir, labels, tcount, flag);
+    if (const unsigned blocks = sw.list_blocks + sw.blocks[0] + sw.blocks[1] + sw.blocks[2]) {
+        k_tc_small<<<blocks, 256, 0, s>>>(o, sw, Dir{plan.dir_lo, plan.dir_hi, plan.dir_amin}, labels, tcount, flag);
         CK_LAUNCH("k_tc_small");
         c.launches++;
     }
+}
+
+void launch_huge(Ctx &c, const Oriented &o, const TcPlan &plan, LabelFilter labels, uint32_t *tcount, uint8_t *flag,
+                 cudaStream_t s) {
+    if (!plan.nverts[6]) return;
+    k_tc_huge<<<152 * 4, 256, 0, s>>>(o, plan.verts[6], plan.nverts[6], labels, tcount, flag);
+    CK_LAUNCH("k_tc_huge");
+    c.launches++;
+}
+
+}  // namespace
+
+void count_triangles(Ctx &c, const Oriented &o, const TcPlan &plan, LabelFilter labels, uint32_t *tcount,
+                     uint8_t *flag, cudaStream_t s) {
+    if (o.n == 0) return;
+    PhaseScope ph(c, "tc");
+    prepare_tc_kernels();
+    uint32_t *ctr = c.work_counter;
+    CK(cudaMemsetAsync(ctr, 0, 24, s));
+    const Dir dir{plan.dir_lo, plan.dir_hi, plan.dir_amin};
+    const bool core = plan.nverts[5] && plan.core_n && !labels.labels;
+    launch_small(c, o, plan, SmallWork{}, labels, tcount, flag, s);
     if (plan.nverts[3]) {
-        k_tc_warp<16, 256, 64, 10><<<152 * 4, 16 * 32, 0, s>>>(o, plan.verts[3], plan.unit_off[3], plan.nverts[3],
-                                                           dir, labels, tcount, flag, ctr);
+        k_tc_warp<16, 256, 64, 10><<<152 * 4, 16 * 32, 0, s>>>(o, bucket_units(plan, 3), dir, labels, tcount, flag, ctr);
         CK_LAUNCH("k_tc_warp64");
         c.launches++;
     }
     if (plan.nverts[4]) {
-        launch_tc_cta<CTA1_THREADS, CTA1_ROUNDS, 2048, 1024, 14, 12>(o, plan, 4, labels, tcount, flag, ctr + 1, 152 * 12,
-                                                                     s);
+        launch_tc_cta<CTA1_THREADS, CTA1_ROUNDS, 2048, 1024, 14, 12>(o, bucket_units(plan, 4), plan.nfwd[4], plan, labels,
+                                                                     tcount, flag, ctr + 1, 152 * 12, s);
         c.launches++;
     }
     if (core) {
         launch_tc_core(o, plan, 5, plan.core_lcap, tcount, flag, ctr + 2, s);
         c.launches++;
     } else if (plan.nverts[5]) {
-        launch_tc_cta<CTA2_THREADS, CTA2_ROUNDS, 16384, 8192, 17, 1>(o, plan, 5, labels, tcount, flag, ctr + 2, 152, s);
+        launch_tc_cta<CTA2_THREADS, CTA2_ROUNDS, 16384, 8192, 17, 1>(o, bucket_units(plan, 5), plan.nfwd[5], plan, labels,
+                                                                     tcount, flag, ctr + 2, 152, s);
         c.launches++;
     }
     if (plan.dense.n) tc_dense_count(c, o, plan, tcount, flag, ctr + 4, s);
-    if (plan.nverts[6]) {
-        k_tc_huge<<<152 * 4, 256, 0, s>>>(o, plan.verts[6], plan.nverts[6], labels, tcount, flag);
-        CK_LAUNCH("k_tc_huge");
+    launch_huge(c, o, plan, labels, tcount, flag, s);
+}
+
+void alloc_internal_work(Ctx &c) {
+    const TcPlan &p = c.wplan;
+    InternalWork &w = c.iwork;
+    const size_t nv = (size_t)p.nverts[3] + p.nverts[4] + p.nverts[5];
+    const size_t units = nv + c.g.m / InternalWork::CHUNK + 1;   // a list of l has at most 1 + l / CHUNK
+    for (int k = 0; k < InternalWork::K; k++) {
+        const bool any = k < 3 ? nv : p.nverts[5];
+        w.verts[k] = any ? c.alloc<uint32_t>(k < 2 ? nv : units) : nullptr;
+        w.chunk[k] = any && k >= 2 ? c.alloc<uint32_t>(units) : nullptr;
+    }
+    w.count = c.work_counter + 8;
+}
+
+void count_internal_triangles(Ctx &c, const Oriented &o, uint32_t *tcount, uint8_t *flag) {
+    PhaseScope ph(c, "wcc_tc");
+    prepare_tc_kernels();
+    const TcPlan &plan = c.wplan;
+    const InternalWork &w = c.iwork;
+    cudaStream_t s = c.stream;
+    uint32_t *ctr = c.work_counter;
+    static_assert(InternalWork::SMALL == 32 && InternalWork::MID == 64 && InternalWork::CTA == 1024 &&
+                  InternalWork::LONGEST == B2, "kernel capacities");
+    static_assert(InternalWork::CHUNK == CTA1_THREADS * CTA1_ROUNDS && InternalWork::CHUNK == CTA2_THREADS * CTA2_ROUNDS,
+                  "partners of a CTA unit");
+    const auto listed = [&](int k, uint32_t per) { return UnitList{w.verts[k], nullptr, 0, w.count + k, w.chunk[k], per}; };
+    const uint32_t nv = plan.nverts[3] + plan.nverts[4] + plan.nverts[5];
+    SmallWork sw{};
+    if (nv) {
+        sw.list = w.verts[0];
+        sw.count = w.count;
+        sw.list_blocks = grid_for((uint64_t)nv * 32, 256, 152 * 8);
+    }
+    launch_small(c, o, plan, sw, LabelFilter{}, tcount, flag, s);
+    const Dir dir{plan.dir_lo, plan.dir_hi, plan.dir_amin};
+    if (nv) {
+        k_tc_warp<16, 256, 64, 10><<<grid_for(2ull * nv, 16, 152 * 4), 16 * 32, 0, s>>>(o, listed(1, 2), dir, LabelFilter{},
+                                                                                     tcount, flag, ctr);
+        CK_LAUNCH("k_tc_warp64");
         c.launches++;
     }
+    if (plan.nverts[4] + plan.nverts[5]) {
+        launch_tc_cta<CTA1_THREADS, CTA1_ROUNDS, 2048, 1024, 14, 12>(
+            o, listed(2, 1), INVALID, plan, LabelFilter{}, tcount, flag, ctr + 1,
+            grid_for(2ull * (plan.nverts[4] + plan.nverts[5]), 1, 152 * 12), s);
+        c.launches++;
+    }
+    if (plan.nverts[5]) {
+        launch_tc_cta<CTA2_THREADS, CTA2_ROUNDS, 16384, 8192, 17, 1>(o, listed(3, 1), INVALID, plan, LabelFilter{}, tcount,
+                                                                     flag, ctr + 2, 152, s);
+        c.launches++;
+    }
+    launch_huge(c, o, plan, LabelFilter{}, tcount, flag, s);
 }
 
 }  // namespace scd
