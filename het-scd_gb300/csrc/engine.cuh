@@ -140,27 +140,29 @@ struct DenseCore {
 // The vertices above the register groups' buckets by the length of their internal out-list,
 // listed anew for every labelling by the pass that makes the internal lists: a community
 // holds a few dozen of a hub's neighbours, so nearly all of them belong to a cheaper kernel
-// than their whole out-list's, or to none (fewer than two internal out-neighbours).
+// than their whole out-list's. (The register groups, up to SMALL, find theirs themselves.)
 // Measured, the CTA kernels of a step by whole out-lists -> by this list: R-MAT scale 22
 // 650 -> 4-21 us, scale 20 210 -> 5 us; 96 planted graphs (register groups only) unchanged.
 struct InternalWork {
-    static constexpr int K = 4;   // register groups, warp units, 128-thread CTA units, 256-thread CTA units
+    static constexpr int K = 3;   // warp units, 128-thread CTA units, 256-thread CTA units
     static constexpr uint32_t SMALL = 32, MID = 64, CTA = 1024, LONGEST = 8192, CHUNK = 512;
     uint32_t *verts[K] = {}, *chunk[K] = {};   // chunk (CTA units only): 512 partners each
     uint32_t *count = nullptr;                 // K words
     // (out-lists above LONGEST keep k_tc_huge)
 };
 // out-degree buckets and their work-unit offsets (built once per oriented graph)
+// The out-lists above the register groups': a bucket for warp units, two for CTA units
+// (1 and 2), one for the longest.
 // Bucket k lists its out-list centres first (nfwd[k] of them) and, for the CTA
 // buckets, then the in-list centres: a vertex b whose edges a -> b with
 // d+(a) < d+(b) (b-centric edges, below) are counted from b's table.
 struct TcPlan {
-    static constexpr int K = 7;
+    static constexpr int K = 4;
     uint32_t *verts[K] = {};
     uint32_t *unit_off[K] = {};
     uint32_t nverts[K] = {};
     uint32_t nfwd[K] = {};
-    uint32_t small_max = 0;   // longest out-list of the register groups (buckets 0 to 2)
+    uint32_t small_max = 0;   // longest out-list of the register groups
     uint32_t dir_lo = 0, dir_hi = 0, dir_amin = 0;   // b-centric iff d+(a) < d+(b),
                                                       // dir_lo < d+(b) <= dir_hi, d+(a) > dir_amin
     DevBuf<uint32_t> tmp[4];   // storage when the plan is temporary: the lists, the unit offsets
@@ -220,8 +222,8 @@ void tc_plan_counting(Ctx &c, const Oriented &o, uint64_t slots, TcPlan &plan, c
 // number of distinct values of row r.
 void sort_rows(Ctx &c, const uint32_t *off, uint32_t nrows, uint32_t *vals, bool dedup, uint32_t *udeg,
                cudaStream_t s);
-void count_triangles(Ctx &c, const Oriented &o, const TcPlan &plan, LabelFilter labels, uint32_t *tcount,
-                     uint8_t *flag, cudaStream_t s);
+void count_triangles(Ctx &c, const Oriented &o, const TcPlan &plan, uint32_t *tcount, uint8_t *flag,
+                     cudaStream_t s);
 // lists for the resident graph's WCC plan (InternalWork), and the count of the internal
 // out-lists o by that plan and those lists
 void alloc_internal_work(Ctx &c);

@@ -542,7 +542,7 @@ k_internal_lists(uint32_t n, uint32_t rows, WarpRows longer, uint32_t most_short
         at = __shfl_sync(FULL, at, 0) + lane;
         if (lane < pend[k]) {
             work.verts[k][at] = pend_v[k];
-            if (k >= 2) work.chunk[k][at] = pend_c[k];
+            if (k >= 1) work.chunk[k][at] = pend_c[k];
         }
         pend[k] = 0;
     };
@@ -567,12 +567,12 @@ k_internal_lists(uint32_t n, uint32_t rows, WarpRows longer, uint32_t most_short
                 }
             }
             if (LISTS && lane == 0) ilen[v] = c;
-            if (LISTS && c >= 2 && len <= InternalWork::LONGEST) {
+            if (LISTS && c > InternalWork::SMALL && len <= InternalWork::LONGEST) {
                 const uint32_t chunks = c <= InternalWork::MID ? 1u : (c + InternalWork::CHUNK - 1) / InternalWork::CHUNK;
                 for (uint32_t ch = 0; ch < chunks; ch++) {
 #pragma unroll
                     for (int k = 0; k < InternalWork::K; k++) {
-                        const uint32_t kk = (c > InternalWork::SMALL) + (c > InternalWork::MID) + (c > InternalWork::CTA);
+                        const uint32_t kk = (c > InternalWork::MID) + (c > InternalWork::CTA);
                         if (kk != (uint32_t)k) continue;
                         if (lane == pend[k]) {
                             pend_v[k] = v;
@@ -645,7 +645,7 @@ void launch_internal_lists(Ctx &c, LabelFilter lf, const Stats &st) {
     WarpRows longer{};
     for (int k = 0; k < WarpRows::K; k++)   // the longest first
         longer.set(k, c.wplan.verts[TcPlan::K - 1 - k], c.wplan.nverts[TcPlan::K - 1 - k]);
-    static_assert(TcPlan::K - WarpRows::K == 3, "the buckets above the register groups");
+    static_assert(TcPlan::K == WarpRows::K, "the buckets above the register groups");
     k_internal_lists<LISTS, STATS><<<grid_for((((uint64_t)g.n + rows - 1) / rows + longer.total) * 32, TPB,
                                               NUM_SMS_HINT * 16), TPB, 0, c.stream>>>(
         g.n, rows, longer, c.wplan.small_max, g.indices, g.nlow, g.adj, lf, c.int_len, c.int_adj, c.slot_flag, c.itcount,

@@ -441,12 +441,12 @@ void launch_dense(const Oriented &o, const DenseCore &d, const TcPlan &plan, con
     k_tc_dense<Q><<<dense_grid(k_tc_dense<Q>, d.n), DENSE_WARPS * 32, 0, s>>>(o, d.verts.get(), d.n, d.num.get(), bits,
                                                                              m.sums, flag, ctr);
     CK_LAUNCH("k_tc_dense");
-    const uint32_t na = plan.nfwd[5], nb = plan.nfwd[4];   // the longer out-lists first
+    const uint32_t na = plan.nfwd[2], nb = plan.nfwd[1];   // the longer out-lists first
     if (na + nb == 0) return;
     k_dense_open<<<grid, 256, 0, s>>>(o, d.verts.get(), d.n, d.num.get(), 128 * Q, flag, m.open, m.row_open);
     CK_LAUNCH("k_dense_open");
     k_tc_fringe<Q><<<dense_grid(k_tc_fringe<Q>, ((uint64_t)na + nb + DENSE_WARPS - 1) / DENSE_WARPS), DENSE_WARPS * 32, 0,
-                     s>>>(o, plan.verts[5], na, plan.verts[4], nb, d.num.get(), bits, m.open, m.row_open, tcount, flag,
+                     s>>>(o, plan.verts[2], na, plan.verts[1], nb, d.num.get(), bits, m.open, m.row_open, tcount, flag,
                           ctr + 1);
     CK_LAUNCH("k_tc_fringe");
     k_dense_close<<<grid, 256, 0, s>>>(o, d.verts.get(), d.n, d.num.get(), 128 * Q, m.open, m.row_open, flag);

@@ -21,10 +21,8 @@
 // table (b's in-lists give the a).  Every triangle a -> b -> c is still found
 // exactly once, at a's table or at b's.
 //
-// With labels, only internal triangles count (all three vertices carry the
-// same valid label): only partners and table entries with the centre's label
-// take part.  (compute_wcc gives the kernels internal out-lists instead, which
-// is faster; the label filter stays for callers with whole out-lists.)
+// compute_wcc counts internal triangles (all three vertices carry the same
+// valid label) by giving the kernels internal out-lists.
 //
 // Work unit = (vertex a, its out-list whole) for a register group, (a, up to
 // 32 consecutive b of out(a)) for one warp, or (centre, up to 512 partners) for
@@ -77,25 +75,25 @@ struct UnitsOf {
     }
 };
 
-// the out-degree bucket of a vertex: bit k for bucket k < 4, bits 4 and 6 for the two CTA
-// buckets, 8 for the last; bit 5 or 7 (in-list centres) when a vertex of a CTA bucket also
-// has a non-empty in-list
+// the out-degree bucket of a vertex above the register groups: bit 0 for the warp bucket, 1 and
+// 3 for the two CTA buckets, 5 for the last; bit 2 or 4 (in-list centres) when a vertex of a CTA
+// bucket also has a non-empty in-list
 struct BucketMask {
     Oriented o;
-    uint32_t upper[TcPlan::K];   // ascending
+    uint32_t upper[TcPlan::K];   // ascending: the register groups' longest, then buckets 0 to K - 2
     bool in_lists;
     const uint32_t *walk;        // 0 for the members of the dense core, which are no out-list centres (nullptr: no core)
     __device__ uint32_t operator[](size_t v) const {
         const uint32_t len = o.len[v];
-        if (len == 0) return 0u;
+        if (len <= upper[0]) return 0u;
         int k = 0;
 #pragma unroll
-        for (int j = 0; j < TcPlan::K - 1; j++) k += len > upper[j];
+        for (int j = 1; j < TcPlan::K; j++) k += len > upper[j];
         const uint32_t out = !walk || walk[v] > 0;
-        if (k < 4) return out << k;
-        if (k == 6) return out << 8;
+        if (k == 0) return out;
+        if (k == 3) return out << 5;
         const uint32_t in = in_lists && o.in_len((uint32_t)v) > 0;
-        return (out | (in << 1)) << (k == 4 ? 4 : 6);
+        return (out | (in << 1)) << (k == 1 ? 1 : 3);
     }
 };
 
@@ -127,40 +125,41 @@ struct UnitList {
     }
 };
 
-// Short out-lists (d+(a) <= G, G = 16 or 32): one group of G lanes per vertex
-// a, no table.  Lane i holds out(a)[i] in a register (out-lists are sorted
-// ascending); the (b, c in out(b)) items of a are flattened by a group scan
-// and taken G at a time, the owner b of an item and the position of c in
-// out(a) are both found by binary search over registers (shuffles).  Per-slot
-// hit counts go to a 32-entry shared array per warp: a hit adds one for b and
-// one for c, both entries of out(a), and flags the (b, c) slot.  An out(b) at
-// least 4x longer than out(a) (a hub's) is not walked: every lane searches its
-// out(a) entry in out(b) instead (alen searches of log2 d+(b) steps).
+// Short out-lists (2 <= d+(a) <= 32). A warp takes `rows` consecutive vertices: bounds and
+// lengths in one coalesced step, then those of more than 16 entries one at a time, those of
+// 9..16 two and those of 2..8 four at a time, a group of G = 32, 16 or 8 lanes each. Lane i of
+// a group holds out(a)[i] in a register (out-lists are sorted ascending); the (b, c in out(b))
+// items of a are flattened by a group scan and taken G at a time; the owner b of an item and
+// the place of c in out(a) are both found by binary search over registers (shuffles). A hit
+// adds one for b and one for c, both entries of out(a), to shared counters and flags the (b, c)
+// slot. An out(b) at least 4x longer than out(a) (a hub's) is not walked: every lane searches
+// its out(a) entry in out(b) instead (alen searches of log2 d+(b) steps).
+//
+// Bound by instructions (issue slots 70-78%). Groups by the list as it is: the internal
+// out-lists of a labelling are a fraction of the whole ones, and with the groups of the whole
+// lists (and vertices gathered from the plan's lists) most lanes idled.
+// Measured: internal count of a step, 96 planted graphs, 466..680 -> 333..660 us (a later one
+// 361..197 -> 239..75), the preprocessing's count 1198 -> 1217 us; Chung-Lu 4M 235 -> 86 us and
+// 2022 -> 2076 us. A table of lane numbers by hash in
+// place of the register search of c took as many instructions and more registers: slower.
+struct SmallShared {
+    uint32_t acc[8][32], beg[8][32], meta[8][32];   // meta: list length << 5 | lane of the vertex
+};
+
 template <int G>
-__device__ __forceinline__ void tc_small(Oriented o, const uint32_t *__restrict__ verts, uint32_t nverts, Dir dir,
-                                         LabelFilter lf, uint32_t *tcount, uint8_t *flag, uint32_t block,
-                                         uint32_t blocks, uint32_t (&acc)[8][32]) {
+__device__ __forceinline__ void tc_small(const Oriented &o, const Dir &dir, uint32_t v0, uint32_t first, uint32_t last,
+                                         uint32_t *tcount, uint8_t *flag, SmallShared &sh) {
     constexpr int PER_WARP = 32 / G;
-    const uint32_t *labels = lf.labels;
     const int lane = threadIdx.x & 31, gl = lane % G, g0 = lane - gl, w = threadIdx.x >> 5;
-    const unsigned gmask = (G == 32) ? FULL : (((1u << G) - 1u) << g0);
-    const uint32_t warps = blocks * 8;
-    for (uint32_t base = ((block * 256 + threadIdx.x) >> 5) * PER_WARP; base < nverts; base += warps * PER_WARP) {
-        const uint32_t vi = base + lane / G;
-        bool live = vi < nverts;
-        const uint32_t a = live ? verts[vi] : 0u;
-        uint32_t la = 0;
-        if (live && labels) {
-            la = labels[a];
-            live = la != INVALID && !lf.frozen(a);
-        }
-        const uint32_t abeg = live ? o.beg[a] : 0u, alen = live ? o.len[a] : 0u;   // alen <= G
+    const unsigned gmask = (G == 32) ? FULL : (((1u << (G & 31)) - 1u) << g0);
+    for (uint32_t i0 = first; i0 < last; i0 += PER_WARP) {
+        const uint32_t i = i0 + lane / G;
+        const uint32_t meta = i < last ? sh.meta[w][i] : 0u, abeg = i < last ? sh.beg[w][i] : 0u;
+        const uint32_t alen = meta >> 5;   // <= G
         const bool in_a = (uint32_t)gl < alen;
-        const uint32_t x = in_a ? o.adj[abeg + gl] : 0xffffffffu;
-        const bool ok = in_a && (!labels || labels[x] == la);   // usable as b and as c
-        const uint32_t dx = ok ? o.len[x] : 0u;
-        const bool walk = ok && !dir.bcentric(alen, dx);        // a -> x is counted here
-        const uint32_t wfull = walk ? dx : 0u, bb = walk ? o.beg[x] : 0u;
+        const uint32_t x = in_a ? o.adj[abeg + gl] : INVALID;
+        const uint32_t dx = in_a ? o.len[x] : 0u, xbeg = in_a ? o.beg[x] : 0u;
+        const uint32_t wfull = dir.bcentric(alen, dx) ? 0u : dx;   // a -> x is counted here
         // a long out(b) is searched for the entries of out(a) (below) instead of walked
         const bool far = wfull >= 32 && wfull >= 4 * alen;
         const uint32_t wb = far ? 0u : wfull;
@@ -171,10 +170,9 @@ __device__ __forceinline__ void tc_small(Oriented o, const uint32_t *__restrict_
             if (gl >= d) incl += y;
         }
         const uint32_t total = __shfl_sync(FULL, incl, G - 1, G), pre = incl - wb;
-        uint32_t tmax = total;
-#pragma unroll
-        for (int d = G; d < 32; d <<= 1) tmax = max(tmax, __shfl_xor_sync(FULL, tmax, d));
-        acc[w][lane] = 0;
+        const uint32_t delta = xbeg - pre;   // item t of this b lies at CSR position delta + t
+        const uint32_t tmax = PER_WARP == 1 ? total : __reduce_max_sync(FULL, total);
+        sh.acc[w][lane] = 0;
         __syncwarp();
         uint32_t hits = 0;
         for (uint32_t t0 = 0; t0 < tmax; t0 += G) {
@@ -183,20 +181,16 @@ __device__ __forceinline__ void tc_small(Oriented o, const uint32_t *__restrict_
 #pragma unroll
             for (int st = G / 2; st > 0; st >>= 1)
                 if (__shfl_sync(FULL, pre, j + st, G) <= t) j += st;
-            const uint32_t bj = __shfl_sync(FULL, bb, j, G), pj = __shfl_sync(FULL, pre, j, G);
             const bool valid = t < total;
-            const uint32_t cpos = bj + (t - pj);
-            const uint32_t cv = valid ? o.adj[cpos] : 0xffffffffu;
+            const uint32_t cpos = __shfl_sync(FULL, delta, j, G) + t;
+            const uint32_t cv = valid ? o.adj[cpos] : INVALID - 1;   // (no entry)
             uint32_t k = 0;   // last entry of out(a) <= c
 #pragma unroll
             for (int st = G / 2; st > 0; st >>= 1)
                 if (__shfl_sync(FULL, x, k + st, G) <= cv) k += st;
-            const uint32_t xk = __shfl_sync(FULL, x, k, G);        // every lane shuffles
-            const int okk = __shfl_sync(FULL, (int)ok, k, G);
-            const bool hit = valid && xk == cv && okk;
-            if (hit) {
-                atomicAdd(&acc[w][g0 + j], 1u);
-                atomicAdd(&acc[w][g0 + k], 1u);
+            if (__shfl_sync(FULL, x, k, G) == cv) {
+                atomicAdd(&sh.acc[w][g0 + j], 1u);
+                atomicAdd(&sh.acc[w][g0 + k], 1u);
                 flag[cpos] = 1;
                 hits++;
             }
@@ -208,14 +202,14 @@ __device__ __forceinline__ void tc_small(Oriented o, const uint32_t *__restrict_
         const unsigned fm = __ballot_sync(FULL, far);
         unsigned fpos = 0;
 #pragma unroll
-        for (int g = 0; g < PER_WARP; g++) fpos |= (G == 32) ? fm : (fm >> (g * G)) & ((1u << G) - 1u);
+        for (int g = 0; g < PER_WARP; g++) fpos |= (G == 32) ? fm : (fm >> (g * G)) & ((1u << (G & 31)) - 1u);
         for (; fpos; fpos &= fpos - 1) {
             const int j = __ffs(fpos) - 1;
             const bool fj = __shfl_sync(FULL, far, j, G);
-            const uint32_t bj = __shfl_sync(FULL, bb, j, G), wj = __shfl_sync(FULL, wfull, j, G);
+            const uint32_t bj = __shfl_sync(FULL, xbeg, j, G), wj = __shfl_sync(FULL, wfull, j, G);
             bool hit = false;
             uint32_t lo = 0;
-            if (fj && ok) {
+            if (fj && in_a) {
                 uint32_t hi = wj;
                 while (lo < hi) {
                     const uint32_t mid = (lo + hi) >> 1;
@@ -230,47 +224,53 @@ __device__ __forceinline__ void tc_small(Oriented o, const uint32_t *__restrict_
                 hits++;
             }
             const uint32_t nb = __popc(__ballot_sync(FULL, hit) & gmask);
-            if (gl == j && nb) acc[w][lane] += nb;
+            if (gl == j) selfc += nb;
         }
         __syncwarp();
-        const uint32_t hc = acc[w][lane] + selfc;
+        const uint32_t hc = sh.acc[w][lane] + selfc;
         if (hc && in_a) {
             atomicAdd(tcount + o.at(x), hc);
             flag[abeg + gl] = 1;
         }
 #pragma unroll
         for (int d = G / 2; d > 0; d >>= 1) hits += __shfl_xor_sync(FULL, hits, d);
-        if (gl == 0 && hits) atomicAdd(tcount + o.at(a), hits);
+        if (gl == 0 && hits) atomicAdd(tcount + o.at(v0 + (meta & 31)), hits);
         __syncwarp();
     }
 }
 
-// The three register-group buckets in one launch, the longest out-lists' blocks first
-struct SmallWork {
-    const uint32_t *verts[3];   // buckets 2, 1, 0: groups of 32, 16 and 8 lanes
-    uint32_t nverts[3], blocks[3];
-    const uint32_t *list, *count;   // and a list made on the device, groups of 32
-    uint32_t list_blocks;
-};
-
-__global__ void __launch_bounds__(256)
-k_tc_small(Oriented o, SmallWork w, Dir dir, LabelFilter lf, uint32_t *tcount, uint8_t *flag) {
-    __shared__ uint32_t acc[8][32];
-    uint32_t b = blockIdx.x;
-    if (b < w.list_blocks) return tc_small<32>(o, w.list, *w.count, dir, lf, tcount, flag, b, w.list_blocks, acc);
-    b -= w.list_blocks;
-    if (b < w.blocks[0]) return tc_small<32>(o, w.verts[0], w.nverts[0], dir, lf, tcount, flag, b, w.blocks[0], acc);
-    b -= w.blocks[0];
-    if (b < w.blocks[1]) return tc_small<16>(o, w.verts[1], w.nverts[1], dir, lf, tcount, flag, b, w.blocks[1], acc);
-    b -= w.blocks[1];
-    tc_small<8>(o, w.verts[2], w.nverts[2], dir, lf, tcount, flag, b, w.blocks[2], acc);
+// walk: 0 for the vertices whose out-list is counted elsewhere (nullptr: none)
+__global__ void __launch_bounds__(256, 8)
+k_tc_small(Oriented o, uint32_t rows, uint32_t max_len, const uint32_t *__restrict__ walk, Dir dir, uint32_t *tcount,
+           uint8_t *flag) {
+    __shared__ SmallShared sh;
+    const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5, warps = (gridDim.x * blockDim.x) >> 5;
+    const unsigned lt = lanemask_lt();
+    const uint32_t units = (o.n + rows - 1) / rows;
+    for (uint32_t unit = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; unit < units; unit += warps) {
+        const uint32_t v0 = unit * rows, v = v0 + lane;
+        uint32_t len = lane < min(rows, o.n - v0) ? o.len[v] : 0u;
+        if (len < 2 || len > max_len || (walk && walk[v] == 0)) len = 0;
+        const unsigned m32 = __ballot_sync(FULL, len > 16), m16 = __ballot_sync(FULL, len > 8) & ~m32,
+                       m8 = __ballot_sync(FULL, len > 0) & ~(m32 | m16);
+        const uint32_t n32 = __popc(m32), n16 = n32 + __popc(m16), n8 = n16 + __popc(m8);
+        if (len) {
+            const uint32_t at = len > 16 ? __popc(m32 & lt) : len > 8 ? n32 + __popc(m16 & lt) : n16 + __popc(m8 & lt);
+            sh.beg[w][at] = o.beg[v];
+            sh.meta[w][at] = len << 5 | lane;
+        }
+        __syncwarp();
+        tc_small<32>(o, dir, v0, 0, n32, tcount, flag, sh);
+        tc_small<16>(o, dir, v0, n32, n16, tcount, flag, sh);
+        tc_small<8>(o, dir, v0, n16, n8, tcount, flag, sh);
+        __syncwarp();
+    }
 }
 
 // Warp units.  Per warp: table of TCAP (key, index) entries, LCAP counters.
 template <int WARPS, int TCAP, int LCAP, int FBITS>
 __global__ void __launch_bounds__(WARPS * 32)
-k_tc_warp(Oriented o, UnitList units, Dir dir, LabelFilter lf, uint32_t *tcount, uint8_t *flag, uint32_t *next_unit) {
-    const uint32_t *labels = lf.labels;
+k_tc_warp(Oriented o, UnitList units, Dir dir, uint32_t *tcount, uint8_t *flag, uint32_t *next_unit) {
     __shared__ uint32_t filt[WARPS][(1 << FBITS) / 32];
     __shared__ uint32_t keys[WARPS][TCAP];
     __shared__ uint16_t idxs[WARPS][TCAP];
@@ -285,8 +285,6 @@ k_tc_warp(Oriented o, UnitList units, Dir dir, LabelFilter lf, uint32_t *tcount,
         if (unit >= n_units) break;
         uint32_t vi, a, ch;
         units.find(unit, vi, a, ch);
-        const uint32_t la = labels ? labels[a] : 0u;
-        if (labels && (la == INVALID || lf.frozen(a))) continue;
         const uint32_t abeg = o.beg[a], alen = o.len[a];
         int bits = 1;
         while ((1u << bits) < 4 * alen) bits++;
@@ -298,7 +296,6 @@ k_tc_warp(Oriented o, UnitList units, Dir dir, LabelFilter lf, uint32_t *tcount,
         __syncwarp();
         for (uint32_t i = lane; i < alen; i += 32) {
             const uint32_t id = o.adj[abeg + i];
-            if (labels && labels[id] != la) continue;   // only internal c can close an internal triangle
             const uint32_t hv = id * HASH_MUL, fi = hv >> (32 - FBITS);
             atomicOr(&filt[w][fi >> 5], 1u << (fi & 31));
             uint32_t h = hv >> (32 - bits);
@@ -311,7 +308,7 @@ k_tc_warp(Oriented o, UnitList units, Dir dir, LabelFilter lf, uint32_t *tcount,
         if (j < alen) {
             b = o.adj[abeg + j];
             const uint32_t db = o.len[b];
-            if ((!labels || labels[b] == la) && !dir.bcentric(alen, db)) {
+            if (!dir.bcentric(alen, db)) {
                 wb = db;
                 bb = o.beg[b];
             }
@@ -401,11 +398,10 @@ k_tc_warp(Oriented o, UnitList units, Dir dir, LabelFilter lf, uint32_t *tcount,
 // MIN_CTAS CTAs share an SM.
 template <int THREADS, int ROUNDS, int TCAP, int LCAP, int FBITS, int MIN_CTAS>
 __global__ void __launch_bounds__(THREADS, MIN_CTAS)
-k_tc_cta(Oriented o, UnitList units, uint32_t nfwd, const uint32_t *__restrict__ walk, Dir dir, LabelFilter lf, uint32_t *tcount, uint8_t *flag,
+k_tc_cta(Oriented o, UnitList units, uint32_t nfwd, const uint32_t *__restrict__ walk, Dir dir, uint32_t *tcount, uint8_t *flag,
          uint32_t *next_unit) {
     constexpr uint32_t PER_UNIT = (uint32_t)THREADS * ROUNDS;
     static_assert(PER_UNIT < 65536, "16-bit hit counts");
-    const uint32_t *labels = lf.labels;
     extern __shared__ uint32_t sm[];
     uint32_t *keys = sm;                                  // TCAP
     uint32_t *cnt = sm + TCAP;                            // LCAP 16-bit counts
@@ -423,11 +419,6 @@ k_tc_cta(Oriented o, UnitList units, uint32_t nfwd, const uint32_t *__restrict__
         uint32_t vi, x, ch;
         units.find(unit, vi, x, ch);
         const bool fwd = vi < nfwd, in_core = !fwd && walk[x] == 0;
-        const uint32_t la = labels ? labels[x] : 0u;
-        if (labels && (la == INVALID || lf.frozen(x))) {
-            __syncthreads();
-            continue;
-        }
         const uint32_t xbeg = o.beg[x], xlen = o.len[x];
         int bits = 1;
         while ((1u << bits) < 2 * xlen) bits++;
@@ -438,7 +429,6 @@ k_tc_cta(Oriented o, UnitList units, uint32_t nfwd, const uint32_t *__restrict__
         __syncthreads();
         for (uint32_t i = threadIdx.x; i < xlen; i += THREADS) {
             const uint32_t id = o.adj[xbeg + i];
-            if (labels && labels[id] != la) continue;   // only internal c can close an internal triangle
             const uint32_t hv = id * HASH_MUL, fi = hv >> (32 - FBITS);
             atomicOr(&filt[fi >> 5], 1u << (fi & 31));
             uint32_t h = hv >> (32 - bits);
@@ -457,7 +447,7 @@ k_tc_cta(Oriented o, UnitList units, uint32_t nfwd, const uint32_t *__restrict__
                 uint32_t dy = walk[y];
                 if (in_core && dy > dir.lo) dy = 0;
                 const bool here = fwd ? !dir.bcentric(xlen, dy) : dir.bcentric(dy, xlen);
-                if (here && (!labels || labels[y] == la)) {
+                if (here) {
                     wb = dy;
                     bb = o.beg[y];
                 }
@@ -561,11 +551,11 @@ void set_tc_attr() {
 }
 
 template <int THREADS, int ROUNDS, int TCAP, int LCAP, int FBITS, int MIN_CTAS>
-void launch_tc_cta(const Oriented &o, const UnitList &units, uint32_t nfwd, const TcPlan &plan, LabelFilter labels,
+void launch_tc_cta(const Oriented &o, const UnitList &units, uint32_t nfwd, const TcPlan &plan,
                    uint32_t *tcount, uint8_t *flag, uint32_t *ctr, unsigned grid, cudaStream_t s) {
     const size_t smem = tc_cta_smem<TCAP, LCAP, FBITS>();
     k_tc_cta<THREADS, ROUNDS, TCAP, LCAP, FBITS, MIN_CTAS><<<grid, THREADS, smem, s>>>(
-        o, units, nfwd, plan.walk(o), Dir{plan.dir_lo, plan.dir_hi, plan.dir_amin}, labels, tcount, flag, ctr);
+        o, units, nfwd, plan.walk(o), Dir{plan.dir_lo, plan.dir_hi, plan.dir_amin}, tcount, flag, ctr);
     CK_LAUNCH("k_tc_cta");
 }
 
@@ -573,7 +563,7 @@ void launch_tc_cta(const Oriented &o, const UnitList &units, uint32_t nfwd, cons
 constexpr int CTA1_THREADS = 128, CTA1_ROUNDS = 4, CTA2_THREADS = 256, CTA2_ROUNDS = 2;
 
 // CTA units of the upper CTA bucket (out-degree in (cta_hi, 8192]) over a core
-// bitmap, when the plan has a core map and no labels filter.  Every out-list
+// bitmap, when the plan has a core map.  Every out-list
 // of such a centre lies in the core, the vertices of degree > cta_hi (their
 // degrees are at least the centre's), so the centre's out-list in core numbers
 // is held exactly by a shared bitmap of core_n bits (plus the outside marker
@@ -778,26 +768,23 @@ void launch_tc_core(const Oriented &o, const TcPlan &plan, int k, uint32_t lcap,
 // by binary search in the sorted out-list in global memory, per-triangle
 // atomics.  Kept for generality.
 __global__ void __launch_bounds__(256)
-k_tc_huge(Oriented o, const uint32_t *__restrict__ verts, uint32_t nverts, LabelFilter lf, uint32_t *tcount,
+k_tc_huge(Oriented o, const uint32_t *__restrict__ verts, uint32_t nverts, uint32_t *tcount,
           uint8_t *flag) {
-    const uint32_t *labels = lf.labels;
     const int lane = threadIdx.x & 31;
     const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
     for (uint32_t vi = 0; vi < nverts; vi++) {
         const uint32_t a = verts[vi];
-        const uint32_t la = labels ? labels[a] : 0u;
-        if (labels && (la == INVALID || lf.frozen(a))) continue;
         const uint32_t abeg = o.beg[a], alen = o.len[a];
+        if (alen <= 32) continue;   // (an internal list of the register groups)
         const uint32_t *A = o.adj + abeg;
         for (uint32_t j = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; j < alen; j += warps) {
             const uint32_t b = A[j];
-            if (labels && labels[b] != la) continue;
             const uint32_t bbeg = o.beg[b], blen = o.len[b];
             uint32_t hits = 0;
             for (uint32_t i = lane; i < blen; i += 32) {
                 const uint32_t c = o.adj[bbeg + i];
                 const uint32_t ic = lower_bound(A, alen, c);
-                if (ic < alen && A[ic] == c && (!labels || labels[c] == la)) {
+                if (ic < alen && A[ic] == c) {
                     hits++;
                     atomicAdd(tcount + o.at(c), 1u);
                     flag[abeg + ic] = 1;
@@ -885,7 +872,7 @@ uint32_t tc_short_lists(const Ctx &c) { return c.tc_b0 > c.tc_small ? c.tc_b0 : 
 
 void tc_plan_lists(Ctx &c, const Oriented &o, TcPlan &plan, uint32_t *lists, uint32_t *bounds, cudaStream_t s,
                    bool in_lists, uint32_t core_from) {
-    const uint32_t sm = c.tc_small, s16 = sm < 16 ? sm : 16, s8 = sm < 8 ? sm : 8, b0 = tc_short_lists(c);
+    const uint32_t sm = c.tc_small, b0 = tc_short_lists(c);
     // the core-bitmap kernel takes the upper CTA bucket from core_from on; the hash
     // kernels' upper bucket (one CTA per SM, 16K-entry tables) from tc_b1 on
     const uint32_t b1 = core_from ? (core_from > b0 ? core_from : b0) : c.tc_b1;
@@ -896,24 +883,24 @@ void tc_plan_lists(Ctx &c, const Oriented &o, TcPlan &plan, uint32_t *lists, uin
     plan.dir_amin = c.tc_amin < sm ? c.tc_amin : sm;
     plan.cta_lo = b0;
     plan.cta_hi = b1;
-    build_lists<TC_LISTS>(BucketMask{o, {s8, s16, sm, b0, b1, B2, 0xffffffffu}, split,
+    build_lists<TC_LISTS>(BucketMask{o, {sm, b0, b1, B2}, split,
                                      plan.dense.n ? plan.dense.walk.get() : nullptr},
                           o.n, lists, bounds, s);
 }
 
 void tc_plan_units(const Oriented &o, TcPlan &plan, uint32_t *lists, const uint32_t *hb, cudaStream_t s, bool owned) {
-    const uint32_t per_unit[TcPlan::K] = {1, 1, 1, 32, CTA1_THREADS * CTA1_ROUNDS, CTA2_THREADS * CTA2_ROUNDS, 1};
+    const uint32_t per_unit[TcPlan::K] = {32, CTA1_THREADS * CTA1_ROUNDS, CTA2_THREADS * CTA2_ROUNDS, 1};
     for (int k = 0; k < TcPlan::K; k++) {
-        const int l = k < 5 ? k : k + (k == 5 ? 1 : 2);   // first list of bucket k
-        const bool cta = k == 4 || k == 5;
+        const int l = k < 2 ? k : k + (k == 2 ? 1 : 2);   // first list of bucket k
+        const bool cta = k == 1 || k == 2;
         plan.verts[k] = lists + hb[l];
         plan.nfwd[k] = hb[l + 1] - hb[l];
         plan.nverts[k] = hb[l + 1 + cta] - hb[l];
         plan.unit_off[k] = nullptr;
         const uint32_t cnt = plan.nverts[k];
-        if (k < 3 || k > 5 || !cnt || owned) continue;
-        plan.tmp[k - 2].alloc((size_t)cnt + 1, s);
-        plan.unit_off[k] = plan.tmp[k - 2].get();
+        if (k == 3 || !cnt || owned) continue;
+        plan.tmp[k + 1].alloc((size_t)cnt + 1, s);
+        plan.unit_off[k] = plan.tmp[k + 1].get();
         scan_exclusive<uint32_t>(UnitsOf{o, plan.verts[k], per_unit[k], plan.nfwd[k]}, plan.unit_off[k], cnt, s);
     }
 }
@@ -939,7 +926,7 @@ void tc_core_map(Ctx &c, const Oriented &o, uint64_t slots, TcPlan &plan, uint32
                  cudaStream_t s) {
     plan.core_adj = plan.core_beg = nullptr;
     plan.core_n = plan.core_lcap = 0;
-    if (o.n == 0 || plan.nverts[5] == 0) return;
+    if (o.n == 0 || plan.nverts[2] == 0) return;
     const uint64_t padded = slots + 3ull * o.n;   // at most: every list padded by three
     if (padded >= 0xffffffffull) return;          // the padded layout is indexed in 32 bits
     DevBuf<uint32_t> cpos((size_t)o.n + 1, s);
@@ -969,7 +956,7 @@ void tc_plan_counting(Ctx &c, const Oriented &o, uint64_t slots, TcPlan &plan, c
     if (o.n <= CORE_BUDGET) {   // every core fits the budget: the lowest split, no host read
         tc_plan(c, o, plan, s, false, true, b0);
         tc_core_map(c, o, slots, plan, o.n, B2, s);   // core_n <= n; counts sized for the cap
-        if (plan.core_n || !plan.nverts[5]) return;
+        if (plan.core_n || !plan.nverts[2]) return;
         tc_plan(c, o, plan, s, false, true);
         return;
     }
@@ -993,7 +980,7 @@ void tc_plan_counting(Ctx &c, const Oriented &o, uint64_t slots, TcPlan &plan, c
         const uint32_t core_n = h[pick], lcap = h[K + pick];
         tc_plan(c, o, plan, s, false, true, cb.t[pick]);
         tc_core_map(c, o, slots, plan, core_n, lcap, s);
-        if (plan.core_n || !plan.nverts[5]) return;
+        if (plan.core_n || !plan.nverts[2]) return;
     }
     tc_plan(c, o, plan, s, false, true);   // no map: the hash kernels' split
 }
@@ -1043,7 +1030,7 @@ double autotune_tc(Ctx &c, std::vector<std::string> *report) {
                         CK(cudaMemsetAsync(tcount.get(), 0, (size_t)g.n * 4, s));
                         CK(cudaMemsetAsync(flag.get(), 0, 2 * (size_t)g.m, s));
                         CK(cudaEventRecord(e0, s));
-                        count_triangles(c, o, plan, LabelFilter{}, tcount.get(), flag.get(), s);
+                        count_triangles(c, o, plan, tcount.get(), flag.get(), s);
                         CK(cudaEventRecord(e1, s));
                         CK(cudaEventSynchronize(e1));
                         float ms = 0;
@@ -1089,31 +1076,31 @@ UnitList bucket_units(const TcPlan &plan, int k) {
     return UnitList{plan.verts[k], plan.unit_off[k], plan.nverts[k], nullptr, nullptr, 1};
 }
 
-void launch_small(Ctx &c, const Oriented &o, const TcPlan &plan, SmallWork sw, LabelFilter labels, uint32_t *tcount,
+void launch_small(Ctx &c, const Oriented &o, uint32_t max_len, const uint32_t *walk, const Dir &dir, uint32_t *tcount,
                   uint8_t *flag, cudaStream_t s) {
-    for (int j = 0; j < 3; j++) {
-        sw.verts[j] = plan.verts[2 - j];
-        sw.nverts[j] = plan.nverts[2 - j];
-        sw.blocks[j] = sw.nverts[j] ? grid_for((uint64_t)sw.nverts[j] * (32 >> j), 256, 152 * 8) : 0u;
-    }
-    if (const unsigned blocks = sw.list_blocks + sw.blocks[0] + sw.blocks[1] + sw.blocks[2]) {
-        k_tc_small<<<blocks, 256, 0, s>>>(o, sw, Dir{plan.dir_lo, plan.dir_hi, plan.dir_amin}, labels, tcount, flag);
-        CK_LAUNCH("k_tc_small");
-        c.launches++;
-    }
+    // 16 vertices a warp, fewer where that would leave SMs short of their 64 warps; a grid of
+    // one unit a warp, because units of dense graphs take 25 times as long as those of sparse
+    // ones and CTAs that are handed out even that out (96 planted graphs, all counts of a run:
+    // 8 CTAs an SM 7.3 ms, 16 6.8 ms, 48 6.0 ms, 128 5.8 ms; with 32 vertices 6.1 ms, with 8 6.0 ms)
+    uint32_t rows = 4;
+    while (rows < 16 && (uint64_t)rows * 2 * NUM_SMS_HINT * 64 <= o.n) rows <<= 1;
+    k_tc_small<<<grid_for(((uint64_t)o.n + rows - 1) / rows * 32, 256, 1u << 20), 256, 0, s>>>(o, rows, max_len, walk, dir, tcount,
+                                                                                                flag);
+    CK_LAUNCH("k_tc_small");
+    c.launches++;
 }
 
-void launch_huge(Ctx &c, const Oriented &o, const TcPlan &plan, LabelFilter labels, uint32_t *tcount, uint8_t *flag,
+void launch_huge(Ctx &c, const Oriented &o, const TcPlan &plan, uint32_t *tcount, uint8_t *flag,
                  cudaStream_t s) {
-    if (!plan.nverts[6]) return;
-    k_tc_huge<<<152 * 4, 256, 0, s>>>(o, plan.verts[6], plan.nverts[6], labels, tcount, flag);
+    if (!plan.nverts[3]) return;
+    k_tc_huge<<<152 * 4, 256, 0, s>>>(o, plan.verts[3], plan.nverts[3], tcount, flag);
     CK_LAUNCH("k_tc_huge");
     c.launches++;
 }
 
 }  // namespace
 
-void count_triangles(Ctx &c, const Oriented &o, const TcPlan &plan, LabelFilter labels, uint32_t *tcount,
+void count_triangles(Ctx &c, const Oriented &o, const TcPlan &plan, uint32_t *tcount,
                      uint8_t *flag, cudaStream_t s) {
     if (o.n == 0) return;
     PhaseScope ph(c, "tc");
@@ -1121,39 +1108,39 @@ void count_triangles(Ctx &c, const Oriented &o, const TcPlan &plan, LabelFilter 
     uint32_t *ctr = c.work_counter;
     CK(cudaMemsetAsync(ctr, 0, 24, s));
     const Dir dir{plan.dir_lo, plan.dir_hi, plan.dir_amin};
-    const bool core = plan.nverts[5] && plan.core_n && !labels.labels;
-    launch_small(c, o, plan, SmallWork{}, labels, tcount, flag, s);
-    if (plan.nverts[3]) {
-        k_tc_warp<16, 256, 64, 10><<<152 * 4, 16 * 32, 0, s>>>(o, bucket_units(plan, 3), dir, labels, tcount, flag, ctr);
+    const bool core = plan.nverts[2] && plan.core_n;
+    launch_small(c, o, plan.small_max, plan.dense.n ? plan.dense.walk.get() : nullptr, dir, tcount, flag, s);
+    if (plan.nverts[0]) {
+        k_tc_warp<16, 256, 64, 10><<<152 * 4, 16 * 32, 0, s>>>(o, bucket_units(plan, 0), dir, tcount, flag, ctr);
         CK_LAUNCH("k_tc_warp64");
         c.launches++;
     }
-    if (plan.nverts[4]) {
-        launch_tc_cta<CTA1_THREADS, CTA1_ROUNDS, 2048, 1024, 14, 12>(o, bucket_units(plan, 4), plan.nfwd[4], plan, labels,
-                                                                     tcount, flag, ctr + 1, 152 * 12, s);
+    if (plan.nverts[1]) {
+        launch_tc_cta<CTA1_THREADS, CTA1_ROUNDS, 2048, 1024, 14, 12>(o, bucket_units(plan, 1), plan.nfwd[1], plan, tcount,
+                                                                     flag, ctr + 1, 152 * 12, s);
         c.launches++;
     }
     if (core) {
-        launch_tc_core(o, plan, 5, plan.core_lcap, tcount, flag, ctr + 2, s);
+        launch_tc_core(o, plan, 2, plan.core_lcap, tcount, flag, ctr + 2, s);
         c.launches++;
-    } else if (plan.nverts[5]) {
-        launch_tc_cta<CTA2_THREADS, CTA2_ROUNDS, 16384, 8192, 17, 1>(o, bucket_units(plan, 5), plan.nfwd[5], plan, labels,
-                                                                     tcount, flag, ctr + 2, 152, s);
+    } else if (plan.nverts[2]) {
+        launch_tc_cta<CTA2_THREADS, CTA2_ROUNDS, 16384, 8192, 17, 1>(o, bucket_units(plan, 2), plan.nfwd[2], plan, tcount,
+                                                                     flag, ctr + 2, 152, s);
         c.launches++;
     }
     if (plan.dense.n) tc_dense_count(c, o, plan, tcount, flag, ctr + 4, s);
-    launch_huge(c, o, plan, labels, tcount, flag, s);
+    launch_huge(c, o, plan, tcount, flag, s);
 }
 
 void alloc_internal_work(Ctx &c) {
     const TcPlan &p = c.wplan;
     InternalWork &w = c.iwork;
-    const size_t nv = (size_t)p.nverts[3] + p.nverts[4] + p.nverts[5];
+    const size_t nv = (size_t)p.nverts[0] + p.nverts[1] + p.nverts[2];
     const size_t units = nv + c.g.m / InternalWork::CHUNK + 1;   // a list of l has at most 1 + l / CHUNK
     for (int k = 0; k < InternalWork::K; k++) {
-        const bool any = k < 3 ? nv : p.nverts[5];
-        w.verts[k] = any ? c.alloc<uint32_t>(k < 2 ? nv : units) : nullptr;
-        w.chunk[k] = any && k >= 2 ? c.alloc<uint32_t>(units) : nullptr;
+        const bool any = k < 2 ? nv : p.nverts[2];
+        w.verts[k] = any ? c.alloc<uint32_t>(k ? units : nv) : nullptr;
+        w.chunk[k] = any && k ? c.alloc<uint32_t>(units) : nullptr;
     }
     w.count = c.work_counter + 8;
 }
@@ -1170,33 +1157,27 @@ void count_internal_triangles(Ctx &c, const Oriented &o, uint32_t *tcount, uint8
     static_assert(InternalWork::CHUNK == CTA1_THREADS * CTA1_ROUNDS && InternalWork::CHUNK == CTA2_THREADS * CTA2_ROUNDS,
                   "partners of a CTA unit");
     const auto listed = [&](int k, uint32_t per) { return UnitList{w.verts[k], nullptr, 0, w.count + k, w.chunk[k], per}; };
-    const uint32_t nv = plan.nverts[3] + plan.nverts[4] + plan.nverts[5];
-    SmallWork sw{};
-    if (nv) {
-        sw.list = w.verts[0];
-        sw.count = w.count;
-        sw.list_blocks = grid_for((uint64_t)nv * 32, 256, 152 * 8);
-    }
-    launch_small(c, o, plan, sw, LabelFilter{}, tcount, flag, s);
+    const uint32_t nv = plan.nverts[0] + plan.nverts[1] + plan.nverts[2];
     const Dir dir{plan.dir_lo, plan.dir_hi, plan.dir_amin};
+    launch_small(c, o, InternalWork::SMALL, nullptr, dir, tcount, flag, s);
     if (nv) {
-        k_tc_warp<16, 256, 64, 10><<<grid_for(2ull * nv, 16, 152 * 4), 16 * 32, 0, s>>>(o, listed(1, 2), dir, LabelFilter{},
-                                                                                     tcount, flag, ctr);
+        k_tc_warp<16, 256, 64, 10><<<grid_for(2ull * nv, 16, 152 * 4), 16 * 32, 0, s>>>(o, listed(0, 2), dir, tcount, flag,
+                                                                                     ctr);
         CK_LAUNCH("k_tc_warp64");
         c.launches++;
     }
-    if (plan.nverts[4] + plan.nverts[5]) {
+    if (plan.nverts[1] + plan.nverts[2]) {
         launch_tc_cta<CTA1_THREADS, CTA1_ROUNDS, 2048, 1024, 14, 12>(
-            o, listed(2, 1), INVALID, plan, LabelFilter{}, tcount, flag, ctr + 1,
-            grid_for(2ull * (plan.nverts[4] + plan.nverts[5]), 1, 152 * 12), s);
+            o, listed(1, 1), INVALID, plan, tcount, flag, ctr + 1,
+            grid_for(2ull * (plan.nverts[1] + plan.nverts[2]), 1, 152 * 12), s);
         c.launches++;
     }
-    if (plan.nverts[5]) {
-        launch_tc_cta<CTA2_THREADS, CTA2_ROUNDS, 16384, 8192, 17, 1>(o, listed(3, 1), INVALID, plan, LabelFilter{}, tcount,
-                                                                     flag, ctr + 2, 152, s);
+    if (plan.nverts[2]) {
+        launch_tc_cta<CTA2_THREADS, CTA2_ROUNDS, 16384, 8192, 17, 1>(o, listed(2, 1), INVALID, plan, tcount, flag,
+                                                                     ctr + 2, 152, s);
         c.launches++;
     }
-    launch_huge(c, o, plan, LabelFilter{}, tcount, flag, s);
+    launch_huge(c, o, plan, tcount, flag, s);
 }
 
 }  // namespace scd

@@ -14,10 +14,12 @@ import scd_gb300
 pytestmark = pytest.mark.gpu
 
 
-def _graph(sizes, density, stray, seed):
+def _graph(sizes, density, stray, seed, n=None, ids=None):
     rng = np.random.default_rng(seed)
-    n, ids = sum(sizes), rng.permutation(sum(sizes))
-    labels, tri, us, vs, at = np.empty(n, np.uint32), np.ones(n, np.int32), [], [], 0
+    n = n or sum(sizes)
+    ids = rng.permutation(n) if ids is None else ids
+    labels = np.full(n, scd_gb300.INVALID_LABEL, np.uint32)
+    tri, us, vs, at = np.ones(n, np.int32), [], [], 0
     for k, s in enumerate(sizes):
         me = np.sort(ids[at:at + s])   # members of any id, so that out-lists mix
         at += s
@@ -46,6 +48,23 @@ def _graph(sizes, density, stray, seed):
 def test_internal_lists(sizes, density, stray, retuned):
     g, labels = _graph(sizes, density, stray, len(sizes))
     want = O.wcc(g, labels, np.bincount(labels))
+    _check(g, labels, want, retuned)
+
+
+@pytest.mark.parametrize("size", [3, 8, 9, 16, 17, 32, 33])
+@pytest.mark.parametrize("bits", [5, 6, 7])
+def test_entries_of_one_slot(size, bits):
+    """A community whose ids all share the slot of the register groups' tables (the upper
+    bits of the multiplicative hash), with every second vertex of another one among them."""
+    n = 64 << bits
+    ids = np.arange(n)
+    same = ids[(ids * 0x9E3779B1 % 2 ** 32) >> (32 - bits) == 5]
+    ids = np.concatenate([same[:size], np.setdiff1d(ids, same)[: 2 * size]])
+    g, labels = _graph([size, 2 * size], 0.8, 300, size, n, ids)
+    _check(g, labels, O.wcc(g, labels, np.bincount(labels[labels != scd_gb300.INVALID_LABEL])), False)
+
+
+def _check(g, labels, want, retuned):
     with scd_gb300.Engine(0) as eng:
         eng.transfer_graph(g)
         if retuned:   # the lists follow the buckets of another split
