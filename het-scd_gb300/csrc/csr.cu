@@ -119,7 +119,8 @@ k_sort_rows_warp_e(const uint32_t *__restrict__ list, uint32_t count, const uint
 // exchange stages, three radix passes are a third of its instructions; the counters of a
 // pass are W x 256 whatever the row's length, hence the two sizes. R-MAT scale 22, both
 // sorts, rows of 513 to 4096: 2.5 ms by the network, 2.2 with one size of 16 warps and ranks
-// by __match_any_sync, 1.66 ms so.)
+// by __match_any_sync, 1.66 ms so; 1.54 ms with four times the resident CTAs, handed out as
+// rows end.)
 template <int W>
 __global__ void __launch_bounds__(W * 32, 64 / W)
 k_sort_rows_radix(const uint32_t *__restrict__ list, uint32_t count, const uint32_t *__restrict__ off, int bits,
@@ -382,12 +383,12 @@ void sort_rows(Ctx &c, const uint32_t *off, uint32_t nrows, uint32_t *vals, bool
     }
     const int vbits = ceil_log2(nrows < 2 ? 2 : nrows);   // values are row numbers
     if (cnt[4]) {
-        k_sort_rows_radix<8><<<grid_for(cnt[4], 1, 152 * 8), 256, 0, s>>>(list[4], cnt[4], off, vbits, vals, dedup, udeg);
+        k_sort_rows_radix<8><<<grid_for(cnt[4], 1, 152 * 32), 256, 0, s>>>(list[4], cnt[4], off, vbits, vals, dedup, udeg);
         CK_LAUNCH("k_sort_rows_radix2048");
         c.launches++;
     }
     if (cnt[5]) {
-        k_sort_rows_radix<16><<<grid_for(cnt[5], 1, 152 * 4), 512, 0, s>>>(list[5], cnt[5], off, vbits, vals, dedup, udeg);
+        k_sort_rows_radix<16><<<grid_for(cnt[5], 1, 152 * 16), 512, 0, s>>>(list[5], cnt[5], off, vbits, vals, dedup, udeg);
         CK_LAUNCH("k_sort_rows_radix4096");
         c.launches++;
     }

@@ -552,7 +552,7 @@ void convert_edges(Ctx &c, const uint32_t *pairs_in, uint64_t count, const std::
     CK(cudaStreamSynchronize(s));
     const uint32_t m1 = hm[0], core_members = hm[1], core_bound = hm[2];
     DevBuf<uint32_t> orow(m1 ? m1 : 1, s), ocol(m1 ? m1 : 1, s), icol(m1 ? m1 : 1, s);
-    k_row_orient<<<grid_for((uint64_t)n1 * 32, TPB), TPB, 0, s>>>(off1.get(), n1, vals.get(), cnt.get(), obeg.get(),
+    k_row_orient<<<grid_for((uint64_t)n1 * 32, TPB, 152 * 256), TPB, 0, s>>>(off1.get(), n1, vals.get(), cnt.get(), obeg.get(),
                                                                   ibeg.get(), orow.get(), ocol.get(), icol.get());
     CK_LAUNCH("k_row_orient");
     k_long_orient<<<152 * 2, LONG_THREADS, 0, s>>>(off1.get(), longs.get(), nlong.get() + 1, vals.get(), cnt.get(),
@@ -642,7 +642,7 @@ void convert_edges(Ctx &c, const uint32_t *pairs_in, uint64_t count, const std::
         const Spread at2(n2, NG == 1);
         DevBuf<uint32_t> fill(at2.size(), s);
         CK(cudaMemsetAsync(fill.get(), 0, at2.size() * 4, s));
-        k_final_fill<<<grid_for(m1, TPB), TPB, 0, s>>>(orow.get(), ocol.get(), oflag.get(), m1, rank.get(), g.indices,
+        k_final_fill<<<grid_for(m1, TPB, 152 * 256), TPB, 0, s>>>(orow.get(), ocol.get(), oflag.get(), m1, rank.get(), g.indices,
                                                       at2, fill.get(), g.adj);
         CK_LAUNCH("k_final_fill");
         sort_rows(c, g.indices, n2, g.adj, false, nullptr, s);
