@@ -444,8 +444,10 @@ void iterate_async(Ctx &c, double threshold, double *trace, int max_trace) {
     c.labels = c.labels_next;
     c.labels_next = t;
     c.cur ^= 1;
-    launch_stats_wcc(c, c.labels, c.st[c.cur], frozen);
-    batch_step(c, threshold, trace, max_trace);
+    const Batch &b = c.b;
+    launch_stats_wcc(c, c.labels, c.st[c.cur], frozen,
+                     BatchStep{b.best_wcc, b.active, b.improved, b.iters, threshold, b.n_active, trace, max_trace});
+    copy_improved(c);
 }
 
 // Kernel nodes of a captured graph (the launches one replay makes).

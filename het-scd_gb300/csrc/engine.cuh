@@ -255,7 +255,7 @@ struct Ctx {
     double alpha = 1.0;
     cudaStream_t stream = nullptr;
     cudaStream_t side = nullptr;
-    cudaStream_t aux = nullptr;                        // improve: the hub kernel beside the other classes
+    cudaStream_t aux = nullptr;                        // improve: the hub kernel, or without hubs the longer rows', beside the other classes
     cudaEvent_t aux_fork = nullptr, aux_join = nullptr;
     std::string err;
     uint64_t launches = 0;
@@ -350,18 +350,29 @@ double compute_wcc(Ctx &c, const uint32_t *labels, const Stats &st);
 // frozen_graphs: vertices of graphs whose loop has ended keep their labels
 // clear (nullable): statistics to clear for the labels this call makes
 void improve(Ctx &c, const uint32_t *labels, const Stats &st, uint32_t *next, bool frozen_graphs, Stats *clear);
-// statistics (st cleared by improve) and WCC of an iteration's labels
-void launch_stats_wcc(Ctx &c, const uint32_t *labels, Stats &st, bool frozen_graphs);
+// per-graph loop control after a WCC (src/main.cpp:68-81): iteration count, best WCC,
+// convergence, whether the labels are the best yet; *n_active receives the graphs still
+// running (active == nullptr: no step)
+struct BatchStep {
+    double *best;
+    uint8_t *active, *improved;
+    int32_t *iters;
+    double threshold;
+    uint32_t *n_active;
+    double *trace;
+    int max_trace;
+};
+// statistics (st cleared by improve) and WCC of an iteration's labels, and the step they decide
+void launch_stats_wcc(Ctx &c, const uint32_t *labels, Stats &st, bool frozen_graphs, const BatchStep &step = BatchStep{});
 double read_wcc(Ctx &c);   // waits for the WCC of graph 0
 // per-graph WCC in c.b.wcc (device); frozen_graphs: skip the graphs of a batch that stopped iterating
 // with_stats: also adds the labels' statistics to st
-void launch_wcc(Ctx &c, const uint32_t *labels, const Stats &st, bool frozen_graphs = false, bool with_stats = false);
+void launch_wcc(Ctx &c, const uint32_t *labels, const Stats &st, bool frozen_graphs = false, bool with_stats = false,
+                const BatchStep &step = BatchStep{});
 void compute_p_ext(Ctx &c);   // launches on the side stream
 void join_p_ext(Ctx &c);      // main stream waits for p_ext (outside captures)
 void host_p_ext(Ctx &c);      // host copies of p_ext (b.h_p_ext, g.p_ext)
-// per-graph loop control after a WCC (src/main.cpp:68-81): iteration count,
-// best WCC, best labels, convergence; *n_active receives the graphs still running
-void batch_step(Ctx &c, double threshold, double *trace = nullptr, int max_trace = 0);
+void copy_improved(Ctx &c);   // best labels of the graphs whose last step improved them
 void batch_reset(Ctx &c);   // best := current WCC, all non-empty graphs active
 
 }  // namespace scd

@@ -1029,6 +1029,34 @@ void improve(Ctx &c, const uint32_t *labels, const Stats &st, uint32_t *next, bo
         CK(cudaEventRecord(c.aux_join, c.aux));
         c.launches++;
     }
+    // without hubs, the classes above the groups' run there: on small graphs both sides are a
+    // chain of latencies (10,000 vertices: 9 of a step's 95 us)
+    const uint32_t upper = k.count[3] + k.count[4] + k.count[5] + k.count[6], groups = k.count[0] + k.count[1] + k.count[2];
+    const bool beside = !k.count[7] && c.aux && upper && groups;
+    cudaStream_t side = beside ? c.aux : s;
+    if (beside) {
+        CK(cudaEventRecord(c.aux_fork, s));
+        CK(cudaStreamWaitEvent(c.aux, c.aux_fork, 0));
+    }
+    if (k.count[3]) {
+        const uint32_t take = take_of(k.count[3], 1, WARP_CTAS * WWARPS);
+        k_improve_warp<<<grid_of(k.count[3], take, WWARPS, WARP_CTAS), WWARPS * 32, 0, side>>>(k.list[3], k.count[3], take, a);
+        CK_LAUNCH("k_improve_warp");
+        c.launches++;
+    }
+    if (k.count[4]) {
+        launch_cta<128, 2048>(k.list[4], k.count[4], a, side, 152 * 16);
+        c.launches++;
+    }
+    if (k.count[5]) {
+        launch_cta<256, 4096>(k.list[5], k.count[5], a, side, 152 * 7);
+        c.launches++;
+    }
+    if (k.count[6]) {
+        launch_cta<512, 8192>(k.list[6], k.count[6], a, side, 152 * 2);
+        c.launches++;
+    }
+    if (beside) CK(cudaEventRecord(c.aux_join, c.aux));
     GroupWork gw{};
     for (int j = 0; j < 3; j++) {   // classes 2, 1, 0: groups of 32, 16 and 8 lanes
         const uint32_t n = k.count[2 - j];
@@ -1042,25 +1070,7 @@ void improve(Ctx &c, const uint32_t *labels, const Stats &st, uint32_t *next, bo
         CK_LAUNCH("k_improve_groups");
         c.launches++;
     }
-    if (k.count[3]) {
-        const uint32_t take = take_of(k.count[3], 1, WARP_CTAS * WWARPS);
-        k_improve_warp<<<grid_of(k.count[3], take, WWARPS, WARP_CTAS), WWARPS * 32, 0, s>>>(k.list[3], k.count[3], take, a);
-        CK_LAUNCH("k_improve_warp");
-        c.launches++;
-    }
-    if (k.count[4]) {
-        launch_cta<128, 2048>(k.list[4], k.count[4], a, s, 152 * 16);
-        c.launches++;
-    }
-    if (k.count[5]) {
-        launch_cta<256, 4096>(k.list[5], k.count[5], a, s, 152 * 7);
-        c.launches++;
-    }
-    if (k.count[6]) {
-        launch_cta<512, 8192>(k.list[6], k.count[6], a, s, 152 * 2);
-        c.launches++;
-    }
-    if (fork) {
+    if (fork || beside) {
         CK(cudaStreamWaitEvent(s, c.aux_join, 0));
     } else if (k.count[7]) {
         k_improve_global<<<grid_for(k.count[7], 1, 152 * 2), GLOBAL_THREADS, 0, s>>>(k.list[7], k.count[7], a,

@@ -129,22 +129,24 @@ __device__ __forceinline__ void intdeg_seg(RowSeg r, const uint32_t *nlow, const
 
 // int_tri_deg (src/wcc.cpp:124-126): per vertex, the internal edges that lie on an
 // internal triangle, counted from the out-slot flags of both endpoints; the out-slots
-// of rows of degree <= 256 as 32-row streams in id order, longer rows as RowWork chunks
+// of rows of degree <= 256 as streams of up to 32 rows in id order, longer rows as RowWork
+// chunks. (A stream's steps are a chain of dependent loads: small graphs have fewer rows in
+// one, so that every SM has its warps. 10,000 vertices, 32 rows 15 us, 4 rows 6 us.)
 __global__ void __launch_bounds__(TPB)
-k_internal_degrees(uint32_t n, RowWork rw, const uint32_t *__restrict__ indices, const uint32_t *__restrict__ nlow,
+k_internal_degrees(uint32_t n, uint32_t rows, RowWork rw, const uint32_t *__restrict__ indices, const uint32_t *__restrict__ nlow,
                    const uint32_t *__restrict__ adj, const uint8_t *__restrict__ flag, int32_t *itdeg,
                    LabelFilter skip) {
     const int lane = threadIdx.x & 31;
     const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
-    const uint32_t groups = (n + 31) / 32, nchunks = rw.nchunks;
+    const uint32_t groups = (n + rows - 1) / rows, nchunks = rw.nchunks;
     for (uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < groups + nchunks; w += warps) {
         if (w >= groups) {   // a piece of a long row
             intdeg_seg<32>(chunk_seg(rw, w - groups, indices), nlow, adj, flag, itdeg, skip);
             continue;
         }
-        const uint32_t u = w * 32 + lane;
+        const uint32_t u = w * rows + lane;
         uint32_t b = 0, len = 0;
-        if (u < n && !skip.frozen(u)) {
+        if (lane < (int)rows && u < n && !skip.frozen(u)) {
             b = indices[u];
             if (indices[u + 1] - b <= RowWork::CHUNK) len = nlow[u];
         }
@@ -242,18 +244,42 @@ k_wcc_partial(const uint32_t *__restrict__ fin_off, const uint32_t *__restrict__
 }
 
 // one block per graph: fixed-order sum of the graph's partials, divided by its n
+// src/main.cpp:68-81 for a graph still iterating (thread 0 of its CTA of k_wcc_final: a launch
+// of its own was 3 us of a small graph's step): count the iteration, remember whether it beat
+// the best WCC, stop when it is below best*(1+threshold)
+__device__ __forceinline__ void batch_step_of(uint32_t g, double w, const BatchStep &st) {
+    st.improved[g] = 0;
+    if (!st.active[g]) return;
+    const double b = st.best[g];
+    const int it = ++st.iters[g];
+    if (st.trace && it <= st.max_trace) st.trace[(size_t)g * st.max_trace + it - 1] = w;
+    if (w > b) st.improved[g] = 1;
+    if (w < dmul(b, dadd(1.0, st.threshold))) {
+        st.active[g] = 0;
+    } else {
+        st.best[g] = w;
+        atomicAdd(st.n_active, 1u);
+    }
+}
+
 __global__ void __launch_bounds__(TPB) k_wcc_final(const double *__restrict__ partial,
                                                    const uint32_t *__restrict__ blk_off,
                                                    const uint32_t *__restrict__ fin_off, double *out,
-                                                   const uint8_t *__restrict__ active = nullptr) {
+                                                   const uint8_t *active, BatchStep step) {
     __shared__ double sh[TPB / 32];
     const uint32_t g = blockIdx.x;
-    if (active && !active[g]) return;
+    if (active && !active[g]) {
+        if (step.active && threadIdx.x == 0) step.improved[g] = 0;
+        return;
+    }
     const uint32_t p0 = blk_off[g], parts = blk_off[g + 1] - p0, n = fin_off[g + 1] - fin_off[g];
     double s = 0.0;
     for (uint32_t i = threadIdx.x; i < parts; i += TPB) s = dadd(s, partial[p0 + i]);
     double r = block_sum_fixed(s, sh);
-    if (threadIdx.x == 0) out[g] = n > 0 ? ddiv(r, (double)n) : 0.0;
+    if (threadIdx.x) return;
+    r = n > 0 ? ddiv(r, (double)n) : 0.0;
+    out[g] = r;
+    if (step.active) batch_step_of(g, r, step);
 }
 
 // ---- p_ext ---------------------------------------------------------------------
@@ -443,27 +469,6 @@ __global__ void k_pext_tree(const uint32_t *__restrict__ fin_off, const uint32_t
 
 // ---- per-graph loop control ---------------------------------------------------
 
-// src/main.cpp:68-81 for every graph still iterating: count the iteration,
-// remember whether it beat the best WCC, stop when it is below best*(1+threshold)
-__global__ void k_batch_step(uint32_t G, const double *__restrict__ wcc, double *best, uint8_t *active,
-                             uint8_t *improved, int32_t *iters, double threshold, uint32_t *n_active, double *trace,
-                             int max_trace) {
-    for (uint32_t g = blockIdx.x * blockDim.x + threadIdx.x; g < G; g += gridDim.x * blockDim.x) {
-        improved[g] = 0;
-        if (!active[g]) continue;
-        const double w = wcc[g], b = best[g];
-        const int it = ++iters[g];
-        if (trace && it <= max_trace) trace[(size_t)g * max_trace + it - 1] = w;
-        if (w > b) improved[g] = 1;
-        if (w < dmul(b, dadd(1.0, threshold))) {
-            active[g] = 0;
-        } else {
-            best[g] = w;
-            atomicAdd(n_active, 1u);
-        }
-    }
-}
-
 __global__ void k_copy_improved(uint32_t n, const uint32_t *__restrict__ gid, const uint8_t *__restrict__ improved,
                                 const uint32_t *__restrict__ labels, uint32_t *best) {
     for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x)
@@ -481,18 +486,11 @@ __global__ void k_batch_reset(uint32_t G, const uint32_t *__restrict__ fin_off, 
 
 }  // namespace
 
-void batch_step(Ctx &c, double threshold, double *trace, int max_trace) {
-    Batch &b = c.b;
-    cudaStream_t s = c.stream;
-    CK(cudaMemsetAsync(b.n_active, 0, 4, s));
-    k_batch_step<<<grid_for(b.G, TPB), TPB, 0, s>>>(b.G, b.wcc, b.best_wcc, b.active, b.improved, b.iters, threshold,
-                                                     b.n_active, trace, max_trace);
-    CK_LAUNCH("k_batch_step");
-    if (c.g.n) {
-        k_copy_improved<<<grid_for(c.g.n, TPB), TPB, 0, s>>>(c.g.n, b.gid, b.improved, c.labels, c.best);
-        CK_LAUNCH("k_copy_improved");
-    }
-    c.launches += 2;
+void copy_improved(Ctx &c) {
+    if (!c.g.n) return;
+    k_copy_improved<<<grid_for(c.g.n, TPB), TPB, 0, c.stream>>>(c.g.n, c.b.gid, c.b.improved, c.labels, c.best);
+    CK_LAUNCH("k_copy_improved");
+    c.launches++;
 }
 
 void batch_reset(Ctx &c) {
@@ -646,11 +644,17 @@ k_internal_lists(uint32_t n, uint32_t rows, WarpRows longer, uint32_t most_short
     }
 }
 
+// rows a warp takes: as many as leave every SM its 32 warps
+uint32_t rows_a_warp(uint32_t n) {
+    uint32_t rows = 4;
+    while (rows < 32 && (uint64_t)rows * 2 * NUM_SMS_HINT * 32 <= n) rows <<= 1;
+    return rows;
+}
+
 template <bool LISTS, bool STATS>
 void launch_internal_lists(Ctx &c, LabelFilter lf, const Stats &st) {
     const Graph &g = c.g;
-    uint32_t rows = 4;   // as many as leave every SM its 32 warps
-    while (rows < 32 && (uint64_t)rows * 2 * NUM_SMS_HINT * 32 <= g.n) rows <<= 1;
+    const uint32_t rows = rows_a_warp(g.n);
     WarpRows longer{};
     for (int k = 0; k < WarpRows::K; k++)   // the longest first
         longer.set(k, c.wplan.verts[TcPlan::K - 1 - k], c.wplan.nverts[TcPlan::K - 1 - k]);
@@ -689,10 +693,12 @@ void collect_stats(Ctx &c, const uint32_t *labels, Stats &st, bool frozen_graphs
     c.launches++;
 }
 
-void launch_wcc(Ctx &c, const uint32_t *labels, const Stats &st, bool frozen_graphs, bool with_stats) {
+void launch_wcc(Ctx &c, const uint32_t *labels, const Stats &st, bool frozen_graphs, bool with_stats,
+                const BatchStep &step) {
     const Graph &g = c.g;
     cudaStream_t s = c.stream;
-    if (g.n == 0) {
+    if (step.active) CK(cudaMemsetAsync(step.n_active, 0, 4, s));
+    if (g.n == 0) {   // (no graph is active)
         CK(cudaMemsetAsync(c.b.wcc, 0, sizeof(double) * c.b.G, s));
         return;
     }
@@ -706,8 +712,9 @@ void launch_wcc(Ctx &c, const uint32_t *labels, const Stats &st, bool frozen_gra
     // the plan's buckets (by full out-degree) stay valid: internal lists are never longer
     const Oriented o{g.indices, c.int_len, c.int_adj, g.n};
     count_internal_triangles(c, o, c.itcount, c.slot_flag);
-    k_internal_degrees<<<grid_for(((uint64_t)(g.n + 31) / 32 + g.rows.nchunks) * 32, TPB), TPB, 0, s>>>(
-        g.n, g.rows, g.indices, c.int_len, c.int_adj, c.slot_flag, c.itdeg, lf);
+    const uint32_t rows = rows_a_warp(g.n);
+    k_internal_degrees<<<grid_for((((uint64_t)g.n + rows - 1) / rows + g.rows.nchunks) * 32, TPB), TPB, 0, s>>>(
+        g.n, rows, g.rows, g.indices, c.int_len, c.int_adj, c.slot_flag, c.itdeg, lf);
     CK_LAUNCH("k_internal_degrees");
     c.launches++;
     if (b.blocks) {
@@ -715,16 +722,16 @@ void launch_wcc(Ctx &c, const uint32_t *labels, const Stats &st, bool frozen_gra
                                                c.itcount, c.itdeg, c.alpha, c.wcc_part, active);
         CK_LAUNCH("k_wcc_partial");
     }
-    k_wcc_final<<<b.G, TPB, 0, s>>>(c.wcc_part, b.blk_off, b.fin_off, b.wcc, active);
+    k_wcc_final<<<b.G, TPB, 0, s>>>(c.wcc_part, b.blk_off, b.fin_off, b.wcc, active, step);
     CK_LAUNCH("k_wcc_final");
     c.launches += 3;
 }
 
 // statistics (st cleared by improve) and WCC of the labels of an iteration
-void launch_stats_wcc(Ctx &c, const uint32_t *labels, Stats &st, bool frozen_graphs) {
+void launch_stats_wcc(Ctx &c, const uint32_t *labels, Stats &st, bool frozen_graphs, const BatchStep &step) {
     const bool fused = stats_from_out_lists(c);
     if (!fused) collect_stats(c, labels, st, frozen_graphs);
-    launch_wcc(c, labels, st, frozen_graphs, fused);
+    launch_wcc(c, labels, st, frozen_graphs, fused, step);
 }
 
 double read_wcc(Ctx &c) {
@@ -766,7 +773,7 @@ void compute_p_ext(Ctx &c) {
             k_pext_tree<<<b.blocks, TPB, 0, s>>>(b.fin_off, b.blk_off, b.blk_gid, term.get(), part.get());
             CK_LAUNCH("k_pext_tree");
         }
-        k_wcc_final<<<b.G, TPB, 0, s>>>(part.get(), b.blk_off, b.fin_off, b.p_ext);
+        k_wcc_final<<<b.G, TPB, 0, s>>>(part.get(), b.blk_off, b.fin_off, b.p_ext, nullptr, BatchStep{});
         CK_LAUNCH("k_wcc_final");
         c.launches += 2;
         // (an empty graph's p_ext is 0 here, NaN in the index-ordered mode like the reference's 0/0)

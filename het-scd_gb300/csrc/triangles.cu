@@ -1078,11 +1078,12 @@ UnitList bucket_units(const TcPlan &plan, int k) {
 
 void launch_small(Ctx &c, const Oriented &o, uint32_t max_len, const uint32_t *walk, const Dir &dir, uint32_t *tcount,
                   uint8_t *flag, cudaStream_t s) {
-    // 16 vertices a warp, fewer where that would leave SMs short of their 64 warps; a grid of
+    // 16 vertices a warp, fewer where that would leave SMs short of their 64 warps (10,000
+    // vertices, a step: 4 a warp 16 us, 1 a warp 10 us); a grid of
     // one unit a warp, because units of dense graphs take 25 times as long as those of sparse
     // ones and CTAs that are handed out even that out (96 planted graphs, all counts of a run:
     // 8 CTAs an SM 7.3 ms, 16 6.8 ms, 48 6.0 ms, 128 5.8 ms; with 32 vertices 6.1 ms, with 8 6.0 ms)
-    uint32_t rows = 4;
+    uint32_t rows = 1;
     while (rows < 16 && (uint64_t)rows * 2 * NUM_SMS_HINT * 64 <= o.n) rows <<= 1;
     k_tc_small<<<grid_for(((uint64_t)o.n + rows - 1) / rows * 32, 256, 1u << 20), 256, 0, s>>>(o, rows, max_len, walk, dir, tcount,
                                                                                                 flag);
