@@ -474,6 +474,11 @@ namespace {
 template <typename F>
 int guarded(scd_ctx *ctx, F &&f) {
     if (!ctx) return SCD_ERR_ARG;
+    struct Blocks {   // this thread's temporaries come from the context's blocks
+        BlockCache *before = BlockCache::current();
+        explicit Blocks(BlockCache *b) { BlockCache::current() = b; }
+        ~Blocks() { BlockCache::current() = before; }
+    } blocks(&ctx->c.blocks);
     try {
         CK(cudaSetDevice(ctx->c.device));
         f(ctx->c);
@@ -509,9 +514,7 @@ void set_labels(Ctx &c, const uint32_t *host_labels) {
         k_max_label<<<grid_for(g.n, TPB), TPB, 0, s>>>(g.n, c.labels, mx.get());
         CK_LAUNCH("k_max_label");
     }
-    uint32_t nc = 0;
-    CK(cudaMemcpyAsync(&nc, mx.get(), 4, cudaMemcpyDeviceToHost, s));
-    CK(cudaStreamSynchronize(s));
+    const uint32_t nc = c.read(mx.get());
     if (nc > g.n) throw Error(SCD_ERR_ARG, "labels must be < n or SCD_INVALID_LABEL");
     c.num_comms = nc;
     c.b.h_comm_off.assign(c.b.G + 1, nc);
@@ -673,6 +676,7 @@ int scd_create(scd_ctx **out, int device_id, int work_group_size, unsigned flags
             CK(cudaDeviceGetStreamPriorityRange(&lowest, &prio));
         }
         CK(cudaStreamCreateWithPriority(&c.stream, cudaStreamNonBlocking, prio));
+        c.blocks.stream = c.stream;
         CK(cudaStreamCreateWithPriority(&c.side, cudaStreamNonBlocking, prio));
         CK(cudaStreamCreateWithPriority(&c.aux, cudaStreamNonBlocking, prio));
         CK(cudaEventCreateWithFlags(&c.aux_fork, cudaEventDisableTiming));
@@ -694,6 +698,7 @@ void scd_destroy(scd_ctx *ctx) {
     cudaSetDevice(c.device);
     resident_destroy(c);
     c.free_all();
+    c.blocks.give_back();
     if (c.stream) cudaStreamSynchronize(c.stream);
     {   // hand the cached pool memory back (arrays still in use elsewhere are not affected)
         cudaMemPool_t pool;

@@ -14,6 +14,7 @@
 //   wcc_part[], wcc_sum         fixed-order WCC reduction
 #pragma once
 
+#include <cstring>
 #include <string>
 #include <vector>
 
@@ -234,7 +235,7 @@ double autotune_tc(Ctx &c, std::vector<std::string> *report);
 void prepare_tc_kernels();
 void prepare_improve_kernels();
 
-constexpr int HOST_PLAN = 2, HOST_SUMS = 56, HOST_WORDS = 64;   // pinned words of a context (Ctx::host_u32)
+constexpr int HOST_PLAN = 2, HOST_SUMS = 56, HOST_READ = 64, HOST_WORDS = 68;   // pinned words of a context (Ctx::host_u32)
 
 struct Ctx;
 // records [start, end) of a phase on the context's stream when profiling
@@ -296,6 +297,7 @@ struct Ctx {
     bool resident = false;            // every iteration skips the graphs that stopped
 
     PhaseTimers timers;
+    BlockCache blocks;                // of the temporaries
     std::vector<void *> owned;        // device allocations freed with the graph
     uint64_t bytes = 0;
 
@@ -316,6 +318,18 @@ struct Ctx {
         return (T *)p;
     }
     void free_all();
+
+    // one value from the device, waited for; through pinned words (a copy to pageable memory
+    // is staged by the driver, 6 us more)
+    template <typename T>
+    T read(const T *dev) {
+        static_assert(sizeof(T) <= 4 * (HOST_WORDS - HOST_READ), "pinned words");
+        T v;
+        CK(cudaMemcpyAsync(host_u32 + HOST_READ, dev, sizeof(T), cudaMemcpyDeviceToHost, stream));
+        CK(cudaStreamSynchronize(stream));
+        std::memcpy(&v, host_u32 + HOST_READ, sizeof(T));
+        return v;
+    }
 };
 
 // preprocess.cu

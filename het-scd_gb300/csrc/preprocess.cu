@@ -422,14 +422,6 @@ __global__ void k_final_offsets(uint32_t G, const uint32_t *__restrict__ ren_off
         fin_off[g] = kscan[ren_off[g]];
 }
 
-template <typename T>
-T read_scalar(const T *dev, cudaStream_t s) {
-    T h;
-    CK(cudaMemcpyAsync(&h, dev, sizeof(T), cudaMemcpyDeviceToHost, s));
-    CK(cudaStreamSynchronize(s));
-    return h;
-}
-
 }  // namespace
 
 void convert_edges(Ctx &c, const uint32_t *pairs_in, uint64_t count, const std::vector<uint64_t> *rec_off_h) {
@@ -460,7 +452,7 @@ void convert_edges(Ctx &c, const uint32_t *pairs_in, uint64_t count, const std::
         }
         raw_off.alloc(NG + 1, s);
         scan_exclusive<uint64_t>(gmax.get(), raw_off.get(), NG, s);
-        if (read_scalar(raw_off.get() + NG, s) >= 0xffffffffull)
+        if (c.read(raw_off.get() + NG) >= 0xffffffffull)
             throw Error(SCD_ERR_LIMIT, "the graphs of a batch need more than 2^32-1 vertex ids together");
         shifted.alloc(2 * count + 1, s);
         if (count) {
@@ -482,7 +474,7 @@ void convert_edges(Ctx &c, const uint32_t *pairs_in, uint64_t count, const std::
     CK(cudaMemsetAsync(mx.get(), 0, 4, s));
     k_reduce_max<uint32_t><<<grid_for(2 * count, TPB, 152 * 16), TPB, 0, s>>>(pairs, 2 * count, mx.get());
     CK_LAUNCH("k_reduce_max");
-    const uint32_t n_raw = read_scalar(mx.get(), s) + 1;
+    const uint32_t n_raw = c.read(mx.get()) + 1;
     if (n_raw == 0) throw Error(SCD_ERR_LIMIT, "vertex id 2^32-1 is not supported");
     DevBuf<uint32_t> rename(n_raw, s);
     CK(cudaMemsetAsync(rename.get(), 0xff, (size_t)n_raw * 4, s));
@@ -496,7 +488,7 @@ void convert_edges(Ctx &c, const uint32_t *pairs_in, uint64_t count, const std::
     scan_exclusive<uint32_t>(PopcountOf{bits.get()}, wpre.get(), words, s);
     k_rename<<<grid_for(n_raw, TPB), TPB, 0, s>>>(rename.get(), n_raw, bits.get(), wpre.get());
     CK_LAUNCH("k_rename");
-    const uint32_t n1 = read_scalar(wpre.get() + words, s);
+    const uint32_t n1 = c.read(wpre.get() + words);
     bits.release();
     wpre.release();
     DevBuf<uint32_t> ren_off(NG + 1, s);   // renamed ids of graph g: [ren_off[g], ren_off[g+1])
@@ -519,7 +511,7 @@ void convert_edges(Ctx &c, const uint32_t *pairs_in, uint64_t count, const std::
     k_pair_degrees<<<G, TPB, 0, s>>>(pairs, count, rename.get(), at1, cnt.get());
     CK_LAUNCH("k_pair_degrees");
     scan_exclusive<uint32_t>(SpreadCounters{cnt.get(), at1}, off1.get(), n1, s);
-    const uint32_t entries = read_scalar(off1.get() + n1, s);
+    const uint32_t entries = c.read(off1.get() + n1);
     DevBuf<uint32_t> vals(entries ? entries : 1, s);
     CK(cudaMemsetAsync(cnt.get(), 0, at1.size() * 4, s));
     k_pair_fill<<<G, TPB, 0, s>>>(pairs, count, rename.get(), off1.get(), at1, cnt.get(), vals.get());
@@ -629,7 +621,7 @@ void convert_edges(Ctx &c, const uint32_t *pairs_in, uint64_t count, const std::
                                                        g.tri_deg);
     CK_LAUNCH("k_rank_of");
     scan_exclusive<uint32_t>(DegreeOf{g.tri_deg}, g.indices, n2, s);
-    const uint32_t m2 = read_scalar(g.indices + n2, s) / 2;
+    const uint32_t m2 = c.read(g.indices + n2) / 2;
     g.m = m2;
     g.adj = c.alloc<uint32_t>(2 * (size_t)m2);
     c.b.G = NG;

@@ -6,39 +6,114 @@
 // (Scan, SegSortKeysFromIndices, ReduceByKey, Reduce; src/cuda.cu:205-345).
 #pragma once
 
+#include <mutex>
+#include <utility>
+
 #include "common.cuh"
 
 namespace scd {
 
 // ---------------------------------------------------------------------------
-// stream-ordered temporary device buffer
+// stream-ordered temporary device buffers
+
+// Blocks of up to 1 MB that a context keeps between its temporaries instead of returning each to
+// the device's pool: a cudaMallocAsync and its free are 1.8 us of host time, and a call on a
+// small graph, bound by the host, makes about ninety of them. Sizes are powers of two; at most
+// 64 blocks of a size and 32 MB together are kept, the rest and (at the context's end) all of
+// them go back. A block is only handed out again for work on the stream it was used on, later in
+// that stream, as cudaFreeAsync and cudaMallocAsync on one stream would. Locked: a resident set
+// lets another thread than the stepping one work on the context.
+class BlockCache {
+public:
+    static constexpr int LOW = 9, HIGH = 20, SIZES = HIGH - LOW + 1, SLOTS = 64;
+    static constexpr size_t KEEP = 32u << 20;
+    cudaStream_t stream = nullptr;   // of the context
+
+    static int size_of(size_t bytes) {   // SIZES: too large to keep
+        int k = 0;
+        while (k < SIZES && bytes > ((size_t)1 << (LOW + k))) k++;
+        return k;
+    }
+    void *get(int k) {
+        {
+            std::lock_guard<std::mutex> hold(lock_);
+            if (n_[k]) {
+                kept_ -= (size_t)1 << (LOW + k);
+                return block_[k][--n_[k]];
+            }
+        }
+        void *p = nullptr;
+        CK(cudaMallocAsync(&p, (size_t)1 << (LOW + k), stream));
+        return p;
+    }
+    void put(void *p, int k) {
+        {
+            std::lock_guard<std::mutex> hold(lock_);
+            if (n_[k] < SLOTS && kept_ + ((size_t)1 << (LOW + k)) <= KEEP) {
+                kept_ += (size_t)1 << (LOW + k);
+                block_[k][n_[k]++] = p;
+                return;
+            }
+        }
+        cudaFreeAsync(p, stream);
+    }
+    void give_back() {
+        std::lock_guard<std::mutex> hold(lock_);
+        for (int k = 0; k < SIZES; k++)
+            while (n_[k]) cudaFreeAsync(block_[k][--n_[k]], stream);
+        kept_ = 0;
+    }
+    // the cache of the context whose call this thread is in
+    static BlockCache *&current() {
+        static thread_local BlockCache *c = nullptr;
+        return c;
+    }
+
+private:
+    std::mutex lock_;
+    void *block_[SIZES][SLOTS];
+    int n_[SIZES] = {};
+    size_t kept_ = 0;
+};
 
 template <typename T>
 struct DevBuf {
     T *p = nullptr;
     size_t n = 0;
     cudaStream_t s = nullptr;
+    BlockCache *cache = nullptr;   // the block came from it (size class k), else from the device's pool
+    int k = 0;
     DevBuf() = default;
     DevBuf(size_t count, cudaStream_t stream) { alloc(count, stream); }
     void alloc(size_t count, cudaStream_t stream) {
         release();
         s = stream;
         n = count;
-        if (count) CK(cudaMallocAsync((void **)&p, count * sizeof(T), stream));
+        if (!count) return;
+        BlockCache *c = BlockCache::current();
+        k = BlockCache::size_of(count * sizeof(T));
+        if (c && c->stream == stream && k < BlockCache::SIZES) {
+            p = (T *)c->get(k);
+            cache = c;
+        } else {
+            CK(cudaMallocAsync((void **)&p, count * sizeof(T), stream));
+        }
     }
     void release() {
-        if (p) cudaFreeAsync(p, s);
+        if (p && cache) cache->put(p, k);
+        else if (p) cudaFreeAsync(p, s);
         p = nullptr;
+        cache = nullptr;
         n = 0;
     }
     ~DevBuf() { release(); }
     DevBuf(const DevBuf &) = delete;
     DevBuf &operator=(const DevBuf &) = delete;
-    DevBuf(DevBuf &&o) noexcept : p(o.p), n(o.n), s(o.s) { o.p = nullptr; o.n = 0; }
+    DevBuf(DevBuf &&o) noexcept { *this = std::move(o); }
     DevBuf &operator=(DevBuf &&o) noexcept {
         release();
-        p = o.p; n = o.n; s = o.s;
-        o.p = nullptr; o.n = 0;
+        p = o.p; n = o.n; s = o.s; cache = o.cache; k = o.k;
+        o.p = nullptr; o.cache = nullptr; o.n = 0;
         return *this;
     }
     T *get() const { return p; }

@@ -139,8 +139,7 @@ uint64_t parse_edge_text(Ctx &c, const char *text, uint64_t bytes, DevBuf<uint32
         k_count_newlines<<<(unsigned)chunks, TPB, 0, s>>>(text, bytes, per.get());
         CK_LAUNCH("k_count_newlines");
         scan_exclusive<uint32_t>((const uint32_t *)per.get(), nl_off.get(), chunks, s);
-        CK(cudaMemcpyAsync(&nl, nl_off.get() + chunks, 4, cudaMemcpyDeviceToHost, s));
-        CK(cudaStreamSynchronize(s));
+        nl = c.read(nl_off.get() + chunks);
     }
     if (nl >= 0xfffffffeu) throw Error(SCD_ERR_LIMIT, "more than 2^32-2 text lines");
     const uint32_t lines = nl + 1;   // the piece after the last newline (possibly empty) is a line too
@@ -157,11 +156,10 @@ uint64_t parse_edge_text(Ctx &c, const char *text, uint64_t bytes, DevBuf<uint32
                                                        err.get());
     CK_LAUNCH("k_parse_lines");
     scan_exclusive<uint32_t>(IsRecord{status.get()}, pos.get(), lines, s);
-    unsigned long long e = 0;
-    uint32_t count = 0;
-    CK(cudaMemcpyAsync(&e, err.get(), 8, cudaMemcpyDeviceToHost, s));
-    CK(cudaMemcpyAsync(&count, pos.get() + lines, 4, cudaMemcpyDeviceToHost, s));
-    CK(cudaStreamSynchronize(s));
+    uint32_t *h = c.host_u32 + HOST_READ;
+    CK(cudaMemcpyAsync(h + 2, pos.get() + lines, 4, cudaMemcpyDeviceToHost, s));
+    const unsigned long long e = c.read(err.get());   // (waits for both)
+    const uint32_t count = h[2];
     c.launches += 4;
     if (e != ~0ull) {
         const uint64_t line = (e >> 2) + 1;
