@@ -34,6 +34,8 @@ RANGE = 54 * 1024 * 32   # row numbers of one bitmap range
 
 
 @pytest.mark.parametrize("lengths,repeats,extra", [
+    (list(range(1, 40)), 2, 0),
+    (list(range(1, 40)) * 800, 2, 1000),   # 32 rows a warp
     ([31, 32, 33, 64, 65, 128, 129, 256, 257], 7, 0),
     ([511, 512, 513, 1023, 1024, 1025, 2048, 4095], 0, 0),
     ([505, 1000, 4089, 4096], 7, 0),
@@ -42,7 +44,7 @@ RANGE = 54 * 1024 * 32   # row numbers of one bitmap range
     ([6000, 9000], 11, RANGE // 2 - 7600),   # one range, just
     ([6000, 9000], 11, RANGE // 2),          # two
     ([6000, 9000], 11, 16 * RANGE // 2 + 5000),   # more than the bitmap takes
-], ids=["warp", "radix", "radix-repeats", "bitmap", "long", "one-range", "two-ranges", "beyond"])
+], ids=["short", "short-many", "warp", "radix", "radix-repeats", "bitmap", "long", "one-range", "two-ranges", "beyond"])
 def test_rows_of_every_form(lengths, repeats, extra):
     pairs = _hubs(lengths, repeats, extra, 3)
     ref, _ = oracle.convert(pairs)
