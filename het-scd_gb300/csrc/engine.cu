@@ -354,7 +354,7 @@ void build_union_structure(Ctx &c, bool always_gid, bool check_symmetry) {
     }
     g.rows.llong = lists + hb[K];
     g.rows.nlong = hb[K + 1] - hb[K];
-    if (n) tc_plan_units(o, c.wplan, tc_lists, htc, s, true);
+    if (n) tc_plan_units(o, 0, c.wplan, tc_lists, htc, s, true);
     alloc_internal_work(c);
     // the pieces of the long rows and the table words of the last class: one more read, if there are any
     const uint32_t n_big = g.cls.count[K - 1];
@@ -1188,7 +1188,7 @@ int scd_autotune(scd_ctx *ctx, uint32_t *small_max, uint32_t *warp_max, uint32_t
         const double ms = autotune_tc(c, &lines);
         if (c.g.n) {   // the WCC plan follows the chosen split
             c.wplan = TcPlan();
-            tc_plan(c, Oriented{c.g.indices, c.g.nlow, c.g.adj, c.g.n}, c.wplan, c.stream, true, false);
+            tc_plan(c, Oriented{c.g.indices, c.g.nlow, c.g.adj, c.g.n}, 0, c.wplan, c.stream, true, false);
             alloc_internal_work(c);
         }
         if (small_max) *small_max = c.tc_small;

@@ -167,6 +167,7 @@ struct TcPlan {
     uint32_t dir_lo = 0, dir_hi = 0, dir_amin = 0;   // b-centric iff d+(a) < d+(b),
                                                       // dir_lo < d+(b) <= dir_hi, d+(a) > dir_amin
     DevBuf<uint32_t> tmp[4];   // storage when the plan is temporary: the lists, the unit offsets
+    DevBuf<uint32_t> owner[K]; // place in its list of every unit's vertex
     // Core map of the upper CTA bucket (tc_core_map): the vertices of degree >
     // cta_hi, numbered 0..core_n-1 in id order.  core_adj holds every out-list
     // in core numbers (core_n for a vertex outside the core), v's list at
@@ -183,10 +184,11 @@ struct TcPlan {
     const uint32_t *walk(const Oriented &o) const { return dense.n ? dense.walk.get() : o.len; }
 };
 struct Ctx;
+// slots: entries of all out-lists (unused when owned)
 // in_lists: also in-list centres (b-centric edges) in the CTA buckets
 // core_from > 0: the upper CTA bucket starts at that out-degree (the core-bitmap
 // kernel's split, for a plan that gets a core map) instead of tc_b1
-void tc_plan(Ctx &c, const Oriented &o, TcPlan &plan, cudaStream_t s, bool owned, bool in_lists,
+void tc_plan(Ctx &c, const Oriented &o, uint64_t slots, TcPlan &plan, cudaStream_t s, bool owned, bool in_lists,
              uint32_t core_from = 0);
 // builds the core map of the upper CTA bucket (from plan.cta_hi) for out-lists
 // o.adj[0..slots) (symmetric degree of v = o.len[v] + o.in_len(v)); core_n: the
@@ -200,8 +202,8 @@ void tc_core_map(Ctx &c, const Oriented &o, uint64_t slots, TcPlan &plan, uint32
 constexpr int TC_LISTS = TcPlan::K + 2;   // the two CTA buckets have an in-list part
 void tc_plan_lists(Ctx &c, const Oriented &o, TcPlan &plan, uint32_t *lists, uint32_t *bounds, cudaStream_t s,
                    bool in_lists, uint32_t core_from);
-void tc_plan_units(const Oriented &o, TcPlan &plan, uint32_t *lists, const uint32_t *host_bounds, cudaStream_t s,
-                   bool owned);
+void tc_plan_units(const Oriented &o, uint64_t slots, TcPlan &plan, uint32_t *lists, const uint32_t *host_bounds,
+                   cudaStream_t s, bool owned);
 // out-degree up to which the walks take a vertex by register groups or a warp
 uint32_t tc_short_lists(const Ctx &c);
 // tc_dense.cu.  pick (2 device words): members and degree bound of the dense core worth

@@ -764,7 +764,7 @@ int scd_resident_add(scd_ctx *set, scd_ctx *src, uint64_t *ids) {
             s.tc_b1 = sp[2];
             s.tc_amin = sp[3];
             s.wplan = TcPlan();
-            if (s.g.n) tc_plan(s, Oriented{s.g.indices, s.g.nlow, s.g.adj, s.g.n}, s.wplan, s.stream, true, false);
+            if (s.g.n) tc_plan(s, Oriented{s.g.indices, s.g.nlow, s.g.adj, s.g.n}, 0, s.wplan, s.stream, true, false);
         }
         ps->lists = lists_of(s);
         ps->nlow = s.g.nlow;

@@ -97,10 +97,11 @@ struct BucketMask {
     }
 };
 
-// The work units of a kernel: those of a plan's bucket (unit_off), or a list made on the device
-// (count set): with `chunk` a (vertex, chunk) per entry, else `per` chunks of every vertex.
+// The work units of a kernel: those of a plan's bucket (unit_off, and owner: the place of a unit's
+// vertex in the list), or a list made on the device (count set): with `chunk` a (vertex, chunk)
+// per entry, else `per` chunks of every vertex.
 struct UnitList {
-    const uint32_t *verts, *unit_off;
+    const uint32_t *verts, *unit_off, *owner;
     uint32_t nverts;
     const uint32_t *count, *chunk;
     uint32_t per;
@@ -113,13 +114,7 @@ struct UnitList {
             ch = chunk ? chunk[vi] : unit % per;
             return;
         }
-        uint32_t lo = 0, hi = nverts + 1;   // unit_off[vi] <= unit < unit_off[vi + 1]
-        while (lo < hi) {
-            const uint32_t mid = (lo + hi) >> 1;
-            if (unit_off[mid] <= unit) lo = mid + 1;
-            else hi = mid;
-        }
-        vi = lo - 1;
+        vi = owner[unit];
         v = verts[vi];
         ch = unit - unit_off[vi];
     }
@@ -278,11 +273,9 @@ k_tc_warp(Oriented o, UnitList units, Dir dir, uint32_t *tcount, uint8_t *flag, 
     __shared__ uint32_t pre[WARPS][32], bbase[WARPS][32], bhits[WARPS][32];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const uint32_t n_units = units.total();
-    while (true) {
-        uint32_t unit = 0;
-        if (lane == 0) unit = atomicAdd(next_unit, 1u);
-        unit = __shfl_sync(FULL, unit, 0);
-        if (unit >= n_units) break;
+    for (uint32_t unit = blockIdx.x * WARPS + w; unit < n_units;) {
+        uint32_t next = 0;   // the first units are the warps' own numbers; asked for early
+        if (lane == 0) next = gridDim.x * WARPS + atomicAdd(next_unit, 1u);
         uint32_t vi, a, ch;
         units.find(unit, vi, a, ch);
         const uint32_t abeg = o.beg[a], alen = o.len[a];
@@ -377,6 +370,7 @@ k_tc_warp(Oriented o, UnitList units, Dir dir, uint32_t *tcount, uint8_t *flag, 
             }
         }
         __syncwarp();
+        unit = __shfl_sync(FULL, next, 0);
     }
 }
 
@@ -408,14 +402,16 @@ k_tc_cta(Oriented o, UnitList units, uint32_t nfwd, const uint32_t *__restrict__
     uint32_t *filt = sm + TCAP + LCAP / 2;                // 2^FBITS bits
     uint16_t *idxs = (uint16_t *)(filt + (1 << FBITS) / 32);   // TCAP
     __shared__ uint32_t pre[THREADS], bbase[THREADS], bhits[THREADS], wsum[THREADS / 32];
-    __shared__ uint32_t s_unit, s_total;
+    __shared__ uint32_t s_unit;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const uint32_t n_units = units.total();
+    if (threadIdx.x == 0) s_unit = blockIdx.x;   // the first units are the CTAs' own numbers
+    __syncthreads();
     while (true) {
-        if (threadIdx.x == 0) s_unit = atomicAdd(next_unit, 1u);
-        __syncthreads();
         const uint32_t unit = s_unit;
         if (unit >= n_units) break;
+        uint32_t next = 0;   // asked for early, needed at the end
+        if (threadIdx.x == 0) next = gridDim.x + atomicAdd(next_unit, 1u);
         uint32_t vi, x, ch;
         units.find(unit, vi, x, ch);
         const bool fwd = vi < nfwd, in_core = !fwd && walk[x] == 0;
@@ -455,21 +451,16 @@ k_tc_cta(Oriented o, UnitList units, uint32_t nfwd, const uint32_t *__restrict__
             uint32_t incl = warp_inclusive_scan(wb);   // block inclusive scan of wb
             if (lane == 31) wsum[w] = incl;
             __syncthreads();
-            if (threadIdx.x == 0) {
-                uint32_t run = 0;
-                for (int k = 0; k < THREADS / 32; k++) {
-                    const uint32_t v = wsum[k];
-                    wsum[k] = run;
-                    run += v;
-                }
-                s_total = run;
+            uint32_t total = 0;
+#pragma unroll
+            for (int k = 0; k < THREADS / 32; k++) {
+                const uint32_t v = wsum[k];
+                if (k < w) incl += v;
+                total += v;
             }
-            __syncthreads();
-            incl += wsum[w];
             pre[threadIdx.x] = incl - wb;
             bbase[threadIdx.x] = bb;
             bhits[threadIdx.x] = 0;
-            const uint32_t total = s_total;
             __syncthreads();
             // warp chunks of 32*ITEMS consecutive items; lane L takes items chunk + L + 32k
             // (coalesced loads) and walks the owner boundaries forward
@@ -534,6 +525,7 @@ k_tc_cta(Oriented o, UnitList units, uint32_t nfwd, const uint32_t *__restrict__
                 flag[xbeg + i] = 1;
             }
         }
+        if (threadIdx.x == 0) s_unit = next;
         __syncthreads();
     }
 }
@@ -583,35 +575,30 @@ constexpr int CTA1_THREADS = 128, CTA1_ROUNDS = 4, CTA2_THREADS = 256, CTA2_ROUN
 template <int THREADS, int K>
 __global__ void __launch_bounds__(THREADS, 6)
 k_tc_core(Oriented o, const uint32_t *__restrict__ cpad, const uint32_t *__restrict__ cbeg, uint32_t core_n,
-          uint32_t kwords, uint32_t lcap, const uint32_t *__restrict__ verts, const uint32_t *__restrict__ unit_off,
-          uint32_t nverts, uint32_t nfwd, const uint32_t *__restrict__ walk, uint32_t per_unit, Dir dir, uint32_t *tcount,
+          uint32_t kwords, uint32_t lcap, UnitList units, uint32_t nfwd, const uint32_t *__restrict__ walk, uint32_t per_unit, Dir dir, uint32_t *tcount,
           uint8_t *flag, uint32_t *next_unit) {
     extern __shared__ __align__(16) uint32_t sm[];
     uint32_t *bm = sm;                           // kwords
     uint32_t *cnt = bm + kwords;                 // lcap hit counts of the centre's members
     uint16_t *pre = (uint16_t *)(cnt + lcap);    // kwords
     __shared__ uint32_t qpre[THREADS], sq0[THREADS], sdl[THREADS], sh[THREADS], wsum[THREADS / 32];
-    __shared__ uint32_t s_unit, s_total, s_xhits;
+    __shared__ uint32_t s_unit, s_xhits;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const uint4 *cq = reinterpret_cast<const uint4 *>(cpad);
     for (uint32_t i = threadIdx.x; i < kwords; i += THREADS) bm[i] = 0;
-    const uint32_t n_units = unit_off[nverts];
+    const uint32_t n_units = units.total();
+    if (threadIdx.x == 0) {
+        s_unit = blockIdx.x;   // the first units are the CTAs' own numbers
+        s_xhits = 0;
+    }
+    __syncthreads();
     while (true) {
-        if (threadIdx.x == 0) {
-            s_unit = atomicAdd(next_unit, 1u);
-            s_xhits = 0;
-        }
-        __syncthreads();
         const uint32_t unit = s_unit;
         if (unit >= n_units) break;
-        uint32_t lo = 0, hi = nverts + 1;
-        while (lo < hi) {
-            const uint32_t mid = (lo + hi) >> 1;
-            if (unit_off[mid] <= unit) lo = mid + 1;
-            else hi = mid;
-        }
-        const uint32_t vi = lo - 1;
-        const uint32_t x = verts[vi], ch = unit - unit_off[vi];
+        uint32_t next = 0;   // asked for early, needed at the end
+        if (threadIdx.x == 0) next = gridDim.x + atomicAdd(next_unit, 1u);
+        uint32_t vi, x, ch;
+        units.find(unit, vi, x, ch);
         const bool fwd = vi < nfwd, in_core = !fwd && walk[x] == 0;
         const uint32_t xbeg = o.beg[x], xlen = o.len[x];
         const uint32_t *xc = cpad + cbeg[x];
@@ -644,21 +631,17 @@ k_tc_core(Oriented o, const uint32_t *__restrict__ cpad, const uint32_t *__restr
             uint32_t incl = warp_inclusive_scan(nq);   // block scan of the quad counts
             if (lane == 31) wsum[w] = incl;
             __syncthreads();   // also orders the bitmap build before the walk
-            if (threadIdx.x == 0) {
-                uint32_t run = 0;
-                for (int k = 0; k < THREADS / 32; k++) {
-                    const uint32_t v = wsum[k];
-                    wsum[k] = run;
-                    run += v;
-                }
-                s_total = run;
+            uint32_t total = 0;
+#pragma unroll
+            for (int k = 0; k < THREADS / 32; k++) {
+                const uint32_t v = wsum[k];
+                if (k < w) incl += v;
+                total += v;
             }
-            __syncthreads();
-            qpre[threadIdx.x] = incl + wsum[w] - nq;
+            qpre[threadIdx.x] = incl - nq;
             sq0[threadIdx.x] = cb >> 2;
             sdl[threadIdx.x] = ob - cb;   // core-array position -> out-slot (mod 2^32)
             sh[threadIdx.x] = 0;
-            const uint32_t total = s_total;
             __syncthreads();
             // warp w walks its own contiguous range of the round's quads, 32 x K at a
             // time (lane L every 32nd: coalesced); each lane finds the owner of its first
@@ -723,7 +706,11 @@ k_tc_core(Oriented o, const uint32_t *__restrict__ cpad, const uint32_t *__restr
         xh = warp_sum(xh);
         if (lane == 0 && xh) atomicAdd(&s_xhits, xh);
         __syncthreads();
-        if (threadIdx.x == 0 && s_xhits) atomicAdd(tcount + o.at(x), s_xhits);
+        if (threadIdx.x == 0) {
+            if (s_xhits) atomicAdd(tcount + o.at(x), s_xhits);
+            s_xhits = 0;
+            s_unit = next;
+        }
         const uint32_t *xa = o.adj + xbeg;
         for (uint32_t i = threadIdx.x; i < xlen; i += THREADS) {
             const uint32_t cc = cnt[i];
@@ -747,6 +734,10 @@ inline size_t tc_core_smem(uint32_t kwords, uint32_t lcap) {
     return (size_t)kwords * 4 + (size_t)lcap * 4 + ((size_t)kwords * 2 + 3) / 4 * 4;
 }
 
+UnitList bucket_units(const TcPlan &plan, int k) {
+    return UnitList{plan.verts[k], plan.unit_off[k], plan.owner[k].get(), plan.nverts[k], nullptr, nullptr, 1};
+}
+
 void launch_tc_core(const Oriented &o, const TcPlan &plan, int k, uint32_t lcap, uint32_t *tcount, uint8_t *flag,
                     uint32_t *ctr, cudaStream_t s) {
     const uint32_t kwords = plan.core_n / 32 + 1;
@@ -758,8 +749,7 @@ void launch_tc_core(const Oriented &o, const TcPlan &plan, int k, uint32_t lcap,
     if (per_sm < 1) throw Error(SCD_ERR_CUDA, "core triangle-count kernel does not fit an SM");
     CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     k_tc_core<CORE_THREADS, CORE_K><<<sms * per_sm, CORE_THREADS, smem, s>>>(
-        o, plan.core_adj, plan.core_beg, plan.core_n, kwords, lcap, plan.verts[k], plan.unit_off[k], plan.nverts[k],
-        plan.nfwd[k], plan.walk(o), CTA2_THREADS * CTA2_ROUNDS, Dir{plan.dir_lo, plan.dir_hi, plan.dir_amin}, tcount,
+        o, plan.core_adj, plan.core_beg, plan.core_n, kwords, lcap, bucket_units(plan, k), plan.nfwd[k], plan.walk(o), CTA2_THREADS * CTA2_ROUNDS, Dir{plan.dir_lo, plan.dir_hi, plan.dir_amin}, tcount,
         flag, ctr);
     CK_LAUNCH("k_tc_core");
 }
@@ -888,7 +878,14 @@ void tc_plan_lists(Ctx &c, const Oriented &o, TcPlan &plan, uint32_t *lists, uin
                           o.n, lists, bounds, s);
 }
 
-void tc_plan_units(const Oriented &o, TcPlan &plan, uint32_t *lists, const uint32_t *hb, cudaStream_t s, bool owned) {
+// owner[u]: the place in its list of the vertex whose unit u is
+__global__ void k_unit_owners(const uint32_t *__restrict__ unit_off, uint32_t count, uint32_t *owner) {
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x)
+        for (uint32_t u = unit_off[i]; u < unit_off[i + 1]; u++) owner[u] = i;
+}
+
+void tc_plan_units(const Oriented &o, uint64_t slots, TcPlan &plan, uint32_t *lists, const uint32_t *hb, cudaStream_t s,
+                   bool owned) {
     const uint32_t per_unit[TcPlan::K] = {32, CTA1_THREADS * CTA1_ROUNDS, CTA2_THREADS * CTA2_ROUNDS, 1};
     for (int k = 0; k < TcPlan::K; k++) {
         const int l = k < 2 ? k : k + (k == 2 ? 1 : 2);   // first list of bucket k
@@ -902,10 +899,15 @@ void tc_plan_units(const Oriented &o, TcPlan &plan, uint32_t *lists, const uint3
         plan.tmp[k + 1].alloc((size_t)cnt + 1, s);
         plan.unit_off[k] = plan.tmp[k + 1].get();
         scan_exclusive<uint32_t>(UnitsOf{o, plan.verts[k], per_unit[k], plan.nfwd[k]}, plan.unit_off[k], cnt, s);
+        // (the out-list centres have at most `slots` partners together, the in-list centres too)
+        plan.owner[k].alloc(cnt + 2 * slots / per_unit[k] + 1, s);
+        k_unit_owners<<<grid_for(cnt, 256), 256, 0, s>>>(plan.unit_off[k], cnt, plan.owner[k].get());
+        CK_LAUNCH("k_unit_owners");
     }
 }
 
-void tc_plan(Ctx &c, const Oriented &o, TcPlan &plan, cudaStream_t s, bool owned, bool in_lists, uint32_t core_from) {
+void tc_plan(Ctx &c, const Oriented &o, uint64_t slots, TcPlan &plan, cudaStream_t s, bool owned, bool in_lists,
+             uint32_t core_from) {
     const size_t most = in_lists ? 2 * (size_t)o.n : o.n;   // an in-list centre is listed twice
     uint32_t *lists;
     if (owned) {
@@ -919,7 +921,7 @@ void tc_plan(Ctx &c, const Oriented &o, TcPlan &plan, cudaStream_t s, bool owned
     uint32_t *hb = c.host_u32 + HOST_PLAN;
     CK(cudaMemcpyAsync(hb, bounds.get(), 4 * (TC_LISTS + 1), cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
-    tc_plan_units(o, plan, lists, hb, s, owned);
+    tc_plan_units(o, slots, plan, lists, hb, s, owned);
 }
 
 void tc_core_map(Ctx &c, const Oriented &o, uint64_t slots, TcPlan &plan, uint32_t core_n, uint32_t lcap,
@@ -946,7 +948,7 @@ void tc_core_map(Ctx &c, const Oriented &o, uint64_t slots, TcPlan &plan, uint32
 
 void tc_plan_counting(Ctx &c, const Oriented &o, uint64_t slots, TcPlan &plan, cudaStream_t s) {
     if (c.flags & SCD_FLAG_TC_HASH || o.n == 0) {
-        tc_plan(c, o, plan, s, false, true);
+        tc_plan(c, o, slots, plan, s, false, true);
         return;
     }
     // the core kernel starts at the lowest candidate bound whose core fits the
@@ -954,10 +956,10 @@ void tc_plan_counting(Ctx &c, const Oriented &o, uint64_t slots, TcPlan &plan, c
     const uint32_t b0 = tc_short_lists(c);
     constexpr int K = CoreBounds::K;
     if (o.n <= CORE_BUDGET) {   // every core fits the budget: the lowest split, no host read
-        tc_plan(c, o, plan, s, false, true, b0);
+        tc_plan(c, o, slots, plan, s, false, true, b0);
         tc_core_map(c, o, slots, plan, o.n, B2, s);   // core_n <= n; counts sized for the cap
         if (plan.core_n || !plan.nverts[2]) return;
-        tc_plan(c, o, plan, s, false, true);
+        tc_plan(c, o, slots, plan, s, false, true);
         return;
     }
     CoreBounds cb{};
@@ -978,11 +980,11 @@ void tc_plan_counting(Ctx &c, const Oriented &o, uint64_t slots, TcPlan &plan, c
         if (tc_core_smem(h[j] / 32 + 1, h[K + j]) <= CORE_SMEM_MAX) pick = j;
     if (pick >= 0) {
         const uint32_t core_n = h[pick], lcap = h[K + pick];
-        tc_plan(c, o, plan, s, false, true, cb.t[pick]);
+        tc_plan(c, o, slots, plan, s, false, true, cb.t[pick]);
         tc_core_map(c, o, slots, plan, core_n, lcap, s);
         if (plan.core_n || !plan.nverts[2]) return;
     }
-    tc_plan(c, o, plan, s, false, true);   // no map: the hash kernels' split
+    tc_plan(c, o, slots, plan, s, false, true);   // no map: the hash kernels' split
 }
 
 void prepare_tc_kernels() {
@@ -1024,7 +1026,7 @@ double autotune_tc(Ctx &c, std::vector<std::string> *report) {
                     c.tc_b1 = b1;
                     c.tc_amin = am;
                     TcPlan plan;
-                    tc_plan(c, o, plan, s, false, true);
+                    tc_plan(c, o, 2 * (uint64_t)g.m, plan, s, false, true);
                     double ms_min = 1e300;
                     for (int rep = 0; rep < 2; rep++) {
                         CK(cudaMemsetAsync(tcount.get(), 0, (size_t)g.n * 4, s));
@@ -1071,10 +1073,6 @@ double autotune_tc(Ctx &c, std::vector<std::string> *report) {
 }
 
 namespace {
-
-UnitList bucket_units(const TcPlan &plan, int k) {
-    return UnitList{plan.verts[k], plan.unit_off[k], plan.nverts[k], nullptr, nullptr, 1};
-}
 
 void launch_small(Ctx &c, const Oriented &o, uint32_t max_len, const uint32_t *walk, const Dir &dir, uint32_t *tcount,
                   uint8_t *flag, cudaStream_t s) {
@@ -1157,7 +1155,7 @@ void count_internal_triangles(Ctx &c, const Oriented &o, uint32_t *tcount, uint8
                   InternalWork::LONGEST == B2, "kernel capacities");
     static_assert(InternalWork::CHUNK == CTA1_THREADS * CTA1_ROUNDS && InternalWork::CHUNK == CTA2_THREADS * CTA2_ROUNDS,
                   "partners of a CTA unit");
-    const auto listed = [&](int k, uint32_t per) { return UnitList{w.verts[k], nullptr, 0, w.count + k, w.chunk[k], per}; };
+    const auto listed = [&](int k, uint32_t per) { return UnitList{w.verts[k], nullptr, nullptr, 0, w.count + k, w.chunk[k], per}; };
     const uint32_t nv = plan.nverts[0] + plan.nverts[1] + plan.nverts[2];
     const Dir dir{plan.dir_lo, plan.dir_hi, plan.dir_amin};
     launch_small(c, o, InternalWork::SMALL, nullptr, dir, tcount, flag, s);
