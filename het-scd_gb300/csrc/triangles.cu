@@ -1135,7 +1135,9 @@ void alloc_internal_work(Ctx &c) {
     const TcPlan &p = c.wplan;
     InternalWork &w = c.iwork;
     const size_t nv = (size_t)p.nverts[0] + p.nverts[1] + p.nverts[2];
-    const size_t units = nv + c.g.m / InternalWork::CHUNK + 1;   // a list of l has at most 1 + l / CHUNK
+    // a list of l has at most 1 + l / CHUNK, and the out-lists of a graph whose rows are not
+    // symmetric may hold all 2m entries
+    const size_t units = nv + 2 * (size_t)c.g.m / InternalWork::CHUNK + 1;
     for (int k = 0; k < InternalWork::K; k++) {
         const bool any = k < 2 ? nv : p.nverts[2];
         w.verts[k] = any ? c.alloc<uint32_t>(k ? units : nv) : nullptr;

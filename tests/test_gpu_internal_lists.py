@@ -73,3 +73,23 @@ def _check(g, labels, want, retuned):
         got = [eng.compute_wcc() for _ in range(2)]
     assert got[0] == got[1]
     assert abs(got[0] - want) <= g.n * 2.0 ** -53 * abs(want)
+
+
+def test_rows_that_are_all_out_list():
+    """A community stored one way (every entry in the row of its larger id): the out-lists hold
+    all entries of the graph, twice what they hold of a symmetric one, and the score, which is
+    made from the out-lists, is the same."""
+    n = 3001   # an even number of entries
+    u, v = np.tril_indices(n, -1)
+    first = np.concatenate([[0], np.cumsum(np.arange(n))])
+    tri, labels = np.full(n, (n - 1) * (n - 2), np.int32), np.zeros(n, np.uint32)
+    one_way = O.Graph(n, u.size // 2, first, v, tri, np.full(n, n - 1))
+    both = np.tile(np.arange(n), (n, 1))[~np.eye(n, dtype=bool)]
+    symmetric = O.Graph(n, u.size, np.arange(n + 1) * (n - 1), both, tri, np.full(n, n - 1))
+    got = []
+    for g in (one_way, symmetric):
+        with scd_gb300.Engine(0) as eng:
+            eng.transfer_graph(g)
+            eng.labels_to_device(labels)
+            got.append(eng.compute_wcc())
+    assert got[0] == got[1]
