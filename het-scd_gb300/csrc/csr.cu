@@ -81,7 +81,7 @@ k_sort_rows_warp(const uint32_t *__restrict__ off, uint32_t nrows, uint32_t rows
     __shared__ RowShared sh;
     const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5, warps = (gridDim.x * blockDim.x) >> 5;
     const unsigned lt = lanemask_lt();
-    const uint32_t units = (nrows + rows - 1) / rows;
+    const uint32_t units = nrows / rows + (nrows % rows != 0);
     for (uint32_t unit = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; unit < units; unit += warps) {
         const uint32_t r0 = unit * rows, r = r0 + lane;
         uint32_t beg = 0, len = 0;

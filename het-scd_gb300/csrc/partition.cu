@@ -111,7 +111,7 @@ __global__ void __launch_bounds__(TPB)
 k_mis_round(uint32_t n, uint32_t rows, WarpRows wr, const uint32_t *__restrict__ indices,
             const uint32_t *__restrict__ adj, const uint32_t *__restrict__ pos, uint8_t *state, uint32_t *undecided) {
     const uint32_t lane = threadIdx.x & 31, warps = (gridDim.x * blockDim.x) >> 5;
-    const uint32_t groups = (n + rows - 1) / rows;
+    const uint32_t groups = n / rows + (n % rows != 0);
     uint32_t left = 0;   // rows of this warp still undecided
     for (uint32_t unit = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; unit < wr.total + groups; unit += warps) {
         if (unit < wr.total) {
@@ -234,7 +234,7 @@ k_claim_labels(uint32_t n, uint32_t rows, WarpRows wr, const uint32_t *__restric
                const uint32_t *__restrict__ adj, const uint32_t *__restrict__ pos, const uint8_t *__restrict__ state,
                uint32_t *labels) {
     const uint32_t lane = threadIdx.x & 31, warps = (gridDim.x * blockDim.x) >> 5;
-    const uint32_t groups = (n + rows - 1) / rows;
+    const uint32_t groups = n / rows + (n % rows != 0);
     for (uint32_t unit = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; unit < wr.total + groups; unit += warps) {
         if (unit < wr.total) {
             const uint32_t v = wr[unit];

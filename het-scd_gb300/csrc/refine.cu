@@ -138,7 +138,7 @@ k_internal_degrees(uint32_t n, uint32_t rows, RowWork rw, const uint32_t *__rest
                    LabelFilter skip) {
     const int lane = threadIdx.x & 31;
     const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
-    const uint32_t groups = (n + rows - 1) / rows, nchunks = rw.nchunks;
+    const uint32_t groups = n / rows + (n % rows != 0), nchunks = rw.nchunks;
     for (uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < groups + nchunks; w += warps) {
         if (w >= groups) {   // a piece of a long row
             intdeg_seg<32>(chunk_seg(rw, w - groups, indices), nlow, adj, flag, itdeg, skip);
@@ -538,7 +538,7 @@ k_internal_lists(uint32_t n, uint32_t rows, WarpRows longer, uint32_t most_short
                  const uint32_t *__restrict__ indices, const uint32_t *__restrict__ nlow, const uint32_t *__restrict__ adj, LabelFilter lf, uint32_t *ilen, uint32_t *iadj, uint8_t *flag,
                  uint32_t *itcount, int32_t *itdeg, Stats st, InternalWork work) {
     const uint32_t lane = threadIdx.x & 31, gl = lane & 7, grp = lane >> 3;
-    const uint32_t warps = (gridDim.x * blockDim.x) >> 5, units = (n + rows - 1) / rows;
+    const uint32_t warps = (gridDim.x * blockDim.x) >> 5, units = n / rows + (n % rows != 0);
     const unsigned gmask = 0xffu << (grp * 8), lt = (1u << lane) - 1u;
     // entries of the work lists, a warp's 32 at a time (one atomic a vertex on one address would
     // be the kernel's time): lane i of the pending ones holds entry i

@@ -241,7 +241,7 @@ k_tc_small(Oriented o, uint32_t rows, uint32_t max_len, const uint32_t *__restri
     __shared__ SmallShared sh;
     const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5, warps = (gridDim.x * blockDim.x) >> 5;
     const unsigned lt = lanemask_lt();
-    const uint32_t units = (o.n + rows - 1) / rows;
+    const uint32_t units = o.n / rows + (o.n % rows != 0);
     for (uint32_t unit = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; unit < units; unit += warps) {
         const uint32_t v0 = unit * rows, v = v0 + lane;
         uint32_t len = lane < min(rows, o.n - v0) ? o.len[v] : 0u;
