@@ -26,6 +26,7 @@
 
 #include "engine.cuh"
 #include "gain_interval.cuh"
+#include "gain_rule.cuh"
 
 namespace scd {
 
@@ -97,21 +98,14 @@ __device__ __forceinline__ Iv interval_any_gain(const ImproveArgs &a, uint32_t l
     return g;
 }
 
-// Can a foreign label seen once never have a positive gain?  With d_in = 1 the terms A and B
-// of the model are 0 (their numerators hold d_in - 1), and the gain is (r - 1) C with
-//   C = -(r-1)(r-2) p_in^3 (q + t) alpha / den
-// for q = (r-1) p_in, t = (ext - 1) / r. Every factor of den is >= 0 if t is 0 or at least 1
-// (p_in <= 1 makes r - q - 1 >= 0; t (t - 1) is the one term that could be negative), and
-// (r-1)(r-2) does not wrap up to r = 46340; for r <= 2 the numerator is 0. Rounding to
-// nearest keeps all these signs, so the FP64 gain is <= 0 and the label is never chosen.
-// `signs`: alpha >= 0 and p_ext >= 0. Most labels of a skewed graph's long rows are seen once
-// (R-MAT scale 21, degree 257..1024: 460 labels a vertex, nearly one per neighbour), and this
-// costs a tenth of an interval.
+// Foreign labels that cannot be chosen, by a rule on signs (gain_rule.cuh); `signs`: alpha >= 0
+// and p_ext >= 0. Most labels of a skewed graph's long rows are seen once (R-MAT scale 21,
+// degree 257..1024: 460 labels a vertex, nearly one per neighbour), and this costs a tenth of
+// an interval.
 __device__ __forceinline__ bool never_gains(const ImproveArgs &a, uint32_t l, uint32_t freq, uint32_t mine, bool signs) {
     if (freq != 1 || l == mine || !signs) return false;
     const int4 cv = a.civ[l];
-    const int r = cv.x, ext = cv.y;
-    return r >= 1 && r <= 46340 && ext >= 1 && __int_as_float(cv.z) >= 0.f && (r <= 2 || ext == 1 || ext - 1 >= r);
+    return seen_once_never_gains(cv.x, cv.y, __int_as_float(cv.z), __int_as_float(cv.w));
 }
 
 // The own label's exact gain is needed unless no foreign label survives the
