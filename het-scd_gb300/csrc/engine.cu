@@ -27,7 +27,8 @@ __global__ void k_nlow(uint32_t n, const uint32_t *__restrict__ indices, const u
 // Is every entry (u, v) of the rows matched by its (v, u)?  Order-independent sums of two
 // 64-bit hashes of (smaller, larger) id, added from the smaller end's row and taken off from
 // the larger's: both are 0 for a symmetric graph, and for another only with the chance of
-// two hash sums meeting. sums[2] counts loops and descents of a row.
+// two hash sums meeting. sums[2] counts loops and descents of a row, sums[3] the entries that
+// are not above the one before.
 __device__ __forceinline__ unsigned long long mix64(unsigned long long z) {   // splitmix64's finaliser
     z = (z ^ (z >> 30)) * 0xbf58476d1ce4e5b9ull;
     z = (z ^ (z >> 27)) * 0x94d049bb133111ebull;
@@ -37,12 +38,14 @@ __device__ __forceinline__ unsigned long long mix64(unsigned long long z) {   //
 __global__ void k_symmetry(uint32_t n, const uint32_t *__restrict__ indices, const uint32_t *__restrict__ adj,
                            unsigned long long *sums) {
     const uint32_t lane = threadIdx.x & 31, warps = (gridDim.x * blockDim.x) >> 5;
-    unsigned long long a = 0, b = 0, bad = 0;
+    unsigned long long a = 0, b = 0, bad = 0, repeats = 0;
     for (uint32_t v = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; v < n; v += warps) {
         const uint32_t beg = indices[v], end = indices[v + 1];
         for (uint32_t i = beg + lane; i < end; i += 32) {
             const uint32_t w = adj[i];
-            bad += w == v || (i > beg && adj[i - 1] > w);
+            const uint32_t before = i > beg ? adj[i - 1] : 0u;
+            bad += w == v || before > w;
+            repeats += i > beg && before >= w;
             const unsigned long long key = v < w ? ((unsigned long long)v << 32) | w : ((unsigned long long)w << 32) | v;
             const unsigned long long h = mix64(key + 0x9e3779b97f4a7c15ull), k = mix64(h ^ 0xd1b54a32d192ed03ull);
             a += v < w ? h : 0ull - h;
@@ -52,10 +55,12 @@ __global__ void k_symmetry(uint32_t n, const uint32_t *__restrict__ indices, con
     a = warp_sum(a);
     b = warp_sum(b);
     bad = warp_sum(bad);
+    repeats = warp_sum(repeats);
     if (lane == 0) {
         if (a) atomicAdd(sums, a);
         if (b) atomicAdd(sums + 1, b);
         if (bad) atomicAdd(sums + 2, bad);
+        if (repeats) atomicAdd(sums + 3, repeats);
     }
 }
 
@@ -335,18 +340,20 @@ void build_union_structure(Ctx &c, bool always_gid, bool check_symmetry) {
         DevBuf<uint32_t> bounds(K + 2 + TC_LISTS + 1, s);
         build_lists<K + 1>(DegreeMask{g.indices}, n, lists, bounds.get(), s);
         tc_plan_lists(c, o, c.wplan, tc_lists, bounds.get() + K + 2, s, false, 0);
-        DevBuf<unsigned long long> sums(3, s);
+        DevBuf<unsigned long long> sums(4, s);
         unsigned long long *hs = (unsigned long long *)(c.host_u32 + HOST_SUMS);
-        hs[0] = hs[1] = hs[2] = 0;
+        hs[0] = hs[1] = hs[2] = hs[3] = 0;
+        static_assert(HOST_SUMS + 8 <= HOST_READ, "planning words");
         if (check_symmetry && n) {
-            CK(cudaMemsetAsync(sums.get(), 0, 24, s));
+            CK(cudaMemsetAsync(sums.get(), 0, 32, s));
             k_symmetry<<<grid_for((uint64_t)n * 32, TPB, NUM_SMS_HINT * 16), TPB, 0, s>>>(n, g.indices, g.adj, sums.get());
             CK_LAUNCH("k_symmetry");
-            CK(cudaMemcpyAsync(hs, sums.get(), 24, cudaMemcpyDeviceToHost, s));
+            CK(cudaMemcpyAsync(hs, sums.get(), 32, cudaMemcpyDeviceToHost, s));
         }
         CK(cudaMemcpyAsync(hb, bounds.get(), 4 * (K + 2 + TC_LISTS + 1), cudaMemcpyDeviceToHost, s));
         CK(cudaStreamSynchronize(s));
         g.symmetric = !(hs[0] | hs[1] | hs[2]);
+        g.distinct = !hs[3];
     }
     for (int k = 0; k < K; k++) {
         g.cls.list[k] = lists + hb[k];

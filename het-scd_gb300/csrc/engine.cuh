@@ -48,6 +48,8 @@ struct Graph {
     // every entry (u, v) has its (v, u), rows ascend, no loops: always so after convert, checked
     // for a transferred graph
     bool symmetric = true;
+    // no row lists an entry twice or out of order: also always so after convert, also checked
+    bool distinct = true;
     // degree buckets of the improve kernels, built once per graph
     DegreeClasses cls;
     RowWork rows;
@@ -144,12 +146,17 @@ struct DenseCore {
 // than their whole out-list's. (The register groups, up to SMALL, find theirs themselves.)
 // Measured, the CTA kernels of a step by whole out-lists -> by this list: R-MAT scale 22
 // 650 -> 4-21 us, scale 20 210 -> 5 us; 96 planted graphs (register groups only) unchanged.
+// Only where rows are distinct (Graph::distinct): of a repeated entry the register groups find
+// the last place and their searches one, the table kernels' walks one for every item, so there a
+// vertex stays with the kind of kernel that its whole out-list chooses.
 struct InternalWork {
     static constexpr int K = 3;   // warp units, 128-thread CTA units, 256-thread CTA units
     static constexpr uint32_t SMALL = 32, MID = 64, CTA = 1024, LONGEST = 8192, CHUNK = 512;
     uint32_t *verts[K] = {}, *chunk[K] = {};   // chunk (CTA units only): 512 partners each
     uint32_t *count = nullptr;                 // K words
     // (out-lists above LONGEST keep k_tc_huge)
+    // internal lists of up to this many entries are not listed (a centre of a triangle has two out-neighbours)
+    static uint32_t above(bool distinct) { return distinct ? SMALL : 1u; }
 };
 // out-degree buckets and their work-unit offsets (built once per oriented graph)
 // The out-lists above the register groups': a bucket for warp units, two for CTA units

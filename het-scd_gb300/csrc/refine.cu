@@ -536,7 +536,7 @@ template <bool LISTS, bool STATS>
 __global__ void __launch_bounds__(TPB)
 k_internal_lists(uint32_t n, uint32_t rows, WarpRows longer, uint32_t most_short,
                  const uint32_t *__restrict__ indices, const uint32_t *__restrict__ nlow, const uint32_t *__restrict__ adj, LabelFilter lf, uint32_t *ilen, uint32_t *iadj, uint8_t *flag,
-                 uint32_t *itcount, int32_t *itdeg, Stats st, InternalWork work) {
+                 uint32_t *itcount, int32_t *itdeg, Stats st, InternalWork work, uint32_t above) {
     const uint32_t lane = threadIdx.x & 31, gl = lane & 7, grp = lane >> 3;
     const uint32_t warps = (gridDim.x * blockDim.x) >> 5, units = n / rows + (n % rows != 0);
     const unsigned gmask = 0xffu << (grp * 8), lt = (1u << lane) - 1u;
@@ -574,7 +574,7 @@ k_internal_lists(uint32_t n, uint32_t rows, WarpRows longer, uint32_t most_short
                 }
             }
             if (LISTS && lane == 0) ilen[v] = c;
-            if (LISTS && c > InternalWork::SMALL && len <= InternalWork::LONGEST) {
+            if (LISTS && c > above && len <= InternalWork::LONGEST) {
                 const uint32_t chunks = c <= InternalWork::MID ? 1u : (c + InternalWork::CHUNK - 1) / InternalWork::CHUNK;
                 for (uint32_t ch = 0; ch < chunks; ch++) {
 #pragma unroll
@@ -662,7 +662,7 @@ void launch_internal_lists(Ctx &c, LabelFilter lf, const Stats &st) {
     k_internal_lists<LISTS, STATS><<<grid_for((((uint64_t)g.n + rows - 1) / rows + longer.total) * 32, TPB,
                                               NUM_SMS_HINT * 16), TPB, 0, c.stream>>>(
         g.n, rows, longer, c.wplan.small_max, g.indices, g.nlow, g.adj, lf, c.int_len, c.int_adj, c.slot_flag, c.itcount,
-        c.itdeg, st, c.iwork);
+        c.itdeg, st, c.iwork, InternalWork::above(g.distinct));
     CK_LAUNCH("k_internal_lists");
 }
 

@@ -223,7 +223,7 @@ struct ResidentSource {
     std::vector<uint32_t> fin_off, comm_off, m;   // per graph of the source union
     UnionLists lists{};
     const uint32_t *nlow = nullptr;
-    bool symmetric = true;
+    bool symmetric = true, distinct = true;      // Graph's
     std::vector<GraphLists> gl;                  // per graph of the source union
     std::vector<uint64_t> ids;
     std::vector<double> wcc0;
@@ -447,11 +447,19 @@ uint32_t rebuild(Ctx &c, ResidentSet &R, std::vector<ResidentSource *> &srcs) {
     c.owned.clear();
     c.bytes = 0;
     R.drop_exec();
-    bool symmetric = true;   // statistics from out-lists: only if every graph's rows allow it
-    for (const ResidentGraph &x : R.graphs) symmetric = symmetric && (x.taken || c.g.symmetric);
-    for (const ResidentSource *ps : srcs) symmetric = symmetric && ps->symmetric;
+    // statistics from out-lists, counts by the internal ones' lengths: only if every graph's rows allow it
+    bool symmetric = true, distinct = true;
+    for (const ResidentGraph &x : R.graphs) {
+        symmetric = symmetric && (x.taken || c.g.symmetric);
+        distinct = distinct && (x.taken || c.g.distinct);
+    }
+    for (const ResidentSource *ps : srcs) {
+        symmetric = symmetric && ps->symmetric;
+        distinct = distinct && ps->distinct;
+    }
     c.g = Graph();
     c.g.symmetric = symmetric;
+    c.g.distinct = distinct;
     c.b = Batch();
     c.wplan = TcPlan();
     c.has_graph = c.has_labels = false;
@@ -769,6 +777,7 @@ int scd_resident_add(scd_ctx *set, scd_ctx *src, uint64_t *ids) {
         ps->lists = lists_of(s);
         ps->nlow = s.g.nlow;
         ps->symmetric = s.g.symmetric;
+        ps->distinct = s.g.distinct;
         ps->gl = graph_lists(s);
         ps->a = arrays_of(s);
         ps->fin_off = s.b.h_fin_off;

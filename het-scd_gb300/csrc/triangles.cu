@@ -234,10 +234,10 @@ __device__ __forceinline__ void tc_small(const Oriented &o, const Dir &dir, uint
     }
 }
 
-// walk: 0 for the vertices whose out-list is counted elsewhere (nullptr: none)
+// walk: 0, or more than most, for the vertices whose out-list is counted elsewhere (nullptr: none)
 __global__ void __launch_bounds__(256, 8)
-k_tc_small(Oriented o, uint32_t rows, uint32_t max_len, const uint32_t *__restrict__ walk, Dir dir, uint32_t *tcount,
-           uint8_t *flag) {
+k_tc_small(Oriented o, uint32_t rows, uint32_t max_len, const uint32_t *__restrict__ walk, uint32_t most, Dir dir,
+           uint32_t *tcount, uint8_t *flag) {
     __shared__ SmallShared sh;
     const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5, warps = (gridDim.x * blockDim.x) >> 5;
     const unsigned lt = lanemask_lt();
@@ -245,7 +245,7 @@ k_tc_small(Oriented o, uint32_t rows, uint32_t max_len, const uint32_t *__restri
     for (uint32_t unit = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; unit < units; unit += warps) {
         const uint32_t v0 = unit * rows, v = v0 + lane;
         uint32_t len = lane < min(rows, o.n - v0) ? o.len[v] : 0u;
-        if (len < 2 || len > max_len || (walk && walk[v] == 0)) len = 0;
+        if (len < 2 || len > max_len || (walk && walk[v] - 1 >= most)) len = 0;
         const unsigned m32 = __ballot_sync(FULL, len > 16), m16 = __ballot_sync(FULL, len > 8) & ~m32,
                        m8 = __ballot_sync(FULL, len > 0) & ~(m32 | m16);
         const uint32_t n32 = __popc(m32), n16 = n32 + __popc(m16), n8 = n16 + __popc(m8);
@@ -758,14 +758,14 @@ void launch_tc_core(const Oriented &o, const TcPlan &plan, int k, uint32_t lcap,
 // by binary search in the sorted out-list in global memory, per-triangle
 // atomics.  Kept for generality.
 __global__ void __launch_bounds__(256)
-k_tc_huge(Oriented o, const uint32_t *__restrict__ verts, uint32_t nverts, uint32_t *tcount,
+k_tc_huge(Oriented o, const uint32_t *__restrict__ verts, uint32_t nverts, uint32_t above, uint32_t *tcount,
           uint8_t *flag) {
     const int lane = threadIdx.x & 31;
     const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
     for (uint32_t vi = 0; vi < nverts; vi++) {
         const uint32_t a = verts[vi];
         const uint32_t abeg = o.beg[a], alen = o.len[a];
-        if (alen <= 32) continue;   // (an internal list of the register groups)
+        if (alen <= above) continue;   // (an internal list of the register groups)
         const uint32_t *A = o.adj + abeg;
         for (uint32_t j = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; j < alen; j += warps) {
             const uint32_t b = A[j];
@@ -1074,8 +1074,8 @@ double autotune_tc(Ctx &c, std::vector<std::string> *report) {
 
 namespace {
 
-void launch_small(Ctx &c, const Oriented &o, uint32_t max_len, const uint32_t *walk, const Dir &dir, uint32_t *tcount,
-                  uint8_t *flag, cudaStream_t s) {
+void launch_small(Ctx &c, const Oriented &o, uint32_t max_len, const uint32_t *walk, uint32_t most, const Dir &dir,
+                  uint32_t *tcount, uint8_t *flag, cudaStream_t s) {
     // 16 vertices a warp, fewer where that would leave SMs short of their 64 warps (10,000
     // vertices, a step: 4 a warp 16 us, 1 a warp 10 us); a grid of
     // one unit a warp, because units of dense graphs take 25 times as long as those of sparse
@@ -1083,16 +1083,16 @@ void launch_small(Ctx &c, const Oriented &o, uint32_t max_len, const uint32_t *w
     // 8 CTAs an SM 7.3 ms, 16 6.8 ms, 48 6.0 ms, 128 5.8 ms; with 32 vertices 6.1 ms, with 8 6.0 ms)
     uint32_t rows = 1;
     while (rows < 16 && (uint64_t)rows * 2 * NUM_SMS_HINT * 64 <= o.n) rows <<= 1;
-    k_tc_small<<<grid_for(((uint64_t)o.n + rows - 1) / rows * 32, 256, 1u << 20), 256, 0, s>>>(o, rows, max_len, walk, dir, tcount,
-                                                                                                flag);
+    k_tc_small<<<grid_for(((uint64_t)o.n + rows - 1) / rows * 32, 256, 1u << 20), 256, 0, s>>>(o, rows, max_len, walk, most, dir,
+                                                                                                tcount, flag);
     CK_LAUNCH("k_tc_small");
     c.launches++;
 }
 
-void launch_huge(Ctx &c, const Oriented &o, const TcPlan &plan, uint32_t *tcount, uint8_t *flag,
+void launch_huge(Ctx &c, const Oriented &o, const TcPlan &plan, uint32_t above, uint32_t *tcount, uint8_t *flag,
                  cudaStream_t s) {
     if (!plan.nverts[3]) return;
-    k_tc_huge<<<152 * 4, 256, 0, s>>>(o, plan.verts[3], plan.nverts[3], tcount, flag);
+    k_tc_huge<<<152 * 4, 256, 0, s>>>(o, plan.verts[3], plan.nverts[3], above, tcount, flag);
     CK_LAUNCH("k_tc_huge");
     c.launches++;
 }
@@ -1108,7 +1108,7 @@ void count_triangles(Ctx &c, const Oriented &o, const TcPlan &plan, uint32_t *tc
     CK(cudaMemsetAsync(ctr, 0, 24, s));
     const Dir dir{plan.dir_lo, plan.dir_hi, plan.dir_amin};
     const bool core = plan.nverts[2] && plan.core_n;
-    launch_small(c, o, plan.small_max, plan.dense.n ? plan.dense.walk.get() : nullptr, dir, tcount, flag, s);
+    launch_small(c, o, plan.small_max, plan.dense.n ? plan.dense.walk.get() : nullptr, INVALID, dir, tcount, flag, s);
     if (plan.nverts[0]) {
         k_tc_warp<16, 256, 64, 10><<<152 * 4, 16 * 32, 0, s>>>(o, bucket_units(plan, 0), dir, tcount, flag, ctr);
         CK_LAUNCH("k_tc_warp64");
@@ -1128,7 +1128,7 @@ void count_triangles(Ctx &c, const Oriented &o, const TcPlan &plan, uint32_t *tc
         c.launches++;
     }
     if (plan.dense.n) tc_dense_count(c, o, plan, tcount, flag, ctr + 4, s);
-    launch_huge(c, o, plan, tcount, flag, s);
+    launch_huge(c, o, plan, 0, tcount, flag, s);
 }
 
 void alloc_internal_work(Ctx &c) {
@@ -1160,7 +1160,7 @@ void count_internal_triangles(Ctx &c, const Oriented &o, uint32_t *tcount, uint8
     const auto listed = [&](int k, uint32_t per) { return UnitList{w.verts[k], nullptr, nullptr, 0, w.count + k, w.chunk[k], per}; };
     const uint32_t nv = plan.nverts[0] + plan.nverts[1] + plan.nverts[2];
     const Dir dir{plan.dir_lo, plan.dir_hi, plan.dir_amin};
-    launch_small(c, o, InternalWork::SMALL, nullptr, dir, tcount, flag, s);
+    launch_small(c, o, InternalWork::SMALL, c.g.distinct ? nullptr : c.g.nlow, plan.small_max, dir, tcount, flag, s);
     if (nv) {
         k_tc_warp<16, 256, 64, 10><<<grid_for(2ull * nv, 16, 152 * 4), 16 * 32, 0, s>>>(o, listed(0, 2), dir, tcount, flag,
                                                                                      ctr);
@@ -1178,7 +1178,7 @@ void count_internal_triangles(Ctx &c, const Oriented &o, uint32_t *tcount, uint8
                                                                      ctr + 2, 152, s);
         c.launches++;
     }
-    launch_huge(c, o, plan, tcount, flag, s);
+    launch_huge(c, o, plan, InternalWork::above(c.g.distinct), tcount, flag, s);
 }
 
 }  // namespace scd
