@@ -491,6 +491,7 @@ void tc_dense_setup(Ctx &c, const Oriented &o, const uint32_t *deg, uint32_t mem
 
 void tc_dense_count(Ctx &c, const Oriented &o, const TcPlan &plan, uint32_t *tcount, uint8_t *flag, uint32_t *ctr,
                     cudaStream_t s) {
+    PhaseScope ph(c, "tc_dense");
     const DenseCore &d = plan.dense;
     const uint32_t words = dense_bits(d.n) / 32;
     const size_t matrix = (size_t)d.n * words;

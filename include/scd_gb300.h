@@ -190,7 +190,8 @@ int scd_stream(scd_ctx *ctx, void **stream);
 /* Phase timers (CUDA events on the context's stream, recorded only when the
  * context was created with SCD_FLAG_PROFILE): accumulated milliseconds and
  * number of timed launches of a phase.  Phases: "convert", "tc" (triangle
- * counting kernel of the preprocessing), "partition", "improve", "stats",
+ * counting kernel of the preprocessing), "tc_dense" (its part around a dense
+ * core, if the graph has one worth having), "partition", "improve", "stats",
  * "wcc_tc" (internal-triangle kernel), "wcc".  scd_profile_reset clears them. */
 int scd_profile_get(scd_ctx *ctx, const char *phase, double *total_ms, uint64_t *count);
 int scd_profile_reset(scd_ctx *ctx);
