@@ -85,6 +85,7 @@ class Lane:
         self.staging = staging
         self.waiting = collections.deque()
         self.in_set = {}
+        self.lost = set()        # ids whose requests failed with a step: dropped should they leave after all
         self.step_running = []   # graphs that iterated in each step
         self.steps = 0
         self.converters = []
@@ -235,6 +236,7 @@ class Server:
             except Exception as e:   # the set is unusable: fail everything it holds
                 with self._lock:
                     reqs = list(lane.in_set.values())
+                    lane.lost.update(lane.in_set)
                     lane.in_set.clear()
                     self._release(reqs)
                 for r in reqs:
@@ -243,6 +245,10 @@ class Server:
             if not out:
                 continue
             with self._lock:
+                out = [o for o in out if o[0] not in lane.lost]
+                # a graph can leave before its converter, back from resident_add, has noted its request
+                while any(i not in lane.in_set for i, *_ in out):
+                    self._lock.wait()
                 done = [(lane.in_set.pop(i), res, st, lab) for i, res, st, lab in out]
                 self._release([r for r, *_ in done])
             for r, res, st, lab in done:
