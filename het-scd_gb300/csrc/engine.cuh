@@ -123,11 +123,11 @@ struct Oriented {
     }
     __device__ __forceinline__ const uint32_t *in_adj() const { return ibeg ? iadj : adj; }
 };
-// Label mode of triangle counting: only triangles whose three vertices carry
-// the same valid label count; with `active`, vertices of graphs of a batch that
-// stopped iterating are skipped (their WCC is no longer read).
+// The labelling that statistics and internal out-lists are made of (where only the graphs that
+// stopped matter, labels is nullptr); with `active`, vertices of graphs of a batch that stopped
+// iterating are skipped (their statistics and WCC are no longer read).
 struct LabelFilter {
-    const uint32_t *labels = nullptr;   // nullptr: count every triangle
+    const uint32_t *labels = nullptr;
     const uint32_t *gid = nullptr;
     const uint8_t *active = nullptr;
     __device__ __forceinline__ bool frozen(uint32_t v) const { return active && !active[gid[v]]; }
@@ -225,13 +225,13 @@ void tc_dense_count(Ctx &c, const Oriented &o, const TcPlan &plan, uint32_t *tco
 // the plan of a full count (preprocessing) over out-lists o.adj[0..slots) with in-list
 // centres: the core split and its core map, or the hash kernels' split
 void tc_plan_counting(Ctx &c, const Oriented &o, uint64_t slots, TcPlan &plan, cudaStream_t s);
-// tcount[o.at(v)] += triangles at v; flag[slot] = 1 for out-slots on a triangle.
-// With labels: internal triangles only.  tcount and flag must be zeroed.
 // Sorts every row of a CSR (offsets off[nrows+1], values vals) ascending in place;
 // with dedup, repeated values of a row become INVALID and udeg[r] receives the
 // number of distinct values of row r.
 void sort_rows(Ctx &c, const uint32_t *off, uint32_t nrows, uint32_t *vals, bool dedup, uint32_t *udeg,
                cudaStream_t s);
+// tcount[o.at(v)] += triangles at v; flag[slot] = 1 for out-slots on a triangle.
+// tcount and flag must be zeroed.
 void count_triangles(Ctx &c, const Oriented &o, const TcPlan &plan, uint32_t *tcount, uint8_t *flag,
                      cudaStream_t s);
 // lists for the resident graph's WCC plan (InternalWork), and the count of the internal

@@ -1,10 +1,10 @@
 // a / b of two integers, rounded as the FP64 division rounds it, without the FP64 pipe.
 //
 // Schoolbook division by digits of 19 bits: a digit is the remainder times a single-precision
-// reciprocal of b, rounded to an integer (signed, within 0.75 of the exact quotient of that
-// remainder), and the next remainder is exact in 64 bits. Three digits give 57 or 58 bits of the
-// quotient and the sign of what is left, which is all that rounding to nearest even needs. The
-// device's FP64 pipe does about two operations a clock and SM and a division takes ten of them
+// reciprocal of b, rounded to an integer (signed, within 0.82 of the exact quotient of that
+// remainder: half a unit, and 2.5 x 2^-23 of a first digit below 2^20), and the next remainder
+// is exact in 64 bits. Three digits give 57 or 58 bits of the quotient and the sign of what is
+// left, which is all that rounding to nearest even needs. The device's FP64 pipe does about two operations a clock and SM and a division takes ten of them
 // with its conversions; this takes about sixty integer and single-precision operations at 64 or
 // more a clock.
 //
@@ -67,7 +67,7 @@ SCD_HD double exact_div(uint32_t a, uint64_t b) {
     for (int i = 0; i < 3; i++) {
         const int digit = div_digit(r, f);
         q = (q << DIGIT) + (uint64_t)(int64_t)digit;
-        r = (int64_t)(((uint64_t)r << DIGIT) - (uint64_t)(int64_t)digit * d);   // |r| <= 0.75 d
+        r = (int64_t)(((uint64_t)r << DIGIT) - (uint64_t)(int64_t)digit * d);   // |r| <= 0.82 d
     }
     if (r < 0) {   // q + r / d with 0 <= r < d
         q--;

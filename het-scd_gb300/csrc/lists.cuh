@@ -21,9 +21,7 @@ constexpr int LISTS_ONE_WARPS = 32, LISTS_ONE_STEPS = 16;
 constexpr uint32_t LISTS_ONE = LISTS_ONE_WARPS * 32 * LISTS_ONE_STEPS;
 
 // The class masks of a warp's steps x 32 (steps <= STEPS) consecutive ids from `first` on (bit
-// k: the id is in class k), and in lane k < K the number of the warp's ids in class k. (A
-// vote for every class: a loop over only the classes that some lane has, its bound from a
-// warp reduction, lost list entries.)
+// k: the id is in class k), and in lane k < K the number of the warp's ids in class k.
 template <int K, int STEPS, typename F>
 __device__ __forceinline__ uint32_t warp_masks(F f, uint32_t n, uint32_t first, uint32_t steps, uint32_t (&m)[STEPS]) {
     static_assert(K <= 32, "a lane per class");

@@ -21,8 +21,9 @@ namespace scd {
 // small graph, bound by the host, makes about ninety of them. Sizes are powers of two; at most
 // 64 blocks of a size and 32 MB together are kept, the rest and (at the context's end) all of
 // them go back. A block is only handed out again for work on the stream it was used on, later in
-// that stream, as cudaFreeAsync and cudaMallocAsync on one stream would. Locked: a resident set
-// lets another thread than the stepping one work on the context.
+// that stream, as cudaFreeAsync and cudaMallocAsync on one stream would. The calls of a resident
+// set do not use it (their temporaries come from the pool). Locked: a block may go back from
+// another thread than the one that takes the next.
 class BlockCache {
 public:
     static constexpr int LOW = 9, HIGH = 20, SIZES = HIGH - LOW + 1, SLOTS = 64;

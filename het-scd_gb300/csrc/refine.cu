@@ -243,7 +243,6 @@ k_wcc_partial(const uint32_t *__restrict__ fin_off, const uint32_t *__restrict__
     }
 }
 
-// one block per graph: fixed-order sum of the graph's partials, divided by its n
 // src/main.cpp:68-81 for a graph still iterating (thread 0 of its CTA of k_wcc_final: a launch
 // of its own was 3 us of a small graph's step): count the iteration, remember whether it beat
 // the best WCC, stop when it is below best*(1+threshold)
@@ -262,6 +261,7 @@ __device__ __forceinline__ void batch_step_of(uint32_t g, double w, const BatchS
     }
 }
 
+// one block per graph: fixed-order sum of the graph's partials, divided by its n
 __global__ void __launch_bounds__(TPB) k_wcc_final(const double *__restrict__ partial,
                                                    const uint32_t *__restrict__ blk_off,
                                                    const uint32_t *__restrict__ fin_off, double *out,
@@ -502,7 +502,14 @@ void batch_reset(Ctx &c) {
 
 namespace {
 
-// One pass over the out-lists of a labelling, for the label-mode triangle count and for
+// a vertex of label l and degree deg with c internal out-edges
+__device__ __forceinline__ void add_stats(const Stats &st, uint32_t l, uint32_t deg, uint32_t c) {
+    atomicAdd(st.sizes + l, 1);
+    if (deg - 2 * c) atomicAdd(st.ext + l, (int)(deg - 2 * c));
+    if (c) atomicAdd(st.intl + l, (int)(2 * c));
+}
+
+// One pass over the out-lists of a labelling, for the internal triangle count and for
 // the community statistics.
 //
 // LISTS: the internal out-lists, i.e. the out-neighbours of v that carry v's (valid)
@@ -525,13 +532,6 @@ namespace {
 // bounds, neighbour, its label), which one vertex per group at a time paid in full.
 // Measured (statistics + lists of a step): 96 planted graphs, 2.6 M vertices, 130 + 227 ->
 // 195 us; Chung-Lu 500k, statistics alone 123 -> 30 us; R-MAT scale 20 89 + 40 -> 80 us.
-// a vertex of label l and degree deg with c internal out-edges
-__device__ __forceinline__ void add_stats(const Stats &st, uint32_t l, uint32_t deg, uint32_t c) {
-    atomicAdd(st.sizes + l, 1);
-    if (deg - 2 * c) atomicAdd(st.ext + l, (int)(deg - 2 * c));
-    if (c) atomicAdd(st.intl + l, (int)(2 * c));
-}
-
 template <bool LISTS, bool STATS>
 __global__ void __launch_bounds__(TPB)
 k_internal_lists(uint32_t n, uint32_t rows, WarpRows longer, uint32_t most_short,
@@ -709,7 +709,6 @@ void launch_wcc(Ctx &c, const uint32_t *labels, const Stats &st, bool frozen_gra
     CK(cudaMemsetAsync(c.work_counter, 0, 64, s));   // the lists' counts and the kernels' unit counters
     if (with_stats) launch_internal_lists<true, true>(c, lf, st);
     else launch_internal_lists<true, false>(c, lf, st);
-    // the plan's buckets (by full out-degree) stay valid: internal lists are never longer
     const Oriented o{g.indices, c.int_len, c.int_adj, g.n};
     count_internal_triangles(c, o, c.itcount, c.slot_flag);
     const uint32_t rows = rows_a_warp(g.n);

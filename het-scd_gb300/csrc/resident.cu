@@ -10,8 +10,8 @@
 //
 //   * every array of a kept graph (CSR, tri, tri_deg, current and best labels,
 //     the statistics of its label range, p_ext, WCC, best WCC, the active flag
-//     and the iteration count) is gathered into the new union by one launch per
-//     array, with its vertex, adjacency and label offsets shifted;
+//     and the iteration count) is gathered into the new union, all arrays in one
+//     launch, with its vertex, adjacency and label offsets shifted;
 //   * the derived structure of the union (degree classes, row work, hash-table
 //     offsets, triangle-counting plan, WCC blocks) is rebuilt;
 //   * the captured iteration is captured again for the new union.

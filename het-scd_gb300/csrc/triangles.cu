@@ -130,7 +130,8 @@ struct UnitList {
 // slot. An out(b) at least 4x longer than out(a) (a hub's) is not walked: every lane searches
 // its out(a) entry in out(b) instead (alen searches of log2 d+(b) steps).
 //
-// Bound by instructions (issue slots 70-78%). Groups by the list as it is: the internal
+// Bound by instructions and the loads in front of them (issue slots 59 % busy on R-MAT scale 20,
+// 62-70 % on 96 planted graphs). Groups by the list as it is: the internal
 // out-lists of a labelling are a fraction of the whole ones, and with the groups of the whole
 // lists (and vertices gathered from the plan's lists) most lanes idled.
 // Measured: internal count of a step, 96 planted graphs, 466..680 -> 333..660 us (a later one
@@ -791,11 +792,10 @@ k_tc_huge(Oriented o, const uint32_t *__restrict__ verts, uint32_t nverts, uint3
     }
 }
 
-// out-degree buckets: (0,16] and (16,S] register groups (S = 0, 16 or 32), (S,B0] warp
-// units, (B0,B1] and (B1,8192] CTA units, > 8192 fallback; B0 <= 64 and B1 <= 1024
-// (the kernels' shared-memory capacities); S, B0, B1 tuned per context
+// out-degrees: up to S (0, 16 or 32) register groups, found by the kernel itself; then the
+// plan's buckets: (S,B0] warp units, (B0,B1] and (B1,8192] CTA units, > 8192 fallback; B0 <= 64
+// and B1 <= 1024 (the kernels' shared-memory capacities); S, B0, B1 tuned per context
 constexpr uint32_t B2 = 8192;
-
 
 // v lies in the core: symmetric degree above the CTA buckets' lower bound
 struct CoreFlag {
