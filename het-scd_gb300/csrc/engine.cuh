@@ -231,8 +231,8 @@ void tc_plan_counting(Ctx &c, const Oriented &o, uint64_t slots, TcPlan &plan, c
 void sort_rows(Ctx &c, const uint32_t *off, uint32_t nrows, uint32_t *vals, bool dedup, uint32_t *udeg,
                cudaStream_t s);
 // tcount[o.at(v)] += triangles at v; flag[slot] = 1 for out-slots on a triangle.
-// tcount and flag must be zeroed.
-void count_triangles(Ctx &c, const Oriented &o, const TcPlan &plan, uint32_t *tcount, uint8_t *flag,
+// tcount and flag must be zeroed.  entries: of all out-lists.
+void count_triangles(Ctx &c, const Oriented &o, uint64_t entries, const TcPlan &plan, uint32_t *tcount, uint8_t *flag,
                      cudaStream_t s);
 // lists for the resident graph's WCC plan (InternalWork), and the count of the internal
 // out-lists o by that plan and those lists

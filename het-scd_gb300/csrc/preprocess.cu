@@ -578,7 +578,7 @@ void convert_edges(Ctx &c, const uint32_t *pairs_in, uint64_t count, const std::
         tc_dense_setup(c, o, cnt.get(), core_members, core_bound, plan.dense, s);
         cnt.release();
         tc_plan_counting(c, o, m1, plan, s);
-        count_triangles(c, o, plan, tcount.get(), oflag.get(), s);
+        count_triangles(c, o, m1, plan, tcount.get(), oflag.get(), s);
     }
     icol.release();
     ibeg.release();

@@ -1032,7 +1032,7 @@ double autotune_tc(Ctx &c, std::vector<std::string> *report) {
                         CK(cudaMemsetAsync(tcount.get(), 0, (size_t)g.n * 4, s));
                         CK(cudaMemsetAsync(flag.get(), 0, 2 * (size_t)g.m, s));
                         CK(cudaEventRecord(e0, s));
-                        count_triangles(c, o, plan, tcount.get(), flag.get(), s);
+                        count_triangles(c, o, g.m, plan, tcount.get(), flag.get(), s);
                         CK(cudaEventRecord(e1, s));
                         CK(cudaEventSynchronize(e1));
                         float ms = 0;
@@ -1074,15 +1074,31 @@ double autotune_tc(Ctx &c, std::vector<std::string> *report) {
 
 namespace {
 
-void launch_small(Ctx &c, const Oriented &o, uint32_t max_len, const uint32_t *walk, uint32_t most, const Dir &dir,
-                  uint32_t *tcount, uint8_t *flag, cudaStream_t s) {
-    // 16 vertices a warp, fewer where that would leave SMs short of their 64 warps (10,000
-    // vertices, a step: 4 a warp 16 us, 1 a warp 10 us); a grid of
-    // one unit a warp, because units of dense graphs take 25 times as long as those of sparse
+// Vertices a warp of k_tc_small takes: up to 16, while every SM has its 64 warps and they hold up to
+// about 96 out-list entries together, or while every SM has 256. A warp's vertices come one after
+// the other and those with the longest walks are neighbours (ids are degree ranks), so with one
+// round of warps on the SMs and many entries in each the kernel waits for a few of them; with few
+// entries in each it is bound by the warps that find nothing to do. Measured, us of the
+// internal counts with 16, 8, 4, 2, 1 a warp (-: fewer warps than 64 an SM): planted graphs of
+// 150,000 vertices, mean degree 10, - 14 17 24, degree 24, - 47 48 57, degree 40, - 101 93 96; of
+// 200,000, degree 30, 81 70 67 75; of 60,000, degree 17, - - 16 19 23; Chung-Lu with 500,000 in
+// eight communities 234 158 124, by their initial labels 29 33 42; R-MAT scale 18 (65,000
+// vertices, 40 entries each), all kernels of the count, in one community - - 1870 1700 1630; 10,000
+// vertices - - 16 - 10.
+uint32_t small_rows(uint32_t n, uint64_t entries) {
+    uint32_t rows = 1, many = 1;
+    while (rows < 16 && (uint64_t)rows * 2 * NUM_SMS_HINT * 64 <= n && rows * 2 * entries <= 96 * (uint64_t)n) rows <<= 1;
+    while (many < 16 && (uint64_t)many * 2 * NUM_SMS_HINT * 256 <= n) many <<= 1;
+    return rows > many ? rows : many;
+}
+
+// entries: of all out-lists
+void launch_small(Ctx &c, const Oriented &o, uint64_t entries, uint32_t max_len, const uint32_t *walk, uint32_t most,
+                  const Dir &dir, uint32_t *tcount, uint8_t *flag, cudaStream_t s) {
+    // a grid of one unit a warp, because units of dense graphs take 25 times as long as those of sparse
     // ones and CTAs that are handed out even that out (96 planted graphs, all counts of a run:
-    // 8 CTAs an SM 7.3 ms, 16 6.8 ms, 48 6.0 ms, 128 5.8 ms; with 32 vertices 6.1 ms, with 8 6.0 ms)
-    uint32_t rows = 1;
-    while (rows < 16 && (uint64_t)rows * 2 * NUM_SMS_HINT * 64 <= o.n) rows <<= 1;
+    // 8 CTAs an SM 7.3 ms, 16 6.8 ms, 48 6.0 ms, 128 5.8 ms; with 32 vertices a warp 6.1 ms, with 8 6.0 ms)
+    const uint32_t rows = small_rows(o.n, entries);
     k_tc_small<<<grid_for(((uint64_t)o.n + rows - 1) / rows * 32, 256, 1u << 20), 256, 0, s>>>(o, rows, max_len, walk, most, dir,
                                                                                                 tcount, flag);
     CK_LAUNCH("k_tc_small");
@@ -1099,7 +1115,7 @@ void launch_huge(Ctx &c, const Oriented &o, const TcPlan &plan, uint32_t above, 
 
 }  // namespace
 
-void count_triangles(Ctx &c, const Oriented &o, const TcPlan &plan, uint32_t *tcount,
+void count_triangles(Ctx &c, const Oriented &o, uint64_t entries, const TcPlan &plan, uint32_t *tcount,
                      uint8_t *flag, cudaStream_t s) {
     if (o.n == 0) return;
     PhaseScope ph(c, "tc");
@@ -1108,7 +1124,7 @@ void count_triangles(Ctx &c, const Oriented &o, const TcPlan &plan, uint32_t *tc
     CK(cudaMemsetAsync(ctr, 0, 24, s));
     const Dir dir{plan.dir_lo, plan.dir_hi, plan.dir_amin};
     const bool core = plan.nverts[2] && plan.core_n;
-    launch_small(c, o, plan.small_max, plan.dense.n ? plan.dense.walk.get() : nullptr, INVALID, dir, tcount, flag, s);
+    launch_small(c, o, entries, plan.small_max, plan.dense.n ? plan.dense.walk.get() : nullptr, INVALID, dir, tcount, flag, s);
     if (plan.nverts[0]) {
         k_tc_warp<16, 256, 64, 10><<<152 * 4, 16 * 32, 0, s>>>(o, bucket_units(plan, 0), dir, tcount, flag, ctr);
         CK_LAUNCH("k_tc_warp64");
@@ -1160,7 +1176,7 @@ void count_internal_triangles(Ctx &c, const Oriented &o, uint32_t *tcount, uint8
     const auto listed = [&](int k, uint32_t per) { return UnitList{w.verts[k], nullptr, nullptr, 0, w.count + k, w.chunk[k], per}; };
     const uint32_t nv = plan.nverts[0] + plan.nverts[1] + plan.nverts[2];
     const Dir dir{plan.dir_lo, plan.dir_hi, plan.dir_amin};
-    launch_small(c, o, InternalWork::SMALL, c.g.distinct ? nullptr : c.g.nlow, plan.small_max, dir, tcount, flag, s);
+    launch_small(c, o, c.g.m, InternalWork::SMALL, c.g.distinct ? nullptr : c.g.nlow, plan.small_max, dir, tcount, flag, s);
     if (nv) {
         k_tc_warp<16, 256, 64, 10><<<grid_for(2ull * nv, 16, 152 * 4), 16 * 32, 0, s>>>(o, listed(0, 2), dir, tcount, flag,
                                                                                      ctr);
