@@ -362,7 +362,6 @@ void build_union_structure(Ctx &c, bool always_gid, bool check_symmetry) {
     g.rows.llong = lists + hb[K];
     g.rows.nlong = hb[K + 1] - hb[K];
     if (n) tc_plan_units(o, 0, c.wplan, tc_lists, htc, s, true);
-    alloc_internal_work(c);
     // the pieces of the long rows and the table words of the last class: one more read, if there are any
     const uint32_t n_big = g.cls.count[K - 1];
     uint32_t *coff = c.alloc<uint32_t>((size_t)g.rows.nlong + 1);
@@ -387,6 +386,7 @@ void build_union_structure(Ctx &c, bool always_gid, bool check_symmetry) {
     }
     c.pin64 = c.alloc<double>(n);
     c.civ = c.alloc<int4>(n);
+    alloc_internal_work(c);
     c.slot_flag = c.alloc<uint8_t>(2 * (size_t)g.m);
     c.itcount = c.alloc<uint32_t>(n);
     c.itdeg = c.alloc<int32_t>(n);

@@ -234,8 +234,8 @@ void sort_rows(Ctx &c, const uint32_t *off, uint32_t nrows, uint32_t *vals, bool
 // tcount and flag must be zeroed.  entries: of all out-lists.
 void count_triangles(Ctx &c, const Oriented &o, uint64_t entries, const TcPlan &plan, uint32_t *tcount, uint8_t *flag,
                      cudaStream_t s);
-// lists for the resident graph's WCC plan (InternalWork), and the count of the internal
-// out-lists o by that plan and those lists
+// lists for the resident graph's WCC plan (InternalWork; in the memory of pin64 and civ), and the
+// count of the internal out-lists o by that plan and those lists
 void alloc_internal_work(Ctx &c);
 void count_internal_triangles(Ctx &c, const Oriented &o, uint32_t *tcount, uint8_t *flag);
 // times the triangle-counting bucket splits on the resident graph, keeps the fastest

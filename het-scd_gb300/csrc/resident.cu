@@ -531,12 +531,12 @@ uint32_t rebuild(Ctx &c, ResidentSet &R, std::vector<ResidentSource *> &srcs) {
             pl.nverts[k] = pl.nfwd[k] = (uint32_t)lcnt[BUCKET0 + k];
         }
         pl.small_max = R.split[0];
-        alloc_internal_work(c);
         pl.dir_lo = pl.dir_hi = 0;   // out-list centres only, as tc_plan builds the WCC plan
         pl.dir_amin = c.tc_amin < c.tc_small ? c.tc_amin : c.tc_small;
         // scratch of the iteration
         c.pin64 = c.alloc<double>(N);
         c.civ = c.alloc<int4>(N);
+        alloc_internal_work(c);
         c.slot_flag = c.alloc<uint8_t>(M2);
         c.itcount = c.alloc<uint32_t>(N);
         c.itdeg = c.alloc<int32_t>(N);

@@ -41,6 +41,8 @@
 // T, numbered densely, so a small shared bitmap holds each one (k_tc_core).
 // T is the lowest of 64, 128, 256, 512, 1024 whose core has at most 128K
 // vertices (R-MAT scale 22: 128; Chung-Lu 8M: 256).
+#include <algorithm>
+
 #include "engine.cuh"
 #include "lists.cuh"
 
@@ -1155,14 +1157,33 @@ void count_triangles(Ctx &c, const Oriented &o, uint64_t entries, const TcPlan &
 void alloc_internal_work(Ctx &c) {
     const TcPlan &p = c.wplan;
     InternalWork &w = c.iwork;
-    const size_t nv = (size_t)p.nverts[0] + p.nverts[1] + p.nverts[2];
-    // a list of l has at most 1 + l / CHUNK, and the out-lists of a graph whose rows are not
-    // symmetric may hold all 2m entries
-    const size_t units = nv + 2 * (size_t)c.g.m / InternalWork::CHUNK + 1;
+    // The lists of a score lie in the memory of the gains' per-community records: an improvement
+    // fills those before it reads them, and both are over before the other begins. (Arrays of their
+    // own were up to 0.7 % of a dense graph's memory; lists that do not fit still get them.)
+    struct Region {
+        uint32_t *at;
+        size_t words;
+    } free_of[2] = {{(uint32_t *)c.civ, 4 * (size_t)c.g.n}, {(uint32_t *)c.pin64, 2 * (size_t)c.g.n}};
+    const auto take = [&](size_t words) {
+        for (Region &r : free_of)
+            if (words <= r.words) {
+                uint32_t *at = r.at;
+                r.at += words;
+                r.words -= words;
+                return at;
+            }
+        return c.alloc<uint32_t>(words);
+    };
+    // A list of l entries has at most 1 + l / CHUNK of its own, and the out-lists of a graph whose
+    // rows are not symmetric may hold all 2m; the lists up to CTA and up to LONGEST have no more
+    // than 2 and 16, and those above CTA are of the last bucket's vertices.
+    static_assert(InternalWork::CTA == 2 * InternalWork::CHUNK && InternalWork::LONGEST == 16 * InternalWork::CHUNK, "chunks");
+    const size_t last = p.nverts[2], nv = (size_t)p.nverts[0] + p.nverts[1] + last;
+    const size_t all = 2 * (size_t)c.g.m / InternalWork::CHUNK + 1;
+    const size_t most[InternalWork::K] = {nv, std::min(2 * nv, nv + all), std::min(16 * last, last + all)};
     for (int k = 0; k < InternalWork::K; k++) {
-        const bool any = k < 2 ? nv : p.nverts[2];
-        w.verts[k] = any ? c.alloc<uint32_t>(k ? units : nv) : nullptr;
-        w.chunk[k] = any && k ? c.alloc<uint32_t>(units) : nullptr;
+        w.verts[k] = most[k] ? take(most[k]) : nullptr;
+        w.chunk[k] = most[k] && k ? take(most[k]) : nullptr;
     }
     w.count = c.work_counter + 8;
 }
