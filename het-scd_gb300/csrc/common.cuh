@@ -26,6 +26,7 @@ struct Error : std::runtime_error {
 
 inline void cuda_check(cudaError_t e, const char *what, const char *file, int line) {
     if (e != cudaSuccess) {
+        cudaGetLastError();   // reported here: not again by the next launch's check
         char buf[512];
         snprintf(buf, sizeof buf, "%s: %s (%s:%d)", what, cudaGetErrorString(e), file, line);
         throw Error(e == cudaErrorMemoryAllocation ? SCD_ERR_OOM : SCD_ERR_CUDA, buf);
