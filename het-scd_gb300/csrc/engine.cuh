@@ -139,6 +139,8 @@ struct DenseCore {
     uint32_t n = 0, bound = 0;
     DevBuf<uint32_t> verts, num;   // members ascending; number of each member (INVALID for the others)
     DevBuf<uint32_t> walk;         // out-degree of every vertex, 0 for members
+    DevBuf<uint32_t> bits, sums;   // two bit matrices (the rows, the open bits); counts of the members' edges
+    DevBuf<uint8_t> row_open;
 };
 // The vertices above the register groups' buckets by the length of their internal out-list,
 // listed anew for every labelling by the pass that makes the internal lists: a community
@@ -218,6 +220,7 @@ uint32_t tc_short_lists(const Ctx &c);
 // degrees deg; 0 members if none is
 void tc_dense_pick(Ctx &c, const uint32_t *off, const uint32_t *vals, uint64_t entries, const uint32_t *olen,
                    const uint32_t *deg, uint32_t n, uint32_t *pick, cudaStream_t s);
+// d.n == 0 if the device has no room for the bit matrices: the walks count everything then
 void tc_dense_setup(Ctx &c, const Oriented &o, const uint32_t *deg, uint32_t members, uint32_t bound, DenseCore &d,
                     cudaStream_t s);
 void tc_dense_count(Ctx &c, const Oriented &o, const TcPlan &plan, uint32_t *tcount, uint8_t *flag, uint32_t *ctr,

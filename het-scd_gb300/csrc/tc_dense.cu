@@ -475,6 +475,17 @@ void tc_dense_setup(Ctx &c, const Oriented &o, const uint32_t *deg, uint32_t mem
                     cudaStream_t s) {
     d = DenseCore();
     if (!members) return;
+    const size_t matrix = (size_t)members * (dense_bits(members) / 32);
+    try {   // (up to 256 MB)
+        d.bits.alloc(2 * matrix, s);
+        d.sums.alloc(members, s);
+        d.row_open.alloc(members, s);
+    } catch (const Error &e) {
+        if (e.status != SCD_ERR_OOM) throw;
+        cudaGetLastError();
+        d = DenseCore();
+        return;
+    }
     d.n = members;
     d.bound = bound;
     d.verts.alloc(members, s);
@@ -495,14 +506,12 @@ void tc_dense_count(Ctx &c, const Oriented &o, const TcPlan &plan, uint32_t *tco
     const DenseCore &d = plan.dense;
     const uint32_t words = dense_bits(d.n) / 32;
     const size_t matrix = (size_t)d.n * words;
-    DevBuf<uint32_t> bits(2 * matrix, s), sums(d.n, s);   // the rows, then the open bits
-    DevBuf<uint8_t> row_open(d.n, s);
-    CK(cudaMemsetAsync(bits.get(), 0, 8 * matrix, s));
-    CK(cudaMemsetAsync(sums.get(), 0, 4 * (size_t)d.n, s));
-    CK(cudaMemsetAsync(row_open.get(), 0, d.n, s));
-    k_dense_fill<<<grid_for((uint64_t)d.n * 32, 256), 256, 0, s>>>(o, d.verts.get(), d.n, d.num.get(), words, bits.get());
+    CK(cudaMemsetAsync(d.bits.get(), 0, 8 * matrix, s));
+    CK(cudaMemsetAsync(d.sums.get(), 0, 4 * (size_t)d.n, s));
+    CK(cudaMemsetAsync(d.row_open.get(), 0, d.n, s));
+    k_dense_fill<<<grid_for((uint64_t)d.n * 32, 256), 256, 0, s>>>(o, d.verts.get(), d.n, d.num.get(), words, d.bits.get());
     CK_LAUNCH("k_dense_fill");
-    const DenseBuffers m{bits.get(), bits.get() + matrix, sums.get(), row_open.get()};
+    const DenseBuffers m{d.bits.get(), d.bits.get() + matrix, d.sums.get(), d.row_open.get()};
     switch (words / 128) {
     case 1: launch_dense<1>(o, d, plan, m, tcount, flag, ctr, s); break;
     case 2: launch_dense<2>(o, d, plan, m, tcount, flag, ctr, s); break;
@@ -513,7 +522,7 @@ void tc_dense_count(Ctx &c, const Oriented &o, const TcPlan &plan, uint32_t *tco
     case 7: launch_dense<7>(o, d, plan, m, tcount, flag, ctr, s); break;
     default: launch_dense<8>(o, d, plan, m, tcount, flag, ctr, s); break;
     }
-    k_dense_counts<<<grid_for(d.n, 256), 256, 0, s>>>(d.verts.get(), d.n, sums.get(), o.at, tcount);
+    k_dense_counts<<<grid_for(d.n, 256), 256, 0, s>>>(d.verts.get(), d.n, d.sums.get(), o.at, tcount);
     CK_LAUNCH("k_dense_counts");
     c.launches += 6;
 }
